@@ -1,0 +1,406 @@
+// The host side of a call as native code: kernels/_host.so, a CPython extension between the Python entry points and
+// the C ABI of libb200attn.so.
+//
+// What bounds a small call is not the GPU but the caller's thread: validating the tensors, filling a ctypes
+// structure field by field, allocating the output and looking up the workspace took 17 - 21 us of Python per
+// attention call and 10 us per softmax, where the launch itself takes 2 - 3 us.  Here the same steps read the
+// tensors' fields directly.
+//
+// Every function takes a call it understands completely - plain CUDA tensors, contiguous, of the shapes and types the
+// kernels read as they are - and returns None for anything else; the Python entry point then validates and converts
+// (and raises, with the messages of utils/validation.py).  Nothing is launched before a call has been accepted, so a
+// call is either served here or by the Python path, never by both.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <dlfcn.h>
+
+#include <cmath>
+#include <limits>
+#include <vector>
+
+#include "../../include/b200attn.h"
+
+namespace {
+
+// ---------------------------------------------------------------------------------------------------------------
+// the library (bound once, from the path the Python side resolved) and the workspaces
+// ---------------------------------------------------------------------------------------------------------------
+struct Library {
+  bool bound = false;
+  decltype(&b200attn_last_error) last_error;
+  decltype(&b200attn_prefill_workspace_bytes) prefill_workspace_bytes;
+  decltype(&b200attn_decode_workspace_bytes) decode_workspace_bytes;
+  decltype(&b200attn_prefill) prefill;
+  decltype(&b200attn_decode) decode;
+  decltype(&b200attn_paged_append) paged_append;
+  decltype(&b200attn_softmax) softmax;
+};
+Library g_lib;
+
+// kernels/_native.py owns the workspaces (one per device and stream, grown on demand); this is a view of its table,
+// asked for again whenever an entry is missing or too small, and emptied by forget() when the owner drops them.
+// Guarded by the GIL like everything in this file.
+struct Workspace {
+  int device;
+  void* stream;
+  void* data;
+  size_t bytes;
+};
+std::vector<Workspace> g_workspaces;
+PyObject* g_workspace_source = nullptr;   // _native.workspace(device, stream, nbytes) -> uint8 tensor
+
+
+
+bool find_workspace(const at::Tensor& like, int device, void* stream, size_t need, void** data, size_t* bytes) {
+  for (const Workspace& w : g_workspaces)
+    if (w.stream == stream && w.device == device && w.bytes >= need) {
+      *data = w.data;
+      *bytes = w.bytes;
+      return true;
+    }
+  PyObject* dev = THPDevice_New(like.device());
+  if (!dev) return false;
+  PyObject* buf = PyObject_CallFunction(g_workspace_source, "NKn", dev, reinterpret_cast<unsigned long long>(stream),
+                                        static_cast<Py_ssize_t>(need));
+  if (!buf) return false;
+  const at::Tensor& t = THPVariable_Unpack(buf);
+  const Workspace w{device, stream, t.data_ptr(), static_cast<size_t>(t.numel())};
+  Py_DECREF(buf);                         // the owner's table keeps it alive
+  bool known = false;
+  for (Workspace& old : g_workspaces)
+    if (old.stream == stream && old.device == device) { old = w; known = true; }
+  if (!known) g_workspaces.push_back(w);
+  *data = w.data;
+  *bytes = w.bytes;
+  return true;
+}
+
+PyObject* fail(const char* what, int status) {
+  PyErr_Format(PyExc_RuntimeError, "%s failed with status %d: %s", what, status, g_lib.last_error());
+  return nullptr;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// arguments
+// ---------------------------------------------------------------------------------------------------------------
+// a plain tensor (no subclass with its own behaviour) on a CUDA device, contiguous; nullptr otherwise
+const at::Tensor* cuda_tensor(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && t.is_contiguous() && !t.is_conj() && !t.is_neg() ? &t : nullptr;
+}
+
+bool small_int(PyObject* o, int* out) {
+  if (!PyLong_CheckExact(o)) return false;
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+  if (v <= 0 || v > std::numeric_limits<int>::max()) return false;
+  *out = static_cast<int>(v);
+  return true;
+}
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kHalf: return B200ATTN_F16;
+    case at::kBFloat16: return B200ATTN_BF16;
+    case at::kFloat: return B200ATTN_F32;
+    default: return -1;
+  }
+}
+
+bool fits_int(int64_t v) { return v >= 0 && v <= std::numeric_limits<int>::max(); }
+
+// one-dimensional int32 / int64 tensor on `dev`, contiguous
+bool index_tensor(const at::Tensor* t, const at::Device& dev) {
+  return t && t->dim() == 1 && (t->scalar_type() == at::kInt || t->scalar_type() == at::kLong) && t->device() == dev;
+}
+bool table_tensor(const at::Tensor* t, const at::Device& dev, int64_t batch) {
+  return t && t->dim() == 2 && t->scalar_type() == at::kInt && t->device() == dev && t->size(0) == batch;
+}
+
+at::Tensor new_like(const at::Tensor& t) {
+  return at::Tensor(at::detail::empty_cuda(t.sizes(), t.scalar_type(), t.device(), std::nullopt));
+}
+
+struct Qkv {
+  const at::Tensor *q, *k, *v;
+  int dtype, device;
+};
+// q, k, v of one supported type on one device
+bool same_kind(PyObject* const* args, Qkv* o) {
+  o->q = cuda_tensor(args[0]);
+  o->k = o->q ? cuda_tensor(args[1]) : nullptr;
+  o->v = o->k ? cuda_tensor(args[2]) : nullptr;
+  if (!o->v) return false;
+  const at::ScalarType st = o->q->scalar_type();
+  o->dtype = dtype_code(st);
+  if (o->dtype < 0 || o->k->scalar_type() != st || o->v->scalar_type() != st) return false;
+  const at::Device dev = o->q->device();
+  if (o->k->device() != dev || o->v->device() != dev || o->q->numel() == 0) return false;
+  o->device = dev.index();
+  return true;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// entry points; arguments are positional, absent optional tensors are None
+// ---------------------------------------------------------------------------------------------------------------
+// prefill(q, k, v, is_causal, q_indptr, kv_indptr, k_table, v_table, page_size, empty_like)
+PyObject* host_prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  Qkv x;
+  if (n != 10 || !g_lib.bound || !same_kind(args, &x)) Py_RETURN_NONE;
+  const at::Tensor &q = *x.q, &k = *x.k, &v = *x.v;
+  const int causal = PyObject_IsTrue(args[3]);
+  if (causal < 0) return nullptr;
+  b200attn_prefill_args_t a = {};
+  a.dtype = x.dtype;
+  a.device = x.device;
+  a.is_causal = causal;
+  const auto qs = q.sizes(), ks = k.sizes();
+  if (ks != v.sizes()) Py_RETURN_NONE;
+  if (args[6] != Py_None) {
+    const at::Tensor *len = cuda_tensor(args[5]), *kt = cuda_tensor(args[6]), *vt = cuda_tensor(args[7]);
+    int page = 0;
+    if (qs.size() != 4 || ks.size() != 3 || ks[2] != qs[3] || !small_int(args[8], &page) || !index_tensor(len, q.device()) ||
+        len->size(0) != qs[0] || !table_tensor(kt, q.device(), qs[0]) || !table_tensor(vt, q.device(), qs[0]) ||
+        kt->size(1) != vt->size(1) || !fits_int(kt->size(1) * page))
+      Py_RETURN_NONE;
+    a.layout = B200ATTN_PAGED;
+    a.batch = static_cast<int>(qs[0]); a.q_heads = static_cast<int>(qs[1]); a.max_q = static_cast<int>(qs[2]);
+    a.head_dim = static_cast<int>(qs[3]); a.kv_heads = static_cast<int>(ks[1]);
+    a.total_kv = ks[0];
+    a.table_stride = kt->size(1);
+    a.page_size = page;
+    a.max_kv = static_cast<int>(kt->size(1) * page);
+    a.kv_indptr = len->data_ptr();
+    a.indptr_is_i64 = len->scalar_type() == at::kLong;
+    a.k_table = static_cast<const int32_t*>(kt->data_ptr());
+    a.v_table = static_cast<const int32_t*>(vt->data_ptr());
+  } else if (args[4] != Py_None) {
+    const at::Tensor *qi = cuda_tensor(args[4]), *ki = cuda_tensor(args[5]);
+    if (qs.size() != 3 || ks.size() != 3 || ks[2] != qs[2] || !index_tensor(qi, q.device()) || !index_tensor(ki, q.device()) ||
+        qi->scalar_type() != ki->scalar_type() || qi->size(0) != ki->size(0) || qi->size(0) < 1 || !fits_int(qi->size(0)))
+      Py_RETURN_NONE;
+    a.layout = B200ATTN_RAGGED;
+    a.batch = static_cast<int>(qi->size(0) - 1);
+    a.q_heads = static_cast<int>(qs[1]); a.head_dim = static_cast<int>(qs[2]); a.kv_heads = static_cast<int>(ks[1]);
+    a.total_q = qs[0];
+    a.total_kv = ks[0];
+    a.q_indptr = qi->data_ptr();
+    a.kv_indptr = ki->data_ptr();
+    a.indptr_is_i64 = qi->scalar_type() == at::kLong;
+  } else {
+    if (qs.size() != 4 || ks.size() != 4 || ks[0] != qs[0] || ks[3] != qs[3] || !fits_int(ks[2])) Py_RETURN_NONE;
+    a.layout = B200ATTN_DENSE;
+    a.batch = static_cast<int>(qs[0]); a.q_heads = static_cast<int>(qs[1]); a.max_q = static_cast<int>(qs[2]);
+    a.head_dim = static_cast<int>(qs[3]); a.kv_heads = static_cast<int>(ks[1]);
+    a.max_kv = static_cast<int>(ks[2]);
+  }
+  if (a.kv_heads <= 0 || a.q_heads % a.kv_heads != 0 || (a.head_dim != 64 && a.head_dim != 128)) Py_RETURN_NONE;
+  a.sm_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(a.head_dim)));
+  // the output comes from the caller's torch.empty_like
+  PyObject* out = PyObject_CallOneArg(args[9], args[0]);
+  if (!out) return nullptr;
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr();
+  a.out = THPVariable_Unpack(out).data_ptr();
+  void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(x.device)).stream();
+  if (!find_workspace(q, x.device, stream, g_lib.prefill_workspace_bytes(&a), &a.workspace, &a.workspace_bytes)) {
+    Py_DECREF(out);
+    return nullptr;
+  }
+  const int rc = g_lib.prefill(&a, stream);
+  if (rc) { Py_DECREF(out); return fail("b200attn_prefill", rc); }
+  return out;
+}
+
+// decode(q, k, v, causal, kv_indptr, k_table, v_table, page_size, spec)
+PyObject* host_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  Qkv x;
+  if (n != 9 || !g_lib.bound || !same_kind(args, &x)) Py_RETURN_NONE;
+  const at::Tensor &q = *x.q, &k = *x.k, &v = *x.v;
+  const bool spec = args[8] == Py_True;
+  const int causal = PyObject_IsTrue(args[3]);
+  if (causal < 0) return nullptr;
+  b200attn_decode_args_t a = {};
+  a.dtype = x.dtype;
+  a.device = x.device;
+  a.causal_drafts = causal;
+  const auto qs = q.sizes(), ks = k.sizes();
+  if (ks != v.sizes() || qs.size() != (spec ? 4u : 3u)) Py_RETURN_NONE;
+  a.batch = static_cast<int>(qs[0]);
+  a.q_heads = static_cast<int>(qs[1]);
+  a.q_len = spec ? static_cast<int>(qs[2]) : 1;
+  a.head_dim = static_cast<int>(qs.back());
+  if (ks.size() < 3 || ks.back() != qs.back() || a.q_len > 16) Py_RETURN_NONE;
+  if (args[5] != Py_None) {
+    const at::Tensor *len = cuda_tensor(args[4]), *kt = cuda_tensor(args[5]), *vt = cuda_tensor(args[6]);
+    int page = 0;
+    if (ks.size() > 4 || !small_int(args[7], &page) || !index_tensor(len, q.device()) || len->size(0) != qs[0] ||
+        !table_tensor(kt, q.device(), qs[0]) || !table_tensor(vt, q.device(), qs[0]) || kt->size(1) != vt->size(1) ||
+        !fits_int(kt->size(1) * page))
+      Py_RETURN_NONE;
+    a.layout = B200ATTN_PAGED;
+    a.kv_heads = static_cast<int>(ks[ks.size() - 2]);
+    a.total_kv = ks.size() == 4 ? ks[0] * ks[1] : ks[0];
+    a.table_stride = kt->size(1);
+    a.page_size = page;
+    a.max_kv = static_cast<int>(kt->size(1) * page);
+    a.kv_indptr = len->data_ptr();
+    a.indptr_is_i64 = len->scalar_type() == at::kLong;
+    a.k_table = static_cast<const int32_t*>(kt->data_ptr());
+    a.v_table = static_cast<const int32_t*>(vt->data_ptr());
+  } else if (args[4] != Py_None) {
+    const at::Tensor* ip = cuda_tensor(args[4]);
+    if (ks.size() != 3 || !index_tensor(ip, q.device()) || ip->size(0) != qs[0] + 1) Py_RETURN_NONE;
+    a.layout = B200ATTN_RAGGED;
+    a.kv_heads = static_cast<int>(ks[1]);
+    a.total_kv = ks[0];
+    a.kv_indptr = ip->data_ptr();
+    a.indptr_is_i64 = ip->scalar_type() == at::kLong;
+  } else {
+    if (ks.size() != 4 || ks[0] != qs[0] || !fits_int(ks[2])) Py_RETURN_NONE;
+    a.layout = B200ATTN_DENSE;
+    a.kv_heads = static_cast<int>(ks[1]);
+    a.max_kv = static_cast<int>(ks[2]);
+  }
+  if (a.kv_heads <= 0 || a.q_heads % a.kv_heads != 0 || (a.head_dim != 64 && a.head_dim != 128)) Py_RETURN_NONE;
+  a.sm_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(a.head_dim)));
+  at::Tensor out = new_like(q);
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.out = out.data_ptr();
+  void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(x.device)).stream();
+  const size_t need = g_lib.decode_workspace_bytes(&a);
+  if (need == 0) {
+    PyErr_Format(PyExc_RuntimeError, "b200attn_decode_workspace_bytes failed: %s", g_lib.last_error());
+    return nullptr;
+  }
+  if (!find_workspace(q, x.device, stream, need, &a.workspace, &a.workspace_bytes)) return nullptr;
+  const int rc = g_lib.decode(&a, stream);
+  if (rc) return fail("b200attn_decode", rc);
+  return THPVariable_Wrap(std::move(out));
+}
+
+// paged_append(cache, table, src, src_indptr, page_size, dst_pos) -> True when the rows are on their way
+PyObject* host_paged_append(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 6 || !g_lib.bound) Py_RETURN_NONE;
+  const at::Tensor *cache = cuda_tensor(args[0]), *table = cuda_tensor(args[1]), *src = cuda_tensor(args[2]),
+                   *indptr = cuda_tensor(args[3]), *pos = args[5] == Py_None ? nullptr : cuda_tensor(args[5]);
+  int page = 0;
+  if (!cache || !src || (args[5] != Py_None && !pos) || !small_int(args[4], &page)) Py_RETURN_NONE;
+  const at::Device dev = src->device();
+  const auto cs = cache->sizes(), ss = src->sizes();
+  if (cache->device() != dev || cache->scalar_type() != src->scalar_type() || ss.size() != 3 || cs.size() < 3 || cs.size() > 4 ||
+      cs[cs.size() - 2] != ss[1] || cs.back() != ss[2] || !table || table->dim() != 2 || !table_tensor(table, dev, table->size(0)) ||
+      !index_tensor(indptr, dev) || indptr->size(0) != table->size(0) + 1 || !fits_int(table->size(0)))
+    Py_RETURN_NONE;
+  if (pos && (pos->dim() != 1 || pos->size(0) != table->size(0) || pos->device() != dev || pos->scalar_type() != indptr->scalar_type()))
+    Py_RETURN_NONE;
+  const int64_t row_bytes = ss[1] * ss[2] * static_cast<int64_t>(src->element_size());
+  if (row_bytes % 16 != 0 || !fits_int(row_bytes) || ss[0] == 0 || table->size(0) == 0) Py_RETURN_NONE;
+  b200attn_paged_append_args_t a = {};
+  a.device = dev.index();
+  void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  if (!find_workspace(*src, a.device, stream, 256, &a.workspace, &a.workspace_bytes)) return nullptr;
+  a.src = src->data_ptr(); a.cache = cache->data_ptr();
+  a.src_indptr = indptr->data_ptr();
+  a.dst_pos = pos ? pos->data_ptr() : nullptr;
+  a.table = static_cast<const int32_t*>(table->data_ptr());
+  a.total_rows = ss[0];
+  a.cache_rows = cs.size() == 4 ? cs[0] * cs[1] : cs[0];
+  a.table_stride = table->size(1);
+  a.row_bytes = static_cast<int>(row_bytes);
+  a.indptr_is_i64 = indptr->scalar_type() == at::kLong;
+  a.batch = static_cast<int>(table->size(0));
+  a.page_size = page;
+  const int rc = g_lib.paged_append(&a, stream);
+  if (rc) return fail("b200attn_paged_append", rc);
+  Py_RETURN_TRUE;
+}
+
+// softmax(x, out, log)
+PyObject* host_softmax(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3 || !g_lib.bound) Py_RETURN_NONE;
+  const at::Tensor *x = cuda_tensor(args[0]), *o = args[1] == Py_None ? nullptr : cuda_tensor(args[1]);
+  if (!x || (args[1] != Py_None && !o) || x->dim() < 1 || x->numel() == 0) Py_RETURN_NONE;
+  b200attn_softmax_args_t a = {};
+  a.dtype = dtype_code(x->scalar_type());
+  if (a.dtype < 0) Py_RETURN_NONE;
+  if (o && (o->sizes() != x->sizes() || o->scalar_type() != x->scalar_type() || o->device() != x->device())) Py_RETURN_NONE;
+  at::Tensor fresh;
+  if (!o) fresh = new_like(*x);
+  a.x = x->data_ptr();
+  a.out = o ? o->data_ptr() : fresh.data_ptr();
+  a.cols = x->sizes().back();
+  a.rows = x->numel() / a.cols;
+  a.log_softmax = args[2] == Py_True;
+  a.device = x->device().index();
+  const int rc = g_lib.softmax(&a, c10::cuda::getCurrentCUDAStream(x->device().index()).stream());
+  if (rc) return fail("b200attn_softmax", rc);
+  if (o) { Py_INCREF(args[1]); return args[1]; }
+  return THPVariable_Wrap(std::move(fresh));
+}
+
+// bind(library path, workspace function)
+PyObject* host_bind(PyObject*, PyObject* args) {
+  const char* path;
+  PyObject* source;
+  if (!PyArg_ParseTuple(args, "sO", &path, &source)) return nullptr;
+  void* h = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  if (!h) { PyErr_Format(PyExc_RuntimeError, "dlopen: %s", dlerror()); return nullptr; }
+  Library l;
+#define B200ATTN_BIND(name)                                                            \
+  l.name = reinterpret_cast<decltype(l.name)>(dlsym(h, "b200attn_" #name));            \
+  if (!l.name) { PyErr_Format(PyExc_RuntimeError, "%s lacks b200attn_" #name, path); return nullptr; }
+  B200ATTN_BIND(last_error)
+  B200ATTN_BIND(prefill_workspace_bytes)
+  B200ATTN_BIND(decode_workspace_bytes)
+  B200ATTN_BIND(prefill)
+  B200ATTN_BIND(decode)
+  B200ATTN_BIND(paged_append)
+  B200ATTN_BIND(softmax)
+#undef B200ATTN_BIND
+  l.bound = true;
+  g_lib = l;
+  Py_INCREF(source);
+  Py_XSETREF(g_workspace_source, source);
+  g_workspaces.clear();
+  Py_RETURN_NONE;
+}
+
+PyObject* host_forget(PyObject*, PyObject*) {
+  g_workspaces.clear();
+  Py_RETURN_NONE;
+}
+
+// C++ exceptions (an allocation that fails, a CUDA error inside torch) become Python's
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  return F(self, args, n);
+  END_HANDLE_TH_ERRORS
+}
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyCFunction fast() {
+  return reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&guarded<F>));
+}
+
+PyMethodDef kMethods[] = {
+    {"prefill", fast<host_prefill>(), METH_FASTCALL, nullptr},
+    {"decode", fast<host_decode>(), METH_FASTCALL, nullptr},
+    {"paged_append", fast<host_paged_append>(), METH_FASTCALL, nullptr},
+    {"softmax", fast<host_softmax>(), METH_FASTCALL, nullptr},
+    {"bind", host_bind, METH_VARARGS, nullptr},
+    {"forget", host_forget, METH_NOARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "Native call path of the attention and softmax entry points.", -1, kMethods,
+                       nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&kModule); }

@@ -143,6 +143,7 @@ class SoftmaxArgs(C.Structure):
 
 _lib: Optional[C.CDLL] = None
 _lib_lock = threading.Lock()
+_HOST_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_host.so")
 
 
 def library_path() -> str:
@@ -191,8 +192,40 @@ def lib() -> C.CDLL:
         got = handle.b200attn_abi_version()
         if got != ABI_VERSION:
             raise RuntimeError(f"{path}: ABI version {got}, expected {ABI_VERSION}")
+        if not os.path.exists(_HOST_PATH):
+            raise RuntimeError(
+                f"_host.so not found at {_HOST_PATH}. Build it with `make -C {os.path.join(_PKG_ROOT, 'csrc')}`."
+            )
         _lib = handle
         return _lib
+
+
+# ---------------------------------------------------------------------------
+# The native call path (csrc/host.cpp).  ``fast`` is bound to the library at its first use; until then, and for calls
+# it does not take (it answers None), the entry points validate and launch from Python.
+# ---------------------------------------------------------------------------
+def _unbound(*_args):
+    """Stands in for the functions of ``_host`` until the first call with CUDA tensors binds them."""
+    if torch.cuda.is_available():
+        bind_host()
+    return None
+
+
+class _Unbound:
+    prefill = decode = paged_append = softmax = staticmethod(_unbound)
+
+
+fast = _Unbound
+
+
+def bind_host() -> None:
+    """Load ``_host`` and hand it the library and the workspace table."""
+    global fast
+    lib()
+    from . import _host
+
+    _host.bind(library_path(), workspace)
+    fast = _host
 
 
 def last_error() -> str:
@@ -229,6 +262,8 @@ def workspace(device: torch.device, stream_ptr: int, nbytes: int) -> torch.Tenso
         size = (size + 255) & ~255
         if buf is not None:
             _retired.setdefault(key, []).append(buf)
+            if fast is not _Unbound:
+                fast.forget()  # its view of the table would keep pointing at the retired buffer
         buf = torch.zeros(size, dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
@@ -249,5 +284,7 @@ def check_device_errors() -> None:
 
 
 def release_workspaces() -> None:
+    if fast is not _Unbound:
+        fast.forget()
     _workspaces.clear()
     _retired.clear()

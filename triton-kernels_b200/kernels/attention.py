@@ -2,7 +2,8 @@
 ``kernels/attention.py``: ``flash_attention_v2`` :749-927 and ``flash_attention_v1`` :249-364).
 
 Host code only validates, allocates the output and calls the sm_100a kernel
-through the C ABI (``b200attn_prefill``).  No Triton, no CPU path.
+through the C ABI (``b200attn_prefill``): natively for the calls ``_host`` takes
+(csrc/host.cpp), from here for the rest.  No Triton, no CPU path.
 """
 from __future__ import annotations
 
@@ -41,6 +42,10 @@ def flash_attention_v2(
 
     Returns a tensor shaped and typed like ``q``.
     """
+    out = _native.fast.prefill(q, k, v, is_causal, q_indptr, kv_indptr, k_block_table, v_block_table, kv_page_size,
+                               torch.empty_like)
+    if out is not None:
+        return out
     prob = validate_prefill(q, k, v, q_indptr, kv_indptr, k_block_table, v_block_table, kv_page_size)
     out = torch.empty_like(q)
     if q.numel() == 0:

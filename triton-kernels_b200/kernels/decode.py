@@ -68,5 +68,8 @@ def decode_attention(
     Paged  : q (B, QH, D), k/v (total_kv_tokens, KVH, D), kv_indptr (B,) context lengths,
              k_block_table / v_block_table (B, max_blocks_per_seq), kv_page_size
     """
+    out = _native.fast.decode(q, k, v, False, kv_indptr, k_block_table, v_block_table, kv_page_size, False)
+    if out is not None:
+        return out
     prob = validate_decode(q, k, v, kv_indptr, k_block_table, v_block_table, kv_page_size, spec=False)
     return _launch_decode(q, k, v, prob, causal=False)

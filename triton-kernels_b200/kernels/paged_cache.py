@@ -29,6 +29,8 @@ def append_paged_kv(
     src_indptr  (B + 1,) prefix sums over ``src`` rows (int32 or int64)
     dst_pos     (B,) position inside each sequence of its first new row; None = 0 (fill from scratch)
     """
+    if _native.fast.paged_append(cache, block_table, src, src_indptr, kv_page_size, dst_pos):
+        return cache
     assert cache.is_cuda and src.is_cuda and block_table.is_cuda and src_indptr.is_cuda, "tensors must be on a CUDA device"
     assert cache.device == src.device == block_table.device == src_indptr.device
     assert cache.dtype == src.dtype, "cache and src must have the same dtype"

@@ -30,6 +30,9 @@ def _validate(x: torch.Tensor, out: Optional[torch.Tensor]) -> None:
 
 
 def _launch(x: torch.Tensor, out: Optional[torch.Tensor], log: bool) -> torch.Tensor:
+    done = _native.fast.softmax(x, out, log)
+    if done is not None:
+        return done
     _validate(x, out)
     out = torch.empty_like(x) if out is None else out
     a = _native.SoftmaxArgs()

@@ -6,6 +6,7 @@ import torch
 
 from utils.validation import validate_decode
 
+from . import _native
 from .decode import _launch_decode
 
 
@@ -30,5 +31,8 @@ def speculative_decode_attention(
     keys (the passed length includes them) and draft row i does not see draft keys
     i+1..M-1; every draft row sees the whole context.
     """
+    out = _native.fast.decode(q, k, v, causal, kv_indptr, k_block_table, v_block_table, kv_page_size, True)
+    if out is not None:
+        return out
     prob = validate_decode(q, k, v, kv_indptr, k_block_table, v_block_table, kv_page_size, spec=True)
     return _launch_decode(q, k, v, prob, causal=bool(causal))
