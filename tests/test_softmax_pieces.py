@@ -1,0 +1,49 @@
+"""Row softmax where the 16-byte piece kernels can go wrong: rows of every misalignment, lengths either side of the
+lines between the kernels (a warp's 4 KiB, a CTA's 64 KiB, one CTA's ring of 224 KiB, a cluster's), rows shorter than a
+piece, and tensors that start off the 16-byte grid (alike in x and out, or not)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+LINES = [4 << 10, 64 << 10, 224 << 10, 448 << 10, 1792 << 10]          # bytes of a row
+
+
+def _check(got, x, log):
+    # the oracle in float64, rounded to the dtype; torch.testing's defaults for the dtype, as in test_softmax.py
+    exp = (torch.log_softmax if log else torch.softmax)(x.cpu().double(), dim=-1).to(x.dtype)
+    torch.testing.assert_close(got.cpu(), exp)
+
+
+@pytest.mark.parametrize("log", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("line", LINES)
+@pytest.mark.parametrize("delta", [-9, -1, 0, 1, 8])
+def test_lengths_around_the_lines(line, delta, dtype, log):
+    from kernels import log_softmax, softmax
+
+    cols = line // torch.finfo(dtype).bits * 8 + delta
+    rows = 301 if line <= 4 << 10 else (151 if line <= 64 << 10 else 3)
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    x = (3 * torch.randn((rows, cols), generator=g, device=DEV)).to(dtype)
+    x[rows // 2, cols // 3:] = -float("inf")
+    _check((log_softmax if log else softmax)(x), x, log)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("cols", [1, 3, 7, 17, 1025, 5003, 60001])
+@pytest.mark.parametrize("shift_x,shift_out", [(0, 0), (1, 1), (3, 3), (1, 2), (0, 1)])
+def test_tensors_off_the_grid(cols, shift_x, shift_out, dtype):
+    from kernels import softmax
+
+    rows = 5
+    g = torch.Generator(device=DEV).manual_seed(cols)
+    raw = torch.randn(rows * cols + 8, generator=g, device=DEV).to(dtype)
+    x = raw[shift_x:shift_x + rows * cols].view(rows, cols)
+    guard = torch.full((rows * cols + 8,), 7.0, device=DEV, dtype=dtype)
+    out = guard[shift_out:shift_out + rows * cols].view(rows, cols)
+    softmax(x, out=out)
+    _check(out, x, False)
+    assert (guard[:shift_out] == 7).all() and (guard[shift_out + rows * cols:] == 7).all()
+    softmax(x, out=x)                                                   # in place
+    assert torch.equal(x, out) or shift_x % 4 != shift_out % 4

@@ -1,0 +1,35 @@
+// Kernel launches with programmatic stream serialisation.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace b200attn {
+
+// Launches `kernel` so that it may be scheduled, and set itself up, while the kernel before it in the stream is still
+// running; the kernel itself blocks (ptx::grid_dep_wait) before it touches memory that anything earlier in the stream
+// may have written or may still read.  Behind a kernel that knows nothing of this, the wait ends when that kernel has
+// completed, like an ordinary launch.  Saves the 1.5 - 2.5 us between the end of one grid and the first instruction of
+// the next.  `cluster` > 1: CTAs per thread-block cluster.
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                             unsigned cluster, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+}  // namespace b200attn

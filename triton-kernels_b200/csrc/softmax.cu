@@ -2,19 +2,19 @@
 //
 // Replaces the reference's small / medium / partial + merge + finalize kernels (kernels/softmax.py:18-150 and
 // :239-375): there a row longer than one block is read twice (three launches when it is split over programs).
-// Here a row is read once, kept on the SM and normalised from there.  Rows whose bytes are a multiple of 16:
-//   softmax_reg_kernel     up to 16 384 fp32 / 16-bit elements: one CTA per row, the row in registers
-//   softmax_pipe_kernel    up to 864 KiB: a CTA, or a cluster of 2, 4 or 8 CTAs, per row; slices of up to 108 KiB arrive
-//                          by bulk copies into a ring of 2 to 8 shared-memory stages, so the next rows load while
-//                          this one is reduced and written
-//   softmax_regc_kernel    up to 1 MiB: the row in the registers of a cluster of eight CTAs
-//   softmax_cluster_kernel up to 1.6 MB: 200 KiB per CTA in shared memory, cluster of eight
-// Any other row:
+// Here a row is read once, kept on the SM and normalised from there:
+//   softmax_warp_kernel    up to 4 KiB: a warp per row, the row in its registers
+//   softmax_reg_kernel     up to 64 KiB: one CTA per row, the row in registers
+//   softmax_ring_kernel    up to 1.75 MiB: a CTA, or a cluster of 2, 4 or 8 CTAs, per row; the row passes through a ring
+//                          of shared-memory chunks filled by bulk copies, the next row loads while this one is reduced
+//                          and written
+// These move 16-byte pieces; the few elements of a row before its first and behind its last 16-byte boundary travel
+// singly, so the row length may be anything.  Rows that are longer, or lie differently in x and out:
 //   softmax_row_kernel     up to 200 KiB: one CTA per row, the row in shared memory
-//   softmax_cluster_kernel up to 1.6 MB (as above)
+//   softmax_cluster_kernel up to 1.6 MB: 200 KiB per CTA in shared memory, cluster of eight
 //   softmax_stream_kernel  beyond: one CTA per row, online (max, sum) pass, then a second read
-// Clusters exchange their (max, sum) pairs through distributed shared memory; the pipelined and register kernels do it
-// with asynchronous remote stores that count on the receiver's mbarrier, because a cluster-wide barrier also waits
+// Clusters exchange their (max, sum) pairs through distributed shared memory; the ring kernel does it with
+// asynchronous remote stores that count on the receiver's mbarrier, because a cluster-wide barrier also waits
 // for the previous row's global stores.
 // All arithmetic is fp32, like the reference's `.to(tl.float32)`: expf for fp32 rows in registers, ex2.approx of
 // (x - max) * log2(e) for 16-bit types and for fp32 rows in the pipelined kernel (tl.exp compiles to the same).  `out` may alias `x`: a row is written only after all of it has been staged (the streaming kernel
@@ -22,9 +22,11 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "sm100_ptx.cuh"
 #include "softmax_launch.h"
 
@@ -36,8 +38,6 @@ namespace {
 
 constexpr int kRowSmemBytes = 200 * 1024;   // row bytes one CTA stages
 constexpr int kMaxCluster = 8;              // portable cluster size
-constexpr int kPipeSliceBytes = 108 * 1024; // longest slice of a row per CTA of the pipelined kernel (two are staged)
-constexpr int kPipeStages = 8;              // shorter slices: as many stages as fit 216 KiB, up to this many
 
 __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -102,49 +102,23 @@ __device__ __forceinline__ void merge_ml(float& m, float& l, float m2, float l2)
   m = g;
 }
 
-// Stage `n` elements of a row in shared memory (16-byte copies when VEC) and return this thread's running max.
-template <typename T, bool VEC>
+// Stage `n` elements of a row in shared memory and return this thread's running max.
+template <typename T>
 __device__ __forceinline__ float stage_row(const T* src, T* row, long long n) {
   float mx = -INFINITY;
-  if constexpr (VEC) {
-    constexpr int E = Vec16<T>::kElems;
-    const long long nv = n / E;
-    const uint4* s4 = reinterpret_cast<const uint4*>(src);
-    uint4* d4 = reinterpret_cast<uint4*>(row);
-    for (long long i = threadIdx.x; i < nv; i += blockDim.x) {
-      const uint4 u = s4[i];       // (plain load: `out` may alias `x`)
-      d4[i] = u;
-      const T* e = reinterpret_cast<const T*>(&u);
-#pragma unroll
-      for (int k = 0; k < E; ++k) mx = fmaxf(mx, ElemTraits<T>::to_float(e[k]));
-    }
-  } else {
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-      const T v = src[i];
-      row[i] = v;
-      mx = fmaxf(mx, ElemTraits<T>::to_float(v));
-    }
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
+    const T v = src[i];            // (plain load: `out` may alias `x`)
+    row[i] = v;
+    mx = fmaxf(mx, ElemTraits<T>::to_float(v));
   }
   return mx;
 }
 
-template <typename T, bool VEC>
+template <typename T>
 __device__ __forceinline__ float row_exp_sum(const T* row, long long n, float m) {
   float s = 0.f;
   if (m == -INFINITY) return 0.f;
-  if constexpr (VEC) {
-    constexpr int E = Vec16<T>::kElems;
-    const long long nv = n / E;
-    const uint4* r4 = reinterpret_cast<const uint4*>(row);
-    for (long long i = threadIdx.x; i < nv; i += blockDim.x) {
-      const uint4 u = r4[i];
-      const T* e = reinterpret_cast<const T*>(&u);
-#pragma unroll
-      for (int k = 0; k < E; ++k) s += fast_or_exact_exp<T>(ElemTraits<T>::to_float(e[k]) - m);
-    }
-  } else {
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) s += fast_or_exact_exp<T>(ElemTraits<T>::to_float(row[i]) - m);
-  }
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) s += fast_or_exact_exp<T>(ElemTraits<T>::to_float(row[i]) - m);
   return s;
 }
 
@@ -156,23 +130,9 @@ __device__ __forceinline__ T finish(float x, float m, float k) {
   else return ElemTraits<T>::from_float(fast_or_exact_exp<T>(x - m) * k);
 }
 
-template <typename T, bool LOG, bool VEC>
+template <typename T, bool LOG>
 __device__ __forceinline__ void write_row(const T* row, T* dst, long long n, float m, float k) {
-  if constexpr (VEC) {
-    constexpr int E = Vec16<T>::kElems;
-    const long long nv = n / E;
-    const uint4* r4 = reinterpret_cast<const uint4*>(row);
-    uint4* d4 = reinterpret_cast<uint4*>(dst);
-    for (long long i = threadIdx.x; i < nv; i += blockDim.x) {
-      uint4 u = r4[i];
-      T* e = reinterpret_cast<T*>(&u);
-#pragma unroll
-      for (int q = 0; q < E; ++q) e[q] = finish<T, LOG>(ElemTraits<T>::to_float(e[q]), m, k);
-      d4[i] = u;
-    }
-  } else {
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) dst[i] = finish<T, LOG>(ElemTraits<T>::to_float(row[i]), m, k);
-  }
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) dst[i] = finish<T, LOG>(ElemTraits<T>::to_float(row[i]), m, k);
 }
 
 // the constant the write pass needs: 1 / l for softmax, log l for log-softmax
@@ -205,141 +165,202 @@ template <typename T> __device__ __forceinline__ uint32_t floats_to_word(const f
   else return __float_as_uint(f[0]);
 }
 
-// CL: the row is spread over the CTAs of a thread-block cluster (CTA `rank` holds the pieces rank * slice ...); each
-// CTA normalises against its own maximum first, the (max, sum) pairs meet in distributed shared memory, and the
-// correction exp(own max - row max) / row sum goes into the constant of the store loop.  The pairs are double
-// buffered by row parity, so one cluster barrier per row is enough.
-template <typename T, bool LOG, int VPT, bool CL>
-__device__ __forceinline__ void softmax_reg_body(const T* x, T* out, long long rows, long long cols) {
+// Where a row lies relative to the 16-byte grid of memory: `head` elements before the first 16-byte boundary, `nv` whole
+// 16-byte pieces, and the rest behind them.  x and out are misaligned by the same amount (the launcher checks), so the
+// pieces of a row are aligned in both; the fewer than 2 E elements around them, the edges, are single loads and stores.
+struct RowSplit { int head, nv, edges; };
+template <typename T> __device__ __forceinline__ RowSplit split_row(const T* row, long long cols) {
   constexpr int E = Vec16<T>::kElems;
-  constexpr int W = E / 4;                           // elements per 32-bit word
-  constexpr float kLog2e = 1.4426950408889634f;
-  __shared__ float scratch[32];
-  __shared__ __align__(8) float2 pairs[2][kMaxCluster];   // CL: every CTA's (max, sum) of the even / odd row in work
-  __shared__ __align__(8) uint64_t pair_bar[2];           // CL: completes when all pairs of that row have landed
-  int nv = static_cast<int>(cols / E);
-  unsigned csize = 1;
-  int rank = 0;
-  if constexpr (CL) {
-    cg::cluster_group cluster = cg::this_cluster();
-    rank = static_cast<int>(cluster.block_rank());
-    csize = cluster.num_blocks();
-    if (threadIdx.x == 0) {
-      ptx::mbar_init(smem_u32(&pair_bar[0]), 1);
-      ptx::mbar_init(smem_u32(&pair_bar[1]), 1);
-      ptx::mbar_fence_init();
-    }
-    cluster.sync();                                  // once: every peer's barriers exist before anyone sends
-    const int slice = (nv + static_cast<int>(csize) - 1) / static_cast<int>(csize);
-    x += static_cast<long long>(slice) * rank * E;   // this CTA's pieces start here within every row
-    out += static_cast<long long>(slice) * rank * E;
-    nv = max(0, min(slice, nv - slice * rank));
-  }
-  const unsigned row_step = gridDim.x / csize;
-  unsigned iter = 0;                                 // rows this CTA has worked on
-  for (long long r = blockIdx.x / csize; r < rows; r += row_step, ++iter) {
-    const unsigned parity = iter & 1u;
-    const uint4* s4 = reinterpret_cast<const uint4*>(x + r * cols);
-    uint4* d4 = reinterpret_cast<uint4*>(out + r * cols);
-    float f[VPT * E];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      if (i < nv) {
-        const uint4 u = s4[i];
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) word_to_floats<T>(w[q], &f[k * E + q * W]);
-#pragma unroll
-        for (int q = 0; q < E; ++q) mx = fmaxf(mx, f[k * E + q]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < E; ++q) f[k * E + q] = -INFINITY;
-      }
-    }
-    const float m = block_max(mx, scratch);
-    float sum = 0.f;
-    if (m != -INFINITY) {
-#pragma unroll
-      for (int j = 0; j < VPT * E; ++j) {
-        // 16-bit outputs round away far more than the approximate exponential loses: exp2((x - m) log2e), the
-        // difference first (it is exact for x near m, whatever the magnitude of m); fp32 outputs need expf.
-        // exp(-inf) = 0 for the padding.
-        float ev;
-        if constexpr (sizeof(T) == 2) ev = fast_exp2((f[j] - m) * kLog2e);
-        else ev = expf(f[j] - m);
-        sum += ev;
-        if constexpr (!LOG) f[j] = ev;
-      }
-    } else if constexpr (CL && !LOG) {
-      // this CTA's part is all -inf but the row may not be: its outputs are zeros
-#pragma unroll
-      for (int j = 0; j < VPT * E; ++j) f[j] = 0.f;
-    }
-    float l = block_sum(sum, scratch);
-    float own = 1.f;                                 // CL: exp(own max - row max)
-    float m_row = m;
-    if constexpr (CL) {
-      // Thread 0 posts this CTA's pair into every CTA's `pairs` (its own included) with asynchronous remote stores
-      // that count bytes on the receiver's barrier: no cluster-wide barrier, no fence that would wait for the
-      // previous row's global stores.  Slot reuse is safe: a peer can send row r + 2 only after it has seen this
-      // CTA's pair of row r + 1, which thread 0 sends after all threads here have read the pairs of row r.
-      const uint32_t bar = smem_u32(&pair_bar[parity]);
-      if (threadIdx.x == 0) {
-        ptx::mbar_arrive_expect_tx(bar, csize * 8u);
-        const uint32_t slot = smem_u32(&pairs[parity][rank]);
-        for (unsigned p = 0; p < csize; ++p) ptx::st_async_pair(slot, bar, p, m, l);
-      }
-      const bool landed = ptx::mbar_wait(bar, (iter >> 1) & 1u);
-      float gm = -INFINITY, gl = 0.f;
-      for (unsigned p = 0; p < csize; ++p) merge_ml(gm, gl, pairs[parity][p].x, pairs[parity][p].y);
-      if (!landed) gl = __int_as_float(0x7fc00000);  // bounded wait ran out: the row comes out as NaN, never a hang
-      own = (m == -INFINITY) ? 0.f : expf(m - gm);
-      m_row = gm;
-      l = gl;
-    }
-    float kk = final_constant<LOG>(m_row, l);
-    if constexpr (CL && !LOG) kk *= own;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      if (i < nv) {
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float t[W];
-#pragma unroll
-          for (int e = 0; e < W; ++e) {
-            const float v = f[k * E + q * W + e];
-            if constexpr (LOG) t[e] = (v - m_row) - kk;
-            else t[e] = m_row == -INFINITY ? __int_as_float(0x7fc00000) : v * kk;
-          }
-          w[q] = floats_to_word<T>(t);
-        }
-        d4[i] = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-    }
-  }
-  // (a CTA may leave right away: it has received every pair sent to it, and its own last pairs have been received
-  // by peers that are still waiting for them or already past that wait)
+  RowSplit s;
+  const int off = static_cast<int>(reinterpret_cast<uintptr_t>(row) & 15) / static_cast<int>(sizeof(T));
+  s.head = static_cast<int>(min(static_cast<long long>(off ? E - off : 0), cols));
+  s.nv = static_cast<int>((cols - s.head) / E);
+  s.edges = static_cast<int>(cols - static_cast<long long>(s.nv) * E);
+  return s;
+}
+// column of edge element i (0 <= i < edges)
+template <typename T> __device__ __forceinline__ long long edge_col(const RowSplit& s, int i) {
+  return i < s.head ? i : static_cast<long long>(s.nv) * Vec16<T>::kElems + i;
 }
 
-template <typename T, bool LOG, int VPT>
-__global__ void __launch_bounds__(1024) softmax_reg_kernel(const T* x, T* out, long long rows, long long cols) {
-  softmax_reg_body<T, LOG, VPT, false>(x, out, rows, cols);
+// exp(x) for the sums and results of rows of type T: 16-bit outputs round away far more than the approximate
+// exponential loses (the difference to the maximum is taken first, so it is exact near the maximum whatever the
+// magnitude); fp32 outputs need expf
+template <typename T> __device__ __forceinline__ float row_exp(float d) {
+  if constexpr (sizeof(T) == 2) return fast_exp2(d * 1.4426950408889634f);
+  else return expf(d);
 }
-// two CTAs per SM while a thread holds 16 elements
+
+// maximum of a 16-byte piece (16-bit values: exact in 16 bits, one packed instruction per two elements)
+template <typename T> __device__ __forceinline__ float piece_max(const uint4& u) {
+  if constexpr (sizeof(T) == 2) {
+    using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+    const T2 a = __hmax2(*reinterpret_cast<const T2*>(&u.x), *reinterpret_cast<const T2*>(&u.y));
+    const T2 b = __hmax2(*reinterpret_cast<const T2*>(&u.z), *reinterpret_cast<const T2*>(&u.w));
+    const T2 c = __hmax2(a, b);
+    float f[2];
+    word_to_floats<T>(*reinterpret_cast<const uint32_t*>(&c), f);
+    return fmaxf(f[0], f[1]);
+  } else {
+    return fmaxf(fmaxf(__uint_as_float(u.x), __uint_as_float(u.y)), fmaxf(__uint_as_float(u.z), __uint_as_float(u.w)));
+  }
+}
+
+// Sum of exp(x - m) over a piece: the difference first (exact near the maximum whatever the magnitude), then
+// ex2.approx of it times log2(e), whose error in a term of the sum is below the rounding of the sum; two elements per
+// instruction where the hardware packs them.  KEEP (fp32 softmax): the terms are the results, they come from expf and
+// replace the elements.
+template <typename T, bool KEEP> __device__ __forceinline__ float piece_exp_sum(uint4& u, float m) {
+  constexpr int W = Vec16<T>::kElems / 4;
+  uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  if constexpr (KEEP) {
+    float s[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      s[q] = expf(__uint_as_float(w[q]) - m);
+      w[q] = __float_as_uint(s[q]);
+    }
+    u = make_uint4(w[0], w[1], w[2], w[3]);
+    return (s[0] + s[1]) + (s[2] + s[3]);
+  } else {
+    const uint64_t nm = ptx::pack_f2(-m, -m);
+    constexpr float kLog2e = 1.4426950408889634f;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; q += 2 / W) {
+      float f[2];
+      if constexpr (W == 2) word_to_floats<T>(w[q], f);
+      else { f[0] = __uint_as_float(w[q]); f[1] = __uint_as_float(w[q + 1]); }
+      float a, b;
+      ptx::unpack_f2(ptx::add_f2(ptx::pack_f2(f[0], f[1]), nm), a, b);
+      s0 += fast_exp2(a * kLog2e);
+      s1 += fast_exp2(b * kLog2e);
+    }
+    return s0 + s1;
+  }
+}
+
+// What the store pass needs of a row: its maximum and log(sum) (log-softmax), 1 / sum (fp32 softmax) or -log2(sum)
+// (16-bit softmax: exp(x - m) / l = exp2((x - m) log2e - log2 l), the division folded into the exponent).  A row of
+// -inf only has m = -inf, and -inf - -inf makes every output NaN, like the sum over no terms it stands for.
+template <typename T, bool LOG> __device__ __forceinline__ float row_constant(float l) {
+  if constexpr (LOG) return logf(l);
+  else if constexpr (sizeof(T) == 2) return -__log2f(l);
+  else return 1.f / l;
+}
+// KEPT: x is exp(x - m) already (fp32 softmax of rows in registers)
+template <typename T, bool LOG, bool KEPT> __device__ __forceinline__ float row_value(float x, float m, float k) {
+  if constexpr (KEPT) return x * k;
+  else if constexpr (LOG) return (x - m) - k;
+  else if constexpr (sizeof(T) == 2) return fast_exp2(fmaf(x - m, 1.4426950408889634f, k));
+  else return expf(x - m) * k;
+}
+template <typename T, bool LOG, bool KEPT> __device__ __forceinline__ uint4 piece_values(const uint4& u, float m, float k) {
+  constexpr int W = Vec16<T>::kElems / 4;
+  uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float f[W];
+    word_to_floats<T>(w[q], f);
+#pragma unroll
+    for (int e = 0; e < W; ++e) f[e] = row_value<T, LOG, KEPT>(f[e], m, k);
+    w[q] = floats_to_word<T>(f);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// ---------------------------------------------------------------------------
+// short rows: a warp per row, the row's 16-byte pieces in the warp's registers (VPT per lane), no barrier of any kind.
+// Bound by HBM, below it by the launch.  A CTA per row spent most of a short row in its two block reductions, and a row
+// whose length is not a multiple of 16 bytes went through single-element copies: 65 536 x 128 bf16 25.0 -> 14.9 us (no
+// two rows' loads overlapped before), 30 001 x 2 047 bf16 139 -> 38 us (0.98 of the copy bandwidth), 64 x 2 048 (a
+// launch) 4.2 -> 2.5 us.
+// ---------------------------------------------------------------------------
+constexpr int kWarpPieces = 32 * 8;   // longest row: eight pieces per lane; beyond, a CTA's registers were faster
+constexpr int kWarpRows = 4;   // warps per CTA
 template <typename T, bool LOG, int VPT>
-__global__ void __launch_bounds__(1024, VPT * (16 / sizeof(T)) <= 16 ? 2 : 1)
-softmax_regc_kernel(const T* x, T* out, long long rows, long long cols) {
-  softmax_reg_body<T, LOG, VPT, true>(x, out, rows, cols);
+__global__ void __launch_bounds__(kWarpRows * 32) softmax_warp_kernel(const T* x, T* out, long long rows, long long cols) {
+  constexpr bool KEEP = sizeof(T) == 4 && !LOG;
+  const int lane = threadIdx.x & 31;
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch_dependents();
+  for (long long r = static_cast<long long>(blockIdx.x) * kWarpRows + (threadIdx.x >> 5); r < rows;
+       r += static_cast<long long>(gridDim.x) * kWarpRows) {
+    const T* src = x + r * cols;
+    T* dst = out + r * cols;
+    const RowSplit sp = split_row(src, cols);
+    const uint4* s4 = reinterpret_cast<const uint4*>(src + sp.head);
+    uint4* d4 = reinterpret_cast<uint4*>(dst + sp.head);
+    uint4 u[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (lane + 32 * k < sp.nv) u[k] = s4[lane + 32 * k];
+    float edge = -INFINITY;
+    if (lane < sp.edges) edge = ElemTraits<T>::to_float(src[edge_col<T>(sp, lane)]);
+    float m = edge;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (lane + 32 * k < sp.nv) m = fmaxf(m, piece_max<T>(u[k]));
+    m = warp_max(m);
+    float s = lane < sp.edges ? row_exp<T>(edge - m) : 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (lane + 32 * k < sp.nv) s += piece_exp_sum<T, KEEP>(u[k], m);
+    const float c = row_constant<T, LOG>(warp_sum(s));
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (lane + 32 * k < sp.nv) d4[lane + 32 * k] = piece_values<T, LOG, KEEP>(u[k], m, c);
+    if (lane < sp.edges) dst[edge_col<T>(sp, lane)] = ElemTraits<T>::from_float(row_value<T, LOG, false>(edge, m, c));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// medium rows: a CTA per row, thread t holds the four 16-byte pieces t, t + blockDim, ...: as many threads as the row
+// needs, and 32 registers, so that 2 048 threads share an SM and up to 128 KiB of rows are in flight on it.  Bound by
+// HBM.  With power-of-two CTAs a quarter of the threads idled on average: 20 000 x 3 001 bf16 161.7 -> 41.3 us, 5 000 x
+// 8 200 fp32 80.7 -> 57.9 us, 16 384 x 16 384 bf16 200 -> 170 us (0.96 of the copy bandwidth).
+// ---------------------------------------------------------------------------
+template <typename T, bool LOG>
+__global__ void __launch_bounds__(1024, 2) softmax_reg_kernel(const T* x, T* out, long long rows, long long cols) {
+  constexpr bool KEEP = sizeof(T) == 4 && !LOG;
+  constexpr int VPT = 4;
+  __shared__ float scratch[2][32];
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch_dependents();
+  const int t = threadIdx.x;
+  for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
+    const T* src = x + r * cols;
+    T* dst = out + r * cols;
+    const RowSplit sp = split_row(src, cols);
+    const uint4* s4 = reinterpret_cast<const uint4*>(src + sp.head);
+    uint4* d4 = reinterpret_cast<uint4*>(dst + sp.head);
+    uint4 u[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (t + k * static_cast<int>(blockDim.x) < sp.nv) u[k] = s4[t + k * static_cast<int>(blockDim.x)];
+    float edge = -INFINITY;
+    if (t < sp.edges) edge = ElemTraits<T>::to_float(src[edge_col<T>(sp, t)]);
+    float m = edge;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (t + k * static_cast<int>(blockDim.x) < sp.nv) m = fmaxf(m, piece_max<T>(u[k]));
+    m = block_max_nolead(m, scratch[0]);   // (each scratch is rewritten only after the other's barrier)
+    float s = t < sp.edges ? row_exp<T>(edge - m) : 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (t + k * static_cast<int>(blockDim.x) < sp.nv) s += piece_exp_sum<T, KEEP>(u[k], m);
+    const float c = row_constant<T, LOG>(block_sum_nolead(s, scratch[1]));
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (t + k * static_cast<int>(blockDim.x) < sp.nv) d4[t + k * static_cast<int>(blockDim.x)] = piece_values<T, LOG, KEEP>(u[k], m, c);
+    if (t < sp.edges) dst[edge_col<T>(sp, t)] = ElemTraits<T>::from_float(row_value<T, LOG, false>(edge, m, c));
+  }
 }
 
 // ---------------------------------------------------------------------------
 // one CTA per row, the row in shared memory
 // ---------------------------------------------------------------------------
-template <typename T, bool LOG, bool VEC>
+template <typename T, bool LOG>
 __global__ void softmax_row_kernel(const T* x, T* out, long long rows, long long cols) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float scratch[32];
@@ -347,17 +368,17 @@ __global__ void softmax_row_kernel(const T* x, T* out, long long rows, long long
   for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
     const T* src = x + r * cols;
     __syncthreads();               // the previous row has been written out of `row`
-    float m = stage_row<T, VEC>(src, row, cols);
+    float m = stage_row<T>(src, row, cols);
     m = block_max(m, scratch);     // (its barriers also publish the staged row)
-    const float l = block_sum(row_exp_sum<T, VEC>(row, cols, m), scratch);
-    write_row<T, LOG, VEC>(row, out + r * cols, cols, m, final_constant<LOG>(m, l));
+    const float l = block_sum(row_exp_sum<T>(row, cols, m), scratch);
+    write_row<T, LOG>(row, out + r * cols, cols, m, final_constant<LOG>(m, l));
   }
 }
 
 // ---------------------------------------------------------------------------
 // one cluster per row: every CTA stages a slice, (max, sum) pairs meet in distributed shared memory
 // ---------------------------------------------------------------------------
-template <typename T, bool LOG, bool VEC>
+template <typename T, bool LOG>
 __global__ void softmax_cluster_kernel(const T* x, T* out, long long rows, long long cols,
                                        long long slice) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -371,9 +392,9 @@ __global__ void softmax_cluster_kernel(const T* x, T* out, long long rows, long 
   const long long nclusters = gridDim.x / csize;
   for (long long r = blockIdx.x / csize; r < rows; r += nclusters) {
     const T* src = x + r * cols + c0;
-    float m = stage_row<T, VEC>(src, row, n);
+    float m = stage_row<T>(src, row, n);
     m = block_max(m, scratch);
-    const float l = block_sum(row_exp_sum<T, VEC>(row, n, m), scratch);
+    const float l = block_sum(row_exp_sum<T>(row, n, m), scratch);
     if (threadIdx.x == 0) { ml[0] = m; ml[1] = l; }
     cluster.sync();                // every CTA's pair is in place
     float gm = -INFINITY, gl = 0.f;
@@ -382,174 +403,191 @@ __global__ void softmax_cluster_kernel(const T* x, T* out, long long rows, long 
       merge_ml(gm, gl, peer[0], peer[1]);
     }
     cluster.sync();                // all pairs have been read: they may be overwritten for the next row
-    write_row<T, LOG, VEC>(row, out + r * cols + c0, n, gm, final_constant<LOG>(gm, gl));
+    write_row<T, LOG>(row, out + r * cols + c0, n, gm, final_constant<LOG>(gm, gl));
     __syncthreads();               // `row` is free again
   }
 }
 
 // ---------------------------------------------------------------------------
-// long rows, pipelined: a CTA (alone, or as one of a cluster of 2, 4 or 8 that share a row) keeps two slices in shared
-// memory; the bulk copy of the next row's slice runs while the current one is reduced and written out, so loads are
-// in flight all the time.  Clusters exchange (max, sum) pairs like softmax_regc_kernel does.
+// long rows: a ring of 15.5 KiB chunks in shared memory.  A producer warp fills it by bulk copies; the other warps take a
+// chunk as soon as it has landed and keep a running (max, sum) per thread (first pass), combine them once per row, and
+// go over the chunks again to write the row (second pass), handing each back to the producer, which fills it with the
+// next row.  So a row is read once, loads run under both passes, and there is one barrier per row.  A row that is
+// longer than the ring, or of which there are too few to keep every SM busy, is shared by a cluster of 2, 4 or 8 CTAs.
+// Bound by HBM with a fixed microsecond per row (the reduction, during which nothing is stored).  The chunk is what the
+// waits and the loop overhead are spread over: 4 pieces per thread against 2 and 1 gave 135, 150 and 160 us on 2 000 x
+// 50 000 fp32; 512 threads against 256 and 384 gave 135, 159 and 140.  Larger clusters than a row needs only cost
+// (cluster 2 / 4: 155 / 220 us).  Before (three barriers per row, a slice of the row as one copy, single-element loads
+// for odd lengths) and now: 2 000 x 50 001 fp32 282 -> 138 us (0.89 of the copy bandwidth), 1 024 x 131 072 fp32
+// 309 -> 198, bf16 151 -> 103, 8 192 x 24 576 fp32 268 -> 249.
 // ---------------------------------------------------------------------------
+constexpr int kRingThreads = 512;                   // threads that compute (the producer warp comes on top)
+constexpr int kRingWarps = kRingThreads / 32;
+constexpr int kRingPer = 4;                         // 16-byte pieces per thread and chunk
+constexpr int kRingChunk = kRingThreads * kRingPer;
+constexpr int kRingSlots = 7;                       // 224 KiB
+constexpr int kRingPieces = kRingChunk * kRingSlots;
+
+// (m, s) <- (m, s) + the elements of a thread's pieces of a chunk; m is the reference of s
+template <typename T> __device__ __forceinline__ void online_add(float& m, float& s, uint4 (&u)[kRingPer]) {
+  float mx = piece_max<T>(u[0]);
+#pragma unroll
+  for (int k = 1; k < kRingPer; ++k) mx = fmaxf(mx, piece_max<T>(u[k]));
+  if (mx > m) {
+    s = (m == -INFINITY) ? 0.f : s * row_exp<T>(m - mx);
+    m = mx;
+  }
+  if (m != -INFINITY) {
+    float t = piece_exp_sum<T, false>(u[0], m);
+#pragma unroll
+    for (int k = 1; k < kRingPer; ++k) t += piece_exp_sum<T, false>(u[k], m);
+    s += t;
+  }
+}
+
 template <typename T, bool LOG>
-__global__ void __launch_bounds__(1024, 1)
-softmax_pipe_kernel(const T* x, T* out, long long rows, long long cols, int slice /* 16-byte pieces per CTA */,
-                    int csize, int stages /* slices staged, 2..kPipeStages */) {
-  constexpr int E = Vec16<T>::kElems;
-  constexpr int W = E / 4;
-  constexpr float kLog2e = 1.4426950408889634f;
+__global__ void __launch_bounds__(kRingThreads + 32, 1)
+softmax_ring_kernel(const T* x, T* out, long long rows, long long cols, int slice /* pieces of a row per CTA */, int csize) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float scratch[2][32];                   // [0] for the maxima, [1] for the sums: each is rewritten only
-                                                     // after the barrier that ends the row
-  __shared__ __align__(8) float2 pairs[2][kMaxCluster];
-  __shared__ __align__(8) uint64_t pair_bar[2];
-  __shared__ __align__(8) uint64_t full_bar[kPipeStages];
+  __shared__ float2 scratch[2][kRingWarps];
+  __shared__ __align__(8) float2 pairs[2][kMaxCluster];    // every CTA's (max, sum) of the even / odd row in work
+  __shared__ __align__(8) uint64_t pair_bar[2];            // completes when all pairs of that row have landed
+  __shared__ __align__(8) uint64_t full[kRingSlots], empty[kRingSlots];
+  uint4* const ring = reinterpret_cast<uint4*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = csize > 1 ? static_cast<int>(cg::this_cluster().block_rank()) : 0;
-  const int nv_row = static_cast<int>(cols / E);
-  const int nv = max(0, min(slice, nv_row - slice * rank));
-  const uint32_t bytes = static_cast<uint32_t>(nv) * 16u;
-  x += static_cast<long long>(slice) * rank * E;
-  out += static_cast<long long>(slice) * rank * E;
-  uint4* const base = reinterpret_cast<uint4*>(smem_raw);   // stage s at base + s * slice
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     for (int i = 0; i < 2; ++i) ptx::mbar_init(smem_u32(&pair_bar[i]), 1);
-    for (int i = 0; i < kPipeStages; ++i) ptx::mbar_init(smem_u32(&full_bar[i]), 1);
+    for (int i = 0; i < kRingSlots; ++i) {
+      ptx::mbar_init(smem_u32(&full[i]), 1);
+      ptx::mbar_init(smem_u32(&empty[i]), kRingWarps);
+    }
     ptx::mbar_fence_init();
   }
   if (csize > 1) cg::this_cluster().sync(); else __syncthreads();
-  const unsigned row_step = gridDim.x / csize;
-  const long long r0 = blockIdx.x / csize;
-  if (threadIdx.x == 0 && nv > 0) {
-    for (int s = 0; s < stages - 1; ++s) {
-      const long long r = r0 + static_cast<long long>(s) * row_step;
-      if (r >= rows) break;
-      ptx::mbar_arrive_expect_tx(smem_u32(&full_bar[s]), bytes);
-      ptx::bulk_load(smem_u32(base + static_cast<size_t>(s) * slice), x + r * cols, bytes, smem_u32(&full_bar[s]));
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch_dependents();
+  const long long row_step = gridDim.x / csize, r0 = blockIdx.x / csize;
+  const int first = slice * rank;                          // this CTA's pieces of every row: first .. first + slice - 1
+  auto my_pieces = [&](const RowSplit& sp) { return max(0, min(slice, sp.nv - first)); };
+
+  if (warp == kRingWarps) {
+    // ------------------------------ producer ------------------------------
+    if (lane == 0) {
+      int slot = 0;
+      unsigned phase = 1;                                  // parity of the wait for a free slot (the first round is free)
+      long long issued = 0;
+      bool ok = true;
+      for (long long r = r0; ok && r < rows; r += row_step) {
+        const T* src = x + r * cols;
+        const RowSplit sp = split_row(src, cols);
+        const uint4* s4 = reinterpret_cast<const uint4*>(src + sp.head) + first;
+        const int n = my_pieces(sp);
+        for (int p = 0; p < n; p += kRingChunk) {
+          if (issued >= kRingSlots) ok = ptx::mbar_wait(smem_u32(&empty[slot]), phase);
+          if (!ok) break;
+          const uint32_t bytes = static_cast<uint32_t>(min(kRingChunk, n - p)) * 16u;
+          ptx::mbar_arrive_expect_tx(smem_u32(&full[slot]), bytes);
+          ptx::bulk_load(smem_u32(ring + slot * kRingChunk), s4 + p, bytes, smem_u32(&full[slot]));
+          ++issued;
+          if (++slot == kRingSlots) { slot = 0; phase ^= 1u; }
+        }
+      }
+      // (a consumer gave up: wait, bounded, for the copies in flight before the CTA's memory goes away)
+      if (!ok)
+        for (int i = 0; i < kRingSlots; ++i) {
+          const unsigned done = static_cast<unsigned>((issued - 1 - i) / kRingSlots);
+          if (issued - 1 - i >= 0) ptx::mbar_wait(smem_u32(&full[(issued - 1 - i) % kRingSlots]), done & 1u);
+        }
     }
+    return;
   }
-  unsigned iter = 0;
-  int b = 0;                                         // stage of this iteration
-  unsigned phase = 0;                                // and the parity its barrier completes with
-  bool ok = true;
+  // ------------------------------ consumers ------------------------------
+  int slot = 0;
+  unsigned phase = 0, iter = 0;
+  bool ok = true;                                          // false: a bounded wait ran out, the rows come out as NaN
   for (long long r = r0; r < rows; r += row_step, ++iter) {
-    if (threadIdx.x == 0 && nv > 0) {
-      // refill the stage the previous iteration used: it was read for the last time before the barrier that ended
-      // that iteration
-      const long long rn = r + static_cast<long long>(stages - 1) * row_step;
-      if (rn < rows) {
-        const int bn = b == 0 ? stages - 1 : b - 1;
-        ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive_expect_tx(smem_u32(&full_bar[bn]), bytes);
-        ptx::bulk_load(smem_u32(base + static_cast<size_t>(bn) * slice), x + rn * cols, bytes, smem_u32(&full_bar[bn]));
-      }
-    }
-    if (nv > 0) ok = ptx::mbar_wait(smem_u32(&full_bar[b]), phase) && ok;
-    uint4* row = base + static_cast<size_t>(b) * slice;
-    float mx = -INFINITY;
-    if constexpr (sizeof(T) == 2) {
-      // the maximum of 16-bit values is exact in 16 bits: one packed instruction per two elements, unpacked once
-      using T2 = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
-      const uint32_t ninf2 = std::is_same<T, __half>::value ? 0xfc00fc00u : 0xff80ff80u;
-      uint32_t acc = ninf2;
-#pragma unroll 2
-      for (int i = threadIdx.x; i < nv; i += 1024) {
-        const uint4 u = row[i];
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    const T* src = x + r * cols;
+    T* dst = out + r * cols;
+    const RowSplit sp = split_row(src, cols);
+    const int n = my_pieces(sp);
+    const int edges = rank == 0 ? sp.edges : 0;
+    float edge = -INFINITY;
+    if (tid < edges) edge = ElemTraits<T>::to_float(src[edge_col<T>(sp, tid)]);
+    const int slot0 = slot;
+    float m = -INFINITY, s = 0.f;
+    for (int p = 0; p < n; p += kRingChunk) {
+      if (ok) ok = ptx::mbar_wait(smem_u32(&full[slot]), phase);
+      const uint4* c4 = ring + slot * kRingChunk + tid;
+      const int left = n - p - tid;
+      uint4 u[kRingPer];
+      if (n - p >= kRingChunk) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const T2 t = __hmax2(*reinterpret_cast<const T2*>(&acc), *reinterpret_cast<const T2*>(&w[q]));
-          acc = *reinterpret_cast<const uint32_t*>(&t);
-        }
-      }
-      float f[2];
-      word_to_floats<T>(acc, f);
-      mx = fmaxf(f[0], f[1]);
-    } else {
-#pragma unroll 2
-      for (int i = threadIdx.x; i < nv; i += 1024) {
-        const uint4 u = row[i];
-        mx = fmaxf(mx, fmaxf(fmaxf(__uint_as_float(u.x), __uint_as_float(u.y)),
-                             fmaxf(__uint_as_float(u.z), __uint_as_float(u.w))));
-      }
-    }
-    const float m = block_max_nolead(mx, scratch[0]);
-    float sum = 0.f;
-    if (m != -INFINITY) {
-#pragma unroll 2
-      for (int i = threadIdx.x; i < nv; i += 1024) {
-        const uint4 u = row[i];
-        uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        for (int k = 0; k < kRingPer; ++k) u[k] = c4[k * kRingThreads];
+      } else {
+        constexpr uint32_t w = sizeof(T) == 4 ? 0xff800000u : (std::is_same<T, __half>::value ? 0xfc00fc00u : 0xff80ff80u);  // -inf
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float f[W];
-          word_to_floats<T>(w[q], f);
-#pragma unroll
-          for (int e = 0; e < W; ++e) {
-            if constexpr (sizeof(T) == 2) {
-              sum += fast_exp2((f[e] - m) * kLog2e);
-            } else {
-              // ex2.approx is within 2^-22 relative, the scaled difference within 2^-24 of its own magnitude: inside
-              // the fp32 tolerance, and what the reference's tl.exp compiles to
-              const float ev = fast_exp2((f[e] - m) * kLog2e);
-              sum += ev;
-              if constexpr (!LOG) w[q] = __float_as_uint(ev);   // fp32 softmax keeps exp(x - m) in place
-            }
-          }
-        }
-        if constexpr (sizeof(T) == 4 && !LOG) row[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int k = 0; k < kRingPer; ++k) u[k] = k * kRingThreads < left ? c4[k * kRingThreads] : make_uint4(w, w, w, w);
       }
+      online_add<T>(m, s, u);
+      if (++slot == kRingSlots) { slot = 0; phase ^= 1u; }
     }
-    float l = block_sum_nolead(sum, scratch[1]);
-    float m_row = m, own = 1.f;
+    if (tid < edges && edge != -INFINITY) {
+      const float mx = fmaxf(m, edge);
+      s = (m == -INFINITY ? 0.f : s * row_exp<T>(m - mx)) + row_exp<T>(edge - mx);
+      m = mx;
+    }
+    if (!ok) { m = 0.f; s = __int_as_float(0x7fc00000); }
+    // the CTA's (max, sum): warps through shuffles, warps of the CTA through shared memory
+    float mw = warp_max(m);
+    float sw = warp_sum(m == -INFINITY ? 0.f : s * row_exp<T>(m - mw));
+    float2* sc = scratch[iter & 1u];
+    if (lane == 0) sc[warp] = make_float2(mw, sw);
+    ptx::named_bar_sync(1, kRingThreads);
+    const float2 pw = lane < kRingWarps ? sc[lane] : make_float2(-INFINITY, 0.f);
+    float gm = warp_max(pw.x);
+    float gl = warp_sum(pw.x != -INFINITY ? pw.y * row_exp<T>(pw.x - gm) : 0.f);
     if (csize > 1) {
+      // Thread 0 posts the CTA's pair into every CTA's `pairs` (its own included) with asynchronous remote stores that
+      // count bytes on the receiver's barrier: no cluster-wide barrier, no fence that would wait for the previous
+      // row's global stores.  Slot reuse is safe: a peer can send row r + 2 only after it has seen this CTA's pair
+      // of row r + 1, which thread 0 sends after all threads here have read the pairs of row r (the barrier above).
       const unsigned parity = iter & 1u;
       const uint32_t bar = smem_u32(&pair_bar[parity]);
-      if (threadIdx.x == 0) {
+      if (tid == 0) {
         ptx::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(csize) * 8u);
-        const uint32_t slot = smem_u32(&pairs[parity][rank]);
-        for (int p = 0; p < csize; ++p) ptx::st_async_pair(slot, bar, p, m, l);
+        const uint32_t to = smem_u32(&pairs[parity][rank]);
+        for (int p = 0; p < csize; ++p) ptx::st_async_pair(to, bar, p, gm, gl);
       }
-      ok = ptx::mbar_wait(bar, (iter >> 1) & 1u) && ok;
-      float gm = -INFINITY, gl = 0.f;
-      for (int p = 0; p < csize; ++p) merge_ml(gm, gl, pairs[parity][p].x, pairs[parity][p].y);
-      own = (m == -INFINITY) ? 0.f : expf(m - gm);
-      m_row = gm;
-      l = gl;
-    }
-    if (!ok) l = __int_as_float(0x7fc00000);         // a bounded wait ran out: NaN rows, never a hang
-    float kk = final_constant<LOG>(m_row, l);
-    if constexpr (!LOG && sizeof(T) == 4) kk *= own;
-    // 16-bit softmax: exp(x - m) / l = exp2((x - m) log2e - log2 l), the division folded into the exponent (l >= 1
-    // whenever the row has a finite maximum)
-    const float neg_log2_l = LOG ? 0.f : -__log2f(l);
-    const bool nan_row = m_row == -INFINITY;
-    uint4* d4 = reinterpret_cast<uint4*>(out + r * cols);
-#pragma unroll 2
-    for (int i = threadIdx.x; i < nv; i += 1024) {
-      const uint4 u = row[i];
-      uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float f[W];
-        word_to_floats<T>(w[q], f);
-#pragma unroll
-        for (int e = 0; e < W; ++e) {
-          if constexpr (LOG) {
-            f[e] = (f[e] - m_row) - kk;
-          } else if constexpr (sizeof(T) == 2) {
-            f[e] = nan_row ? __int_as_float(0x7fc00000) : fast_exp2(fmaf(f[e] - m_row, kLog2e, neg_log2_l));
-          } else {
-            // (a slice of -inf only still holds -inf, not exp: its outputs are zeros unless the whole row is -inf)
-            f[e] = nan_row ? __int_as_float(0x7fc00000) : (m == -INFINITY ? 0.f : f[e] * kk);
-          }
-        }
-        w[q] = floats_to_word<T>(f);
+      if (ok) ok = ptx::mbar_wait(bar, (iter >> 1) & 1u);
+      gm = -INFINITY;
+      for (int p = 0; p < csize; ++p) gm = fmaxf(gm, pairs[parity][p].x);
+      gl = 0.f;
+      for (int p = 0; p < csize; ++p) {
+        const float2 q = pairs[parity][p];
+        gl += q.x == -INFINITY && gm != -INFINITY ? 0.f : q.y * row_exp<T>(q.x - gm);
       }
-      d4[i] = make_uint4(w[0], w[1], w[2], w[3]);
+      if (!ok) gl = __int_as_float(0x7fc00000);
     }
-    __syncthreads();                                 // `row` may be refilled
-    if (++b == stages) { b = 0; phase ^= 1u; }
+    const float c = row_constant<T, LOG>(gl);
+    uint4* d4 = reinterpret_cast<uint4*>(dst + sp.head) + first;
+    int back = slot0;
+    for (int p = 0; p < n; p += kRingChunk) {
+      const uint4* c4 = ring + back * kRingChunk + tid;
+      uint4* o4 = d4 + p + tid;
+      const int left = n - p - tid;
+      uint4 u[kRingPer];
+#pragma unroll
+      for (int k = 0; k < kRingPer; ++k)
+        if (k * kRingThreads < left) u[k] = c4[k * kRingThreads];
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(smem_u32(&empty[back]));
+#pragma unroll
+      for (int k = 0; k < kRingPer; ++k)
+        if (k * kRingThreads < left) o4[k * kRingThreads] = piece_values<T, LOG, false>(u[k], gm, c);
+      if (++back == kRingSlots) back = 0;
+    }
+    if (tid < edges) dst[edge_col<T>(sp, tid)] = ElemTraits<T>::from_float(row_value<T, LOG, false>(edge, gm, c));
   }
 }
 
@@ -582,121 +620,105 @@ int set_smem_limit(K kernel, size_t bytes) {
   return ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
 }
 
-template <typename T, bool LOG, bool VEC>
-int launch_typed(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t stream) {
+// CTAs that share a row of `nv` pieces in the ring kernel: as few as hold it, more when there are so few rows that SMs
+// would stay idle (as long as a CTA still has two chunks of the row).
+inline int ring_cluster(long long rows, long long nv, int sm_count) {
+  int csize = 1;
+  while ((nv + csize - 1) / csize > kRingPieces) csize *= 2;
+  while (csize < kMaxCluster && rows * csize * 2 <= sm_count && nv > 4LL * csize * kRingChunk) csize *= 2;
+  return csize;
+}
+
+// Rows whose 16-byte pieces can be copied as they are (x and out misaligned by the same amount).
+template <typename T, bool LOG>
+int launch_pieces(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t stream) {
+  const T* x = static_cast<const T*>(a.x);
+  T* out = static_cast<T*>(a.out);
+  const long long rows = a.rows, cols = a.cols;
+  constexpr int E = Vec16<T>::kElems;
+  const long long nv = cols / E;
+  cudaError_t e = cudaSuccess;
+  if (nv <= kWarpPieces) {
+    int vpt = 1;
+    while (32 * vpt < nv) vpt *= 2;
+    const long long max_grid = static_cast<long long>(sm_count) * (2048 / (kWarpRows * 32)) * 4;
+    const dim3 grid(static_cast<unsigned>(std::min<long long>((rows + kWarpRows - 1) / kWarpRows, max_grid)));
+    switch (vpt) {
+      case 1: e = launch_dependent(softmax_warp_kernel<T, LOG, 1>, grid, kWarpRows * 32, 0, stream, 1, x, out, rows, cols); break;
+      case 2: e = launch_dependent(softmax_warp_kernel<T, LOG, 2>, grid, kWarpRows * 32, 0, stream, 1, x, out, rows, cols); break;
+      case 4: e = launch_dependent(softmax_warp_kernel<T, LOG, 4>, grid, kWarpRows * 32, 0, stream, 1, x, out, rows, cols); break;
+      default: e = launch_dependent(softmax_warp_kernel<T, LOG, 8>, grid, kWarpRows * 32, 0, stream, 1, x, out, rows, cols); break;
+    }
+  } else if (nv <= 4 * 1024) {
+    // four pieces per thread whatever the length; rows are dealt in small portions (16 resident grids' worth of CTAs),
+    // which measured 2 - 7 % above 4 and keeps CTAs from running in step
+    const int threads = static_cast<int>(((nv + 3) / 4 + 31) / 32 * 32);
+    const long long max_grid = static_cast<long long>(sm_count) * (2048 / threads) * 16;
+    const dim3 grid(static_cast<unsigned>(std::min<long long>(rows, max_grid)));
+    e = launch_dependent(softmax_reg_kernel<T, LOG>, grid, threads, 0, stream, 1, x, out, rows, cols);
+  } else {
+    const int csize = ring_cluster(rows, nv, sm_count);
+    const int slice = static_cast<int>((nv + csize - 1) / csize);
+    const size_t smem = static_cast<size_t>(kRingPieces) * 16;
+    auto kernel = softmax_ring_kernel<T, LOG>;
+    int rc = set_smem_limit(kernel, smem);
+    if (rc) return rc;
+    // one CTA per SM; how many clusters of a size the GPU holds at once is asked of the driver once (the answer depends
+    // on the device model only, and only B200 is accepted)
+    static std::atomic<int> resident[4];
+    const int log_c = csize == 1 ? 0 : (csize == 2 ? 1 : (csize == 4 ? 2 : 3));
+    int n = resident[log_c].load(std::memory_order_relaxed);
+    if (n == 0) {
+      n = sm_count;
+      if (csize > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(sm_count / csize * csize), 1, 1);
+        cfg.blockDim = dim3(kRingThreads + 32, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = csize;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveClusters(softmax)");
+        n = std::max(1, n);
+      }
+      resident[log_c].store(n, std::memory_order_relaxed);
+    }
+    const long long clusters = std::min<long long>(rows, n);
+    e = launch_dependent(kernel, dim3(static_cast<unsigned>(clusters * csize)), kRingThreads + 32, smem, stream,
+                         static_cast<unsigned>(csize), x, out, rows, cols, slice, csize);
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "softmax kernel launch");
+  return B200ATTN_OK;
+}
+
+// Everything else: rows that x and out place differently on the 16-byte grid, and rows beyond what a cluster's ring holds.
+template <typename T, bool LOG>
+int launch_elements(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t stream) {
   const T* x = static_cast<const T*>(a.x);
   T* out = static_cast<T*>(a.out);
   const long long rows = a.rows, cols = a.cols;
   const size_t row_bytes = static_cast<size_t>(cols) * sizeof(T);
-  constexpr int E = 16 / static_cast<int>(sizeof(T));
-  constexpr int kMaxVpt = 32 / E;                      // 32 elements per thread
-  constexpr int kPrefVpt = 16 / E;                     // 16 elements per thread: 32 registers, two 1024-thread CTAs per SM
-  if (VEC && cols / E <= 1024LL * kPrefVpt) {
-    const int nv = static_cast<int>(cols / E);
-    int threads = 64;
-    while (threads < 1024 && threads * 4 < nv) threads *= 2;
-    int vpt = 1;
-    while (threads * vpt < nv) vpt *= 2;
-    const long long max_grid = static_cast<long long>(sm_count) * (2048 / threads) * 4;
-    const unsigned grid = static_cast<unsigned>(std::min<long long>(rows, max_grid));
-    switch (vpt) {
-      case 1: softmax_reg_kernel<T, LOG, 1><<<grid, threads, 0, stream>>>(x, out, rows, cols); break;
-      case 2: softmax_reg_kernel<T, LOG, 2><<<grid, threads, 0, stream>>>(x, out, rows, cols); break;
-      case 4: softmax_reg_kernel<T, LOG, 4><<<grid, threads, 0, stream>>>(x, out, rows, cols); break;
-      default: break;                                 // (not reached: vpt <= kPrefVpt <= 4)
-    }
-  } else if (VEC && row_bytes <= static_cast<size_t>(kPipeSliceBytes) * kMaxCluster) {
-    // measured against the alternatives below on every length from 24 576 elements up: the pipelined kernel wins
-    const long long nv = cols / E;
-    int csize = 1;
-    while ((nv + csize - 1) / csize * 16 > kPipeSliceBytes) csize *= 2;
-    const int slice = static_cast<int>((nv + csize - 1) / csize);
-    const int stages = std::max(2, std::min<int>(kPipeStages, 2 * kPipeSliceBytes / (slice * 16)));
-    const size_t smem = static_cast<size_t>(slice) * 16 * stages;
-    auto kernel = softmax_pipe_kernel<T, LOG>;
-    int rc = set_smem_limit(kernel, smem);
-    if (rc) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(1024, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csize;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = csize > 1 ? 1 : 0;
-    // the grid is exactly what the GPU holds at once (each CTA or cluster loops over rows)
-    thread_local int key_csize = 0, resident = 0;
-    thread_local size_t key_smem = 0;
-    if (key_csize != csize || key_smem != smem) {
-      int n = 0;
-      if (csize > 1) {
-        cfg.gridDim = dim3(static_cast<unsigned>(sm_count / csize * csize), 1, 1);
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveClusters(softmax)");
-      } else {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 1024, smem);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(softmax)");
-        n *= sm_count;
-      }
-      resident = std::max(1, n);
-      key_csize = csize;
-      key_smem = smem;
-    }
-    const long long clusters = std::min<long long>(rows, resident);
-    cfg.gridDim = dim3(static_cast<unsigned>(clusters * csize), 1, 1);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, x, out, rows, cols, slice, csize, stages);
-    if (e != cudaSuccess) return cuda_fail(e, "softmax pipelined kernel launch");
-  } else if (VEC && cols / E <= 1024LL * kMaxVpt * kMaxCluster) {
-    // up to 1 MiB: the row in the registers of eight CTAs, 32 elements per thread
-    const int csize = kMaxCluster;
-    auto kernel = softmax_regc_kernel<T, LOG, kMaxVpt>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(1024, 1, 1);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csize;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    // the grid is exactly the clusters the GPU holds at once (each loops over rows); asked of the driver once.  The
-    // answer depends on the device model only, and only B200 is accepted.
-    static int cached = 0;
-    if (cached == 0) {
-      cfg.gridDim = dim3(static_cast<unsigned>(sm_count / csize * csize), 1, 1);
-      int n = 0;
-      cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-      if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveClusters(softmax)");
-      cached = std::max(1, n);
-    }
-    const long long clusters = std::min<long long>(rows, cached);
-    cfg.gridDim = dim3(static_cast<unsigned>(clusters * csize), 1, 1);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, x, out, rows, cols);
-    if (e != cudaSuccess) return cuda_fail(e, "softmax register cluster kernel launch");
-  } else if (row_bytes <= static_cast<size_t>(kRowSmemBytes)) {
-    // threads: enough for 16-byte pieces to keep every lane busy on short rows, 1024 on long ones
+  if (row_bytes <= static_cast<size_t>(kRowSmemBytes)) {
     int threads = 64;
     while (threads < 1024 && static_cast<long long>(threads) * 8 < cols) threads *= 2;
-    const size_t smem = (row_bytes + 15) & ~static_cast<size_t>(15);
-    int rc = set_smem_limit(softmax_row_kernel<T, LOG, VEC>, smem);
+    int rc = set_smem_limit(softmax_row_kernel<T, LOG>, row_bytes);
     if (rc) return rc;
     const long long max_grid = static_cast<long long>(sm_count) * 32;
     const unsigned grid = static_cast<unsigned>(std::min<long long>(rows, max_grid));
-    softmax_row_kernel<T, LOG, VEC><<<grid, threads, smem, stream>>>(x, out, rows, cols);
+    softmax_row_kernel<T, LOG><<<grid, threads, row_bytes, stream>>>(x, out, rows, cols);
   } else if (row_bytes <= static_cast<size_t>(kRowSmemBytes) * kMaxCluster) {
     // more CTAs per row while a slice stays above 64 KiB (fp32) / 128 KiB (16-bit), measured: smaller CTAs share an SM
     // and one's loads overlap another's stores
     int csize = 2;
     while (csize < kMaxCluster && (static_cast<size_t>(kRowSmemBytes) * csize < row_bytes || row_bytes / csize > (sizeof(T) == 4 ? 64 : 128) * 1024)) csize *= 2;
-    long long slice = (cols + csize - 1) / csize;
-    slice = ((slice + E - 1) / E) * E;                 // slices start on 16-byte boundaries of the row
+    const long long slice = (cols + csize - 1) / csize;
     const size_t smem = static_cast<size_t>(slice) * sizeof(T);
-    int rc = set_smem_limit(softmax_cluster_kernel<T, LOG, VEC>, smem);
+    int rc = set_smem_limit(softmax_cluster_kernel<T, LOG>, smem);
     if (rc) return rc;
     const int per_sm = std::max<int>(1, std::min<int>(2, static_cast<int>((220 * 1024) / (smem + 1024))));
     const long long clusters = std::min<long long>(rows, std::max(1, sm_count * per_sm / csize));
@@ -712,7 +734,7 @@ int launch_typed(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t st
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, softmax_cluster_kernel<T, LOG, VEC>, x, out, rows, cols, slice);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, softmax_cluster_kernel<T, LOG>, x, out, rows, cols, slice);
     if (e != cudaSuccess) return cuda_fail(e, "softmax cluster kernel launch");
   } else {
     const unsigned grid = static_cast<unsigned>(std::min<long long>(rows, static_cast<long long>(sm_count) * 2));
@@ -725,13 +747,11 @@ int launch_typed(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t st
 
 template <typename T>
 int launch_dtype(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t stream) {
-  // 16-byte copies need every row to start on a 16-byte boundary
-  const bool vec = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 &&
-                   (static_cast<size_t>(a.cols) * sizeof(T)) % 16 == 0;
-  if (a.log_softmax) {
-    return vec ? launch_typed<T, true, true>(a, sm_count, stream) : launch_typed<T, true, false>(a, sm_count, stream);
-  }
-  return vec ? launch_typed<T, false, true>(a, sm_count, stream) : launch_typed<T, false, false>(a, sm_count, stream);
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(a.x), oa = reinterpret_cast<uintptr_t>(a.out);
+  const bool pieces = (xa & 15) == (oa & 15) && xa % sizeof(T) == 0 &&
+                      a.cols / Vec16<T>::kElems <= static_cast<long long>(kRingPieces) * kMaxCluster;
+  if (a.log_softmax) return pieces ? launch_pieces<T, true>(a, sm_count, stream) : launch_elements<T, true>(a, sm_count, stream);
+  return pieces ? launch_pieces<T, false>(a, sm_count, stream) : launch_elements<T, false>(a, sm_count, stream);
 }
 
 }  // namespace
