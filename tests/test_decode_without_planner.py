@@ -1,0 +1,60 @@
+"""The fp32 decode kernel's row blocks."""
+import pytest
+import torch
+
+from helpers import assert_close_both
+from oracle import sdpa_ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _problem(gen, lens, qh, kvh, d, dtype, m=0):
+    shape = (qh, d) if m == 0 else (qh, m, d)
+    qs = [torch.randn(shape, generator=gen).to(dtype).to(DEV) for _ in lens]
+    ks = [torch.randn((n, kvh, d), generator=gen).to(dtype).to(DEV) for n in lens]
+    vs = [torch.randn((n, kvh, d), generator=gen).to(dtype).to(DEV) for n in lens]
+    return qs, ks, vs
+
+
+def _call(qs, ks, vs, layout, m, page=16, index=torch.int32):
+    from kernels import decode_attention, speculative_decode_attention
+
+    q = torch.stack(qs)
+    if layout == "ragged":
+        (k, ip), (v, _) = sdpa_ref.pack_ragged(ks, index), sdpa_ref.pack_ragged(vs, index)
+        kw = {"kv_indptr": ip}
+    elif layout == "dense":
+        k, v = (torch.stack([x.transpose(0, 1) for x in t]).contiguous() for t in (ks, vs))
+        kw = {}
+    else:
+        k, kt, n = sdpa_ref.pack_paged(ks, page, permute_seed=1, extra_pages=2, pad_value=-1, poison=float("nan"))
+        v, vt, _ = sdpa_ref.pack_paged(vs, page, permute_seed=2, extra_pages=2, pad_value=-1, poison=float("nan"))
+        kw = {"kv_indptr": n, "k_block_table": kt, "v_block_table": vt, "kv_page_size": page}
+    return decode_attention(q, k, v, **kw) if m == 0 else speculative_decode_attention(q, k, v, causal=True, **kw)
+
+
+def _reference(qs, ks, vs, qh, kvh, m):
+    f = [[t.float() for t in x] for x in (qs, ks, vs)]
+    refs = sdpa_ref.decode_reference(*f, qh, kvh) if m == 0 else sdpa_ref.spec_decode_reference(*f, qh, kvh, True)
+    return torch.stack(refs)
+
+
+# q rows per KV head: blocks of 1, 2 and 4 rows, blocks with rows left over, three blocks (no key split); more than 16 rows
+# multiply in 16 bits, on another kernel
+@pytest.mark.parametrize("group", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("layout", ["ragged", "paged"])
+def test_fp32_row_blocks(group, d, layout):
+    gen = torch.Generator().manual_seed(group * 7 + d)
+    lens = [1, 31, 64, 65, 200, 1111]
+    qs, ks, vs = _problem(gen, lens, 2 * group, 2, d, torch.float32)
+    out = _call(qs, ks, vs, layout, 0)
+    # 64-bit reference.  A score is a sum of d products of N(0, 1) numbers, a weight its exponential, an output a sum of
+    # weighted values: relative errors of a few d * 2^-24 (scores of up to 5 / sqrt(d) * d) - 2e-5 covers them.
+    f = [[t.double().cpu() for t in x] for x in (qs, ks, vs)]
+    for i, n in enumerate(lens):
+        k = f[1][i].repeat_interleave(group, 1)
+        w = torch.softmax(torch.einsum("hd,nhd->hn", f[0][i], k) / d ** 0.5, -1)
+        want = torch.einsum("hn,nhd->hd", w, f[2][i].repeat_interleave(group, 1))
+        torch.testing.assert_close(out[i].double().cpu(), want, atol=2e-5, rtol=2e-5)

@@ -1519,13 +1519,27 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------------------
-// fp32 kernel: fp32 FMA dot products, one warp per q row, lanes split head_dim
+// fp32 kernel: fp32 FMA dot products.
+//
+// A key row is held by D / 8 lanes, eight floats each, so a warp has 32 / (D / 8) rows in hand per load instruction
+// (4 at head_dim 64, 2 at 128) and a dot product is three or four shuffles instead of the five that a row spread over
+// the whole warp takes; the RB query rows of a block share every key row that is loaded.  Each lane group keeps an
+// online softmax of its own over its keys, so that nothing but the dot products crosses lanes inside the loop; the
+// groups of a warp are merged once at the end, the warps of a row in emit_and_merge.
+// kKeys rows of K and V per lane group are loaded one step ahead of their use, into registers: the kernel is bound by
+// the bytes in flight.
 // ---------------------------------------------------------------------------
-template <int D>
-__global__ void __launch_bounds__(128) decode_simt_kernel(const DecodeParams p) {
+constexpr int kSimtThreads = 128;
+
+// rows of a block: the q rows that share a K/V read (a fourth one would cost registers that the loads need)
+template <int D, int RB>
+__global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_ticket;
-  constexpr int VEC = D / 32;  // floats per lane
+  constexpr int kGroup = D / 8;              // lanes that share a key row
+  constexpr int kRowsWarp = 32 / kGroup;     // key rows of a warp per load instruction
+  constexpr int kKeys = 2;                   // key rows of a lane group per step
+  constexpr int kStep = kRowsWarp * kKeys;   // keys of a warp per step
   ptx::grid_dep_wait();      // the planner's records are complete and visible from here on
   const int n_items = p.header[2];
   // heads vary fastest across CTAs: the CTAs that run side by side walk the same pages and read
@@ -1534,98 +1548,149 @@ __global__ void __launch_bounds__(128) decode_simt_kernel(const DecodeParams p) 
   if (item >= n_items) return;
   const int h = blockIdx.x - item * p.kv_heads;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = blockDim.x >> 5;
+  const int sub = lane / kGroup, gl = lane % kGroup;
+  constexpr int nwarps = kSimtThreads / 32;
   const int R = p.rows;
 
-  const int b = find_sequence(p.item_start, p.batch, item);
-  const int item0 = p.item_start[b];
-  const int c = item - item0;
-  const int n_chunks = p.item_start[b + 1] - item0;
-  const SeqInfo si = seq_info(p, b);
-  const int len = si.len;
-  const int chunk = seq_chunk(len, n_chunks, p.header[1], p.equal_split);
-  const int t_begin = c * chunk;
-  const int t_end = min(len, t_begin + chunk);
+  const int4 rec0 = __ldg(p.item_info + 2 * item);
+  const int4 rec1 = __ldg(p.item_info + 2 * item + 1);
+  const int b = rec0.x, c = rec0.y, n_chunks = rec0.z, item0 = rec0.w;
+  const long long seq_start = (static_cast<long long>(rec1.w) << 32) | static_cast<unsigned int>(rec1.z);
+  const int len = rec1.x;
+  const int t_begin = c * rec1.y;
+  const int t_end = min(len, t_begin + rec1.y);
 
-  float* comb_o = reinterpret_cast<float*>(smem);                            // [KS][R][D], KS * R <= max(R, warps)
-  float* comb_ml = comb_o + static_cast<size_t>(max(R, nwarps)) * D;         // [KS][R][2]
-  const float* kg = static_cast<const float*>(p.k);
-  const float* vg = static_cast<const float*>(p.v);
+  float* comb_o = reinterpret_cast<float*>(smem);                       // [KS][R][D]
+  const int blocks = (R + RB - 1) / RB;                                 // blocks of RB rows
+  const int KS = (blocks <= nwarps && nwarps % blocks == 0) ? nwarps / blocks : 1;   // warps that split a block's keys
+  float* comb_ml = comb_o + static_cast<size_t>(KS) * R * D;            // [KS][R][2]
+  const float* kg = static_cast<const float*>(p.k) + gl * 4;
+  const float* vg = static_cast<const float*>(p.v) + gl * 4;
   const float* qg = static_cast<const float*>(p.q) +
                     ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
   const float sl2 = p.scale_log2;
+  constexpr int kHalf = D / 2;               // a lane holds 4 floats at gl * 4 and 4 at D / 2 + gl * 4
 
-  // A warp owns one q row (lanes split head_dim) and takes four keys per step: four independent dot products and
-  // shuffle reductions in flight, one online-softmax update for the four.  With fewer rows than warps (plain decode
-  // with a small GQA group) the warps of a row split its keys in groups of four and leave one partial each, which
-  // emit_and_merge combines like the key slices of the tensor-core kernel.
-  constexpr int TB = 4;
-  const int KS = (R <= nwarps && nwarps % R == 0) ? nwarps / R : 1;
-  for (int rr = warp; rr < R * KS; rr += nwarps) {
-    const int r = rr % R, ks = rr / R;
-    float qv[VEC], acc[VEC];
+  for (int rr = warp; rr < blocks * KS; rr += nwarps) {
+    const int r0 = (rr % blocks) * RB, ks = rr / blocks;
+    float4 q0[RB], q1[RB], a0[RB], a1[RB];
+    float m[RB], l[RB];
+    int vis[RB];                             // keys [0, vis) of the sequence are visible to the row
+    int stop = 0, all = t_end;               // keys any row of the block sees; keys every row sees
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) { qv[i] = qg[static_cast<long long>(r) * D + lane * VEC + i]; acc[i] = 0.f; }
-    const int lim = p.causal ? (len - p.q_len + (r % p.q_len)) : (len - 1);
-    const int stop = min(t_end, lim + 1);
-    float m = -INFINITY, l = 0.f;
-    for (int t = t_begin + ks * TB; t < stop; t += KS * TB) {
-      float dot[TB], vv[TB][VEC];
+    for (int i = 0; i < RB; ++i) {
+      const int r = min(r0 + i, R - 1);      // (rows past the last repeat it and are not written)
+      q0[i] = __ldg(reinterpret_cast<const float4*>(qg + static_cast<long long>(r) * D) + gl);
+      q1[i] = __ldg(reinterpret_cast<const float4*>(qg + static_cast<long long>(r) * D + kHalf) + gl);
+      a0[i] = a1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      m[i] = -INFINITY;
+      l[i] = 0.f;
+      vis[i] = min(t_end, p.causal ? len - p.q_len + (r % p.q_len) + 1 : len);
+      stop = max(stop, vis[i]);
+      all = min(all, vis[i]);
+    }
+    float4 k0[kKeys], k1[kKeys], v0[kKeys], v1[kKeys];
+    bool on[kKeys];
+    // issues the loads of the step that starts at key t
+    auto load = [&](int t) {
 #pragma unroll
-      for (int j = 0; j < TB; ++j) {
-        dot[j] = -INFINITY;                       // a key past the end, or on a page outside the cache, weighs nothing
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) vv[j][i] = 0.f;
-        if (t + j >= stop) continue;
-        const long long ko = row_offset(p, p.k_table, b, h, si.start, t + j, D);
-        const long long vo = (p.layout == B200ATTN_PAGED) ? row_offset(p, p.v_table, b, h, si.start, t + j, D) : ko;
-        if (ko < 0 || vo < 0) {
-          if (lane == 0) p.header[0] = DEV_ERR_PAGE_RANGE;
+      for (int j = 0; j < kKeys; ++j) {
+        const int key = t + j * kRowsWarp + sub;
+        k0[j] = k1[j] = v0[j] = v1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        on[j] = key < stop;
+        if (!on[j]) continue;
+        const long long ko = row_offset(p, p.k_table, b, h, seq_start, key, D);
+        const long long vo = (p.layout == B200ATTN_PAGED) ? row_offset(p, p.v_table, b, h, seq_start, key, D) : ko;
+        if (ko < 0 || vo < 0) {              // a key on a page outside the cache weighs nothing
+          if (gl == 0) p.header[0] = DEV_ERR_PAGE_RANGE;
+          on[j] = false;
           continue;
         }
-        float kv[VEC];
-        if constexpr (VEC == 4) {
-          const float4 k4 = __ldg(reinterpret_cast<const float4*>(kg + ko) + lane);
-          const float4 v4 = __ldg(reinterpret_cast<const float4*>(vg + vo) + lane);
-          kv[0] = k4.x; kv[1] = k4.y; kv[2] = k4.z; kv[3] = k4.w;
-          vv[j][0] = v4.x; vv[j][1] = v4.y; vv[j][2] = v4.z; vv[j][3] = v4.w;
-        } else {
-          const float2 k2 = __ldg(reinterpret_cast<const float2*>(kg + ko) + lane);
-          const float2 v2 = __ldg(reinterpret_cast<const float2*>(vg + vo) + lane);
-          kv[0] = k2.x; kv[1] = k2.y;
-          vv[j][0] = v2.x; vv[j][1] = v2.y;
+        k0[j] = __ldg(reinterpret_cast<const float4*>(kg + ko));
+        k1[j] = __ldg(reinterpret_cast<const float4*>(kg + ko + kHalf));
+        v0[j] = __ldg(reinterpret_cast<const float4*>(vg + vo));
+        v1[j] = __ldg(reinterpret_cast<const float4*>(vg + vo + kHalf));
+      }
+    };
+    int t = t_begin + ks * kStep;
+    load(t);
+    for (; t < stop; t += KS * kStep) {
+      float4 ck0[kKeys], ck1[kKeys], cv0[kKeys], cv1[kKeys];
+      bool con[kKeys];
+#pragma unroll
+      for (int j = 0; j < kKeys; ++j) { ck0[j] = k0[j]; ck1[j] = k1[j]; cv0[j] = v0[j]; cv1[j] = v1[j]; con[j] = on[j]; }
+      load(t + KS * kStep);
+      const bool whole = t + kStep <= all;   // every row sees every key of the step
+      float dot[RB][kKeys];
+#pragma unroll
+      for (int i = 0; i < RB; ++i) {
+#pragma unroll
+        for (int j = 0; j < kKeys; ++j) {
+          float d = q0[i].x * ck0[j].x;
+          d = fmaf(q0[i].y, ck0[j].y, d); d = fmaf(q0[i].z, ck0[j].z, d); d = fmaf(q0[i].w, ck0[j].w, d);
+          d = fmaf(q1[i].x, ck1[j].x, d); d = fmaf(q1[i].y, ck1[j].y, d);
+          d = fmaf(q1[i].z, ck1[j].z, d); d = fmaf(q1[i].w, ck1[j].w, d);
+          dot[i][j] = d;
         }
-        float d = 0.f;
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) d = fmaf(qv[i], kv[i], d);
-        dot[j] = d;
       }
-      // (-inf + -inf stays -inf through the reduction: every lane of the warp took the same branch for key j)
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
+      for (int off = kGroup / 2; off > 0; off >>= 1) {
 #pragma unroll
-        for (int j = 0; j < TB; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], off);
+        for (int i = 0; i < RB; ++i) {
+#pragma unroll
+          for (int j = 0; j < kKeys; ++j) dot[i][j] += __shfl_xor_sync(0xffffffffu, dot[i][j], off);
+        }
       }
-      float mn = m;
 #pragma unroll
-      for (int j = 0; j < TB; ++j) { dot[j] *= sl2; mn = fmaxf(mn, dot[j]); }
-      if (mn == -INFINITY) continue;              // nothing visible yet
-      const float a = fast_exp2(m - mn);          // m == -inf: exp2(-inf) = 0
-      l *= a;
+      for (int i = 0; i < RB; ++i) {
+        float mn = m[i];
+        bool see[kKeys];
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) acc[i] *= a;
+        for (int j = 0; j < kKeys; ++j) {
+          see[j] = con[j] && (whole || t + j * kRowsWarp + sub < vis[i]);
+          dot[i][j] = see[j] ? dot[i][j] * sl2 : -INFINITY;
+          mn = fmaxf(mn, dot[i][j]);
+        }
+        const float ms = mn == -INFINITY ? 0.f : mn;    // nothing visible yet: every weight below is 0
+        const float a = fast_exp2(m[i] - ms);           // m == -inf: 0
+        m[i] = mn;
+        l[i] *= a;
+        a0[i].x *= a; a0[i].y *= a; a0[i].z *= a; a0[i].w *= a;
+        a1[i].x *= a; a1[i].y *= a; a1[i].z *= a; a1[i].w *= a;
 #pragma unroll
-      for (int j = 0; j < TB; ++j) {
-        const float pw = fast_exp2(dot[j] - mn);
-        l += pw;
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) acc[i] = fmaf(pw, vv[j][i], acc[i]);
+        for (int j = 0; j < kKeys; ++j) {
+          // (a key that the row does not see is left out rather than weighed with 0: its V may be anything)
+          if (!whole && !see[j]) continue;
+          const float w = fast_exp2(dot[i][j] - ms);
+          l[i] += w;
+          a0[i].x = fmaf(w, cv0[j].x, a0[i].x); a0[i].y = fmaf(w, cv0[j].y, a0[i].y);
+          a0[i].z = fmaf(w, cv0[j].z, a0[i].z); a0[i].w = fmaf(w, cv0[j].w, a0[i].w);
+          a1[i].x = fmaf(w, cv1[j].x, a1[i].x); a1[i].y = fmaf(w, cv1[j].y, a1[i].y);
+          a1[i].z = fmaf(w, cv1[j].z, a1[i].z); a1[i].w = fmaf(w, cv1[j].w, a1[i].w);
+        }
       }
-      m = mn;
     }
+    // merge the lane groups of the warp, then leave one partial per (key slice, row)
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) comb_o[(static_cast<size_t>(ks) * R + r) * D + lane * VEC + i] = acc[i];
-    if (lane == 0) { comb_ml[(ks * R + r) * 2] = m; comb_ml[(ks * R + r) * 2 + 1] = l; }
+    for (int i = 0; i < RB; ++i) {
+      float g = m[i];
+#pragma unroll
+      for (int off = kGroup; off < 32; off <<= 1) g = fmaxf(g, __shfl_xor_sync(0xffffffffu, g, off));
+      const float w = m[i] == -INFINITY ? 0.f : fast_exp2(m[i] - g);
+      float x[9] = {a0[i].x, a0[i].y, a0[i].z, a0[i].w, a1[i].x, a1[i].y, a1[i].z, a1[i].w, l[i]};
+#pragma unroll
+      for (int e = 0; e < 9; ++e) {
+        x[e] *= w;
+#pragma unroll
+        for (int off = kGroup; off < 32; off <<= 1) x[e] += __shfl_xor_sync(0xffffffffu, x[e], off);
+      }
+      if (r0 + i < R && sub == 0) {
+        const size_t row = static_cast<size_t>(ks) * R + r0 + i;
+        *reinterpret_cast<float4*>(comb_o + row * D + gl * 4) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4*>(comb_o + row * D + kHalf + gl * 4) = make_float4(x[4], x[5], x[6], x[7]);
+        if (gl == 0) { comb_ml[row * 2] = g; comb_ml[row * 2 + 1] = x[8]; }
+      }
+    }
   }
   __syncthreads();
   emit_and_merge<float, D>(p, b, h, c, n_chunks, item0, comb_o, comb_ml, KS, R, &s_ticket);
@@ -1817,7 +1882,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   // Equal items per sequence and longest-first order let the greedy CTA dispatch pair long and short items: with two
   // or three whole waves the grid drains almost level (measured on B200, 16-token pages: 0.80 -> 0.84 of the copy
   // bandwidth for paged decode, 0.68 -> 0.76 for speculative decode).
-  p.equal_split = a.dtype != B200ATTN_F32 ? 1 : 0;
+  p.equal_split = 1;
   p.scale_log2 = a.sm_scale * 1.4426950408889634f;
 
   decode_plan_kernel<<<1, kPlanThreads, 0, stream>>>(p);
@@ -1827,10 +1892,19 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   const dim3 grid(static_cast<unsigned>(w.max_items) * a.kv_heads, 1);
   const int D = a.head_dim;
   if (a.dtype == B200ATTN_F32) {
-    const size_t smem = sizeof(float) * static_cast<size_t>(std::max(p.rows, 4)) * (D + 2);   // 4 warps: see the kernel
+    // (four warps leave at most 4 / blocks-of-rows partials per row: see the kernel)
+    const int rb = p.rows >= 3 ? 4 : p.rows;
+    const size_t smem = sizeof(float) * static_cast<size_t>(std::max(p.rows, 4 * rb)) * (D + 2);
     int rc = 0;
-    if (D == 128) { rc = set_smem(decode_simt_kernel<128>, smem); if (rc) return rc; launch_after_planner(decode_simt_kernel<128>, grid, 128, smem, stream, p); }
-    else          { rc = set_smem(decode_simt_kernel<64>, smem);  if (rc) return rc; launch_after_planner(decode_simt_kernel<64>, grid, 128, smem, stream, p); }
+#define B200ATTN_LAUNCH_SIMT(DIM, RB)                                                                 \
+    do {                                                                                              \
+      rc = set_smem(decode_simt_kernel<DIM, RB>, smem);                                               \
+      if (rc) return rc;                                                                              \
+      launch_after_planner(decode_simt_kernel<DIM, RB>, grid, kSimtThreads, smem, stream, p);         \
+    } while (0)
+    if (D == 128) { if (rb == 1) B200ATTN_LAUNCH_SIMT(128, 1); else if (rb == 2) B200ATTN_LAUNCH_SIMT(128, 2); else B200ATTN_LAUNCH_SIMT(128, 4); }
+    else          { if (rb == 1) B200ATTN_LAUNCH_SIMT(64, 1);  else if (rb == 2) B200ATTN_LAUNCH_SIMT(64, 2);  else B200ATTN_LAUNCH_SIMT(64, 4); }
+#undef B200ATTN_LAUNCH_SIMT
   } else if (p.rows > 16) {
     // many q rows per KV head: one 128-row tcgen05 tile with Q and P in tensor memory
     CUtensorMap tk, tv;

@@ -28,7 +28,6 @@ class DecodePlan:
     threads: int
     wave_items: int = 0      # items of one KV head resident at once (one wave); 0: a single wave is never planned
     item_overhead: int = 0   # start-up + merge of an item in keys of streaming time (the planner's cost estimate)
-    equal_split: bool = True
 
 
 def decode_pass_group(group: int, q_len: int) -> int:
@@ -77,8 +76,7 @@ def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: i
     wide = rows > 16           # more than one 16-row tile: the tcgen05 kernel, two resident CTAs per SM (else three)
     wave = 0 if fp32 else max(1, (sm_count * (2 if wide else 3)) // max(1, kv_heads))
     overhead = 0 if fp32 else (448 if wide else 128)
-    return DecodePlan(target, min_chunk, target + batch, tiles, slices, 32 * (tiles * slices + 1), wave, overhead,
-                      not fp32)
+    return DecodePlan(target, min_chunk, target + batch, tiles, slices, 32 * (tiles * slices + 1), wave, overhead)
 
 
 def _round_up(x: int, m: int) -> int:
@@ -87,8 +85,6 @@ def _round_up(x: int, m: int) -> int:
 
 def _item_tokens(plan: DecodePlan, length: int, n: int, chunk: int) -> int:
     """Keys per item of a sequence cut into ``n`` items (csrc/decode.cu seq_chunk)."""
-    if not plan.equal_split:
-        return chunk
     return max(DECODE_TILE_TOKENS, _round_up(-(-length // n), DECODE_TILE_TOKENS))
 
 
