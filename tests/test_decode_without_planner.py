@@ -1,4 +1,5 @@
-"""The fp32 decode kernel's row blocks."""
+"""The fp32 decode kernel's row blocks; calls that follow one another on a stream
+without a synchronisation in between."""
 import pytest
 import torch
 
@@ -58,3 +59,48 @@ def test_fp32_row_blocks(group, d, layout):
         w = torch.softmax(torch.einsum("hd,nhd->hn", f[0][i], k) / d ** 0.5, -1)
         want = torch.einsum("hn,nhd->hd", w, f[2][i].repeat_interleave(group, 1))
         torch.testing.assert_close(out[i].double().cpu(), want, atol=2e-5, rtol=2e-5)
+
+
+@pytest.mark.parametrize("qh,m", [(8, 0), (64, 5)], ids=["decode", "speculative"])   # warp-level and tcgen05 kernel
+def test_calls_in_a_row_see_each_other(qh, m):
+    """Each call reads what the one before it wrote (cache rows, scores, fp16 copies), each has its launch set up while
+    that one is still running: the outputs are those of the same calls one at a time."""
+    from kernels import append_paged_kv, decode_attention, flash_attention_v2, softmax, speculative_decode_attention
+
+    gen = torch.Generator().manual_seed(9)
+    batch, kvh, d, page, steps = 4, 8, 128, 16, 24
+    pages = 20
+    table = torch.randperm(batch * pages, generator=gen).to(torch.int32).view(batch, pages).to(DEV)
+    q0 = torch.randn((batch, qh, d) if m == 0 else (batch, qh, m, d), generator=gen).to(torch.bfloat16).to(DEV)
+    new = torch.randn((batch * 8, kvh, d), generator=gen).to(torch.bfloat16).to(DEV)
+    indptr = torch.arange(0, 8 * batch + 1, 8, dtype=torch.int32, device=DEV)
+    pq = torch.randn((1, 8, 128, d), generator=gen).to(DEV)
+
+    def run(sync):
+        wait = torch.cuda.synchronize if sync else (lambda: None)
+        k = torch.zeros((batch * pages * page, kvh, d), dtype=torch.bfloat16, device=DEV)
+        v = torch.zeros_like(k)
+        x, y, outs = q0, pq, []
+        for s in range(steps):
+            pos = torch.full((batch,), 8 * s, dtype=torch.int32, device=DEV)
+            lens = pos + 8
+            wait()
+            append_paged_kv(k, table, new, indptr, page, dst_pos=pos)
+            wait()
+            append_paged_kv(v, table, softmax(new), indptr, page, dst_pos=pos)
+            wait()
+            kw = dict(kv_indptr=lens, k_block_table=table, v_block_table=table, kv_page_size=page)
+            x = decode_attention(x, k, v, **kw) if m == 0 else speculative_decode_attention(x, k, v, causal=True, **kw)
+            wait()
+            x = softmax(x)
+            wait()
+            y = flash_attention_v2(y, y, y, is_causal=True)
+            wait()
+            y = softmax(y)
+            wait()
+            outs += [x, y]
+        torch.cuda.synchronize()
+        return [*outs, k, v]
+
+    for a, b in zip(run(True), run(False)):
+        assert torch.equal(a, b)

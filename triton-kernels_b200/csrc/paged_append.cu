@@ -3,7 +3,9 @@
 // reference's fixtures (tests/test_attention.py:101-134, benchmarks/attention.py:351-431).  Pure byte movement:
 // one warp per token row, 16-byte pieces, every source and destination byte touched once.
 #include "common.cuh"
+#include "launch.cuh"
 #include "paged_append_launch.h"
+#include "sm100_ptx.cuh"
 
 namespace b200attn {
 
@@ -14,6 +16,8 @@ __global__ void __launch_bounds__(256) paged_append_kernel(const PagedAppendPara
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   const int pieces = p.row_bytes >> 4;
+  ptx::grid_dep_launch_dependents();
+  ptx::grid_dep_wait();
   for (long long row = warp; row < p.total_rows; row += nwarps) {
     // sequence that owns this source row: last b with indptr[b] <= row
     int lo = 0, hi = p.batch;
@@ -40,7 +44,7 @@ __global__ void __launch_bounds__(256) paged_append_kernel(const PagedAppendPara
     const long long dst_row = static_cast<long long>(page) * p.page_size + (pos - lp * p.page_size);
     const uint4* src = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.src) + row * p.row_bytes);
     uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.cache) + dst_row * p.row_bytes);
-    for (int i = lane; i < pieces; i += 32) dst[i] = __ldg(src + i);
+    for (int i = lane; i < pieces; i += 32) dst[i] = __ldcg(src + i);
   }
 }
 
@@ -59,8 +63,7 @@ int launch_paged_append(const b200attn_paged_append_args_t& a, int sm_count, cud
   long long blocks = (warps_needed + 7) / 8;              // 8 warps per block
   const long long cap = static_cast<long long>(sm_count) * 16;
   if (blocks > cap) blocks = cap;
-  paged_append_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_dependent(paged_append_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1, p);
   if (e != cudaSuccess) return cuda_fail(e, "paged_append_kernel launch");
   return B200ATTN_OK;
 }

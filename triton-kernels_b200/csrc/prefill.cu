@@ -30,6 +30,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "launch.cuh"
 #include "prefill_launch.h"
 #include "sm100_ptx.cuh"
 #include "tensor_map.h"
@@ -151,9 +152,11 @@ __device__ __forceinline__ bool find_ragged_work(const PrefillParams& p, int x, 
 // same cast in registers, kernels/attention.py:547,572,594,614) and the result is written back as fp32.
 __global__ void __launch_bounds__(256) cast_f32_to_f16_kernel(const float4* __restrict__ src, uint2* __restrict__ dst,
                                                               long long n4) {
+  ptx::grid_dep_launch_dependents();
+  ptx::grid_dep_wait();
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float4 f = __ldg(src + i);
+    const float4 f = __ldcg(src + i);
     uint2 u;
     u.x = ElemTraits<__half>::pack2(f.x, f.y);
     u.y = ElemTraits<__half>::pack2(f.z, f.w);
@@ -306,6 +309,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tc_fence_before();
     named_bar_sync(1, kThreads);
     tc_fence_after();
+    // (by one thread, once this CTA holds its tensor memory: a later kernel's CTA that took it first would wait for this
+    // grid while this grid waits for it)
+    if (warp == kMmaWarp) ptx::grid_dep_launch_dependents();
   }
   const uint32_t tmem = warp == kProducerWarp ? 0u : ctrl->tmem_base;   // (the producer never uses it)
   volatile int* abort_flag = &ctrl->abort_flag;
@@ -313,6 +319,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   if (warp == kProducerWarp) {
     // =========================== scheduler + TMA producer ===========================
     if (lane == 0) { prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); }
+    // everything the other warps read or write outside this CTA follows an item published or a tile loaded below
+    ptx::grid_dep_wait();
     bool ok = true;
     int pair_e = 0;       // K/V pairs issued so far, across items
     int pair_lo = 0;      // first pair of the current item
@@ -1024,9 +1032,10 @@ namespace {
 // lse[...] its log-sum-exp (log2 domain): out = sum_s 2^(lse_s - max) part_s / sum_s 2^(lse_s - max)
 // (the reference's merge kernel, kernels/attention.py:659-746, on normalised instead of raw accumulators).
 template <typename OutT, int D>
-__global__ void __launch_bounds__(256) prefill_merge_kernel(const OutT* __restrict__ part, const float* __restrict__ lse,
-                                                            OutT* __restrict__ out, long long rows_per_batch, int batch,
-                                                            int parts) {
+__global__ void __launch_bounds__(256) prefill_merge_kernel(const OutT* part, const float* lse, OutT* out,
+                                                            long long rows_per_batch, int batch, int parts) {
+  ptx::grid_dep_launch_dependents();
+  ptx::grid_dep_wait();
   constexpr int VEC = 16 / sizeof(OutT);          // elements per 16-byte piece
   constexpr int PIECES = D / VEC;
   const long long total = static_cast<long long>(batch) * rows_per_batch * PIECES;
@@ -1036,17 +1045,17 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const OutT* __restri
     const long long row = idx / PIECES;                    // (b, h, r) flattened
     const long long b = row / rows_per_batch, hr = row - b * rows_per_batch;
     float mx = -INFINITY;
-    for (int sp = 0; sp < parts; ++sp) mx = fmaxf(mx, __ldg(lse + (b * parts + sp) * rows_per_batch + hr));
+    for (int sp = 0; sp < parts; ++sp) mx = fmaxf(mx, __ldcg(lse + (b * parts + sp) * rows_per_batch + hr));
     float acc[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
     float wsum = 0.f;
     for (int sp = 0; sp < parts; ++sp) {
       const long long prow = (b * parts + sp) * rows_per_batch + hr;
-      const float l = __ldg(lse + prow);
+      const float l = __ldcg(lse + prow);
       const float w = (l == -INFINITY) ? 0.f : fast_exp2(l - mx);
       wsum += w;
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(part + prow * D) + piece);
+      const uint4 u = __ldcg(reinterpret_cast<const uint4*>(part + prow * D) + piece);
       const OutT* e = reinterpret_cast<const OutT*>(&u);
 #pragma unroll
       for (int i = 0; i < VEC; ++i) acc[i] += w * ElemTraits<OutT>::to_float(e[i]);
@@ -1175,11 +1184,10 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
       const long long n4 = static_cast<long long>(cnt[i] / 4);  // head_dim is a multiple of 4
       if (n4 == 0) continue;
       const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, static_cast<long long>(sm_count) * 16));
-      cast_f32_to_f16_kernel<<<blocks, 256, 0, stream>>>(static_cast<const float4*>(src[i]),
-                                                         reinterpret_cast<uint2*>(ws + off[i]), n4);
+      const cudaError_t ce = launch_dependent(cast_f32_to_f16_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1,
+                                              static_cast<const float4*>(src[i]), reinterpret_cast<uint2*>(ws + off[i]), n4);
+      if (ce != cudaSuccess) return cuda_fail(ce, "cast kernel launch");
     }
-    cudaError_t ce = cudaGetLastError();
-    if (ce != cudaSuccess) return cuda_fail(ce, "cast kernel launch");
     a.q = ws + c.q_off; a.k = ws + c.k_off; a.v = ws + c.v_off;
     a.dtype = B200ATTN_F16;
   }
@@ -1254,10 +1262,10 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
     const size_t smem = std::max<size_t>(SmemPlan<DIM>::kTotal + 1024, 120 * 1024);                      \
     if (a.layout == B200ATTN_PAGED) {                                                                    \
       if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_kernel<TYPE, DIM, OUT, true>), smem))) return rc; \
-      prefill_kernel<TYPE, DIM, OUT, true><<<grid, kThreads, smem, stream>>>(tq, tk, tv, p);             \
+      launch_dependent(prefill_kernel<TYPE, DIM, OUT, true>, grid, kThreads, smem, stream, 1, tq, tk, tv, p);  \
     } else {                                                                                             \
       if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_kernel<TYPE, DIM, OUT, false>), smem))) return rc; \
-      prefill_kernel<TYPE, DIM, OUT, false><<<grid, kThreads, smem, stream>>>(tq, tk, tv, p);            \
+      launch_dependent(prefill_kernel<TYPE, DIM, OUT, false>, grid, kThreads, smem, stream, 1, tq, tk, tv, p); \
     }                                                                                                    \
   } while (0)
   if (f32) {
@@ -1275,8 +1283,9 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
     const long long pieces = static_cast<long long>(a.batch) * rows_per_batch * (D / (f32 ? 4 : 8));
     const int blocks = static_cast<int>(std::min<long long>((pieces + 255) / 256, static_cast<long long>(sm_count) * 8));
 #define B200ATTN_LAUNCH_MERGE(OUT, DIM)                                                                              \
-    prefill_merge_kernel<OUT, DIM><<<blocks, 256, 0, stream>>>(static_cast<const OUT*>(p.out), p.lse,                 \
-                                                               static_cast<OUT*>(a_in.out), rows_per_batch, a.batch, p.kv_split)
+    launch_dependent(prefill_merge_kernel<OUT, DIM>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1,          \
+                     static_cast<const OUT*>(p.out), static_cast<const float*>(p.lse), static_cast<OUT*>(a_in.out),   \
+                     rows_per_batch, a.batch, p.kv_split)
     if (f32) { if (D == 128) B200ATTN_LAUNCH_MERGE(float, 128); else B200ATTN_LAUNCH_MERGE(float, 64); }
     else if (a.dtype == B200ATTN_BF16) { if (D == 128) B200ATTN_LAUNCH_MERGE(__nv_bfloat16, 128); else B200ATTN_LAUNCH_MERGE(__nv_bfloat16, 64); }
     else { if (D == 128) B200ATTN_LAUNCH_MERGE(__half, 128); else B200ATTN_LAUNCH_MERGE(__half, 64); }
