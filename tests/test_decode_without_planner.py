@@ -1,5 +1,5 @@
-"""The fp32 decode kernel's row blocks; calls that follow one another on a stream
-without a synchronisation in between."""
+"""Decode calls with few (sequence, KV head) pairs plan inside the kernel; the fp32 kernel's row blocks; calls that follow
+one another on a stream without a synchronisation in between."""
 import pytest
 import torch
 
@@ -8,6 +8,7 @@ from oracle import sdpa_ref
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
+PAIRS = 96                    # csrc/decode_launch.h kInlinePairs
 
 
 def _problem(gen, lens, qh, kvh, d, dtype, m=0):
@@ -39,6 +40,33 @@ def _reference(qs, ks, vs, qh, kvh, m):
     f = [[t.float() for t in x] for x in (qs, ks, vs)]
     refs = sdpa_ref.decode_reference(*f, qh, kvh) if m == 0 else sdpa_ref.spec_decode_reference(*f, qh, kvh, True)
     return torch.stack(refs)
+
+
+# batch x KV heads on both sides of the line; one KV head (most items per pair); lengths around tiles, one key, long
+@pytest.mark.parametrize("batch,qh,kvh", [(1, 8, 1), (1, 32, 8), (12, 8, 8), (13, 8, 8), (48, 4, 2), (49, 4, 2), (96, 2, 1),
+                                          (97, 2, 1), (1, 96, 96), (1, 97, 97)])
+@pytest.mark.parametrize("layout,page,index", [("dense", 0, None), ("ragged", 0, torch.int32), ("ragged", 0, torch.int64),
+                                               ("paged", 16, None), ("paged", 24, None)])
+def test_both_plans_over_layouts(batch, qh, kvh, layout, page, index):
+    gen = torch.Generator().manual_seed(batch * 131 + qh)
+    base = [300] if layout == "dense" else [1, 63, 64, 65, 127, 129, 640, 1000, 2500]
+    lens = [base[i % len(base)] for i in range(batch)] if batch > 1 else [5000]
+    for m in (0, 2):
+        qs, ks, vs = _problem(gen, lens, qh, kvh, 64, torch.bfloat16, m)
+        out = _call(qs, ks, vs, layout, m, page or 16, index or torch.int32)
+        assert_close_both(out, _reference(qs, ks, vs, qh, kvh, m), torch.bfloat16, max(lens), f"{layout} {batch}x{kvh} m{m}")
+
+
+def test_empty_sequences_without_planner():
+    gen = torch.Generator().manual_seed(5)
+    lens = [0, 700, 0, 3, 0]
+    for dtype in (torch.float16, torch.float32):
+        qs, ks, vs = _problem(gen, lens, 8, 2, 64, dtype)
+        out = _call(qs, ks, vs, "ragged", 0)
+        live = [i for i, n in enumerate(lens) if n]
+        ref = _reference([qs[i] for i in live], [ks[i] for i in live], [vs[i] for i in live], 8, 2, 0)
+        assert_close_both(out[live], ref, dtype, 700)
+        assert (out[[0, 2, 4]] == 0).all()
 
 
 # q rows per KV head: blocks of 1, 2 and 4 rows, blocks with rows left over, three blocks (no key split); more than 16 rows

@@ -92,15 +92,6 @@ __device__ __forceinline__ long long row_offset(const DecodeParams& p, const int
   }
 }
 
-__device__ __forceinline__ int find_sequence(const int* item_start, int batch, int item) {
-  int lo = 0, hi = batch;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (item_start[mid] <= item) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
 // Fills `rows` combined rows with NaN accumulators and (m, l) = (0, 1); every thread of the CTA takes part.
 __device__ __forceinline__ void poison_rows(float* comb_o, float* comb_ml, int rows, int d) {
   const float nan = __int_as_float(0x7fc00000);
@@ -113,6 +104,18 @@ __device__ __forceinline__ void poison_rows(float* comb_o, float* comb_ml, int r
 // t = 0 .. nt-1 of the CTA that drew the last ticket: g = max m; O = sum 2^(m-g) acc / sum 2^(m-g) l
 // (kernels/decode.py:186-197).  Leaves the ticket counter at zero for the next call.
 // ---------------------------------------------------------------------------
+// Draws the next merge ticket of a (sequence, kv head) pair.
+__device__ __forceinline__ int draw_ticket(const DecodeParams& p, int pair) {
+  if (!p.inline_plan) return atomicAdd(p.counters + pair, 1);
+  const int shift = (pair & 1) * 16;
+  return (atomicAdd(reinterpret_cast<unsigned*>(p.header) + kTicketWord + (pair >> 1), 1u << shift) >> shift) & 0xffff;
+}
+// Leaves the pair's ticket counter at zero for the next call; `n` tickets were drawn.
+__device__ __forceinline__ void reset_ticket(const DecodeParams& p, int pair, int n) {
+  if (!p.inline_plan) p.counters[pair] = 0;
+  else atomicSub(reinterpret_cast<unsigned*>(p.header) + kTicketWord + (pair >> 1), static_cast<unsigned>(n) << ((pair & 1) * 16));
+}
+
 template <typename T, int D>
 __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h, int n_chunks, int item0, T* out,
                                              int t, int nt) {
@@ -186,7 +189,7 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h
       }
     }
   }
-  if (t == 0) p.counters[b * p.kv_heads + h] = 0;  // leave the counter ready for the next call
+  if (t == 0) reset_ticket(p, b * p.kv_heads + h, n_chunks);
 }
 
 // ---------------------------------------------------------------------------
@@ -240,7 +243,7 @@ __device__ __forceinline__ void emit_and_merge(const DecodeParams& p, int b, int
   // publish the partial, draw a ticket; the last arrival merges (nobody waits)
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) *s_ticket = atomicAdd(p.counters + b * p.kv_heads + h, 1);
+  if (threadIdx.x == 0) *s_ticket = draw_ticket(p, b * p.kv_heads + h);
   __syncthreads();
   if (*s_ticket != n_chunks - 1) return;
   merge_chunks<T, D>(p, b, h, n_chunks, item0, out, threadIdx.x, blockDim.x);
@@ -249,11 +252,9 @@ __device__ __forceinline__ void emit_and_merge(const DecodeParams& p, int b, int
 // ---------------------------------------------------------------------------
 // Planner
 // ---------------------------------------------------------------------------
-// Keys per work item of a sequence of `len` keys that is split into `n` items.  Equal split: every item covers the
-// same number of keys (a multiple of the 64-key tile), the last takes what is left.  Otherwise: the planner's chunk
-// size, i.e. full chunks and one remainder.
-__device__ __forceinline__ int seq_chunk(int len, int n, int global_chunk, int equal_split) {
-  if (!equal_split) return global_chunk;
+// Keys per work item of a sequence of `len` keys that is split into `n` items: every item covers the same number of
+// keys (a multiple of the 64-key tile), the last takes what is left.
+__device__ __forceinline__ int seq_chunk(int len, int n) {
   const int per = (len + n - 1) / n;
   const int c = ((per + kTileN - 1) / kTileN) * kTileN;
   return c < kTileN ? kTileN : c;
@@ -328,11 +329,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
       if (v < 1) v = 1;
       n += v;
       if (with_largest) {
-        int per = ck;
-        if (p.equal_split) {
-          per = ((ceil_div_fast(len, v, __frcp_rn(static_cast<float>(v))) + kTileN - 1) / kTileN) * kTileN;
-          if (per < kTileN) per = kTileN;
-        }
+        int per = ((ceil_div_fast(len, v, __frcp_rn(static_cast<float>(v))) + kTileN - 1) / kTileN) * kTileN;
+        if (per < kTileN) per = kTileN;
         biggest = max(biggest, min(len, per));
       }
     }
@@ -429,7 +427,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     const int len = len_of(b);
     const int first = b == 0 ? 0 : (cached ? s_first[b] : p.item_start[b]);
     const int n = (cached ? s_first[b + 1] : p.item_start[b + 1]) - first;
-    const int per = seq_chunk(len, n, chunk, p.equal_split);
+    const int per = seq_chunk(len, n);
     const int rem = max(0, len - (n - 1) * per);
     if (n > 1) atomicAdd(&s_hist[size_class(per)], n - 1);
     atomicAdd(&s_hist[size_class(rem)], 1);
@@ -444,7 +442,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     const SeqInfo si = seq_info(p, b);
     const int first = b == 0 ? 0 : (cached ? s_first[b] : p.item_start[b]);
     const int n = (cached ? s_first[b + 1] : p.item_start[b + 1]) - first;
-    const int per = seq_chunk(si.len, n, chunk, p.equal_split);
+    const int per = seq_chunk(si.len, n);
     const int rem = max(0, si.len - (n - 1) * per);
     const int4 rec1 = make_int4(si.len, per, static_cast<int>(si.start & 0xffffffffll), static_cast<int>(si.start >> 32));
     if (n > 1) {
@@ -474,6 +472,132 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     p.header[3] = 0;          // tickets drawn and not merged yet (tcgen05 kernel)
     p.header[4] = 0;          // units drawn beyond the CTAs' first ones (tcgen05 kernel)
   }
+}
+
+// A CTA's work item, from the planner's records or worked out by the CTA itself.
+struct DecodeItem {
+  long long start;            // ragged: first row of the sequence
+  int b, c, n_chunks, item0;  // sequence, chunk, chunks of the sequence, item number of its first chunk
+  int len, per;               // keys of the sequence, keys per item
+};
+
+struct InlinePlan {
+  long long tot[kInlinePairs / 32];
+  int len[kInlinePairs], n[kInlinePairs], per[kInlinePairs];
+  int items[2][32], biggest[32];
+  DecodeItem mine;
+  int found, over;
+};
+
+// The planner's choices (same candidates, same estimate) made by a CTA of at least kInlinePairs threads for itself.
+// Items are numbered sequence by sequence, the sequences with the longest items first.  Returns false when there is no
+// item of that number.
+__device__ __forceinline__ bool plan_inline(const DecodeParams& p, int item, InlinePlan& s, DecodeItem& out) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  SeqInfo mine;
+  mine.start = 0;
+  mine.len = 0;
+  if (tid < p.batch) mine = seq_info(p, tid);
+  if (tid < kInlinePairs) {
+    s.len[tid] = mine.len;
+    long long w = mine.len;
+    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if (lane == 0) s.tot[warp] = w;
+  }
+  if (tid < 32) { s.items[0][tid] = 0; s.items[1][tid] = 0; s.biggest[tid] = 0; }
+  if (tid == 0) { s.found = 0; s.over = 0; }
+  __syncthreads();
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < kInlinePairs / 32; ++w) t += s.tot[w];
+  // candidate `lane` of either target; the warps share the sequences
+  auto candidate = [&](int target) -> int {
+    long long base = t <= 0x7fffffff ? (static_cast<unsigned>(t) + target - 1) / static_cast<unsigned>(target) : (t + target - 1) / target;
+    base = ((base + kTileN - 1) / kTileN) * kTileN;
+    if (base < p.min_chunk) base = p.min_chunk;
+    if (base > (1 << 29)) base = 1 << 29;
+    const long long cand = base + (base * lane) / 32;
+    return static_cast<int>(((cand + kTileN - 1) / kTileN) * kTileN);
+  };
+  const bool try_wave = p.wave_items > 0 && p.wave_items < p.target_items && p.batch <= p.wave_items;
+  const int ck0 = candidate(p.target_items), ck1 = try_wave ? candidate(p.wave_items) : ck0;
+  {
+    const float inv0 = 1.f / static_cast<float>(ck0), inv1 = 1.f / static_cast<float>(ck1);
+    int n0 = 0, n1 = 0, big = 0;
+    for (int b = warp; b < p.batch; b += nwarps) {
+      const int len = s.len[b];
+      n0 += max(1, ceil_div_fast(len, ck0, inv0));
+      const int v = max(1, ceil_div_fast(len, ck1, inv1));
+      n1 += v;
+      const int per = ((ceil_div_fast(len, v, __frcp_rn(static_cast<float>(v))) + kTileN - 1) / kTileN) * kTileN;
+      big = max(big, min(len, max(per, kTileN)));
+    }
+    if (warp < p.batch) {
+      atomicAdd(&s.items[0][lane], n0);
+      atomicAdd(&s.items[1][lane], n1);
+      atomicMax(&s.biggest[lane], big);
+    }
+  }
+  __syncthreads();
+  int chunk;
+  {
+    const int n0 = s.items[0][lane], n1 = s.items[1][lane];
+    const unsigned fit0 = __ballot_sync(0xffffffffu, n0 <= p.target_items);
+    const int pick0 = fit0 ? __ffs(fit0) - 1 : 31;
+    chunk = __shfl_sync(0xffffffffu, ck0, pick0);
+    const int items0 = __shfl_sync(0xffffffffu, n0, pick0);
+    const unsigned fit1 = __ballot_sync(0xffffffffu, n1 <= p.wave_items);
+    if (try_wave && items0 > p.wave_items && fit1) {
+      const int pick1 = __ffs(fit1) - 1;
+      const float ovh = static_cast<float>(p.item_overhead);
+      const float n_several = static_cast<float>(items0);
+      const float several = (static_cast<float>(t) + n_several * ovh) / static_cast<float>(p.wave_items) +
+                            0.5f * (static_cast<float>(t) / n_several + ovh);
+      const float one = static_cast<float>(s.biggest[pick1]) + ovh;
+      const int ck = __shfl_sync(0xffffffffu, ck1, pick1);
+      if (one < several) chunk = ck;
+    }
+  }
+  int n = 0, per = 0;
+  if (tid < p.batch) {
+    n = max(1, ceil_div_fast(mine.len, chunk, 1.f / static_cast<float>(chunk)));
+    per = seq_chunk(mine.len, n);
+    s.n[tid] = n;
+    s.per[tid] = per;
+  }
+  __syncthreads();
+  if (tid < p.batch) {
+    int first = 0, total = 0;
+    for (int b = 0; b < p.batch; ++b) {
+      const int pb = s.per[b], nb = s.n[b];
+      total += nb;
+      if (pb > per || (pb == per && b < tid)) first += nb;
+    }
+    if (blockIdx.x == 0 && tid == 0) { p.header[1] = chunk; p.header[2] = total; }   // (for inspection)
+    if (item >= first && item < first + n) {
+      s.mine = DecodeItem{mine.start, tid, item - first, n, first, mine.len, per};
+      s.found = 1;
+    }
+    // more items than the grid was sized for (prefix sums that are not monotonic): reported, and no item is run
+    if (first + n > static_cast<int>(gridDim.x) / p.kv_heads) {
+      p.header[0] = DEV_ERR_PLAN;
+      s.over = 1;
+    }
+  }
+  __syncthreads();
+  out = s.mine;
+  return s.found != 0 && s.over == 0;
+}
+
+__device__ __forceinline__ bool decode_item(const DecodeParams& p, int item, InlinePlan& s, DecodeItem& out) {
+  if (p.inline_plan) return plan_inline(p, item, s, out);
+  if (item >= p.header[2]) return false;
+  const int4 rec0 = p.item_info[2 * item];
+  const int4 rec1 = p.item_info[2 * item + 1];
+  out.b = rec0.x; out.c = rec0.y; out.n_chunks = rec0.z; out.item0 = rec0.w;
+  out.len = rec1.x; out.per = rec1.y;
+  out.start = (static_cast<long long>(rec1.w) << 32) | static_cast<unsigned int>(rec1.z);
+  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -572,12 +696,13 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
   constexpr int KSTEPS = D / 16;
 
   ptx::grid_dep_launch_dependents();
-  ptx::grid_dep_wait();      // the planner's records are complete and visible from here on
-  const int n_items = p.header[2];
+  ptx::grid_dep_wait();      // what earlier launches wrote (the planner's records among it) is visible from here on
   // heads vary fastest across CTAs: the CTAs that run side by side walk the same pages and read
   // neighbouring head slices of each token row, which keeps DRAM rows open
+  __shared__ InlinePlan s_plan;
   const int item = blockIdx.x / p.kv_heads;
-  if (item >= n_items) return;
+  DecodeItem it;
+  if (!decode_item(p, item, s_plan, it)) return;
   const int h = blockIdx.x - item * p.kv_heads;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NMT = p.n_mtiles;
@@ -587,16 +712,10 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
   const int rows_pad = NMT * 16;
   const bool is_producer = warp == n_cwarps;
 
-  const int4 rec0 = p.item_info[2 * item];
-  const int4 rec1 = p.item_info[2 * item + 1];
-  const int b = rec0.x, c = rec0.y, n_chunks = rec0.z, item0 = rec0.w;
-  const int chunk = rec1.y;              // keys per item of this sequence
-  SeqInfo si;
-  si.len = rec1.x;
-  si.start = (static_cast<long long>(rec1.w) << 32) | static_cast<unsigned int>(rec1.z);
-  const int len = si.len;
-  const int t_begin = c * chunk;
-  const int t_end = min(len, t_begin + chunk);
+  const int b = it.b, c = it.c, n_chunks = it.n_chunks, item0 = it.item0;
+  const int len = it.len;
+  const int t_begin = c * it.per;
+  const int t_end = min(len, t_begin + it.per);
   const int ntiles = t_end > t_begin ? (t_end - t_begin + kTileN - 1) / kTileN : 0;
 
   // smem: [stages (1024-byte aligned)] [Q rows] [control]
@@ -640,7 +759,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     // =========================== TMA producer ===========================
     if (lane == 0) { ptx::prefetch_tensormap(&tm_k); ptx::prefetch_tensormap(&tm_v); }
     int h_coord = h;
-    long long row0 = si.start;               // ragged
+    long long row0 = it.start;               // ragged
     if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(b) * p.kv_heads + h) * p.max_kv; }
     bool ok = true;
     int issued = 0;
@@ -1544,25 +1663,24 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeP
   constexpr int kKeys = 2;                   // key rows of a lane group per step
   constexpr int kStep = kRowsWarp * kKeys;   // keys of a warp per step
   ptx::grid_dep_launch_dependents();
-  ptx::grid_dep_wait();      // the planner's records are complete and visible from here on
-  const int n_items = p.header[2];
+  ptx::grid_dep_wait();      // what earlier launches wrote (the planner's records among it) is visible from here on
   // heads vary fastest across CTAs: the CTAs that run side by side walk the same pages and read
   // neighbouring head slices of each token row, which keeps DRAM rows open
+  __shared__ InlinePlan s_plan;
   const int item = blockIdx.x / p.kv_heads;
-  if (item >= n_items) return;
+  DecodeItem it;
+  if (!decode_item(p, item, s_plan, it)) return;
   const int h = blockIdx.x - item * p.kv_heads;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane / kGroup, gl = lane % kGroup;
   constexpr int nwarps = kSimtThreads / 32;
   const int R = p.rows;
 
-  const int4 rec0 = p.item_info[2 * item];
-  const int4 rec1 = p.item_info[2 * item + 1];
-  const int b = rec0.x, c = rec0.y, n_chunks = rec0.z, item0 = rec0.w;
-  const long long seq_start = (static_cast<long long>(rec1.w) << 32) | static_cast<unsigned int>(rec1.z);
-  const int len = rec1.x;
-  const int t_begin = c * rec1.y;
-  const int t_end = min(len, t_begin + rec1.y);
+  const int b = it.b, c = it.c, n_chunks = it.n_chunks, item0 = it.item0;
+  const long long seq_start = it.start;
+  const int len = it.len;
+  const int t_begin = c * it.per;
+  const int t_end = min(len, t_begin + it.per);
 
   float* comb_o = reinterpret_cast<float*>(smem);                       // [KS][R][D]
   const int blocks = (R + RB - 1) / RB;                                 // blocks of RB rows
@@ -1867,16 +1985,29 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   p.box_shift = 6;
   p.target_items = w.target_items; p.min_chunk = w.min_chunk; p.max_items = w.max_items;
   p.wave_items = w.wave_items; p.item_overhead = w.item_overhead;
-  // Equal items per sequence and longest-first order let the greedy CTA dispatch pair long and short items: with two
-  // or three whole waves the grid drains almost level (measured on B200, 16-token pages: 0.80 -> 0.84 of the copy
-  // bandwidth for paged decode, 0.68 -> 0.76 for speculative decode).
-  p.equal_split = 1;
   p.scale_log2 = a.sm_scale * 1.4426950408889634f;
 
-  cudaError_t e = launch_dependent(decode_plan_kernel, dim3(1), kPlanThreads, 0, stream, 1, p);
+  // Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's
+  // launch, 4 to 5 us in front of the kernel, goes.  The line is the number of merge tickets that fit into the header,
+  // the only part of a workspace that may be relied on to be zero without a launch; beyond it a call streams for longer
+  // and the planner is a smaller part of it.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
+  // keys of two heads 17.2 -> 13.0, four drafts for 16 short sequences 15.1 -> 12.9, 7 x 30 201 keys at 0.98 of the copy
+  // bandwidth.
+  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
+  p.inline_plan = (a.dtype == B200ATTN_F32 || p.rows <= 16) && pairs <= kInlinePairs ? 1 : 0;
+  unsigned grid_items = static_cast<unsigned>(w.max_items);
+  cudaError_t e = cudaSuccess;
+  if (p.inline_plan) {
+    // no more items than this, whatever the lengths are: an item has min_chunk keys or ends a sequence
+    const long long keys = a.layout == B200ATTN_RAGGED ? a.total_kv
+                           : a.batch * (a.layout == B200ATTN_DENSE ? static_cast<long long>(a.max_kv) : a.table_stride * a.page_size);
+    grid_items = static_cast<unsigned>(std::min<long long>(w.max_items, keys / w.min_chunk + a.batch));
+  } else {
+    e = launch_dependent(decode_plan_kernel, dim3(1), kPlanThreads, 0, stream, 1, p);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "decode_plan_kernel launch");
 
-  const dim3 grid(static_cast<unsigned>(w.max_items) * a.kv_heads, 1);
+  const dim3 grid(grid_items * a.kv_heads, 1);
   const int D = a.head_dim;
   if (a.dtype == B200ATTN_F32) {
     // (four warps leave at most 4 / blocks-of-rows partials per row: see the kernel)

@@ -8,6 +8,11 @@
 
 namespace b200attn {
 
+// Merge tickets of calls without a planner launch: 16 bits per (sequence, KV head) pair in the workspace header, the
+// only part of a workspace that keeps its contents between calls (every call leaves them at zero).
+constexpr int kTicketWord = 16;                     // first header word that holds tickets
+constexpr int kInlinePairs = 2 * (64 - kTicketWord);
+
 // Kernel parameter block (passed by value).
 struct DecodeParams {
   const void* q;
@@ -17,7 +22,7 @@ struct DecodeParams {
   const void* kv_indptr;
   const int* k_table;
   const int* v_table;
-  int* header;       // [0] error code, [1] chunk tokens, [2] number of work items
+  int* header;       // [0] error code, [1] chunk tokens, [2] number of work items, [kTicketWord ...] inline-plan tickets
   int* item_start;   // [batch + 1] prefix of per-sequence chunk counts
   int* counters;     // [batch * kv_heads] merge tickets
   int4* item_info;   // [max_items][2]: {sequence, chunk, chunks of the sequence, first item of the sequence}, {len, -, start lo, start hi}
@@ -46,8 +51,8 @@ struct DecodeParams {
   int wave_items;    // items of one KV head that are resident at once (one wave of CTAs); 0: never plan a single wave
   int item_overhead; // start-up and merge of a work item, in keys of streaming time (planner's cost estimate)
   int min_chunk;
-  int equal_split;   // 1: a sequence's items are of equal size; 0: full chunks and one remainder
   int max_items;
+  int inline_plan;   // 1: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs)
   float scale_log2;  // sm_scale * log2(e)
 };
 
