@@ -28,6 +28,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "cast.cuh"
 #include "common.cuh"
 #include "decode_launch.h"
 #include "launch.cuh"
@@ -1907,17 +1908,6 @@ namespace {
 int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, const DecodeWsLayout& w,
                        int pass_group, int head0, bool f32_out);
 
-// fp32 -> fp16, four elements per thread (every tensor here is a whole number of head_dim rows)
-__global__ void __launch_bounds__(256) decode_cast_f16_kernel(const float4* __restrict__ src, uint2* __restrict__ dst,
-                                                              size_t n4) {
-  ptx::grid_dep_launch_dependents();
-  ptx::grid_dep_wait();
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const float4 x = __ldcg(src + i);
-    dst[i] = make_uint2(ElemTraits<__half>::pack2(x.x, x.y), ElemTraits<__half>::pack2(x.z, x.w));
-  }
-}
 }  // namespace
 
 int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, bool allow_cast) {
@@ -1932,17 +1922,13 @@ int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t st
   if (w.cast_kv_elems > 0) {
     // fp16 copies of q, k, v (see decode_ws_layout); the launches below read them and write fp32 rows
     unsigned char* ws = static_cast<unsigned char*>(a.workspace);
-    const void* src[3] = {a.q, a.k, a.v};
     void* dst[3] = {ws + w.cast_q_off, ws + w.cast_k_off, ws + w.cast_v_off};
-    const size_t elems[3] = {w.cast_q_elems, w.cast_kv_elems, w.cast_kv_elems};
-    for (int i = 0; i < 3; ++i) {
-      const size_t n4 = elems[i] / 4;
-      if (n4 == 0) continue;
-      const unsigned blocks = static_cast<unsigned>(std::min<size_t>((n4 + 255) / 256, static_cast<size_t>(sm_count) * 16));
-      const cudaError_t e = launch_dependent(decode_cast_f16_kernel, dim3(blocks), 256, 0, stream, 1,
-                                             static_cast<const float4*>(src[i]), static_cast<uint2*>(dst[i]), n4);
-      if (e != cudaSuccess) return cuda_fail(e, "decode_cast_f16_kernel launch");
-    }
+    const long long q4 = static_cast<long long>(w.cast_q_elems / 4), kv4 = static_cast<long long>(w.cast_kv_elems / 4);
+    const CastJob job = {{static_cast<const float4*>(a.q), static_cast<const float4*>(a.k), static_cast<const float4*>(a.v)},
+                         {static_cast<uint2*>(dst[0]), static_cast<uint2*>(dst[1]), static_cast<uint2*>(dst[2])},
+                         {q4, kv4, kv4}};
+    const cudaError_t e = launch_cast(job, sm_count, stream);
+    if (e != cudaSuccess) return cuda_fail(e, "cast kernel launch");
     b.q = dst[0]; b.k = dst[1]; b.v = dst[2];
     b.dtype = B200ATTN_F16;
   }

@@ -29,6 +29,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "cast.cuh"
 #include "common.cuh"
 #include "launch.cuh"
 #include "prefill_launch.h"
@@ -146,22 +147,6 @@ __device__ __forceinline__ bool find_ragged_work(const PrefillParams& p, int x, 
     base += __shfl_sync(0xffffffffu, incl, 31);
   }
   return false;
-}
-
-// fp32 inputs: q, k and v are first rounded to fp16 into the workspace (the reference's kernel does the
-// same cast in registers, kernels/attention.py:547,572,594,614) and the result is written back as fp32.
-__global__ void __launch_bounds__(256) cast_f32_to_f16_kernel(const float4* __restrict__ src, uint2* __restrict__ dst,
-                                                              long long n4) {
-  ptx::grid_dep_launch_dependents();
-  ptx::grid_dep_wait();
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float4 f = __ldcg(src + i);
-    uint2 u;
-    u.x = ElemTraits<__half>::pack2(f.x, f.y);
-    u.y = ElemTraits<__half>::pack2(f.z, f.w);
-    dst[i] = u;
-  }
 }
 
 __device__ __forceinline__ ItemWork decode_item(const PrefillParams& p, int item, int lane) {
@@ -1177,17 +1162,13 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
   if (f32) {
     const CastPlan c = cast_plan(a_in);
     unsigned char* ws = static_cast<unsigned char*>(a_in.workspace);
-    const void* src[3] = {a_in.q, a_in.k, a_in.v};
-    const size_t off[3] = {c.q_off, c.k_off, c.v_off};
-    const size_t cnt[3] = {c.q_elems, c.kv_elems, c.kv_elems};
-    for (int i = 0; i < 3; ++i) {
-      const long long n4 = static_cast<long long>(cnt[i] / 4);  // head_dim is a multiple of 4
-      if (n4 == 0) continue;
-      const int blocks = static_cast<int>(std::min<long long>((n4 + 255) / 256, static_cast<long long>(sm_count) * 16));
-      const cudaError_t ce = launch_dependent(cast_f32_to_f16_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1,
-                                              static_cast<const float4*>(src[i]), reinterpret_cast<uint2*>(ws + off[i]), n4);
-      if (ce != cudaSuccess) return cuda_fail(ce, "cast kernel launch");
-    }
+    const long long q4 = static_cast<long long>(c.q_elems / 4), kv4 = static_cast<long long>(c.kv_elems / 4);
+    const CastJob job = {{static_cast<const float4*>(a_in.q), static_cast<const float4*>(a_in.k), static_cast<const float4*>(a_in.v)},
+                         {reinterpret_cast<uint2*>(ws + c.q_off), reinterpret_cast<uint2*>(ws + c.k_off),
+                          reinterpret_cast<uint2*>(ws + c.v_off)},
+                         {q4, kv4, kv4}};
+    const cudaError_t ce = launch_cast(job, sm_count, stream);
+    if (ce != cudaSuccess) return cuda_fail(ce, "cast kernel launch");
     a.q = ws + c.q_off; a.k = ws + c.k_off; a.v = ws + c.v_off;
     a.dtype = B200ATTN_F16;
   }
