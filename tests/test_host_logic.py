@@ -240,3 +240,33 @@ def test_fp32_copies_are_capped_by_scratch_size():
     small, large = need(100_000), need(10_000_000)
     assert small >= 2 * 2 * 100_000 * 8 * 128            # fp16 copies of k and v
     assert large < small                                 # 41 GB of fp32 cache: no copies, fp32 kernel
+
+
+@pytest.mark.parametrize("qh,kvh,m", [(64, 8, 5), (8, 1, 5), (64, 4, 2), (128, 64, 9), (96, 3, 3)])
+def test_dealt_out_batches(qh, kvh, m):
+    """A batch dealt out to the CTAs of the persistent kernel: cuts in order, no item shorter than min_chunk except whole
+    sequences, and no slot with more than a stretch of the line plus what the snapping of two cuts adds."""
+    from utils.launch_config import decode_cuts, decode_items, decode_plan
+
+    g = torch.Generator().manual_seed(3 * qh + m)
+    dealt = 0
+    for batch, lo, hi in [(32, 1024, 32768), (1, 50000, 50000), (3, 1, 90000), (200, 0, 2000), (700, 0, 9000), (64, 8192, 8192),
+                          (4096, 1, 300), (40, 0, 300)]:
+        lens = torch.randint(lo, hi + 1, (batch,), generator=g).tolist()
+        plan = decode_plan(148, batch, qh, kvh, m)
+        cuts = decode_cuts(plan, lens)
+        if cuts is None:
+            continue
+        dealt += 1
+        assert cuts == sorted(cuts) and cuts[0] == (0, 0) and len(cuts) * kvh <= 2 * 148
+        inner = [c for c in cuts if c[1] > 0]
+        assert len(set(inner)) == len(inner) and sum(decode_items(plan, lens)) == batch + len(inner) <= plan.max_items
+        ends = {}
+        for b, t in inner:
+            assert t % 64 == 0 and t - ends.get(b, 0) >= plan.min_chunk and lens[b] - t >= plan.min_chunk
+            ends[b] = t
+        # keys and items of each slot
+        at = [sum(lens[:b]) + t for b, t in cuts] + [sum(lens)]
+        stretch = -(-(sum(lens) + (batch + plan.slots - 1) * plan.item_overhead) // plan.slots)
+        assert max(y - x for x, y in zip(at, at[1:])) <= max(stretch + 64, plan.min_chunk) + 2 * plan.min_chunk + 64
+    assert dealt >= 2

@@ -44,6 +44,7 @@ constexpr int kMaxStages = 4;
 constexpr int kPlanThreads = 1024;
 constexpr int kPlanBuckets = 32;    // size classes of the execution order (longest items first)
 constexpr int kPlanLenCache = 4096; // sequences whose lengths the planner keeps in shared memory
+constexpr int kPlanMaxSlots = 512;  // slots of the persistent kernel that the planner deals out
 
 struct SeqInfo {
   long long start;  // ragged: first row of the sequence
@@ -278,6 +279,9 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   __shared__ int s_chunk;
   __shared__ int s_cand_chunk[kPlanThreads / 32], s_cand_items[kPlanThreads / 32], s_cand_max[kPlanThreads / 32];
   __shared__ int s_pick_items;
+  __shared__ int s_slots;                            // > 0: the batch is dealt out to that many slots
+  __shared__ int s_rank[kPlanMaxSlots];              // cuts inside sequences among the slot boundaries 1 .. i
+  __shared__ int s_cut[kPlanMaxSlots];               // their keys, in order
   __shared__ int s_hist[kPlanBuckets];     // items per size class, then the class's first execution slot
   __shared__ int s_cursor[kPlanBuckets];
   __shared__ int s_len[kPlanLenCache];      // sequence lengths, read from global memory once
@@ -288,6 +292,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();      // (the call before may still be using the records and tickets that are written below)
   if (tid < kPlanBuckets) { s_hist[tid] = 0; s_cursor[tid] = 0; }
+  if (tid == 0) s_slots = 0;
   const bool cached = p.batch <= kPlanLenCache;
   auto len_of = [&](int b) -> int { return cached ? s_len[b] : seq_info(p, b).len; };
 
@@ -357,6 +362,13 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     s_carry = 0;
   }
   __syncthreads();
+  // Estimated run time of a plan in several waves, in keys: the average load of a resident CTA plus half an item.
+  const float ovh = static_cast<float>(p.item_overhead);
+  auto several_cost = [&]() -> float {
+    const float n = static_cast<float>(s_pick_items);
+    return (static_cast<float>(t) + n * ovh) / static_cast<float>(p.wave_items) + 0.5f * (static_cast<float>(t) / n + ovh);
+  };
+  float best = p.wave_items > 0 ? several_cost() : 0.f;   // (read by thread 0 only)
   // (a batch of more sequences than a wave has CTAs cannot fit one: every sequence is at least one item)
   if (p.wave_items > 0 && p.wave_items < p.target_items && s_pick_items > p.wave_items && p.batch <= p.wave_items) {
     evaluate(p.wave_items, true);
@@ -367,54 +379,113 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
         if (s_cand_items[k] <= p.wave_items) { pick = k; break; }
       }
       if (pick >= 0) {
-        const float ovh = static_cast<float>(p.item_overhead);
-        const float n_several = static_cast<float>(s_pick_items);
-        const float several = (static_cast<float>(t) + n_several * ovh) / static_cast<float>(p.wave_items) +
-                              0.5f * (static_cast<float>(t) / n_several + ovh);
         const float one = static_cast<float>(s_cand_max[pick]) + ovh;
-        if (one < several) s_chunk = s_cand_chunk[pick];
+        if (one < best) { best = one; s_chunk = s_cand_chunk[pick]; }
       }
     }
+  }
+  // Dealing out: the persistent kernel's CTAs of a KV head ("slots") each take one stretch of the sequences laid end to
+  // end, all of the same length with item_overhead keys added per item, cutting sequences where a stretch ends.  That is
+  // about one item per sequence and one per slot instead of three per slot, and no slot ends later than another.
+  const long long line = t + static_cast<long long>(p.batch + p.slots - 1) * p.item_overhead;
+  if (tid == 0 && p.slots > 1 && p.slots <= kPlanMaxSlots && cached && line < (1 << 30) && s_pick_items > p.wave_items) {
+    if (static_cast<float>(line) / static_cast<float>(p.slots) < best) s_slots = p.slots;
   }
   for (int i = tid; i < p.batch * p.kv_heads; i += kPlanThreads) p.counters[i] = 0;
   __syncthreads();
   const int chunk = s_chunk;
 
-  for (int base = 0; base < p.batch; base += kPlanThreads) {
-    const int b = base + tid;
-    int v = 0;
-    if (b < p.batch) {
-      const int len = len_of(b);
-      v = (len + chunk - 1) / chunk;
-      if (v < 1) v = 1;
-    }
-    int incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int n = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += n;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-      int w = s_warp[lane];
+  // inclusive prefix sums over 0 .. n - 1, in thread order
+  auto prefix = [&](int n, auto value, auto put) {
+    for (int base = 0; base < n; base += kPlanThreads) {
+      const int b = base + tid;
+      int incl = b < n ? value(b) : 0;
       for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += n;
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
       }
-      s_warp[lane] = w;  // inclusive over warps
+      if (lane == 31) s_warp[warp] = incl;
+      __syncthreads();
+      if (warp == 0) {
+        int w = s_warp[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+          const int x = __shfl_up_sync(0xffffffffu, w, o);
+          if (lane >= o) w += x;
+        }
+        s_warp[lane] = w;  // inclusive over warps
+      }
+      __syncthreads();
+      const int carry = s_carry;
+      const int before = warp > 0 ? s_warp[warp - 1] : 0;
+      if (b < n) put(b, carry + before + incl);
+      __syncthreads();
+      if (tid == 0) s_carry = carry + s_warp[31];
+      __syncthreads();
     }
+  };
+  const int slots = s_slots;
+  if (slots > 0) {
+    // s_first[b]: where sequence b starts on the line
+    prefix(p.batch, [&](int b) { return s_len[b] + p.item_overhead; }, [&](int b, int incl) { s_first[b + 1] = incl; });
+    if (tid == 0) { s_first[0] = 0; s_carry = 0; }
     __syncthreads();
-    const int carry = s_carry;
-    const int before = warp > 0 ? s_warp[warp - 1] : 0;
-    if (b < p.batch) {
-      p.item_start[b + 1] = carry + before + incl;
-      if (cached) s_first[b + 1] = carry + before + incl;
+    const int end = s_first[p.batch];
+    int stretch = ((static_cast<int>(line) + slots - 1) / slots + kTileN - 1) / kTileN * kTileN;
+    if (stretch < p.min_chunk) stretch = p.min_chunk;
+    // boundary `tid` between slot tid - 1 and slot tid: key cut_t of sequence cut_b; a piece shorter than min_chunk is
+    // left with the rest of its sequence
+    int cut_b = p.batch, cut_t = 0;
+    const long long x = static_cast<long long>(tid) * stretch;
+    if (tid < slots && x < end) {
+      int lo = 0, hi = p.batch;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (s_first[mid] <= x) lo = mid; else hi = mid;
+      }
+      cut_b = lo;
+      const int off = static_cast<int>(x) - s_first[lo] - p.item_overhead;
+      cut_t = off > 0 ? (off + kTileN / 2) / kTileN * kTileN : 0;
+      if (cut_t < p.min_chunk) cut_t = 0;
+      else if (s_len[lo] - cut_t < p.min_chunk) { cut_b = lo + 1; cut_t = 0; }
     }
-    __syncthreads();
-    if (tid == 0) s_carry = carry + s_warp[31];
-    __syncthreads();
+    prefix(slots, [&](int) { return cut_t > 0 ? 1 : 0; }, [&](int i, int incl) {
+      s_rank[i] = incl;
+      if (cut_t > 0) s_cut[incl - 1] = cut_t;
+    });
+    int* slot_first = reinterpret_cast<int*>(p.item_info + 2 * static_cast<long long>(p.max_items)) - (slots + 1);   // behind the records in use
+    if (tid < slots) slot_first[tid] = cut_b + s_rank[tid];
+    // cuts before sequence b, i.e. at boundaries that lie before its start
+    auto cuts_before = [&](int b) -> int {
+      const int pos = s_first[b];
+      const int k = min(slots - 1, (pos + stretch - 1) / stretch - 1);
+      return k > 0 ? s_rank[k] : 0;
+    };
+    for (int b = tid; b < p.batch; b += kPlanThreads) {
+      const SeqInfo si = seq_info(p, b);
+      const int r = cuts_before(b), first = b + r, n = cuts_before(b + 1) - r + 1;
+      p.item_start[b + 1] = first + n;
+      for (int c = 0; c < n && first + c < p.max_items; ++c) {
+        p.item_info[2 * (first + c)] = make_int4(b, c | (n << 16), first, c > 0 ? s_cut[r + c - 1] : 0);
+        p.item_info[2 * (first + c) + 1] = make_int4(si.len, c + 1 < n ? s_cut[r + c] : si.len,
+                                                     static_cast<int>(si.start & 0xffffffffll), static_cast<int>(si.start >> 32));
+      }
+    }
+    if (tid == 0) {
+      const int n_items = p.batch + s_rank[slots - 1];
+      slot_first[slots] = n_items;
+      p.item_start[0] = 0;
+      p.header[1] = p.min_chunk;   // (the smallest item: a batch that is dealt out has no chunk size)
+      p.header[2] = n_items;
+      p.header[3] = 0;
+      p.header[4] = 0;
+      p.header[5] = slots;
+    }
+    return;
   }
-  __syncthreads();
+  prefix(p.batch, [&](int b) { return max(1, (len_of(b) + chunk - 1) / chunk); }, [&](int b, int incl) {
+    p.item_start[b + 1] = incl;
+    if (cached) s_first[b + 1] = incl;
+  });
   // Per-item records, so that a CTA learns everything about its work item from one 32-byte read.  Records are laid
   // out in execution order: longest items first (by size class), so that the CTAs still running when the grid
   // drains are the short ones.  item_start keeps the per-sequence (logical) numbering, which is what the partial
@@ -445,21 +516,20 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     const int n = (cached ? s_first[b + 1] : p.item_start[b + 1]) - first;
     const int per = seq_chunk(si.len, n);
     const int rem = max(0, si.len - (n - 1) * per);
-    const int4 rec1 = make_int4(si.len, per, static_cast<int>(si.start & 0xffffffffll), static_cast<int>(si.start >> 32));
+    auto put = [&](int slot, int c) {
+      const int t0 = c * per;
+      p.item_info[2 * slot] = make_int4(b, c | (n << 16), first, t0);
+      p.item_info[2 * slot + 1] = make_int4(si.len, min(si.len, t0 + per), static_cast<int>(si.start & 0xffffffffll),
+                                            static_cast<int>(si.start >> 32));
+    };
     if (n > 1) {
       const int q = size_class(per);
       const int pos = s_hist[q] + atomicAdd(&s_cursor[q], n - 1);
-      for (int c = 0; c < n - 1 && pos + c < p.max_items; ++c) {
-        p.item_info[2 * (pos + c)] = make_int4(b, c, n, first);
-        p.item_info[2 * (pos + c) + 1] = rec1;
-      }
+      for (int c = 0; c < n - 1 && pos + c < p.max_items; ++c) put(pos + c, c);
     }
     const int q = size_class(rem);
     const int pos = s_hist[q] + atomicAdd(&s_cursor[q], 1);
-    if (pos < p.max_items) {
-      p.item_info[2 * pos] = make_int4(b, n - 1, n, first);
-      p.item_info[2 * pos + 1] = rec1;
-    }
+    if (pos < p.max_items) put(pos, n - 1);
   }
   if (tid == 0) {
     p.item_start[0] = 0;
@@ -472,6 +542,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     p.header[2] = n_items;
     p.header[3] = 0;          // tickets drawn and not merged yet (tcgen05 kernel)
     p.header[4] = 0;          // units drawn beyond the CTAs' first ones (tcgen05 kernel)
+    p.header[5] = 0;
   }
 }
 
@@ -479,7 +550,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
 struct DecodeItem {
   long long start;            // ragged: first row of the sequence
   int b, c, n_chunks, item0;  // sequence, chunk, chunks of the sequence, item number of its first chunk
-  int len, per;               // keys of the sequence, keys per item
+  int len, t_begin, t_end;    // keys of the sequence, the item's keys
 };
 
 struct InlinePlan {
@@ -576,7 +647,8 @@ __device__ __forceinline__ bool plan_inline(const DecodeParams& p, int item, Inl
     }
     if (blockIdx.x == 0 && tid == 0) { p.header[1] = chunk; p.header[2] = total; }   // (for inspection)
     if (item >= first && item < first + n) {
-      s.mine = DecodeItem{mine.start, tid, item - first, n, first, mine.len, per};
+      s.mine = DecodeItem{mine.start, tid, item - first, n, first, mine.len, (item - first) * per,
+                          min(mine.len, (item - first + 1) * per)};
       s.found = 1;
     }
     // more items than the grid was sized for (prefix sums that are not monotonic): reported, and no item is run
@@ -595,8 +667,8 @@ __device__ __forceinline__ bool decode_item(const DecodeParams& p, int item, Inl
   if (item >= p.header[2]) return false;
   const int4 rec0 = p.item_info[2 * item];
   const int4 rec1 = p.item_info[2 * item + 1];
-  out.b = rec0.x; out.c = rec0.y; out.n_chunks = rec0.z; out.item0 = rec0.w;
-  out.len = rec1.x; out.per = rec1.y;
+  out.b = rec0.x; out.c = rec0.y & 0xffff; out.n_chunks = static_cast<unsigned>(rec0.y) >> 16; out.item0 = rec0.z;
+  out.len = rec1.x; out.t_begin = rec0.w; out.t_end = rec1.y;
   out.start = (static_cast<long long>(rec1.w) << 32) | static_cast<unsigned int>(rec1.z);
   return true;
 }
@@ -715,8 +787,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
 
   const int b = it.b, c = it.c, n_chunks = it.n_chunks, item0 = it.item0;
   const int len = it.len;
-  const int t_begin = c * it.per;
-  const int t_end = min(len, t_begin + it.per);
+  const int t_begin = it.t_begin, t_end = it.t_end;
   const int ntiles = t_end > t_begin ? (t_end - t_begin + kTileN - 1) / kTileN : 0;
 
   // smem: [stages (1024-byte aligned)] [Q rows] [control]
@@ -1081,11 +1152,11 @@ __device__ __forceinline__ UmmaUnit umma_unit(const DecodeParams& p, int u) {
   w.h = u - item * p.kv_heads;
   const int4 rec0 = p.item_info[2 * item];
   const int4 rec1 = p.item_info[2 * item + 1];
-  w.b = rec0.x; w.c = rec0.y; w.n_chunks = rec0.z; w.item0 = rec0.w;
+  w.b = rec0.x; w.c = rec0.y & 0xffff; w.n_chunks = static_cast<unsigned>(rec0.y) >> 16; w.item0 = rec0.z;
   w.len = rec1.x;
   w.seq_start = (static_cast<long long>(rec1.w) << 32) | static_cast<unsigned int>(rec1.z);
-  w.t_begin = w.c * rec1.y;                       // rec1.y: keys per item of this sequence
-  w.t_end = min(w.len, w.t_begin + rec1.y);
+  w.t_begin = rec0.w;
+  w.t_end = rec1.y;
   w.ntiles = w.t_end > w.t_begin ? (w.t_end - w.t_begin + kTileN - 1) / kTileN : 0;
   return w;
 }
@@ -1178,7 +1249,19 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
       ctrl->published = r + 1;
       mbar_arrive(smem_u32(&ctrl->unit_full[r % kUmmaUnitRing]));
     };
-    int u = me < n_units ? me : n_units;
+    // Dealt out (slots > 0): the CTA's units are the items of its slot, in order.  Else its first unit is its own index.
+    const int slots = p.header[5];
+    int u = me, u_end = n_units;
+    if (slots > 0) {
+      const int slot = me / p.kv_heads;
+      const int* slot_first = reinterpret_cast<const int*>(p.item_info + 2 * static_cast<long long>(p.max_items)) - (slots + 1);
+      u = n_units;
+      if (slot < slots) {
+        u = __ldcg(slot_first + slot) * p.kv_heads + me % p.kv_heads;
+        u_end = __ldcg(slot_first + slot + 1) * p.kv_heads;
+      }
+    }
+    if (u >= u_end) u = n_units;
     if (lane == 0) publish(0, u);
     for (int r = 0; ok && u < n_units; ++r) {
       const UmmaUnit w = umma_unit(p, u);
@@ -1274,7 +1357,8 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
         if (!ok || *abort_flag) { ok = false; break; }
       }
       if (lane == 0) {
-        u_next = min(G + atomicAdd(p.header + 4, 1), n_units);
+        u_next = slots > 0 ? u + p.kv_heads : min(G + atomicAdd(p.header + 4, 1), n_units);
+        if (u_next >= u_end) u_next = n_units;
         publish(r + 1, u_next);
       }
       u_next = __shfl_sync(0xffffffffu, u_next, 0);
@@ -1680,8 +1764,7 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeP
   const int b = it.b, c = it.c, n_chunks = it.n_chunks, item0 = it.item0;
   const long long seq_start = it.start;
   const int len = it.len;
-  const int t_begin = c * it.per;
-  const int t_end = min(len, t_begin + it.per);
+  const int t_begin = it.t_begin, t_end = it.t_end;
 
   float* comb_o = reinterpret_cast<float*>(smem);                       // [KS][R][D]
   const int blocks = (R + RB - 1) / RB;                                 // blocks of RB rows
@@ -1971,6 +2054,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   p.box_shift = 6;
   p.target_items = w.target_items; p.min_chunk = w.min_chunk; p.max_items = w.max_items;
   p.wave_items = w.wave_items; p.item_overhead = w.item_overhead;
+  p.slots = a.dtype != B200ATTN_F32 && p.rows > 16 ? 2 * sm_count / a.kv_heads : 0;
   p.scale_log2 = a.sm_scale * 1.4426950408889634f;
 
   // Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's

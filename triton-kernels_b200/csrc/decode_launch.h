@@ -22,10 +22,10 @@ struct DecodeParams {
   const void* kv_indptr;
   const int* k_table;
   const int* v_table;
-  int* header;       // [0] error code, [1] chunk tokens, [2] number of work items, [kTicketWord ...] inline-plan tickets
+  int* header;       // [0] error code, [1] chunk tokens, [2] number of work items, [5] slots dealt out, [kTicketWord ...] inline-plan tickets
   int* item_start;   // [batch + 1] prefix of per-sequence chunk counts
   int* counters;     // [batch * kv_heads] merge tickets
-  int4* item_info;   // [max_items][2]: {sequence, chunk, chunks of the sequence, first item of the sequence}, {len, -, start lo, start hi}
+  int4* item_info;   // [max_items][2]: {sequence, chunk + (chunks << 16), first item of the sequence, first key}, {len, end key, start lo, start hi}
   float* part_ml;    // [slot][rows][2]  (running max in log2 units, running sum)
   float* part_o;     // [slot][rows][D]  un-normalised accumulators
   long long total_kv;
@@ -52,6 +52,7 @@ struct DecodeParams {
   int item_overhead; // start-up and merge of a work item, in keys of streaming time (planner's cost estimate)
   int min_chunk;
   int max_items;
+  int slots;         // persistent kernel: CTAs per KV head that the planner may deal the batch out to; 0: none
   int inline_plan;   // 1: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs)
   float scale_log2;  // sm_scale * log2(e)
 };

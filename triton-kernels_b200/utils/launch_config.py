@@ -10,7 +10,7 @@ library's own ``b200attn_decode_workspace_bytes`` in the GPU tests so that the t
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import List, Sequence
+from typing import List, Optional, Sequence, Tuple
 
 DECODE_TILE_TOKENS = 64       # keys per cp.async stage
 PREFILL_BLOCK_M = 128         # query rows per tensor-core tile
@@ -28,6 +28,7 @@ class DecodePlan:
     threads: int
     wave_items: int = 0      # items of one KV head resident at once (one wave); 0: a single wave is never planned
     item_overhead: int = 0   # start-up + merge of an item in keys of streaming time (the planner's cost estimate)
+    slots: int = 0           # CTAs per KV head of the persistent kernel that a batch may be dealt out to
 
 
 def decode_pass_group(group: int, q_len: int) -> int:
@@ -73,17 +74,18 @@ def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: i
     min_chunk = max(128, by_rows)
     tiles = -(-rows // 16)
     slices = 4 if tiles <= 2 else (2 if tiles <= 4 else 1)
-    wide = rows > 16           # more than one 16-row tile: the tcgen05 kernel, two resident CTAs per SM (else three)
+    wide = rows > 16 and not fp32   # more than one 16-row tile: the tcgen05 kernel, two resident CTAs per SM (else three)
     wave = 0 if fp32 else max(1, (sm_count * (2 if wide else 3)) // max(1, kv_heads))
     overhead = 0 if fp32 else (448 if wide else 128)
-    return DecodePlan(target, min_chunk, target + batch, tiles, slices, 32 * (tiles * slices + 1), wave, overhead)
+    return DecodePlan(target, min_chunk, target + batch, tiles, slices, 32 * (tiles * slices + 1), wave, overhead,
+                      2 * sm_count // max(1, kv_heads) if wide else 0)
 
 
 def _round_up(x: int, m: int) -> int:
     return -(-x // m) * m
 
 
-def _item_tokens(plan: DecodePlan, length: int, n: int, chunk: int) -> int:
+def _item_tokens(length: int, n: int) -> int:
     """Keys per item of a sequence cut into ``n`` items (csrc/decode.cu seq_chunk)."""
     return max(DECODE_TILE_TOKENS, _round_up(-(-length // n), DECODE_TILE_TOKENS))
 
@@ -97,32 +99,72 @@ def _pick_chunk(plan: DecodePlan, lens: Sequence[int], target: int):
     for k in range(32):
         chunk = _round_up(base + (base * k) // 32, DECODE_TILE_TOKENS)
         counts = [max(1, -(-n // chunk)) for n in lens]
-        biggest = max([min(n, _item_tokens(plan, n, c, chunk)) for n, c in zip(lens, counts)], default=0)
+        biggest = max([min(n, _item_tokens(n, c)) for n, c in zip(lens, counts)], default=0)
         last = (chunk, sum(counts), biggest)
         if last[1] <= target:
             return last + (True,)
     return last + (False,)
 
 
+def _plan_lengths(plan: DecodePlan, lens: Sequence[int]):
+    """(chunk, dealt): the chunk size for several waves or a single one, and whether the batch is dealt out instead."""
+    total = sum(lens)
+    chunk, items, _, _ = _pick_chunk(plan, lens, plan.target_items)
+    best = 0.0
+    if plan.wave_items > 0:
+        best = (total + items * plan.item_overhead) / plan.wave_items + 0.5 * (total / items + plan.item_overhead)
+    if 0 < plan.wave_items < plan.target_items and items > plan.wave_items:
+        w_chunk, _, w_biggest, found = _pick_chunk(plan, lens, plan.wave_items)
+        if found and w_biggest + plan.item_overhead < best:
+            best, chunk = w_biggest + plan.item_overhead, w_chunk
+    line = total + (len(lens) + plan.slots - 1) * plan.item_overhead
+    dealt = (1 < plan.slots <= 512 and len(lens) <= 4096 and line < 1 << 30 and items > plan.wave_items
+             and line / plan.slots < best)
+    return chunk, dealt
+
+
+def decode_cuts(plan: DecodePlan, lengths: Sequence[int]) -> Optional[List[Tuple[int, int]]]:
+    """First (sequence, key) of every slot when the batch is dealt out to the CTAs of the persistent kernel, one past the
+    last sequence for slots that get nothing; None when it is planned in chunks."""
+    lens = [max(0, int(n)) for n in lengths]
+    if not _plan_lengths(plan, lens)[1]:
+        return None
+    ovh, starts = plan.item_overhead, [0]
+    for n in lens:
+        starts.append(starts[-1] + n + ovh)
+    line = sum(lens) + (len(lens) + plan.slots - 1) * ovh
+    stretch = max(_round_up(-(-line // plan.slots), DECODE_TILE_TOKENS), plan.min_chunk)
+    cuts = []
+    for i in range(plan.slots):
+        x = i * stretch
+        b, t = len(lens), 0
+        if x < starts[-1]:
+            b = max(j for j in range(len(lens)) if starts[j] <= x)
+            off = x - starts[b] - ovh
+            t = (off + DECODE_TILE_TOKENS // 2) // DECODE_TILE_TOKENS * DECODE_TILE_TOKENS if off > 0 else 0
+            if t < plan.min_chunk:
+                t = 0
+            elif lens[b] - t < plan.min_chunk:
+                b, t = b + 1, 0
+        cuts.append((b, t))
+    return cuts
+
+
 def decode_chunk_tokens(plan: DecodePlan, lengths: Sequence[int]) -> int:
     """Chunk size the device planner picks for these lengths: the smallest of 32 candidates between
     total / target_items and twice that which splits the batch into at most target_items items - or, when the
     batch also fits a single wave of resident CTAs and the estimate favours it (largest item + per-item overhead
-    against the average load of a resident CTA + half an item), the single-wave chunk."""
-    lens = [max(0, int(n)) for n in lengths]
-    total = sum(lens)
-    chunk, items, _, _ = _pick_chunk(plan, lens, plan.target_items)
-    if 0 < plan.wave_items < plan.target_items and items > plan.wave_items:
-        w_chunk, _, w_biggest, found = _pick_chunk(plan, lens, plan.wave_items)
-        if found:
-            several = (total + items * plan.item_overhead) / plan.wave_items + 0.5 * (total / items + plan.item_overhead)
-            if w_biggest + plan.item_overhead < several:
-                chunk = w_chunk
-    return chunk
+    against the average load of a resident CTA + half an item), the single-wave chunk.  A batch that is dealt out has no
+    chunk size; its items have at least min_chunk keys (or are whole sequences)."""
+    chunk, dealt = _plan_lengths(plan, [max(0, int(n)) for n in lengths])
+    return plan.min_chunk if dealt else chunk
 
 
 def decode_items(plan: DecodePlan, lengths: Sequence[int]) -> List[int]:
     """Work items (KV chunks) per sequence; their sum never exceeds plan.max_items."""
+    cuts = decode_cuts(plan, lengths)
+    if cuts is not None:
+        return [1 + sum(1 for c, t in cuts if c == b and t > 0) for b in range(len(lengths))]
     chunk = decode_chunk_tokens(plan, lengths)
     return [max(1, -(-max(0, int(n)) // chunk)) for n in lengths]
 
