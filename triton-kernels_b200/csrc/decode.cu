@@ -72,28 +72,6 @@ __device__ __forceinline__ SeqInfo seq_info(const DecodeParams& p, int b) {
   return s;
 }
 
-// element offset of row `t` of sequence `b`, head `h`; -1 when the block table entry is out of range
-__device__ __forceinline__ long long row_offset(const DecodeParams& p, const int* table, int b, int h,
-                                                long long seq_start, int t, int D) {
-  if (p.layout == B200ATTN_DENSE) {
-    return ((static_cast<long long>(b) * p.kv_heads + h) * p.max_kv + t) * D;
-  } else if (p.layout == B200ATTN_RAGGED) {
-    return ((seq_start + t) * p.kv_heads + h) * D;
-  } else {
-    int lp, off;
-    if (p.page_shift >= 0) {
-      lp = t >> p.page_shift;
-      off = t & (p.page_size - 1);
-    } else {
-      lp = t / p.page_size;
-      off = t - lp * p.page_size;
-    }
-    const int page = __ldg(table + static_cast<long long>(b) * p.table_stride + lp);
-    if (page < 0 || page >= p.num_pages) return -1;
-    return ((static_cast<long long>(page) * p.page_size + off) * p.kv_heads + h) * D;
-  }
-}
-
 // Fills `rows` combined rows with NaN accumulators and (m, l) = (0, 1); every thread of the CTA takes part.
 __device__ __forceinline__ void poison_rows(float* comb_o, float* comb_ml, int rows, int d) {
   const float nan = __int_as_float(0x7fc00000);
@@ -1733,19 +1711,22 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
 // the whole warp takes; the RB query rows of a block share every key row that is loaded.  Each lane group keeps an
 // online softmax of its own over its keys, so that nothing but the dot products crosses lanes inside the loop; the
 // groups of a warp are merged once at the end, the warps of a row in emit_and_merge.
-// kKeys rows of K and V per lane group are loaded one step ahead of their use, into registers: the kernel is bound by
-// the bytes in flight.
+// What bounds the kernel is the bytes in flight: every lane copies the 16-byte pieces that it will use itself
+// (cp.async, kSimtDepth steps ahead) into a ring of its own in shared memory, so nothing waits for another lane and the
+// registers stay free for the rows; block-table entries are read one step before the copies that need them.
 // ---------------------------------------------------------------------------
 constexpr int kSimtThreads = 128;
+constexpr int kSimtDepth = 4;                // steps whose copies are in flight
+constexpr int kSimtKeys = 2;                 // key rows of a lane group per step
+constexpr size_t kSimtRingBytes = static_cast<size_t>(kSimtThreads) * kSimtDepth * kSimtKeys * 4 * 16;
 
-// rows of a block: the q rows that share a K/V read (a fourth one would cost registers that the loads need)
 template <int D, int RB>
-__global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(kSimtThreads, 3) decode_simt_kernel(const DecodeParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_ticket;
   constexpr int kGroup = D / 8;              // lanes that share a key row
   constexpr int kRowsWarp = 32 / kGroup;     // key rows of a warp per load instruction
-  constexpr int kKeys = 2;                   // key rows of a lane group per step
+  constexpr int kKeys = kSimtKeys;
   constexpr int kStep = kRowsWarp * kKeys;   // keys of a warp per step
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();      // what earlier launches wrote (the planner's records among it) is visible from here on
@@ -1766,7 +1747,7 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeP
   const int len = it.len;
   const int t_begin = it.t_begin, t_end = it.t_end;
 
-  float* comb_o = reinterpret_cast<float*>(smem);                       // [KS][R][D]
+  float* comb_o = reinterpret_cast<float*>(smem + kSimtRingBytes);      // [KS][R][D]
   const int blocks = (R + RB - 1) / RB;                                 // blocks of RB rows
   const int KS = (blocks <= nwarps && nwarps % blocks == 0) ? nwarps / blocks : 1;   // warps that split a block's keys
   float* comb_ml = comb_o + static_cast<size_t>(KS) * R * D;            // [KS][R][2]
@@ -1775,6 +1756,12 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeP
   const float* qg = static_cast<const float*>(p.q) +
                     ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
   const float sl2 = p.scale_log2;
+  const uint32_t ring = smem_u32(smem) + tid * 16;
+  // dense and ragged rows: element offset of key 0, and from one key to the next
+  const bool dense = p.layout == B200ATTN_DENSE;
+  const long long kv_base = dense ? (static_cast<long long>(b) * p.kv_heads + h) * p.max_kv * D
+                                  : (seq_start * p.kv_heads + h) * D;
+  const int kv_stride = dense ? D : p.kv_heads * D;
   constexpr int kHalf = D / 2;               // a lane holds 4 floats at gl * 4 and 4 at D / 2 + gl * 4
 
   for (int rr = warp; rr < blocks * KS; rr += nwarps) {
@@ -1795,37 +1782,80 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeP
       stop = max(stop, vis[i]);
       all = min(all, vis[i]);
     }
-    float4 k0[kKeys], k1[kKeys], v0[kKeys], v1[kKeys];
-    bool on[kKeys];
-    // issues the loads of the step that starts at key t
-    auto load = [&](int t) {
+    // block-table entries of the step at key t, K's and V's of every key row of the lane's group
+    const bool paged = p.layout == B200ATTN_PAGED;
+    const int* ktab = paged ? p.k_table + static_cast<long long>(b) * p.table_stride : nullptr;
+    const int* vtab = paged ? p.v_table + static_cast<long long>(b) * p.table_stride : nullptr;
+    int kp[kKeys], vp[kKeys];
+    auto fetch_pages = [&](int t) {
 #pragma unroll
       for (int j = 0; j < kKeys; ++j) {
         const int key = t + j * kRowsWarp + sub;
-        k0[j] = k1[j] = v0[j] = v1[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        on[j] = key < stop;
-        if (!on[j]) continue;
-        const long long ko = row_offset(p, p.k_table, b, h, seq_start, key, D);
-        const long long vo = (p.layout == B200ATTN_PAGED) ? row_offset(p, p.v_table, b, h, seq_start, key, D) : ko;
-        if (ko < 0 || vo < 0) {              // a key on a page outside the cache weighs nothing
-          if (gl == 0) p.header[0] = DEV_ERR_PAGE_RANGE;
-          on[j] = false;
-          continue;
+        kp[j] = vp[j] = 0;
+        if (paged && key < stop) {
+          const int lp = p.page_shift >= 0 ? key >> p.page_shift : key / p.page_size;
+          kp[j] = ktab[lp];
+          vp[j] = vtab[lp];
         }
-        k0[j] = *reinterpret_cast<const float4*>(kg + ko);
-        k1[j] = *reinterpret_cast<const float4*>(kg + ko + kHalf);
-        v0[j] = *reinterpret_cast<const float4*>(vg + vo);
-        v1[j] = *reinterpret_cast<const float4*>(vg + vo + kHalf);
       }
     };
+    unsigned on = 0;                         // kKeys bits per step in flight, the newest lowest: the key is there
+    // issues the copies of the step at key t into slot `slot` of the lane's ring (zeros for keys that are not there)
+    auto copy = [&](int t, int slot) {
+#pragma unroll
+      for (int j = 0; j < kKeys; ++j) {
+        const int key = t + j * kRowsWarp + sub;
+        bool there = key < stop;
+        long long ko = 0, vo = 0;
+        if (there) {
+          if (paged) {
+            const bool bad = kp[j] < 0 || kp[j] >= p.num_pages || vp[j] < 0 || vp[j] >= p.num_pages;
+            if (bad) p.header[0] = DEV_ERR_PAGE_RANGE;   // a key on a page outside the cache weighs nothing
+            there = !bad;
+            const int off = p.page_shift >= 0 ? key & (p.page_size - 1) : key % p.page_size;
+            if (there) {
+              ko = ((static_cast<long long>(kp[j]) * p.page_size + off) * p.kv_heads + h) * D;
+              vo = ((static_cast<long long>(vp[j]) * p.page_size + off) * p.kv_heads + h) * D;
+            }
+          } else {
+            ko = vo = kv_base + static_cast<long long>(key) * kv_stride;
+          }
+        }
+        const int bytes = there ? 16 : 0;
+        const uint32_t dst = ring + static_cast<uint32_t>((slot * kKeys + j) * 4) * (kSimtThreads * 16);
+        cp_async16(dst, kg + ko, bytes);
+        cp_async16(dst + kSimtThreads * 16, kg + ko + kHalf, bytes);
+        cp_async16(dst + 2 * kSimtThreads * 16, vg + vo, bytes);
+        cp_async16(dst + 3 * kSimtThreads * 16, vg + vo + kHalf, bytes);
+        on = (on << 1) | (there ? 1u : 0u);
+      }
+      cp_async_commit();
+    };
     int t = t_begin + ks * kStep;
-    load(t);
+    fetch_pages(t);
+#pragma unroll
+    for (int s = 0; s < kSimtDepth - 1; ++s) {
+      const int ts = t + s * KS * kStep;
+      copy(ts, s);
+      fetch_pages(ts + KS * kStep);
+    }
+    int slot = 0;
     for (; t < stop; t += KS * kStep) {
+      {
+        const int ts = t + (kSimtDepth - 1) * KS * kStep;
+        copy(ts, (slot + kSimtDepth - 1) % kSimtDepth);     // (the slot was read in the step before)
+        fetch_pages(ts + KS * kStep);
+      }
+      cp_async_wait<kSimtDepth - 1>();
       float4 ck0[kKeys], ck1[kKeys], cv0[kKeys], cv1[kKeys];
       bool con[kKeys];
 #pragma unroll
-      for (int j = 0; j < kKeys; ++j) { ck0[j] = k0[j]; ck1[j] = k1[j]; cv0[j] = v0[j]; cv1[j] = v1[j]; con[j] = on[j]; }
-      load(t + KS * kStep);
+      for (int j = 0; j < kKeys; ++j) {
+        const float4* piece = reinterpret_cast<const float4*>(smem) + tid + (slot * kKeys + j) * 4 * kSimtThreads;
+        ck0[j] = piece[0]; ck1[j] = piece[kSimtThreads]; cv0[j] = piece[2 * kSimtThreads]; cv1[j] = piece[3 * kSimtThreads];
+        con[j] = (on >> ((kSimtDepth - 1) * kKeys + kKeys - 1 - j)) & 1u;
+      }
+      slot = (slot + 1) % kSimtDepth;
       const bool whole = t + kStep <= all;   // every row sees every key of the step
       float dot[RB][kKeys];
 #pragma unroll
@@ -1876,6 +1906,7 @@ __global__ void __launch_bounds__(kSimtThreads) decode_simt_kernel(const DecodeP
         }
       }
     }
+    cp_async_wait<0>();
     // merge the lane groups of the warp, then leave one partial per (key slice, row)
 #pragma unroll
     for (int i = 0; i < RB; ++i) {
@@ -1944,20 +1975,16 @@ DecodeWsLayout decode_ws_layout(const b200attn_decode_args_t& a, int sm_count, b
   // Fewer, longer CTAs amortise start-up and merge; the planner keeps the item count at or below this, so the grid
   // is a whole number of waves.  (Measured on B200, paged decode and speculative decode: 4 / 6 / 8 / 12 / 16 per SM
   // give 0.84 / 0.83 / 0.81 / 0.80 / 0.78 and 0.71 / 0.70 / 0.73 / 0.67 / 0.64 of the copy bandwidth without the
-  // whole-wave rule, 0.76 for speculative decode with it.)  The fp32 kernel keeps eight.
-  const int per_sm = f32_kernel ? 8 : 6;
+  // whole-wave rule, 0.76 for speculative decode with it.)
+  const int per_sm = 6;
   long long target = (static_cast<long long>(sm_count) * per_sm) / std::max(1, a.kv_heads);
   if (target < 1) target = 1;
   w.target_items = static_cast<int>(target);
-  // one wave of the tensor-core kernels: 2 (tcgen05 kernel, more than 16 rows) or 3 resident CTAs per SM; their
-  // per-item start-up + merge cost in keys of streaming time (from the sweeps quoted in the planner)
-  w.wave_items = 0;
-  w.item_overhead = 0;
-  if (!f32_kernel) {
-    const bool wide = rows > 16;
-    w.wave_items = static_cast<int>(std::max<long long>(1, (static_cast<long long>(sm_count) * (wide ? 2 : 3)) / std::max(1, a.kv_heads)));
-    w.item_overhead = wide ? 448 : 128;
-  }
+  // one wave: 2 (tcgen05 kernel, more than 16 rows) or 3 resident CTAs per SM; per-item start-up + merge cost in keys of
+  // streaming time (from the sweeps quoted in the planner)
+  const bool wide = rows > 16 && !f32_kernel;
+  w.wave_items = static_cast<int>(std::max<long long>(1, (static_cast<long long>(sm_count) * (wide ? 2 : 3)) / std::max(1, a.kv_heads)));
+  w.item_overhead = wide ? 448 : 128;
   // keep the partial write (rows x D fp32) small next to the chunk's K/V bytes
   int min_chunk = 128;
   const int by_rows = ((rows * 8 + kTileN - 1) / kTileN) * kTileN;
@@ -2082,7 +2109,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   if (a.dtype == B200ATTN_F32) {
     // (four warps leave at most 4 / blocks-of-rows partials per row: see the kernel)
     const int rb = p.rows >= 3 ? 4 : p.rows;
-    const size_t smem = sizeof(float) * static_cast<size_t>(std::max(p.rows, 4 * rb)) * (D + 2);
+    const size_t smem = kSimtRingBytes + sizeof(float) * static_cast<size_t>(std::max(p.rows, 4 * rb)) * (D + 2);
     int rc = 0;
 #define B200ATTN_LAUNCH_SIMT(DIM, RB)                                                                 \
     do {                                                                                              \

@@ -67,16 +67,15 @@ def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: i
     # fp32 inputs of a speculative-decode call (several q rows per head) run the tensor-core kernels on fp16 copies
     # and are planned like 16-bit inputs (unless k and v would need more than 8 GiB of copies: csrc/decode.cu)
     fp32 = fp32 and rows <= 16 and q_len <= 1
-    # six (item, kv head) CTAs per SM for the tensor-core kernels (a whole number of waves at 2 or 3 resident CTAs
-    # per SM), eight for the fp32 kernel
-    target = max(1, (sm_count * (8 if fp32 else 6)) // max(1, kv_heads))
+    # six (item, kv head) CTAs per SM (a whole number of waves at 2 or 3 resident CTAs per SM)
+    target = max(1, (sm_count * 6) // max(1, kv_heads))
     by_rows = -(-(rows * 8) // DECODE_TILE_TOKENS) * DECODE_TILE_TOKENS
     min_chunk = max(128, by_rows)
     tiles = -(-rows // 16)
     slices = 4 if tiles <= 2 else (2 if tiles <= 4 else 1)
     wide = rows > 16 and not fp32   # more than one 16-row tile: the tcgen05 kernel, two resident CTAs per SM (else three)
-    wave = 0 if fp32 else max(1, (sm_count * (2 if wide else 3)) // max(1, kv_heads))
-    overhead = 0 if fp32 else (448 if wide else 128)
+    wave = max(1, (sm_count * (2 if wide else 3)) // max(1, kv_heads))
+    overhead = 448 if wide else 128
     return DecodePlan(target, min_chunk, target + batch, tiles, slices, 32 * (tiles * slices + 1), wave, overhead,
                       2 * sm_count // max(1, kv_heads) if wide else 0)
 
