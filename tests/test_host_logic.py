@@ -251,7 +251,7 @@ def test_dealt_out_batches(qh, kvh, m):
     g = torch.Generator().manual_seed(3 * qh + m)
     dealt = 0
     for batch, lo, hi in [(32, 1024, 32768), (1, 50000, 50000), (3, 1, 90000), (200, 0, 2000), (700, 0, 9000), (64, 8192, 8192),
-                          (4096, 1, 300), (40, 0, 300)]:
+                          (4096, 1, 300), (40, 0, 300), (60, 9000, 70000)]:
         lens = torch.randint(lo, hi + 1, (batch,), generator=g).tolist()
         plan = decode_plan(148, batch, qh, kvh, m)
         cuts = decode_cuts(plan, lens)

@@ -118,7 +118,7 @@ def _plan_lengths(plan: DecodePlan, lens: Sequence[int]):
             best, chunk = w_biggest + plan.item_overhead, w_chunk
     line = total + (len(lens) + plan.slots - 1) * plan.item_overhead
     dealt = (1 < plan.slots <= 512 and len(lens) <= 4096 and line < 1 << 30 and items > plan.wave_items
-             and line / plan.slots < best)
+             and line / plan.slots + plan.min_chunk < best)
     return chunk, dealt
 
 
