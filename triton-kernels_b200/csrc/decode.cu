@@ -683,50 +683,76 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
   return __all_sync(0xffffffffu, ok);
 }
 
-// Block-table read-ahead of a producer warp for paged caches: lane i owns box i of a 64-key tile (`on` only when a
-// tile has at most 32 boxes).  fetch() issues the two table reads of the tile that starts at key t0 and leaves the
-// raw entries in the caller's registers; row() turns an entry into the cache row of the lane's box, once the entry is
-// needed (checking it then, so that nothing waits for the read before).
+// Block-table read-ahead of a producer warp for paged caches (`on`: a 64-key tile has at most 32 boxes).  The warp holds
+// the raw entries of 32 boxes of its item, one per lane, for K and for V, and those of the next 32, read when the first
+// became current: a table read is waited for once in 32 boxes, long after it was issued, instead of a tile after it
+// (32 x 16 384 keys in 16-key pages, head_dim 128: 388 -> 365 us with 40 rows per KV head, 483 -> 417 with
+// 128; dense K/V of that size 341 and 380).
+// Entries are checked when they are used, so that nothing waits for the read before.  Registers are plain scalars: an
+// array indexed by a loop counter would live in local memory.
 constexpr int kNoPage = static_cast<int>(0x80000000u);
 struct PageAhead {
   const int* ktab;
   const int* vtab;
-  int lane, boxes, box_rows;
+  int lane, boxes, box_shift, page_shift, page_size;
   bool on;
-  __device__ __forceinline__ PageAhead(const DecodeParams& p, int b, int lane_) : lane(lane_) {
-    boxes = kTileN >> p.box_shift;
-    box_rows = 1 << p.box_shift;
+  int t_begin, t_end;          // the item's keys
+  int kp, vp, kp_next, vp_next;
+  __device__ __forceinline__ PageAhead(const DecodeParams& p, int lane_) : lane(lane_) {
+    box_shift = p.box_shift;
+    boxes = kTileN >> box_shift;
     on = p.layout == B200ATTN_PAGED && boxes <= 32;
     page_shift = p.page_shift;
     page_size = p.page_size;
-    ktab = on ? p.k_table + static_cast<long long>(b) * p.table_stride : nullptr;
-    vtab = on ? p.v_table + static_cast<long long>(b) * p.table_stride : nullptr;
+    ktab = vtab = nullptr;
+    t_begin = t_end = 0;
+    kp = vp = kp_next = vp_next = kNoPage;
   }
-  __device__ __forceinline__ void retarget(const DecodeParams& p, int b) {
-    if (on) {
-      ktab = p.k_table + static_cast<long long>(b) * p.table_stride;
-      vtab = p.v_table + static_cast<long long>(b) * p.table_stride;
-    }
-  }
-  __device__ __forceinline__ void fetch(int t0, int t_end, int& kp, int& vp) const {
-    const int t = t0 + lane * box_rows;
-    kp = vp = kNoPage;
-    if (lane < boxes && t < t_end) {
+  __device__ __forceinline__ void read(int first_box, int& k, int& v) const {
+    const int t = t_begin + ((first_box + lane) << box_shift);
+    k = v = kNoPage;
+    if (t < t_end) {
       // (page size known only at run time; a shift when it is a power of two)
-      kp = __ldg(ktab + page_of(t));
-      vp = __ldg(vtab + page_of(t));
+      const int lp = page_shift >= 0 ? (t >> page_shift) : t / page_size;
+      k = __ldg(ktab + lp);
+      v = __ldg(vtab + lp);
     }
   }
-  int page_shift, page_size;
-  __device__ __forceinline__ int page_of(int t) const { return page_shift >= 0 ? (t >> page_shift) : t / page_size; }
-  __device__ __forceinline__ int row(const DecodeParams& p, int page, int t0) const {
-    if (page == kNoPage) return -1;
-    const int t = t0 + lane * box_rows;
+  __device__ __forceinline__ void start(const DecodeParams& p, int b, int begin, int end) {
+    if (!on) return;
+    ktab = p.k_table + static_cast<long long>(b) * p.table_stride;
+    vtab = p.v_table + static_cast<long long>(b) * p.table_stride;
+    t_begin = begin;
+    t_end = end;
+    read(0, kp, vp);
+    read(32, kp_next, vp_next);
+  }
+  // cache row of an entry's box at key t, -1 when there is none
+  __device__ __forceinline__ int row(const DecodeParams& p, int page, int t) const {
     const int off = page_shift >= 0 ? (t & (page_size - 1)) : t % page_size;
     // an entry outside the cache is reported and replaced by page 0: never dereferenced, output stays finite
     const bool bad = page < 0 || page >= p.num_pages;
     if (bad) p.header[0] = DEV_ERR_PAGE_RANGE;
-    return p.num_pages > 0 ? (bad ? 0 : page) * p.page_size + off : -1;
+    return (bad ? 0 : page) * p.page_size + off;
+  }
+  // rows of the lane's box of tile number `tile` of the item (called for every tile, in order); returns the boxes that
+  // the tile has
+  __device__ __forceinline__ int tile_rows(const DecodeParams& p, int tile, int& kr, int& vr) {
+    const int at = (tile * boxes) & 31;
+    if (at == 0 && tile > 0) {
+      kp = kp_next;
+      vp = vp_next;
+      read(tile * boxes + 32, kp_next, vp_next);
+    }
+    const int k = __shfl_sync(0xffffffffu, kp, (at + lane) & 31), v = __shfl_sync(0xffffffffu, vp, (at + lane) & 31);
+    const int t0 = t_begin + tile * kTileN;
+    const int n = p.num_pages > 0 ? min(boxes, (t_end - t0 + (1 << box_shift) - 1) >> box_shift) : 0;
+    kr = vr = -1;
+    if (lane < n) {
+      kr = row(p, k, t0 + (lane << box_shift));
+      vr = row(p, v, t0 + (lane << box_shift));
+    }
+    return n;
   }
 };
 
@@ -815,12 +841,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(b) * p.kv_heads + h) * p.max_kv; }
     bool ok = true;
     int issued = 0;
-    // Paged caches with at most one box per lane and tile: the block-table entries of a tile are read one tile ahead,
-    // into two plain registers (an array indexed by a loop counter would live in local memory and the read would be
-    // waited for at once), so that the table read is over by the time the tile's stage comes free.
-    const PageAhead ahead(p, b, lane);
-    int kp_next = kNoPage, vp_next = kNoPage;
-    if (ahead.on && ntiles > 0) ahead.fetch(t_begin, t_end, kp_next, vp_next);
+    PageAhead ahead(p, lane);
+    ahead.start(p, b, t_begin, t_end);
     for (int tile = 0; tile < ntiles; ++tile) {
       const int stage = tile % kStages, use = tile / kStages;
       if (use > 0) {
@@ -839,15 +861,14 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
           ptx::tma_load_4d(vdst, &tm_v, bar, 0, row, 0, h_coord);
         }
       } else if (ahead.on) {
-        const int kr = ahead.row(p, kp_next, t0), vr = ahead.row(p, vp_next, t0);
-        int count = (kr >= 0) + (vr >= 0);
-        for (int off = 16; off > 0; off >>= 1) count += __shfl_xor_sync(0xffffffffu, count, off);
-        if (lane == 0) ptx::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(count) * ahead.box_rows * 128 * CHUNKS);
+        int kr, vr;
+        const int count = ahead.tile_rows(p, tile, kr, vr);
+        const uint32_t box_bytes = 128u * CHUNKS << ahead.box_shift;
+        if (lane == 0) ptx::mbar_arrive_expect_tx(bar, static_cast<uint32_t>(2 * count) * box_bytes);
         __syncwarp();
-        const uint32_t boff = static_cast<uint32_t>(lane) * ahead.box_rows * 128 * CHUNKS;
+        const uint32_t boff = static_cast<uint32_t>(lane) * box_bytes;
         if (kr >= 0) ptx::tma_load_4d(kdst + boff, &tm_k, bar, 0, kr, 0, h_coord);
         if (vr >= 0) ptx::tma_load_4d(vdst + boff, &tm_v, bar, 0, vr, 0, h_coord);
-        if (tile + 1 < ntiles) ahead.fetch(t0 + kTileN, t_end, kp_next, vp_next);
       } else {
         // one box of box_rows keys per (lane, round); only pages that hold keys of this chunk are fetched
         const int boxes = kTileN >> p.box_shift;
@@ -1220,10 +1241,7 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
     bool ok = true;
     int g = 0;                                   // tiles issued so far, over all units
     const int box_rows = 1 << p.box_shift;
-    // block-table entries are read one tile ahead, across units too (see PageAhead)
-    PageAhead ahead(p, 0, lane);
-    int kp_next = kNoPage, vp_next = kNoPage;
-    int ahead_g = -1;                            // running tile index the entries in kp_next / vp_next belong to
+    PageAhead ahead(p, lane);                    // (a unit's first entries are read when it is drawn)
     auto publish = [&](int r, int u) {            // lane 0
       ctrl->unit_ring[r % kUmmaUnitRing] = u;
       ctrl->published = r + 1;
@@ -1245,7 +1263,7 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
     if (lane == 0) publish(0, u);
     for (int r = 0; ok && u < n_units; ++r) {
       const UmmaUnit w = umma_unit(p, u);
-      ahead.retarget(p, w.b);
+      if (r == 0) ahead.start(p, w.b, w.t_begin, w.t_end);
       int h_coord = w.h;
       long long row0 = w.seq_start;
       if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(w.b) * p.kv_heads + w.h) * p.max_kv; }
@@ -1270,22 +1288,15 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
             }
           }
         } else if (ahead.on) {
-          if (ahead_g != g) ahead.fetch(t0, w.t_end, kp_next, vp_next);   // first tile of the CTA, or after an empty unit
-          const int kr = ahead.row(p, kp_next, t0), vr = ahead.row(p, vp_next, t0);
-          int count = (kr >= 0) + (vr >= 0);
-          for (int off = 16; off > 0; off >>= 1) count += __shfl_xor_sync(0xffffffffu, count, off);
-          if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(count) * box_rows * 128 * CHUNKS);
+          int kr, vr;
+          const int count = ahead.tile_rows(p, tile, kr, vr);
+          if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(2 * count) * box_rows * 128 * CHUNKS);
           __syncwarp();
           const uint32_t roff = static_cast<uint32_t>(lane) * box_rows * 128;
 #pragma unroll
           for (int cc = 0; cc < CHUNKS; ++cc) {
             if (kr >= 0) tma_load_3d(kdst + cc * CHUNK_BYTES + roff, &tm_k, bar, cc * 64, h_coord, kr);
             if (vr >= 0) tma_load_3d(vdst + cc * CHUNK_BYTES + roff, &tm_v, bar, cc * 64, h_coord, vr);
-          }
-          // read ahead: the next tile of this unit (the first tile of the next unit: after the draw below)
-          if (tile + 1 < w.ntiles) {
-            ahead.fetch(t0 + kTileN, w.t_end, kp_next, vp_next);
-            ahead_g = g + 1;
           }
         } else {
           const int boxes = kTileN >> p.box_shift;
@@ -1344,11 +1355,7 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
       u_next = __shfl_sync(0xffffffffu, u_next, 0);
       if (u_next < n_units) {
         const UmmaUnit w2 = umma_unit(p, u_next);
-        if (ahead.on && w2.ntiles > 0) {
-          ahead.retarget(p, w2.b);
-          ahead.fetch(w2.t_begin, w2.t_end, kp_next, vp_next);
-          ahead_g = g;
-        }
+        ahead.start(p, w2.b, w2.t_begin, w2.t_end);
         const T* q2 = static_cast<const T*>(p.q) +
                       ((static_cast<long long>(w2.b) * p.q_heads + static_cast<long long>(w2.h) * p.head_stride + p.head0) * p.q_len) * D;
         for (int i = lane; i < (R * D * static_cast<int>(sizeof(T))) / 128; i += 32) prefetch_l2(reinterpret_cast<const char*>(q2) + i * 128);
