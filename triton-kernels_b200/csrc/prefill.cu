@@ -307,6 +307,19 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // everything the other warps read or write outside this CTA follows an item published or a tile loaded below
     ptx::grid_dep_wait();
     bool ok = true;
+    // Paged K/V with at most 32 boxes per tile: the warp holds the raw block-table entries of 32 boxes of the item, one per
+    // lane, for K and for V, and those of the next 32, read when the first became current, so that no table read stands
+    // between "stage free" and "copies issued" (the ring is only two pairs deep).  Against a read per pair, one pair ahead,
+    // causal with 16-key pages: 4 x 2 048 tokens, 32/8 heads, head_dim 128 187 -> 165 us, 2 x 4 096 325 -> 280, 5 x 8 181
+    // at head_dim 64 600 -> 523 (dense K/V: 146, 255, 503).  (Plain registers: an array indexed by a loop counter would
+    // live in local memory.)
+    constexpr int kNoPage = static_cast<int>(0x80000000u);
+    const int box_shift = kPaged ? 31 - __clz(p.box_rows) : 0;
+    const int pf_boxes = kPaged ? kBN >> box_shift : 0;
+    const bool pf = kPaged && pf_boxes <= 32;
+    const bool page_pow2 = (p.page_size & (p.page_size - 1)) == 0;
+    const int page_shift = 31 - __clz(p.page_size);
+    int pg_k = kNoPage, pg_v = kNoPage, pg_k_next = kNoPage, pg_v_next = kNoPage;
     int pair_e = 0;       // K/V pairs issued so far, across items
     int pair_lo = 0;      // first pair of the current item
     for (int k = 0; ok; ++k) {
@@ -329,6 +342,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         mbar_arrive(smem_u32(&ctrl->sched_full[k & 1]));
       }
       if (item < 0) break;
+      const int* vtab = kPaged ? p.v_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
+      const int* ktab = kPaged ? p.k_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
+      auto read_page = [&](const int* tab, int first_box) -> int {
+        const int t = (first_box + lane) << box_shift, tg = t + w.kv_tok0;
+        return t < w.len_k ? __ldg(tab + (page_pow2 ? tg >> page_shift : tg / p.page_size)) : kNoPage;
+      };
+      if (pf && w.nkv_max > 0) {
+        pg_k = read_page(ktab, 0);
+        pg_v = read_page(vtab, 0);
+        if (w.len_k > (32 << box_shift)) {
+          pg_k_next = read_page(ktab, 32);
+          pg_v_next = read_page(vtab, 32);
+        }
+      }
       if (k >= 1 && lane == 0) {
         // the previous item is still running: pull this item's Q tiles and first K/V tiles into L2 now, so the
         // copies issued once the Q buffer is free only pay an L2 round trip
@@ -368,21 +395,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // (the last one V alone).  Stage = pair % 2; its V buffer is ring buffer 2 * stage, its K buffer 2 * stage + 1.
       pair_lo = pair_e;
       const int npairs = w.nkv_max > 0 ? w.nkv_max + 1 : 0;
-      // Paged K/V with at most 32 boxes per tile (one per lane): the raw block-table entries of a pair's boxes (V of
-      // tile pi - 1, K of tile pi) are read one pair ahead, into two plain registers, so that the table read is not
-      // between "stage free" and "copies issued" (the ring is only two pairs deep).
-      constexpr int kNoPage = static_cast<int>(0x80000000u);
-      const int pf_boxes = kPaged ? kBN / p.box_rows : 0;
-      const bool pf = kPaged && pf_boxes <= 32;
-      int pg_v = kNoPage, pg_k = kNoPage;
-      auto fetch_pages = [&](int pi) {
-        const int tv = (pi - 1) * kBN + lane * p.box_rows, tk = pi * kBN + lane * p.box_rows;
-        pg_v = (lane < pf_boxes && pi >= 1 && tv < w.len_k)
-                   ? __ldg(p.v_table + static_cast<long long>(w.b) * p.table_stride + (tv + w.kv_tok0) / p.page_size) : kNoPage;
-        pg_k = (lane < pf_boxes && pi < w.nkv_max && tk < w.len_k)
-                   ? __ldg(p.k_table + static_cast<long long>(w.b) * p.table_stride + (tk + w.kv_tok0) / p.page_size) : kNoPage;
-      };
-      if (pf && npairs > 0) fetch_pages(0);
       for (int pi = 0; pi < npairs && ok; ++pi, ++pair_e) {
         const int stage = pair_e % kStages;
         const int use = pair_e / kStages;
@@ -395,7 +407,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const int jv = pi - 1, jk = pi;               // tile indices of the V and the K of this pair
         const uint32_t vdst = smem_base + Plan::kRingOff + (2 * stage) * Plan::kTileBytes;
         const uint32_t kdst = vdst + Plan::kTileBytes;
-        if (p.layout != B200ATTN_PAGED) {
+        if (!kPaged) {
           if (lane == 0) {
             mbar_arrive_expect_tx(bar, (has_v ? Plan::kTileBytes : 0) + (has_k ? Plan::kTileBytes : 0));
             for (int c = 0; c < Plan::kChunks; ++c) {
@@ -408,19 +420,30 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
           }
         } else if (pf) {
-          // one box per lane and operand from the prefetched table entries
+          // one box per lane and operand from the entries read ahead
+          if (has_k && pi > 0 && ((pi * pf_boxes) & 31) == 0) {
+            pg_k = pg_k_next;
+            pg_k_next = read_page(ktab, pi * pf_boxes + 32);
+          }
+          if (jv > 0 && ((jv * pf_boxes) & 31) == 0) {
+            pg_v = pg_v_next;
+            pg_v_next = read_page(vtab, jv * pf_boxes + 32);
+          }
+          auto boxes_of = [&](int t0) -> int { return min(pf_boxes, (w.len_k - t0 + p.box_rows - 1) >> box_shift); };
+          const int nk = has_k && p.num_pages > 0 ? boxes_of(jk * kBN) : 0;
+          const int nv = has_v && p.num_pages > 0 ? boxes_of(jv * kBN) : 0;
           auto row_of = [&](int page, int t) -> int {
-            if (page == kNoPage) return -1;
             // an entry outside the cache is reported and replaced by page 0: never dereferenced, output stays finite
             const bool bad = page < 0 || page >= p.num_pages;
             if (bad) p.header[0] = DEV_ERR_PAGE_RANGE;
-            return p.num_pages > 0 ? (bad ? 0 : page) * p.page_size + (t + w.kv_tok0) % p.page_size : -1;
+            const int tg = t + w.kv_tok0;
+            return (bad ? 0 : page) * p.page_size + (page_pow2 ? tg & (p.page_size - 1) : tg % p.page_size);
           };
-          const int rv = row_of(pg_v, jv * kBN + lane * p.box_rows);
-          const int rk = row_of(pg_k, jk * kBN + lane * p.box_rows);
-          int count = (rv >= 0) + (rk >= 0);
-          for (int o = 16; o > 0; o >>= 1) count += __shfl_xor_sync(0xffffffffu, count, o);
-          if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(count) * p.box_rows * 128 * Plan::kChunks);
+          const int ek = __shfl_sync(0xffffffffu, pg_k, (jk * pf_boxes + lane) & 31);
+          const int ev = __shfl_sync(0xffffffffu, pg_v, (jv * pf_boxes + lane) & 31);
+          const int rk = lane < nk ? row_of(ek, jk * kBN + (lane << box_shift)) : -1;
+          const int rv = lane < nv ? row_of(ev, jv * kBN + (lane << box_shift)) : -1;
+          if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(nk + nv) * p.box_rows * 128 * Plan::kChunks);
           __syncwarp();
           for (int c = 0; c < Plan::kChunks; ++c) {
             if (rv >= 0)
@@ -428,7 +451,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (rk >= 0)
               tma_load_3d(kdst + c * Plan::kChunkBytes + lane * p.box_rows * 128, &tm_k, bar, c * 64, w.kv_head_coord, rk);
           }
-          if (pi + 1 < npairs) fetch_pages(pi + 1);
         } else {
           // one box of `box_rows` tokens per lane per round and operand; only pages that exist are fetched
           const int boxes = kBN / p.box_rows;
@@ -445,8 +467,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (bad) p.header[0] = DEV_ERR_PAGE_RANGE;
             return p.num_pages > 0 ? (bad ? 0 : page) * p.page_size + (tg - lp * p.page_size) : -1;
           };
-          const int* vtab = p.v_table + static_cast<long long>(w.b) * p.table_stride;
-          const int* ktab = p.k_table + static_cast<long long>(w.b) * p.table_stride;
           for (int i = lane; i < boxes; i += 32) {
             const int rv = has_v ? page_row(vtab, jv * kBN + i * p.box_rows) : -1;
             const int rk = has_k ? page_row(ktab, jk * kBN + i * p.box_rows) : -1;
