@@ -423,16 +423,20 @@ __global__ void softmax_cluster_kernel(const T* x, T* out, long long rows, long 
 // ---------------------------------------------------------------------------
 constexpr int kRingThreads = 512;                   // threads that compute (the producer warp comes on top)
 constexpr int kRingWarps = kRingThreads / 32;
-constexpr int kRingPer = 4;                         // 16-byte pieces per thread and chunk
-constexpr int kRingChunk = kRingThreads * kRingPer;
-constexpr int kRingSlots = 7;                       // 224 KiB
-constexpr int kRingPieces = kRingChunk * kRingSlots;
+// PER 16-byte pieces per thread and chunk.  Four; three where that lets the ring hold more rows, because a row's last
+// chunk would be nearly empty and still take a slot (12 135 x 32 960 bf16 361 -> 319 us).
+template <int PER> struct Ring {
+  static constexpr int kChunk = kRingThreads * PER;
+  static constexpr int kSlots = PER == 4 ? 7 : 9;          // 224 and 216 KiB
+  static int chunks(long long slice) { return static_cast<int>((slice + kChunk - 1) / kChunk); }
+};
+constexpr int kRingPieces = Ring<4>::kChunk * Ring<4>::kSlots;
 
 // (m, s) <- (m, s) + the elements of a thread's pieces of a chunk; m is the reference of s
-template <typename T> __device__ __forceinline__ void online_add(float& m, float& s, uint4 (&u)[kRingPer]) {
+template <typename T, int PER> __device__ __forceinline__ void online_add(float& m, float& s, uint4 (&u)[PER]) {
   float mx = piece_max<T>(u[0]);
 #pragma unroll
-  for (int k = 1; k < kRingPer; ++k) mx = fmaxf(mx, piece_max<T>(u[k]));
+  for (int k = 1; k < PER; ++k) mx = fmaxf(mx, piece_max<T>(u[k]));
   if (mx > m) {
     s = (m == -INFINITY) ? 0.f : s * row_exp<T>(m - mx);
     m = mx;
@@ -440,14 +444,15 @@ template <typename T> __device__ __forceinline__ void online_add(float& m, float
   if (m != -INFINITY) {
     float t = piece_exp_sum<T, false>(u[0], m);
 #pragma unroll
-    for (int k = 1; k < kRingPer; ++k) t += piece_exp_sum<T, false>(u[k], m);
+    for (int k = 1; k < PER; ++k) t += piece_exp_sum<T, false>(u[k], m);
     s += t;
   }
 }
 
-template <typename T, bool LOG>
+template <typename T, bool LOG, int PER>
 __global__ void __launch_bounds__(kRingThreads + 32, 1)
 softmax_ring_kernel(const T* x, T* out, long long rows, long long cols, int slice /* pieces of a row per CTA */, int csize) {
+  constexpr int kRingPer = PER, kRingChunk = Ring<PER>::kChunk, kRingSlots = Ring<PER>::kSlots;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float2 scratch[2][kRingWarps];
   __shared__ __align__(8) float2 pairs[2][kMaxCluster];    // every CTA's (max, sum) of the even / odd row in work
@@ -529,7 +534,7 @@ softmax_ring_kernel(const T* x, T* out, long long rows, long long cols, int slic
 #pragma unroll
         for (int k = 0; k < kRingPer; ++k) u[k] = k * kRingThreads < left ? c4[k * kRingThreads] : make_uint4(w, w, w, w);
       }
-      online_add<T>(m, s, u);
+      online_add<T, PER>(m, s, u);
       if (++slot == kRingSlots) { slot = 0; phase ^= 1u; }
     }
     if (tid < edges && edge != -INFINITY) {
@@ -625,7 +630,7 @@ int set_smem_limit(K kernel, size_t bytes) {
 inline int ring_cluster(long long rows, long long nv, int sm_count) {
   int csize = 1;
   while ((nv + csize - 1) / csize > kRingPieces) csize *= 2;
-  while (csize < kMaxCluster && rows * csize * 2 <= sm_count && nv > 4LL * csize * kRingChunk) csize *= 2;
+  while (csize < kMaxCluster && rows * csize * 2 <= sm_count && nv > 4LL * csize * Ring<4>::kChunk) csize *= 2;
   return csize;
 }
 
@@ -660,7 +665,9 @@ int launch_pieces(const b200attn_softmax_args_t& a, int sm_count, cudaStream_t s
     const int csize = ring_cluster(rows, nv, sm_count);
     const int slice = static_cast<int>((nv + csize - 1) / csize);
     const size_t smem = static_cast<size_t>(kRingPieces) * 16;
-    auto kernel = softmax_ring_kernel<T, LOG>;
+    const int c4 = Ring<4>::chunks(slice), c3 = Ring<3>::chunks(slice);
+    const bool three = c3 <= Ring<3>::kSlots && Ring<3>::kSlots * c4 * 5 >= Ring<4>::kSlots * c3 * 6;
+    auto kernel = three ? softmax_ring_kernel<T, LOG, 3> : softmax_ring_kernel<T, LOG, 4>;
     int rc = set_smem_limit(kernel, smem);
     if (rc) return rc;
     // one CTA per SM; how many clusters of a size the GPU holds at once is asked of the driver once (the answer depends
