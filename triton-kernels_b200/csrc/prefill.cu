@@ -14,14 +14,20 @@
 //   warp  17   : tcgen05.mma issuer and TMEM owner; the warp stays converged, one elected lane issues
 // TMEM (512 columns): S0 | S1 | O0 | O1.  Per KV tile j and slot s:
 //   S_s = Q_s K_j^T   (SS MMA, 128x128xD)            -> commit s_full[s]
-//   the slot's warps read S_s, mask, keep a running max / sum per row in the exp2 domain, rescale O_s in TMEM only
-//   when the max moved by more than 2^8, and write P_s as packed 16-bit (16x128b layout) over the first 32 columns
-//   of each 64-column half of S_s                                     -> arrive p_ready[s]
+//   the slot's warps exponentiate S_s (exp2 domain) against each row's reference, keep the row sums, and write P_s as
+//   packed 16-bit (16x128b layout) over the first 32 columns of each 64-column half of S_s -> arrive p_ready[s]
+//   (a row's reference, the maximum when it was set, moves only when the sums say that it has to; O_s is then rescaled)
 //   O_s += P_s V_j    (TS MMA, A from TMEM, V is the MN-major B operand) -> commit o_done[s]
 // The two slots are interleaved so that one slot's softmax overlaps the other's MMAs.  At the end of an item the
-// MMA warp issues the first score tile of the next item behind the last PVs, and the softmax warps finish the old
-// item's epilogue lazily: O is normalised and read out at the end of the next item's first tile and stored while
-// the tensor cores work on that tile.
+// MMA warp issues the first score tile of the next item behind the last PVs, and the softmax warps read O out, normalise
+// and store it while that tile is computed.
+//
+// What bounds it.  Long launches run at the board's 1 000 W (1.6 GHz instead of 1.97): there the time is the energy of a
+// tile, and an instruction left out per score counts for more than a shorter chain of waits.  The softmax is therefore as
+// few instructions per pair of scores as there can be: one packed FMA, two exponentials, one packed add, one conversion,
+// and no row maximum.  Against a pass for the maximum before them and a quarter of the exponentials as polynomials on the
+// FMA pipes: 2 x 2 048 causal tokens, 32/8 heads, D 128, 86.2 -> 81.1 us; sixteen ragged sequences of 128 to 4 096
+// 1 077 -> 1 001; 8 x 2 048 without a mask 586 -> 546.
 //
 // Every mbarrier wait is bounded; on expiry the role records DEV_ERR_WAIT_EXPIRED
 // in the workspace header and falls through to the common teardown (TMEM is freed).
@@ -51,17 +57,11 @@ constexpr int kSoftmaxWarps = 16;  // 4 warpgroups: (slot 0 | slot 1) x (columns
 constexpr int kThreads = 576;
 constexpr int kProducerWarp = 16;
 constexpr int kMmaWarp = 17;
-constexpr float kRescaleThreshold = 8.0f;  // log2 units
-// Of every 4 pairs of scores, this many are exponentiated on the FMA pipes (range reduction + cubic
-// polynomial, relative error 7.5e-5, far below the 16-bit rounding of P) instead of the MUFU unit,
-// which at 16 results per clock per SM is as scarce as the tensor pipe at head_dim 128.
-#ifndef B200ATTN_EXP_EMU_OF4
-#define B200ATTN_EXP_EMU_OF4 1
-#endif
-constexpr int kExpEmuOf4 = B200ATTN_EXP_EMU_OF4;
-
-
-
+// A tile's exponentials against the reference that stands are good as long as a thread's 32 of them, of a row, sum up to
+// no more than kMaxPartialSum (P then fits 16 bits, and so does every one of them).  When that is not so the row's maximum
+// lies five powers of two or more above its reference; a reference moves when the maximum is kRescaleThreshold above it.
+constexpr float kMaxPartialSum = 1024.0f;
+constexpr float kRescaleThreshold = 3.0f;  // log2 units
 // Everything one work item needs; decoded once by the scheduler warp.  An item is two 128-row query tiles
 // ("slots") that share one KV head: with an even GQA group the same 128 rows of two neighbouring q heads (equal
 // causal extents, so both slots always have work), otherwise two consecutive row tiles of one q head.
@@ -272,7 +272,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       for (int i = 0; i < kStages; ++i) { mbar_init(smem_u32(&ctrl->kv_full[i]), 1); mbar_init(smem_u32(&ctrl->kv_empty[i]), 1); }
       for (int s = 0; s < kSlots; ++s) {
         mbar_init(smem_u32(&ctrl->s_full[s]), 1);
-        mbar_init(smem_u32(&ctrl->p_ready[s]), 2 * kBM);
+        mbar_init(smem_u32(&ctrl->p_ready[s]), 8);         // one arrival per softmax warp of the slot
         mbar_init(smem_u32(&ctrl->o_done[s]), 1);
         mbar_init(smem_u32(&ctrl->o_free[s]), 8);          // one arrival per softmax warp of the slot
       }
@@ -680,16 +680,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const float sl2 = p.scale_log2;
     int tile_cnt = 0;     // score tiles of this slot consumed so far (barrier phases run across items)
     bool ok = true;
-    // The epilogue of an item is finished lazily: O is read out of tensor memory at the end of the first score
-    // tile of the slot's next item (its PV is the first thing that overwrites O) and the global stores are issued
-    // after that tile's P has been handed over, so they drain while the tensor cores work on it.
-    bool pend = false;        // an item's output is still in tensor memory
-    bool pend_acc = false;    // ... and it has an accumulator (false: the slot had no keys, the output is zero)
-    int pend_phase = 0;       // o_done phase of its last PV
-    int pend_rows = 0;        // rows of the tile that exist in the sequence
-    float pend_la = 0.f, pend_lb = 0.f;   // row sums of rows A and B
-    long long pend_off = 0;   // element offset of row A's first output column
-    long long pend_stride = 0;   // elements between consecutive rows of the output
+    // The epilogue of an item runs while the first score tile of the slot's next item is computed.
+    bool out_acc = false;     // the item has an accumulator (false: the slot had no keys, the output is zero)
+    int out_phase = 0;       // o_done phase of its last PV
+    int out_rows = 0;        // rows of the tile that exist in the sequence
+    float out_la = 0.f, out_lb = 0.f;   // row sums of rows A and B
+    long long out_off = 0;   // element offset of row A's first output column
+    long long out_stride = 0;   // elements between consecutive rows of the output
     constexpr bool k16 = !std::is_same<OutT, float>::value;
     auto quad_max = [](float v) {
       v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
@@ -724,25 +721,18 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       }
     };
-    auto flush = [&](bool hand_over) -> bool {
-      if (pend_acc) {
-        if (!warp_wait(smem_u32(&ctrl->o_done[s]), pend_phase)) return false;
+    auto write_out = [&]() -> bool {
+      if (out_acc) {
+        if (!warp_wait(smem_u32(&ctrl->o_done[s]), out_phase)) return false;
       }
       tc_fence_after();
-      const float inv_a = pend_la > 0.f ? 1.f / pend_la : 0.f;
-      const float inv_b = pend_lb > 0.f ? 1.f / pend_lb : 0.f;
-      auto o_is_free = [&]() {
+      const float inv_a = out_la > 0.f ? 1.f / out_la : 0.f;
+      const float inv_b = out_lb > 0.f ? 1.f / out_lb : 0.f;
+      auto o_is_read = [&]() {
         // O has been read out: the MMA warp may start the next item's PV into it
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->o_free[s]));
-      };
-      auto hand = [&]() {
-        if (hand_over) {
-          // this tile's P goes to the MMA warp before the stores are issued
-          tc_fence_before();
-          mbar_arrive(smem_u32(&ctrl->p_ready[s]));
-        }
       };
       constexpr int kChunksO = D / 64;
       if constexpr (k16) {
@@ -753,14 +743,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < kChunksO; ++c) {
           uint32_t v[32];
-          if (pend_acc) {
+          if (out_acc) {
             tmem_ld_16x256b_x8(tO + c * 64, v);
             tmem_wait_ld();
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
-          if (c == kChunksO - 1) o_is_free();
+          if (c == kChunksO - 1) o_is_read();
           uint32_t a[8], b[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -776,13 +766,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             line[c][1][m] = b[2 * m];  line[c][1][4 + m] = b[2 * m + 1];
           }
         }
-        hand();
 #pragma unroll
         for (int ab = 0; ab < 2; ++ab) {
-          if (rowA + 8 * ab < pend_rows) {
+          if (rowA + 8 * ab < out_rows) {
 #pragma unroll
             for (int c = 0; c < kChunksO; ++c) {
-              T* out = static_cast<T*>(p.out) + pend_off + ab * 8 * pend_stride + c * 64 + q * 16;
+              T* out = static_cast<T*>(p.out) + out_off + ab * 8 * out_stride + c * 64 + q * 16;
               const uint32_t (&u)[8] = line[c][ab];
               if (p.out_align32) {
                 st_global_v8(out, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7]);
@@ -798,26 +787,25 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < kChunksO; ++c) {
           uint32_t v[32];
-          if (pend_acc) {
+          if (out_acc) {
             tmem_ld_16x256b_x8(tO + c * 64, v);
             tmem_wait_ld();
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
-          if (c == kChunksO - 1) { o_is_free(); hand(); }
-          float* out = static_cast<float*>(p.out) + pend_off + c * 64 + q * 2;
+          if (c == kChunksO - 1) o_is_read();
+          float* out = static_cast<float*>(p.out) + out_off + c * 64 + q * 2;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            if (rowA < pend_rows)
+            if (rowA < out_rows)
               *reinterpret_cast<float2*>(out + i * 8) = make_float2(__uint_as_float(v[4 * i]) * inv_a, __uint_as_float(v[4 * i + 1]) * inv_a);
-            if (rowA + 8 < pend_rows)
-              *reinterpret_cast<float2*>(out + 8 * pend_stride + i * 8) =
+            if (rowA + 8 < out_rows)
+              *reinterpret_cast<float2*>(out + 8 * out_stride + i * 8) =
                   make_float2(__uint_as_float(v[4 * i + 2]) * inv_b, __uint_as_float(v[4 * i + 3]) * inv_b);
           }
         }
       }
-      pend = false;
       return true;
     };
     for (int k = 0; ok; ++k) {
@@ -830,195 +818,192 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const int n = w.nkv[s];
       const int m0s = w.m0[s];
       const int len_k = w.len_k;
-      const int row_abs = m0s + rowA - w.kv_tok0;       // query index of row A relative to the item's first key (row B: + 8)
-      if (pend && n == 0) {
-        // no score tile in this item to hang the previous item's epilogue on
-        ok = flush(false);
-        if (!ok) break;
-      }
+      const int row0_abs = m0s + qd * 32 + h * 16 - w.kv_tok0;   // query index of the warp's first row relative to the item's first key
       float m_a = -INFINITY, m_b = -INFINITY;   // exponent references currently baked into O and l
       float l_a = 0.f, l_b = 0.f;               // partial row sums over this thread's columns
       for (int j = 0; j < n; ++j, ++tile_cnt) {
         ok = warp_wait(smem_u32(&ctrl->s_full[s]), tile_cnt & 1);
-        if (!ok || *abort_flag) { ok = false; break; }
+        if (!ok) break;
         tc_fence_after();
-        // masking is needed only on the tile that holds the sequence end or the causal diagonal; `lim` is the last
-        // visible column of the tile for the row
-        int lim_a = len_k - 1 - j * kBN, lim_b = lim_a;
-        if (p.is_causal) { lim_a = min(lim_a, row_abs - j * kBN); lim_b = min(lim_b, row_abs + 8 - j * kBN); }
-        const bool masked = min(lim_a, lim_b) < kBN - 1;
-        if (masked) {
-          // The mask is written into the score tile itself (-inf over the hidden columns) before the two passes
-          // below, which then have one form for every tile: a masked copy of their bodies, run once per item from a
-          // cold instruction cache, cost more than this extra round trip through tensor memory.
-#pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
-            uint32_t v[32];
-            tmem_ld_16x256b_x8(tS + c * 64, v);
-            tmem_wait_ld();
-            const int ta = lim_a - c * 64 - 2 * q, tb = lim_b - c * 64 - 2 * q;
+        // Last visible column of the tile for the first and for the last of the warp's sixteen rows (the same for all rows
+        // without a causal mask): hidden columns exist only on the tile that holds the sequence end or the diagonal.
+        int lo = len_k - 1 - j * kBN, hi = lo;
+        if (p.is_causal) { lo = min(lo, row0_abs - j * kBN); hi = min(hi, row0_abs + 15 - j * kBN); }
+        uint64_t rs_a = pack_f2(0.f, 0.f), rs_b = pack_f2(0.f, 0.f);
+        const uint64_t sl2_2 = pack_f2(sl2, sl2);
+        uint64_t nega_2, negb_2;     // minus the exponent references of rows A and B
+        auto exp_pair = [&](uint32_t x0, uint32_t x1, uint64_t neg2, uint64_t& rs) -> uint32_t {
+          const uint64_t t2 = fma_f2(pack_f2(__uint_as_float(x0), __uint_as_float(x1)), sl2_2, neg2);
+          float a, b;
+          unpack_f2(t2, a, b);
+          const float p0 = fast_exp2(a), p1 = fast_exp2(b);
+          rs = add_f2(rs, pack_f2(p0, p1));
+          return ElemTraits<T>::pack2(p0, p1);
+        };
+        // 32 columns of both rows: exponentials, row sums, P as packed 16-bit in the 16x128b layout (the pair of columns
+        // 8 i + 2 q + {0, 1} is packed column 4 i + q)
+        auto exp_quarter = [&](const uint32_t (&v)[16], uint32_t* pq) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < 4; ++i) {
+            pq[2 * i] = exp_pair(v[4 * i], v[4 * i + 1], nega_2, rs_a);
+            pq[2 * i + 1] = exp_pair(v[4 * i + 2], v[4 * i + 3], negb_2, rs_b);
+          }
+        };
+        float sum_a, sum_b;     // row sums over this thread's columns
+        auto pair_sum = [](uint64_t v) {
+          float x, y;
+          unpack_f2(v, x, y);
+          return x + y;
+        };
+        // One pass where no row's exponent reference has to move, which is nearly every tile but an item's first: the
+        // scores are exponentiated, as they arrive, against the reference that stands, and the sums, needed anyhow, tell
+        // afterwards whether it could stand: no maximum is computed, no exponential waits for one, nothing is exchanged
+        // between threads, and the tile is read from tensor memory once.  P stays in registers until the verdict: if a row
+        // has to move, the scores are still there for the two passes below.
+        bool done = false;
+        if (j > 0 && lo >= kBN - 1) {
+          // (a row without a reference yet has -inf here: its sum is then no number and the verdict is no)
+          nega_2 = pack_f2(-m_a, -m_a);
+          negb_2 = pack_f2(-m_b, -m_b);
+          uint32_t pk[2][16];
+          uint32_t v0[16], v1[16];
+          tmem_ld_16x256b_x4(tS, v0);
+          tmem_wait_ld_regs(v0);
+          tmem_ld_16x256b_x4(tS + 32, v1);
+          exp_quarter(v0, pk[0]);
+          tmem_wait_ld_regs(v1);
+          tmem_ld_16x256b_x4(tS + 64, v0);
+          exp_quarter(v1, pk[0] + 8);
+          tmem_wait_ld_regs(v0);
+          tmem_ld_16x256b_x4(tS + 96, v1);
+          exp_quarter(v0, pk[1]);
+          tmem_wait_ld_regs(v1);
+          exp_quarter(v1, pk[1] + 8);
+          sum_a = pair_sum(rs_a);
+          sum_b = pair_sum(rs_b);
+          done = __all_sync(0xffffffffu, sum_a <= kMaxPartialSum && sum_b <= kMaxPartialSum);   // (false for NaN)
+          if (done) {
+            tmem_st_16x128b_x8(tS, pk[0]);
+            tmem_st_16x128b_x8(tS + ptx::kPHalfStride, pk[1]);
+          }
+        }
+        if (!done) {
+          // Two passes, 32 columns at a time: an item's first tile, a tile with hidden columns, a row whose reference moves.
+          // Columns hidden from all sixteen rows are neither read nor exponentiated.
+          auto mask_quarter = [&](uint32_t (&v)[16], int c) {
+            const int ta = min(len_k - 1, p.is_causal ? row0_abs + (lane >> 2) : 0x7fffffff) - j * kBN - c * 32 - 2 * q;
+            const int tb = min(len_k - 1, p.is_causal ? row0_abs + (lane >> 2) + 8 : 0x7fffffff) - j * kBN - c * 32 - 2 * q;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
 #pragma unroll
               for (int e = 0; e < 2; ++e) {
                 v[4 * i + e] = (8 * i + e > ta) ? 0xff800000u : v[4 * i + e];           // -inf
                 v[4 * i + 2 + e] = (8 * i + e > tb) ? 0xff800000u : v[4 * i + 2 + e];
               }
             }
-            tmem_st_16x256b_x8(tS + c * 64, v);
-          }
-          tmem_wait_st();
-        }
-        float mx_a, mx_b;
-        uint32_t v_hi[32];     // columns 64..127 of the tile stay in registers from pass 1 to pass 2
-        {
-          // pass 1: row maxima.  Columns 0..63 are read again in pass 2 (all 128 scores cannot be held across it).
-          uint32_t v[32];
-          tmem_ld_16x256b_x8(tS, v);
-          tmem_ld_16x256b_x8(tS + 64, v_hi);
-          tmem_wait_ld();
-          float a0 = fmaxf(__uint_as_float(v[0]), __uint_as_float(v[1]));
-          float b0 = fmaxf(__uint_as_float(v[2]), __uint_as_float(v[3]));
-#pragma unroll
-          for (int i = 1; i < 8; ++i) {
-            a0 = max3(a0, __uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]));
-            b0 = max3(b0, __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            a0 = max3(a0, __uint_as_float(v_hi[4 * i]), __uint_as_float(v_hi[4 * i + 1]));
-            b0 = max3(b0, __uint_as_float(v_hi[4 * i + 2]), __uint_as_float(v_hi[4 * i + 3]));
-          }
-          mx_a = quad_max(a0);
-          mx_b = quad_max(b0);
-        }
-        const float mn_a = fmaxf(m_a, mx_a * sl2), mn_b = fmaxf(m_b, mx_b * sl2);
-        const bool need_a = (mn_a - m_a) > kRescaleThreshold;   // false for NaN / (-inf)-(-inf)
-        const bool need_b = (mn_b - m_b) > kRescaleThreshold;
-        float alpha_a = 1.f, alpha_b = 1.f;
-        if (need_a) { alpha_a = fast_exp2(m_a - mn_a); m_a = mn_a; l_a *= alpha_a; }
-        if (need_b) { alpha_b = fast_exp2(m_b - mn_b); m_b = mn_b; l_b *= alpha_b; }
-        if (j > 0 && __any_sync(0xffffffffu, need_a || need_b)) {
-          // PV(j-1) has landed in O once S(j) is visible (the MMAs complete in issue order); waiting on its
-          // barrier phase is then immediate, and skipping the wait on other tiles is harmless because the
-          // barrier can never run two phases ahead of this warp
-          ok = warp_wait(smem_u32(&ctrl->o_done[s]), (tile_cnt - 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          // (rare: 16 columns at a time and not unrolled, so that the scores held in registers stay there)
+          };
+          float mx_a = -INFINITY, mx_b = -INFINITY;       // maxima over this thread's columns
+          rs_a = rs_b = pack_f2(0.f, 0.f);
 #pragma unroll 1
-          for (int c = 0; c < D / 16; ++c) {
-            uint32_t ov[8];
-            tmem_ld_16x256b_x2(tO + c * 16, ov);
-            tmem_wait_ld();
+          for (int c = 0; c < 4 && c * 32 <= hi; ++c) {
+            uint32_t v[16];
+            tmem_ld_16x256b_x4(tS + c * 32, v);
+            tmem_wait_ld_regs(v);
+            if (lo < c * 32 + 31) mask_quarter(v, c);
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              ov[4 * i] = __float_as_uint(__uint_as_float(ov[4 * i]) * alpha_a);
-              ov[4 * i + 1] = __float_as_uint(__uint_as_float(ov[4 * i + 1]) * alpha_a);
-              ov[4 * i + 2] = __float_as_uint(__uint_as_float(ov[4 * i + 2]) * alpha_b);
-              ov[4 * i + 3] = __float_as_uint(__uint_as_float(ov[4 * i + 3]) * alpha_b);
+            for (int i = 0; i < 4; ++i) {
+              mx_a = max3(mx_a, __uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]));
+              mx_b = max3(mx_b, __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
             }
-            tmem_st_16x256b_x2(tO + c * 16, ov);
           }
-        }
-        const float neg_a = (m_a == -INFINITY) ? 0.f : -m_a, neg_b = (m_b == -INFINITY) ? 0.f : -m_b;
-        uint64_t rs_a = pack_f2(0.f, 0.f), rs_b = pack_f2(0.f, 0.f);
-        const uint64_t sl2_2 = pack_f2(sl2, sl2), nega_2 = pack_f2(neg_a, neg_a), negb_2 = pack_f2(neg_b, neg_b);
-        auto exp_pair = [&](uint32_t x0, uint32_t x1, uint64_t neg2, uint64_t& rs, bool emulate) -> uint32_t {
-          const uint64_t t2 = fma_f2(pack_f2(__uint_as_float(x0), __uint_as_float(x1)), sl2_2, neg2);
-          float p0, p1;
-          if (emulate) {
-            // 2^t = 2^n * 2^r with n = round(t), r in [-0.5, 0.5]; n is read off the magic-number sum
-            float a, b;
-            unpack_f2(t2, a, b);
-            const uint64_t tc = pack_f2(fmaxf(a, -126.f), fmaxf(b, -126.f));
-            const uint64_t tm = add_f2(tc, pack_f2(12582912.f, 12582912.f));
-            const uint64_t nf = add_f2(tm, pack_f2(-12582912.f, -12582912.f));
-            const uint64_t r = fma_f2(nf, pack_f2(-1.f, -1.f), tc);
-            uint64_t pq = fma_f2(r, pack_f2(0.055171482f, 0.055171482f), pack_f2(0.2426109f, 0.2426109f));
-            pq = fma_f2(pq, r, pack_f2(0.69326097f, 0.69326097f));
-            pq = fma_f2(pq, r, pack_f2(0.99992812f, 0.99992812f));
-            float q0, q1, m0f, m1f;
-            unpack_f2(pq, q0, q1);
-            unpack_f2(tm, m0f, m1f);
-            p0 = __uint_as_float(__float_as_uint(q0) + (__float_as_uint(m0f) << 23));
-            p1 = __uint_as_float(__float_as_uint(q1) + (__float_as_uint(m1f) << 23));
-          } else {
-            float a, b;
-            unpack_f2(t2, a, b);
-            p0 = fast_exp2(a);
-            p1 = fast_exp2(b);
-          }
-          rs = add_f2(rs, pack_f2(p0, p1));
-          return ElemTraits<T>::pack2(p0, p1);
-        };
-        // pass 2, 64 columns at a time: exponentials, row sums, P as packed 16-bit in the 16x128b layout (the pair of
-        // columns 8 i + 2 q + {0, 1} of a half is packed column 4 i + q).  Each half of P goes over the first 32
-        // columns of its own half of S (kPHalfStride apart), so the upper half, still in registers, is done first
-        // and only the lower half is read from tensor memory a second time.
-        auto exp_half = [&](const uint32_t (&v)[32], uint32_t dst) {
-          uint32_t pk[16];
+          mx_a = quad_max(mx_a);
+          mx_b = quad_max(mx_b);
+          const float mn_a = fmaxf(m_a, mx_a * sl2), mn_b = fmaxf(m_b, mx_b * sl2);
+          const bool need_a = (mn_a - m_a) > kRescaleThreshold;   // false for NaN / (-inf)-(-inf)
+          const bool need_b = (mn_b - m_b) > kRescaleThreshold;
+          float alpha_a = 1.f, alpha_b = 1.f;
+          if (need_a) { alpha_a = fast_exp2(m_a - mn_a); m_a = mn_a; l_a *= alpha_a; }
+          if (need_b) { alpha_b = fast_exp2(m_b - mn_b); m_b = mn_b; l_b *= alpha_b; }
+          if (j > 0 && __any_sync(0xffffffffu, need_a || need_b)) {
+            // PV(j-1) has landed in O once S(j) is visible (the MMAs complete in issue order); waiting on its
+            // barrier phase is then immediate, and skipping the wait on other tiles is harmless because the
+            // barrier can never run two phases ahead of this warp
+            ok = warp_wait(smem_u32(&ctrl->o_done[s]), (tile_cnt - 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 0; c < D / 16; ++c) {
+              uint32_t ov[8];
+              tmem_ld_16x256b_x2(tO + c * 16, ov);
+              tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const bool emu = (i & 3) < kExpEmuOf4;
-            pk[2 * i] = exp_pair(v[4 * i], v[4 * i + 1], nega_2, rs_a, emu);
-            pk[2 * i + 1] = exp_pair(v[4 * i + 2], v[4 * i + 3], negb_2, rs_b, emu);
+              for (int i = 0; i < 2; ++i) {
+                ov[4 * i] = __float_as_uint(__uint_as_float(ov[4 * i]) * alpha_a);
+                ov[4 * i + 1] = __float_as_uint(__uint_as_float(ov[4 * i + 1]) * alpha_a);
+                ov[4 * i + 2] = __float_as_uint(__uint_as_float(ov[4 * i + 2]) * alpha_b);
+                ov[4 * i + 3] = __float_as_uint(__uint_as_float(ov[4 * i + 3]) * alpha_b);
+              }
+              tmem_st_16x256b_x2(tO + c * 16, ov);
+            }
           }
-          tmem_st_16x128b_x8(dst, pk);
-        };
-        exp_half(v_hi, tS + ptx::kPHalfStride);
-        {
-          uint32_t v[32];
-          tmem_ld_16x256b_x8(tS, v);
-          tmem_wait_ld();
-          exp_half(v, tS);
+          const float neg_a = (m_a == -INFINITY) ? 0.f : -m_a, neg_b = (m_b == -INFINITY) ? 0.f : -m_b;
+          nega_2 = pack_f2(neg_a, neg_a);
+          negb_2 = pack_f2(neg_b, neg_b);
+          // P of a quarter goes over scores that have been read: quarters 0 and 1 over the first 32 columns, 2 and 3 over
+          // the first 32 of the upper half
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t pq[8];
+            if (c * 32 <= hi) {
+              uint32_t v[16];
+              tmem_ld_16x256b_x4(tS + c * 32, v);
+              tmem_wait_ld_regs(v);
+              if (lo < c * 32 + 31) mask_quarter(v, c);
+              exp_quarter(v, pq);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) pq[i] = 0u;
+            }
+            tmem_st_16x128b_x4(tS + (c >> 1) * ptx::kPHalfStride + (c & 1) * 16, pq);
+          }
+          sum_a = pair_sum(rs_a);
+          sum_b = pair_sum(rs_b);
         }
-        {
-          float r0, r1;
-          unpack_f2(rs_a, r0, r1);
-          l_a += r0 + r1;
-          unpack_f2(rs_b, r0, r1);
-          l_b += r0 + r1;
-        }
+        l_a += sum_a;
+        l_b += sum_b;
         tmem_wait_st();
-        if (pend) {
-          // first tile of an item: the previous item's O must leave tensor memory before this tile's PV
-          ok = flush(true);
-          if (!ok) break;
-        } else {
-          tc_fence_before();
-          mbar_arrive(smem_u32(&ctrl->p_ready[s]));
-        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ctrl->p_ready[s]));
       }
       if (!ok) break;
-      // ---------------- the item's epilogue becomes pending ----------------
+      // ---------------- the item's epilogue ----------------
       const int len_q = w.len_q;
       const bool slot_live = w.valid && m0s < len_q;
       const long long qrow0 = w.out_row0[s];
       const int qhead = w.q_head[s];
-      pend = true;
-      pend_acc = n > 0;
-      pend_phase = (tile_cnt - 1) & 1;
-      pend_rows = slot_live ? min(kBM, len_q - m0s) : 0;
-      pend_la = quad_sum(l_a);
-      pend_lb = quad_sum(l_b);
+      out_acc = n > 0;
+      out_phase = (tile_cnt - 1) & 1;
+      out_rows = slot_live ? min(kBM, len_q - m0s) : 0;
+      out_la = quad_sum(l_a);
+      out_lb = quad_sum(l_b);
       if (p.lse != nullptr && q == 0) {
         // split KV range: the merge needs every row's log-sum-exp (log2 domain; -inf for a row that saw no key)
         float* lse = p.lse + qrow0 + m0s + rowA;
-        if (rowA < (slot_live ? min(kBM, len_q - m0s) : 0)) lse[0] = pend_la > 0.f ? m_a + log2f(pend_la) : -INFINITY;
-        if (rowA + 8 < (slot_live ? min(kBM, len_q - m0s) : 0)) lse[8] = pend_lb > 0.f ? m_b + log2f(pend_lb) : -INFINITY;
+        if (rowA < (slot_live ? min(kBM, len_q - m0s) : 0)) lse[0] = out_la > 0.f ? m_a + log2f(out_la) : -INFINITY;
+        if (rowA + 8 < (slot_live ? min(kBM, len_q - m0s) : 0)) lse[8] = out_lb > 0.f ? m_b + log2f(out_lb) : -INFINITY;
       }
       if (p.layout == B200ATTN_RAGGED) {
-        pend_stride = static_cast<long long>(p.q_heads) * D;
-        pend_off = ((qrow0 + m0s + rowA) * p.q_heads + qhead) * D;
+        out_stride = static_cast<long long>(p.q_heads) * D;
+        out_off = ((qrow0 + m0s + rowA) * p.q_heads + qhead) * D;
       } else {
-        pend_stride = D;
-        pend_off = (qrow0 + m0s + rowA) * D;
+        out_stride = D;
+        out_off = (qrow0 + m0s + rowA) * D;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));
+      ok = write_out();
     }
-    if (ok && pend) ok = flush(false);
     if (!ok && lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
   }
 
