@@ -737,24 +737,34 @@ struct PageAhead {
     if (bad) p.header[0] = DEV_ERR_PAGE_RANGE;
     return (bad ? 0 : page) * p.page_size + off;
   }
-  // rows of the lane's box of tile number `tile` of the item (called for every tile, in order); returns the boxes that
+  // entries for tile number `tile` of the item become current (called for every tile, in order); returns the boxes that
   // the tile has
-  __device__ __forceinline__ int tile_rows(const DecodeParams& p, int tile, int& kr, int& vr) {
-    const int at = (tile * boxes) & 31;
-    if (at == 0 && tile > 0) {
+  __device__ __forceinline__ int advance(const DecodeParams& p, int tile) {
+    if (((tile * boxes) & 31) == 0 && tile > 0) {
       kp = kp_next;
       vp = vp_next;
       read(tile * boxes + 32, kp_next, vp_next);
     }
+    const int t0 = t_begin + tile * kTileN;
+    return p.num_pages > 0 ? min(boxes, (t_end - t0 + (1 << box_shift) - 1) >> box_shift) : 0;
+  }
+  // rows of the lane's box of that tile, for K and for V
+  __device__ __forceinline__ int tile_rows(const DecodeParams& p, int tile, int& kr, int& vr) {
+    const int n = advance(p, tile), at = (tile * boxes) & 31;
     const int k = __shfl_sync(0xffffffffu, kp, (at + lane) & 31), v = __shfl_sync(0xffffffffu, vp, (at + lane) & 31);
     const int t0 = t_begin + tile * kTileN;
-    const int n = p.num_pages > 0 ? min(boxes, (t_end - t0 + (1 << box_shift) - 1) >> box_shift) : 0;
     kr = vr = -1;
     if (lane < n) {
       kr = row(p, k, t0 + (lane << box_shift));
       vr = row(p, v, t0 + (lane << box_shift));
     }
     return n;
+  }
+  // row of any box of that tile (of the first `n`), of K (op 0) or of V; -1 beyond
+  __device__ __forceinline__ int box_row(const DecodeParams& p, int tile, int n, int box, int op) const {
+    const int at = (tile * boxes) & 31;
+    const int k = __shfl_sync(0xffffffffu, kp, (at + box) & 31), v = __shfl_sync(0xffffffffu, vp, (at + box) & 31);
+    return box < n && op < 2 ? row(p, op ? v : k, t_begin + tile * kTileN + (box << box_shift)) : -1;
   }
 };
 
@@ -1101,10 +1111,15 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
 // re-read by ldmatrix once per 16-row tile.  Here the rows are padded to one 128-row tcgen05 tile whose A operands
 // live in tensor memory (Q is written there once per work unit, P once per key tile), so shared memory is read
 // exactly once per K/V byte, by the tensor core.  Per 64-key tile: S = Q K^T (TS MMA, 128 x 64 x D) -> the softmax
-// warps (thread = q row, only the warps that hold real rows work) read S from TMEM, mask, keep the running max / sum
-// in the exp2 domain with the lazy 2^8 rescale, write P as packed 16-bit over S -> O += P V (TS MMA, V is the
-// MN-major B operand).  Two CTAs share an SM (256 TMEM columns, 3 stages of 64 keys each), which overlaps one CTA's
-// softmax with the other's MMAs.
+// warps (thread = q row, only the warps that hold real rows work) exponentiate S against the row's standing reference,
+// keep the row sums, write P as packed 16-bit over S -> O += P V (TS MMA, V is the MN-major B operand).  Two CTAs share
+// an SM (256 TMEM columns, 3 stages of 64 keys each), which overlaps one CTA's softmax with the other's MMAs.
+//
+// What bounds it.  A tile is a chain: scores seen 270 cycles after the issue, 830 of softmax, 550 of MMAs; and a stage is
+// away for 360 (freed and noticed) + 600 to 1 200 (its copies issued by three warps) + 2 200 (under load).  Long batches run
+// at the board's power limit on top of that (32 sequences of 1 000 to 33 000 keys: 1.37 GHz).  Against one issuing warp, a
+// pass for the maximum, and stages given back only when the next had arrived: 8 x 8 192 keys of one head, D 64, 28.5 -> 25.1
+// us; 4 x 8 192, D 128, 50.6 -> 48.2; 16 x 16 384 and 128 rows 75 -> 68; one sequence of 8 192 in pages 43.5 -> 40.2.
 //
 // The kernel is persistent: the grid is one wave (two CTAs per SM); a CTA starts with unit (item, kv head) number
 // blockIdx.x of the planner's longest-first list and its producer warp draws further units from a counter in the
@@ -1117,6 +1132,13 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
 // ---------------------------------------------------------------------------
 constexpr int kUmmaStages = 3;
 constexpr int kUmmaTmemCols = 256;
+// A tile's 64 exponentials of a row against the reference that stands are good as long as their sum is at most this (P then
+// fits 16 bits); when it is not, the row's maximum lies four powers of two or more above its reference, and a reference
+// moves when the maximum is kMoveThreshold above it.
+constexpr float kMaxRowSum = 1024.0f;
+constexpr float kMoveThreshold = 3.0f;   // log2 units
+constexpr int kUmmaThreads = 256;     // four softmax warps, three that issue copies, the MMA warp
+constexpr int kUmmaIssuers = 3;       // warps that share the copies of a stage
 constexpr int kUmmaUnitRing = 4;      // units the producer may be ahead of the slowest consumer
 constexpr int kUmmaMaxClaims = 1;     // merges a CTA takes per sweep of the ticket counters in its teardown
 constexpr int kMergeClaimed = 1 << 30; // added to a pair's ticket counter by the CTA that merges it
@@ -1167,7 +1189,7 @@ __device__ __forceinline__ UmmaUnit umma_unit(const DecodeParams& p, int u) {
 // T: element type of q, k, v as the kernel reads them; OutT: element type of the output rows (T, or float when the
 // inputs are fp16 copies of fp32 tensors).
 template <typename T, int D, typename OutT = T>
-__global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_constant__ CUtensorMap tm_k,
+__global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __grid_constant__ CUtensorMap tm_k,
                                                              const __grid_constant__ CUtensorMap tm_v,
                                                              const DecodeParams p) {
   using namespace ptx;
@@ -1180,28 +1202,38 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
   constexpr int kSCol = kQCols;               // S (64 fp32 columns); P overwrites its first 32
   constexpr int kOCol = kQCols + kTileN;      // O (D fp32 columns)
   static_assert(kOCol + D <= kUmmaTmemCols, "TMEM budget");
-  constexpr int kProducer = 4, kMma = 5;
+  // (with up to 64 rows only the first two softmax warps work: the producer and the MMA warp are not among their neighbours
+  // in the SM's four partitions)
+  constexpr int kHelper = 4, kProducer = 6, kMma = 7;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int R = p.rows;
   const int active_warps = (R + 31) >> 5;      // softmax warps that own real rows
   const int n_softmax = active_warps * 32;
+  // A warp issues a box every 95 to 130 cycles, whatever the box's size, and different warps do not hold one another up: the
+  // sixteen boxes of a stage of 16-key pages took one warp 1 580 of the 2 540 cycles that a CTA had for a tile.  (Pages that
+  // are cut into more boxes than a warp has lanes are left to the producer.)
+  const int boxes_log2 = p.layout == B200ATTN_PAGED ? 6 - p.box_shift : 0;
+  const bool shared_issue = boxes_log2 <= 5;
 
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   UmmaCtrl* ctrl = reinterpret_cast<UmmaCtrl*>(smem + kUmmaStages * STAGE_BYTES);
   const uint32_t smem_base = smem_u32(smem);
 
   if (tid == 0) {
-    for (int i = 0; i < kUmmaStages; ++i) { mbar_init(smem_u32(&ctrl->full[i]), 1); mbar_init(smem_u32(&ctrl->empty[i]), 1); }
+    for (int i = 0; i < kUmmaStages; ++i) {
+      mbar_init(smem_u32(&ctrl->full[i]), shared_issue ? kUmmaIssuers : 1);
+      mbar_init(smem_u32(&ctrl->empty[i]), 1);
+    }
     mbar_init(smem_u32(&ctrl->q_ready), n_softmax);
     mbar_init(smem_u32(&ctrl->s_full), 1);
-    mbar_init(smem_u32(&ctrl->p_ready), n_softmax);
+    mbar_init(smem_u32(&ctrl->p_ready), active_warps);
     mbar_init(smem_u32(&ctrl->o_done), 1);
     mbar_init(smem_u32(&ctrl->o_free), n_softmax);
     mbar_init(smem_u32(&ctrl->rows_out), n_softmax);
     for (int i = 0; i < kUmmaUnitRing; ++i) {
       mbar_init(smem_u32(&ctrl->unit_full[i]), 1);
-      mbar_init(smem_u32(&ctrl->unit_empty[i]), 1 + active_warps);
+      mbar_init(smem_u32(&ctrl->unit_empty[i]), 1 + active_warps + (shared_issue ? kUmmaIssuers - 1 : 0));
     }
     ctrl->published = 0;
     ctrl->abort_flag = 0;
@@ -1237,12 +1269,42 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
     if (lane == 0) mbar_arrive(smem_u32(&ctrl->unit_empty[r % kUmmaUnitRing]));
   };
 
+  // Issuing warp `part`'s share of a stage: every kUmmaIssuers-th (box, operand, column block) of the tile.
+  auto issue_share = [&](const UmmaUnit& w, PageAhead& ahead, int tile, int stage, int part) {
+    const bool paged = p.layout == B200ATTN_PAGED;
+    const int t0 = w.t_begin + tile * kTileN;
+    const int boxes = 1 << boxes_log2, total = 2 * CHUNKS << boxes_log2;
+    const uint32_t box_bytes = static_cast<uint32_t>(kTileN >> boxes_log2) * 128;
+    const uint32_t bar = smem_u32(&ctrl->full[stage]);
+    const int n = paged ? ahead.advance(p, tile) : 1;
+    int h_coord = w.h;
+    long long row0 = w.seq_start;
+    if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(w.b) * p.kv_heads + w.h) * p.max_kv; }
+    // boxes of the share in this tile: the indices part, part + kUmmaIssuers, ... whose box is one of the first n
+    int count = 0;
+    for (int base = 0; base < total; base += 32 * kUmmaIssuers) {
+      const int idx = base + lane * kUmmaIssuers + part;
+      count += __popc(__ballot_sync(0xffffffffu, idx < total && (idx & (boxes - 1)) < n));
+    }
+    if (lane == 0) {
+      if (count > 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(count) * box_bytes);
+      else mbar_arrive(bar);
+    }
+    __syncwarp();
+    for (int base = 0; base < total; base += 32 * kUmmaIssuers) {
+      const int idx = base + lane * kUmmaIssuers + part;
+      const int box = idx & (boxes - 1), rest = idx >> boxes_log2, op = rest & 1, cc = rest >> 1;
+      const int row = paged ? ahead.box_row(p, tile, n, box, idx < total ? op : 2) : (idx < total ? static_cast<int>(row0 + t0) : -1);
+      const uint32_t dst = smem_base + stage * STAGE_BYTES + op * TILE_BYTES + cc * CHUNK_BYTES + box * box_bytes;
+      if (row >= 0) tma_load_3d(dst, op ? &tm_v : &tm_k, bar, cc * 64, h_coord, row);
+    }
+  };
+
   if (warp == kProducer) {
     // =========================== TMA producer ===========================
     if (lane == 0) { prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); }
     bool ok = true;
     int g = 0;                                   // tiles issued so far, over all units
-    const int box_rows = 1 << p.box_shift;
     PageAhead ahead(p, lane);                    // (a unit's first entries are read when it is drawn)
     auto publish = [&](int r, int u) {            // lane 0
       ctrl->unit_ring[r % kUmmaUnitRing] = u;
@@ -1266,41 +1328,21 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
     for (int r = 0; ok && u < n_units; ++r) {
       const UmmaUnit w = umma_unit(p, u);
       if (r == 0) ahead.start(p, w.b, w.t_begin, w.t_end);
-      int h_coord = w.h;
-      long long row0 = w.seq_start;
-      if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(w.b) * p.kv_heads + w.h) * p.max_kv; }
       for (int tile = 0; tile < w.ntiles; ++tile) {
         const int stage = g % kUmmaStages, use = g / kUmmaStages;
         if (use > 0) {
           ok = warp_wait(smem_u32(&ctrl->empty[stage]), (use - 1) & 1);
           if (!ok || *abort_flag) { ok = false; break; }
         }
-        const int t0 = w.t_begin + tile * kTileN;
-        const uint32_t kdst = smem_base + stage * STAGE_BYTES;
-        const uint32_t vdst = kdst + TILE_BYTES;
-        const uint32_t bar = smem_u32(&ctrl->full[stage]);
-        if (p.layout != B200ATTN_PAGED) {
-          if (lane == 0) {
-            mbar_arrive_expect_tx(bar, STAGE_BYTES);
-            const int row = static_cast<int>(row0 + t0);
-#pragma unroll
-            for (int cc = 0; cc < CHUNKS; ++cc) {
-              tma_load_3d(kdst + cc * CHUNK_BYTES, &tm_k, bar, cc * 64, h_coord, row);
-              tma_load_3d(vdst + cc * CHUNK_BYTES, &tm_v, bar, cc * 64, h_coord, row);
-            }
-          }
-        } else if (ahead.on) {
-          int kr, vr;
-          const int count = ahead.tile_rows(p, tile, kr, vr);
-          if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(2 * count) * box_rows * 128 * CHUNKS);
-          __syncwarp();
-          const uint32_t roff = static_cast<uint32_t>(lane) * box_rows * 128;
-#pragma unroll
-          for (int cc = 0; cc < CHUNKS; ++cc) {
-            if (kr >= 0) tma_load_3d(kdst + cc * CHUNK_BYTES + roff, &tm_k, bar, cc * 64, h_coord, kr);
-            if (vr >= 0) tma_load_3d(vdst + cc * CHUNK_BYTES + roff, &tm_v, bar, cc * 64, h_coord, vr);
-          }
+        if (shared_issue) {
+          issue_share(w, ahead, tile, stage, 0);
         } else {
+          const int t0 = w.t_begin + tile * kTileN;
+          const uint32_t kdst = smem_base + stage * STAGE_BYTES;
+          const uint32_t vdst = kdst + TILE_BYTES;
+          const uint32_t bar = smem_u32(&ctrl->full[stage]);
+          const int box_rows = 1 << p.box_shift;
+          const int h_coord = w.h;
           const int boxes = kTileN >> p.box_shift;
           const int* ktab = p.k_table + static_cast<long long>(w.b) * p.table_stride;
           const int* vtab = p.v_table + static_cast<long long>(w.b) * p.table_stride;
@@ -1370,6 +1412,34 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
       for (int t = max(0, g - kUmmaStages); t < g; ++t)
         mbar_wait(smem_u32(&ctrl->full[t % kUmmaStages]), (t / kUmmaStages) & 1);
     }
+  } else if (warp >= kHelper && warp < kHelper + kUmmaIssuers - 1) {
+    // =========================== further issuing warps ===========================
+    if (shared_issue) {
+      bool ok = true;
+      int g = 0;
+      PageAhead ahead(p, lane);
+      for (int r = 0; ok; ++r) {
+        const int u = unit_at(r);
+        if (u < 0) { ok = false; break; }
+        unit_done(r);
+        if (u >= n_units) break;
+        const UmmaUnit w = umma_unit(p, u);
+        ahead.start(p, w.b, w.t_begin, w.t_end);
+        for (int tile = 0; tile < w.ntiles; ++tile, ++g) {
+          const int stage = g % kUmmaStages, use = g / kUmmaStages;
+          if (use > 0) {
+            ok = warp_wait(smem_u32(&ctrl->empty[stage]), (use - 1) & 1);
+            if (!ok || *abort_flag) { ok = false; break; }
+          }
+          issue_share(w, ahead, tile, stage, 1 + warp - kHelper);
+        }
+      }
+      if (!ok) {
+        if (lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
+        for (int t = max(0, g - kUmmaStages); t < g; ++t)
+          mbar_wait(smem_u32(&ctrl->full[t % kUmmaStages]), (t / kUmmaStages) & 1);
+      }
+    }
   } else if (warp == kMma) {
     // =========================== MMA issuer ===========================
     constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
@@ -1408,12 +1478,8 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
       issue_s(g);
       for (int tile = 0; tile < w.ntiles && ok; ++tile, ++g) {
         const int stage = g % kUmmaStages;
-        // what does not depend on the softmax warps comes before the wait for their P: the next K tile (loaded long
-        // ago in steady state), the zero fill of V rows past the end, the operand descriptor
-        if (tile + 1 < w.ntiles) {
-          ok = warp_wait(smem_u32(&ctrl->full[(g + 1) % kUmmaStages]), ((g + 1) / kUmmaStages) & 1);
-          if (!ok) break;
-        }
+        // what does not depend on the softmax warps comes before the wait for their P: the zero fill of V rows past the
+        // end, the operand descriptors
         const int valid = w.len - (w.t_begin + tile * kTileN);
         if (valid < kTileN) {
           // keys past the sequence end carry P == 0 but their V rows may hold anything: zero them so 0 * x stays 0
@@ -1439,9 +1505,15 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
         tc_fence_after();
         mma_ts_batch4(tmem + kOCol, tmem + kSCol, vb, idesc_o, tile > 0 ? 1u : 0u, lead);
         mma_commit_lead(smem_u32(&ctrl->o_done), lead);
-        if (tile + 1 < w.ntiles) issue_s(g + 1);
-        // K_tile was read by S(tile) (complete: its P has come back) and V_tile by the PV just issued
+        // K_tile was read by S(tile) (complete: its P has come back) and V_tile by the PV just issued: the stage goes back
+        // to the issuing warps before this warp waits for the next one
         mma_commit_lead(smem_u32(&ctrl->empty[stage]), lead);
+        if (tile + 1 < w.ntiles) {
+          ok = warp_wait(smem_u32(&ctrl->full[(g + 1) % kUmmaStages]), ((g + 1) / kUmmaStages) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          issue_s(g + 1);
+        }
       }
       if (ok) unit_done(r);
     }
@@ -1506,66 +1578,110 @@ __global__ void __launch_bounds__(192, 2) decode_umma_kernel(const __grid_consta
       float m_used = -INFINITY, l_run = 0.f;               // per-row softmax state
       int lim = w.len - 1;                                 // last visible key of this row
       if (p.causal) lim = w.len - p.q_len + (row % p.q_len);
+      const int first_lim = p.causal ? w.len - p.q_len : w.len - 1;      // the smallest of all rows
       for (int tile = 0; tile < w.ntiles; ++tile, ++g) {
         ok = warp_wait(smem_u32(&ctrl->s_full), g & 1);
-        if (!ok || *abort_flag) { ok = false; break; }
+        if (!ok) break;
         tc_fence_after();
-        const int limit = lim - (w.t_begin + tile * kTileN);   // columns 0..limit of this tile are visible
-        uint32_t ca[32], cb[32];
-        tmem_ld32(tS, ca);
-        tmem_ld32(tS + 32, cb);
-        tmem_wait_ld();
-        if (limit < kTileN - 1) {
+        const int t0 = w.t_begin + tile * kTileN;
+        const int limit = lim - t0;             // columns 0..limit of this tile are visible
+        uint64_t rs;
+        float neg_m;
+        // 16 columns: exponentials, their sum, P as packed 16-bit
+        auto exp_part = [&](const uint32_t (&v)[16], uint32_t* pq) {
+          const uint64_t sl2_2 = pack_f2(sl2, sl2), neg_2 = pack_f2(neg_m, neg_m);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (i > limit) ca[i] = 0xff800000u;          // -inf
-            if (32 + i > limit) cb[i] = 0xff800000u;
+          for (int i = 0; i < 8; ++i) {
+            float a, b;
+            unpack_f2(fma_f2(pack_f2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sl2_2, neg_2), a, b);
+            a = fast_exp2(a);
+            b = fast_exp2(b);
+            rs = add_f2(rs, pack_f2(a, b));
+            pq[i] = ElemTraits<T>::pack2(a, b);
           }
+        };
+        auto row_sum = [&]() {
+          float a, b;
+          unpack_f2(rs, a, b);
+          return a + b;
+        };
+        float sum;
+        bool done = false;
+        // One pass where no row's exponent reference has to move, which is nearly every tile but a unit's first: against the
+        // reference that stands, with the sum to tell whether it could (see kMaxRowSum); P stays in registers until then.
+        if (tile > 0 && first_lim - t0 >= kTileN - 1) {
+          uint32_t va[16], vb[16], pk[32];
+          rs = pack_f2(0.f, 0.f);
+          neg_m = -m_used;             // (+inf for a row without a reference yet: the sum is then no number)
+          tmem_ld16(tS, va);
+          tmem_wait_ld_regs(va);
+          tmem_ld16(tS + 16, vb);
+          exp_part(va, pk);
+          tmem_wait_ld_regs(vb);
+          tmem_ld16(tS + 32, va);
+          exp_part(vb, pk + 8);
+          tmem_wait_ld_regs(va);
+          tmem_ld16(tS + 48, vb);
+          exp_part(va, pk + 16);
+          tmem_wait_ld_regs(vb);
+          exp_part(vb, pk + 24);
+          sum = row_sum();
+          done = __all_sync(0xffffffffu, sum <= kMaxRowSum);
+          if (done) tmem_st32(tS, pk);
         }
-        float ma = max3(__uint_as_float(ca[0]), __uint_as_float(ca[1]), __uint_as_float(ca[2]));
-        float mb = max3(__uint_as_float(cb[0]), __uint_as_float(cb[1]), __uint_as_float(cb[2]));
+        if (!done) {
+          // two passes, 16 columns at a time: a unit's first tile, hidden columns, a reference that moves
+          auto load_part = [&](uint32_t (&v)[16], int c) {
+            tmem_ld16(tS + c * 16, v);
+            tmem_wait_ld_regs(v);
 #pragma unroll
-        for (int i = 3; i + 1 < 32; i += 2) {
-          ma = max3(ma, __uint_as_float(ca[i]), __uint_as_float(ca[i + 1]));
-          mb = max3(mb, __uint_as_float(cb[i]), __uint_as_float(cb[i + 1]));
-        }
-        const float mx = max3(ma, mb, fmaxf(__uint_as_float(ca[31]), __uint_as_float(cb[31]))) * sl2;
-        const bool need = (mx - m_used) > 8.f;
-        float alpha = 1.f;
-        if (need) { alpha = fast_exp2(m_used - mx); m_used = mx; l_run *= alpha; }
-        if (tile > 0 && __any_sync(0xffffffffu, need)) {
-          // PV(tile-1) has completed once S(tile) is visible (MMAs complete in issue order); the wait is immediate
-          ok = warp_wait(smem_u32(&ctrl->o_done), (g - 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
+            for (int i = 0; i < 16; ++i)
+              if (c * 16 + i > limit) v[i] = 0xff800000u;          // -inf
+          };
+          float mx = -INFINITY;
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t v[16];
+            load_part(v, c);
 #pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc) {
-            uint32_t ov[32];
-            tmem_ld32(tO + cc * 32, ov);
-            tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-            tmem_st32(tO + cc * 32, ov);
+            for (int i = 0; i < 16; i += 2) mx = max3(mx, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
           }
-        }
-        const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
-        float rs = 0.f;
-        uint32_t pk[32];
+          mx *= sl2;
+          const bool need = (mx - m_used) > kMoveThreshold;
+          float alpha = 1.f;
+          if (need) { alpha = fast_exp2(m_used - mx); m_used = mx; l_run *= alpha; }
+          if (tile > 0 && __any_sync(0xffffffffu, need)) {
+            // PV(tile-1) has completed once S(tile) is visible (MMAs complete in issue order); the wait is immediate
+            ok = warp_wait(smem_u32(&ctrl->o_done), (g - 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int cc = 0; cc < D / 16; ++cc) {
+              uint32_t ov[16];
+              tmem_ld16(tO + cc * 16, ov);
+              tmem_wait_ld_regs(ov);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(ca[2 * i]), sl2, neg_m));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(ca[2 * i + 1]), sl2, neg_m));
-          const float p2 = fast_exp2(fmaf(__uint_as_float(cb[2 * i]), sl2, neg_m));
-          const float p3 = fast_exp2(fmaf(__uint_as_float(cb[2 * i + 1]), sl2, neg_m));
-          rs += (p0 + p1) + (p2 + p3);
-          pk[i] = ElemTraits<T>::pack2(p0, p1);
-          pk[16 + i] = ElemTraits<T>::pack2(p2, p3);
+              for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
+              tmem_st16(tO + cc * 16, ov);
+            }
+          }
+          neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+          rs = pack_f2(0.f, 0.f);
+          // (P of a part lies over scores that have been read)
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t v[16], pq[8];
+            load_part(v, c);
+            exp_part(v, pq);
+            tmem_st8(tS + c * 8, pq);
+          }
+          sum = row_sum();
         }
-        l_run += rs;
-        tmem_st32(tS, pk);
+        l_run += sum;
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(smem_u32(&ctrl->p_ready));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ctrl->p_ready));
       }
       if (!ok) break;
       // the next unit (published by the producer when it issued this unit's last copy, its Q rows already on their
@@ -2159,7 +2275,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     do {                                                                 \
       rc = set_smem(decode_umma_kernel<TYPE, DIM, OUT>, smem);           \
       if (rc) return rc;                                                 \
-      launch_dependent(decode_umma_kernel<TYPE, DIM, OUT>, grid, 192, smem, stream, 1, tk, tv, p); \
+      launch_dependent(decode_umma_kernel<TYPE, DIM, OUT>, grid, kUmmaThreads, smem, stream, 1, tk, tv, p); \
     } while (0)
     if (f32_out) {
       if (D == 128) B200ATTN_LAUNCH_UMMA(__half, 128, float); else B200ATTN_LAUNCH_UMMA(__half, 64, float);
