@@ -24,6 +24,9 @@
 //       and takes a ticket.  In the one-CTA-per-unit kernels (emit_and_merge) the CTA that draws the last ticket of
 //       its (sequence, kv head) performs the log-sum-exp merge; in the persistent kernel a CTA that has run out of
 //       units claims complete pairs and merges them.  No CTA ever waits for another.
+//   Calls that are all latency (short sequences, cluster_size) skip planner, partials and tickets: a cluster of up to eight
+//       CTAs of the warp-level or the fp32 kernel shares a (sequence, kv head) pair and merges through distributed shared
+//       memory; there, and only there, a CTA waits (with a limit) for the others of its cluster.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -71,6 +74,12 @@ __device__ __forceinline__ SeqInfo seq_info(const DecodeParams& p, int b) {
   }
   return s;
 }
+
+struct DecodeItem {
+  long long start;            // ragged: first row of the sequence
+  int b, c, n_chunks, item0;  // sequence, chunk, chunks of the sequence, item number of its first chunk
+  int len, t_begin, t_end;    // keys of the sequence, the item's keys
+};
 
 // Fills `rows` combined rows with NaN accumulators and (m, l) = (0, 1); every thread of the CTA takes part.
 __device__ __forceinline__ void poison_rows(float* comb_o, float* comb_ml, int rows, int d) {
@@ -227,6 +236,124 @@ __device__ __forceinline__ void emit_and_merge(const DecodeParams& p, int b, int
   __syncthreads();
   if (*s_ticket != n_chunks - 1) return;
   merge_chunks<T, D>(p, b, h, n_chunks, item0, out, threadIdx.x, blockDim.x);
+}
+
+// ---------------------------------------------------------------------------
+// Short sequences: no plan, no partials in global memory, no tickets.
+//
+// The CTAs of a cluster cut a (sequence, kv head) pair's keys into equal parts of whole tiles, and every output element
+// has an owner among them: each CTA sends its partial of the element, and the (m, l) of its row, into the owner's shared
+// memory by asynchronous stores that count on the owner's mbarrier, and the owner merges and writes.  In a planned call of
+// 12 us (16 sequences of 2 048 keys, two KV heads, D 64) planning took 3.3 us, publishing a partial and drawing its ticket
+// 1.5, and the merge by the CTA that drew the last one 3.3: 12.8 -> 8.0 us a call.
+// ---------------------------------------------------------------------------
+struct ClusterPart {
+  int rank, size;        // of this CTA in its cluster, of the cluster
+  int total, share;      // 16-byte pieces of the pair's output rows in fp32, pieces of a CTA's share
+};
+
+template <int D>
+__device__ __forceinline__ ClusterPart cluster_part(const DecodeParams& p) {
+  ClusterPart c;
+  c.size = p.cluster;
+  c.rank = static_cast<int>(blockIdx.x) % c.size;
+  c.total = p.rows * (D / 4);
+  c.share = (c.total + c.size - 1) / c.size;
+  return c;
+}
+
+// Before anything else: the receiving barrier, armed with the bytes that will be sent to this CTA.  The second half of the
+// cluster barrier (cluster_emit) tells that every CTA has got this far.
+template <int D>
+__device__ __forceinline__ void cluster_begin(const DecodeParams& p, const ClusterPart& c, uint64_t* bar) {
+  if (threadIdx.x == 0) {
+    const int first = c.rank * c.share, n = min(c.share, c.total - first);
+    ptx::mbar_init(smem_u32(bar), 1);
+    ptx::mbar_fence_init();
+    if (n > 0) {
+      const int rows = (first + n - 1) / (D / 4) - first / (D / 4) + 1;
+      ptx::mbar_arrive_expect_tx(smem_u32(bar), static_cast<uint32_t>(c.size * (n * 16 + rows * 8)));
+    }
+  }
+  __syncwarp();
+  ptx::cluster_arrive();
+}
+
+// The keys of sequence b that are this CTA's.
+__device__ __forceinline__ void cluster_item(const DecodeParams& p, const ClusterPart& c, int b, DecodeItem& it) {
+  const SeqInfo si = seq_info(p, b);
+  const int tiles = (si.len + kTileN - 1) / kTileN, per = ((tiles + c.size - 1) / c.size) * kTileN;
+  it.start = si.start;
+  it.b = b;
+  it.c = c.rank;
+  it.n_chunks = 1;
+  it.item0 = 0;
+  it.len = si.len;
+  it.t_begin = min(si.len, c.rank * per);
+  it.t_end = min(si.len, it.t_begin + per);
+}
+
+// `recv`: shared memory for the pieces ([CTA][share] of 16 bytes) and the rows' (m, l) ([CTA][row]) sent to this CTA.
+template <typename T, int D>
+__device__ __forceinline__ void cluster_emit(const DecodeParams& p, const ClusterPart& cp, int b, int h, const float* comb_o,
+                                             const float* comb_ml, int KS, int rows_pad, unsigned char* recv, uint64_t* bar) {
+  constexpr int D4 = D / 4;
+  const int R = p.rows;
+  const uint32_t bar_s = smem_u32(bar), recv_o = smem_u32(recv), recv_ml = recv_o + cp.size * cp.share * 16;
+  ptx::cluster_wait();
+  for (int idx = threadIdx.x; idx < cp.total; idx += blockDim.x) {
+    const int r = idx / D4, d4 = idx - r * D4;
+    float mg = -INFINITY;
+    for (int k = 0; k < KS; ++k) mg = fmaxf(mg, comb_ml[(k * rows_pad + r) * 2]);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+    for (int k = 0; k < KS; ++k) {
+      const float mk = comb_ml[(k * rows_pad + r) * 2];
+      const float w = (mk == -INFINITY) ? 0.f : fast_exp2(mk - mg);
+      const float4 o = *reinterpret_cast<const float4*>(comb_o + (static_cast<size_t>(k) * rows_pad + r) * D + d4 * 4);
+      acc.x += w * o.x; acc.y += w * o.y; acc.z += w * o.z; acc.w += w * o.w;
+      l += w * comb_ml[(k * rows_pad + r) * 2 + 1];
+    }
+    const int owner = idx / cp.share, j = idx - owner * cp.share;
+    const uint32_t slot = recv_o + (cp.rank * cp.share + j) * 16;
+    ptx::st_async_pair(slot, bar_s, owner, acc.x, acc.y);
+    ptx::st_async_pair(slot + 8, bar_s, owner, acc.z, acc.w);
+    if (d4 == 0 || j == 0) ptx::st_async_pair(recv_ml + (cp.rank * R + r) * 8, bar_s, owner, mg, l);
+  }
+  const int first = cp.rank * cp.share, n = min(cp.share, cp.total - first);
+  if (n <= 0) return;                    // (nothing is sent to this CTA)
+  // (four times a wait of its own: a CTA of the cluster that gave up on a copy still sends its rows, as NaN)
+  bool ok = false;
+  for (int i = 0; i < 4 && !ok; ++i) ok = ptx::mbar_wait(bar_s, 0);
+  if (!ok) p.header[0] = DEV_ERR_WAIT_EXPIRED;
+  T* out = static_cast<T*>(p.out) +
+           ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
+  const float4* po = reinterpret_cast<const float4*>(recv);
+  const float2* pm = reinterpret_cast<const float2*>(recv + static_cast<size_t>(cp.size) * cp.share * 16);
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const int r = (first + j) / D4, d4 = first + j - r * D4;
+    float mg = -INFINITY;
+    for (int c = 0; c < cp.size; ++c) mg = fmaxf(mg, pm[c * R + r].x);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float l = 0.f;
+    for (int c = 0; c < cp.size; ++c) {
+      const float2 ml = pm[c * R + r];
+      const float4 o = po[c * cp.share + j];
+      const float w = (ml.x == -INFINITY) ? 0.f : fast_exp2(ml.x - mg);
+      acc.x += w * o.x; acc.y += w * o.y; acc.z += w * o.z; acc.w += w * o.w;
+      l += w * ml.y;
+    }
+    const float inv = !ok ? __int_as_float(0x7fc00000) : (l > 0.f ? 1.f / l : (l == l ? 0.f : l));
+    T* dst = out + static_cast<long long>(r) * D + d4 * 4;
+    if constexpr (sizeof(T) == 2) {
+      uint2 u;
+      u.x = ElemTraits<T>::pack2(acc.x * inv, acc.y * inv);
+      u.y = ElemTraits<T>::pack2(acc.z * inv, acc.w * inv);
+      *reinterpret_cast<uint2*>(dst) = u;
+    } else {
+      *reinterpret_cast<float4*>(dst) = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -527,11 +654,6 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
 }
 
 // A CTA's work item, from the planner's records or worked out by the CTA itself.
-struct DecodeItem {
-  long long start;            // ragged: first row of the sequence
-  int b, c, n_chunks, item0;  // sequence, chunk, chunks of the sequence, item number of its first chunk
-  int len, t_begin, t_end;    // keys of the sequence, the item's keys
-};
 
 struct InlinePlan {
   long long tot[kInlinePairs / 32];
@@ -773,7 +895,8 @@ struct PageAhead {
 // NB: 16-key blocks a consumer warp handles per step (2 when a warp owns 32 or more keys of a stage).
 // T: element type of q, k, v as the kernel reads them; OutT: element type of the output rows (T, or float when the
 // inputs are fp16 copies of fp32 tensors).
-template <typename T, int D, int kStages, int NB, int kMaxThreads, int kMinBlocks, typename OutT = T>
+// kCluster: a cluster of CTAs per (sequence, kv head) pair, nothing planned (see ClusterPart).
+template <typename T, int D, int kStages, int NB, int kMaxThreads, int kMinBlocks, typename OutT, bool kCluster>
 __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(const __grid_constant__ CUtensorMap tm_k,
                                                          const __grid_constant__ CUtensorMap tm_v,
                                                          const DecodeParams p) {
@@ -786,15 +909,28 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
   constexpr int STAGE_BYTES = 2 * TILE_BYTES;
   constexpr int KSTEPS = D / 16;
 
+  ClusterPart part = {};
+  __shared__ uint64_t recv_bar;
+  if constexpr (kCluster) {
+    part = cluster_part<D>(p);
+    if (part.size > 1) cluster_begin<D>(p, part, &recv_bar);
+  }
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();      // what earlier launches wrote (the planner's records among it) is visible from here on
   // heads vary fastest across CTAs: the CTAs that run side by side walk the same pages and read
   // neighbouring head slices of each token row, which keeps DRAM rows open
-  __shared__ InlinePlan s_plan;
-  const int item = blockIdx.x / p.kv_heads;
   DecodeItem it;
-  if (!decode_item(p, item, s_plan, it)) return;
-  const int h = blockIdx.x - item * p.kv_heads;
+  int h;
+  if constexpr (kCluster) {
+    const int pair = blockIdx.x / part.size;
+    h = pair % p.kv_heads;
+    cluster_item(p, part, pair / p.kv_heads, it);
+  } else {
+    __shared__ InlinePlan s_plan;
+    const int item = blockIdx.x / p.kv_heads;
+    if (!decode_item(p, item, s_plan, it)) return;
+    h = blockIdx.x - item * p.kv_heads;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NMT = p.n_mtiles;
   const int n_cwarps = (blockDim.x >> 5) - 1;   // consumer warps
@@ -1100,6 +1236,14 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     // output as well as in the error word.
     poison_rows(comb_o, comb_ml, KS * rows_pad, D);
     __syncthreads();
+  }
+  if constexpr (kCluster) {
+    // (behind the control block, rounded up to 16 bytes)
+    unsigned char* recv = reinterpret_cast<unsigned char*>(ctrl) + ((sizeof(DecodeCtrl) + 15) & ~size_t(15));
+    if (part.size > 1) {
+      cluster_emit<OutT, D>(p, part, b, h, comb_o, comb_ml, KS, rows_pad, recv, &recv_bar);
+      return;
+    }
   }
   emit_and_merge<OutT, D>(p, b, h, c, n_chunks, item0, comb_o, comb_ml, KS, rows_pad, &ctrl->ticket);
 }
@@ -1847,7 +1991,7 @@ constexpr int kSimtDepth = 4;                // steps whose copies are in flight
 constexpr int kSimtKeys = 2;                 // key rows of a lane group per step
 constexpr size_t kSimtRingBytes = static_cast<size_t>(kSimtThreads) * kSimtDepth * kSimtKeys * 4 * 16;
 
-template <int D, int RB>
+template <int D, int RB, bool kCluster>
 __global__ void __launch_bounds__(kSimtThreads, 3) decode_simt_kernel(const DecodeParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_ticket;
@@ -1855,15 +1999,28 @@ __global__ void __launch_bounds__(kSimtThreads, 3) decode_simt_kernel(const Deco
   constexpr int kRowsWarp = 32 / kGroup;     // key rows of a warp per load instruction
   constexpr int kKeys = kSimtKeys;
   constexpr int kStep = kRowsWarp * kKeys;   // keys of a warp per step
+  ClusterPart part = {};
+  __shared__ uint64_t recv_bar;
+  if constexpr (kCluster) {
+    part = cluster_part<D>(p);
+    if (part.size > 1) cluster_begin<D>(p, part, &recv_bar);
+  }
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();      // what earlier launches wrote (the planner's records among it) is visible from here on
   // heads vary fastest across CTAs: the CTAs that run side by side walk the same pages and read
   // neighbouring head slices of each token row, which keeps DRAM rows open
-  __shared__ InlinePlan s_plan;
-  const int item = blockIdx.x / p.kv_heads;
   DecodeItem it;
-  if (!decode_item(p, item, s_plan, it)) return;
-  const int h = blockIdx.x - item * p.kv_heads;
+  int h;
+  if constexpr (kCluster) {
+    const int pair = blockIdx.x / part.size;
+    h = pair % p.kv_heads;
+    cluster_item(p, part, pair / p.kv_heads, it);
+  } else {
+    __shared__ InlinePlan s_plan;
+    const int item = blockIdx.x / p.kv_heads;
+    if (!decode_item(p, item, s_plan, it)) return;
+    h = blockIdx.x - item * p.kv_heads;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = lane / kGroup, gl = lane % kGroup;
   constexpr int nwarps = kSimtThreads / 32;
@@ -2057,6 +2214,13 @@ __global__ void __launch_bounds__(kSimtThreads, 3) decode_simt_kernel(const Deco
     }
   }
   __syncthreads();
+  if constexpr (kCluster) {
+    unsigned char* recv = reinterpret_cast<unsigned char*>(comb_ml + ((static_cast<size_t>(KS) * R * 2 + 3) & ~size_t(3)));
+    if (part.size > 1) {
+      cluster_emit<float, D>(p, part, b, h, comb_o, comb_ml, KS, R, recv, &recv_bar);
+      return;
+    }
+  }
   emit_and_merge<float, D>(p, b, h, c, n_chunks, item0, comb_o, comb_ml, KS, R, &s_ticket);
 }
 
@@ -2179,6 +2343,32 @@ int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t st
 
 namespace {
 // `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
+// CTAs per (sequence, KV head) pair when the call runs without a plan, 0 when it is planned.  Up to eight CTAs share a pair,
+// as long as all of them are resident at once (three on an SM).  The line is drawn by the bytes of K and V in a part, from
+// the lengths that the host can know of, and by what a plan is there for:
+//   dense: every part is as long as any other, there is nothing to plan.  bf16, 32/8 heads, D 128, planned -> not, us: 1 x
+//     2 048 13.9 -> 9.0, 6 x 2 048 18.0 -> 14.5, 6 x 8 192 42.2 -> 38.2, 25 x 2 048 48.5 -> 39.2; fp32, D 64, 13 x 2 048
+//     29.9 -> 25.8.  With few pairs a plan cuts finer (1 x 8 192 19.3 -> 19.2, fp32, D 128 1 x 4 096 22.4 -> 32.2).
+//   paged: the longest sequence is known (the table's width), the others may be shorter, and a plan would make use of that:
+//     a quarter of the dense limit, where the worst case, half of the keys not there, still breaks even.
+//   ragged: the average is known; half of that again, and no part longer than 1 MiB whatever the lengths.
+int cluster_size(const b200attn_decode_args_t& a, int sm_count) {
+  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
+  if (pairs <= 0) return 0;
+  const bool ragged = a.layout == B200ATTN_RAGGED, dense = a.layout == B200ATTN_DENSE;
+  const long long keys = ragged ? (a.total_kv + a.batch - 1) / a.batch
+                         : dense ? a.max_kv : a.table_stride * static_cast<long long>(a.page_size);
+  const long long tiles = (keys + kTileN - 1) / kTileN;
+  const long long tile_bytes = 2ll * kTileN * a.head_dim * (a.dtype == B200ATTN_F32 ? 4 : 2);
+  long long c = 8;
+  while (c > 1 && (pairs * c > 3ll * sm_count || tiles <= c / 2)) c /= 2;
+  const bool full = pairs * c >= 2ll * sm_count;
+  const long long limit = (dense ? (full ? 512 : 256) : ragged ? (full ? 64 : 128) : (full ? 128 : 256)) * 1024ll;
+  if ((tiles + c - 1) / c * tile_bytes > limit) return 0;
+  if (ragged && a.total_kv / kTileN * tile_bytes > c * (1ll << 20)) return 0;
+  return static_cast<int>(c);
+}
+
 int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, const DecodeWsLayout& w,
                        int pass_group, int head0, bool f32_out, bool built_in) {
   DecodeParams p;
@@ -2220,7 +2410,8 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   // the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
   // in every call.
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
-  p.inline_plan = !built_in && (a.dtype == B200ATTN_F32 || p.rows <= 16) && pairs <= kInlinePairs ? 1 : 0;
+  p.cluster = a.dtype == B200ATTN_F32 || p.rows <= 16 ? cluster_size(a, sm_count) : 0;
+  p.inline_plan = !built_in && !p.cluster && (a.dtype == B200ATTN_F32 || p.rows <= 16) && pairs <= kInlinePairs ? 1 : 0;
   unsigned grid_items = static_cast<unsigned>(w.max_items);
   cudaError_t e = cudaSuccess;
   if (p.inline_plan) {
@@ -2228,23 +2419,29 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     const long long keys = a.layout == B200ATTN_RAGGED ? a.total_kv
                            : a.batch * (a.layout == B200ATTN_DENSE ? static_cast<long long>(a.max_kv) : a.table_stride * a.page_size);
     grid_items = static_cast<unsigned>(std::min<long long>(w.max_items, keys / w.min_chunk + a.batch));
-  } else {
+  } else if (!p.cluster) {
     e = launch_dependent(decode_plan_kernel, dim3(1), kPlanThreads, 0, stream, 1, p);
   }
   if (e != cudaSuccess) return cuda_fail(e, "decode_plan_kernel launch");
 
-  const dim3 grid(grid_items * a.kv_heads, 1);
+  const dim3 grid(p.cluster ? static_cast<unsigned>(pairs * p.cluster) : grid_items * a.kv_heads, 1);
   const int D = a.head_dim;
+  // shared memory of the pieces and the rows' (m, l) that the CTAs of a cluster send to one another, and their alignment
+  const size_t recv_bytes = p.cluster ? static_cast<size_t>(p.cluster) * ((p.rows * (D / 4) + p.cluster - 1) / p.cluster * 16 + p.rows * 8) + 32 : 0;
   if (a.dtype == B200ATTN_F32) {
     // (four warps leave at most 4 / blocks-of-rows partials per row: see the kernel)
     const int rb = p.rows >= 3 ? 4 : p.rows;
-    const size_t smem = kSimtRingBytes + sizeof(float) * static_cast<size_t>(std::max(p.rows, 4 * rb)) * (D + 2);
+    const size_t smem = kSimtRingBytes + sizeof(float) * static_cast<size_t>(std::max(p.rows, 4 * rb)) * (D + 2) + recv_bytes;
     int rc = 0;
 #define B200ATTN_LAUNCH_SIMT(DIM, RB)                                                                 \
     do {                                                                                              \
-      rc = set_smem(decode_simt_kernel<DIM, RB>, smem);                                               \
-      if (rc) return rc;                                                                              \
-      launch_dependent(decode_simt_kernel<DIM, RB>, grid, kSimtThreads, smem, stream, 1, p);         \
+      if (p.cluster) {                                                                                \
+        if ((rc = set_smem(decode_simt_kernel<DIM, RB, true>, smem))) return rc;                      \
+        launch_dependent(decode_simt_kernel<DIM, RB, true>, grid, kSimtThreads, smem, stream, p.cluster, p); \
+      } else {                                                                                        \
+        if ((rc = set_smem(decode_simt_kernel<DIM, RB, false>, smem))) return rc;                     \
+        launch_dependent(decode_simt_kernel<DIM, RB, false>, grid, kSimtThreads, smem, stream, 1, p); \
+      }                                                                                               \
     } while (0)
     if (D == 128) { if (rb == 1) B200ATTN_LAUNCH_SIMT(128, 1); else if (rb == 2) B200ATTN_LAUNCH_SIMT(128, 2); else B200ATTN_LAUNCH_SIMT(128, 4); }
     else          { if (rb == 1) B200ATTN_LAUNCH_SIMT(64, 1);  else if (rb == 2) B200ATTN_LAUNCH_SIMT(64, 2);  else B200ATTN_LAUNCH_SIMT(64, 4); }
@@ -2297,7 +2494,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     const int stages = 2;
     const size_t stage_bytes = static_cast<size_t>(stages) * 2 * kTileN * D * 2;
     const size_t comb_bytes = sizeof(float) * static_cast<size_t>(ksl) * nmt * 16 * (D + 2);
-    const size_t smem = 1024 + std::max(stage_bytes, comb_bytes) + static_cast<size_t>(nmt) * 16 * D * 2 + sizeof(DecodeCtrl);
+    const size_t smem = 1024 + std::max(stage_bytes, comb_bytes) + static_cast<size_t>(nmt) * 16 * D * 2 + sizeof(DecodeCtrl) + recv_bytes;
     // tensor maps over K and V: (D, heads, tokens), one box = 64 elements x 1 head x box_rows keys
     CUtensorMap tk, tv;
     int rc = 0;
@@ -2319,9 +2516,13 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     }
 #define B200ATTN_LAUNCH_DECODE_V(TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT)                               \
     do {                                                                                                  \
-      rc = set_smem(decode_mma_kernel<TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT>, smem);                  \
-      if (rc) return rc;                                                                                  \
-      launch_dependent(decode_mma_kernel<TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT>, grid, threads, smem, stream, 1, tk, tv, p);\
+      if (p.cluster) {                                                                                    \
+        if ((rc = set_smem(decode_mma_kernel<TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT, true>, smem))) return rc; \
+        launch_dependent(decode_mma_kernel<TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT, true>, grid, threads, smem, stream, p.cluster, tk, tv, p); \
+      } else {                                                                                            \
+        if ((rc = set_smem(decode_mma_kernel<TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT, false>, smem))) return rc; \
+        launch_dependent(decode_mma_kernel<TYPE, DIM, STAGES, NBLK, MAXT, MINB, OUT, false>, grid, threads, smem, stream, 1, tk, tv, p); \
+      }                                                                                                   \
     } while (0)
 #define B200ATTN_LAUNCH_DECODE(TYPE, DIM, OUT) B200ATTN_LAUNCH_DECODE_V(TYPE, DIM, 2, 1, 160, 3, OUT)
     if (f32_out) {

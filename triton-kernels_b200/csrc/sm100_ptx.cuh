@@ -1,7 +1,7 @@
 // Inline-PTX wrappers for the Blackwell (sm_100a) features the kernels use: mbarrier, TMA tiled loads and untiled bulk
 // loads, tensor memory (TMEM) allocation / load / store, tcgen05.mma with shared-memory descriptors.  Every copy lands
-// in the issuing CTA's own shared memory; the only cluster traffic is st_async_pair (8-byte remote stores between the
-// CTAs of a softmax cluster).
+// in the issuing CTA's own shared memory; the only cluster traffic is st_async_pair (8-byte remote stores between the CTAs of
+// a softmax or decode cluster).
 #pragma once
 
 #include <cuda.h>
@@ -74,6 +74,10 @@ __device__ __forceinline__ void st_async_pair(uint32_t slot, uint32_t bar, uint3
       ::"r"(slot), "r"(bar), "r"(cta_rank), "f"(a), "f"(b)
       : "memory");
 }
+
+// Cluster-wide barrier in two halves; every thread of every CTA takes part.  (Only in grids launched with a cluster size.)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 
 // Untiled bulk copy global -> this CTA's shared memory; both addresses 16-byte aligned, `bytes` a multiple of 16.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
