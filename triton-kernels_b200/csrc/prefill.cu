@@ -57,6 +57,7 @@ constexpr int kSoftmaxWarps = 16;  // 4 warpgroups: (slot 0 | slot 1) x (columns
 constexpr int kThreads = 576;
 constexpr int kProducerWarp = 16;
 constexpr int kMmaWarp = 17;
+constexpr int kQBufs = 3;          // Q tiles: the two of the current item and the first of the next
 // A tile's exponentials against the reference that stands are good as long as a thread's 32 of them, of a row, sum up to
 // no more than kMaxPartialSum (P then fits 16 bits, and so does every one of them).  When that is not so the row's maximum
 // lies five powers of two or more above its reference; a reference moves when the maximum is kRescaleThreshold above it.
@@ -83,14 +84,13 @@ struct ItemWork {
 
 // shared-memory control block placed after the tiles
 struct __align__(8) Control {
-  uint64_t q_full;
-  uint64_t q_empty;
+  uint64_t q_full[kQBufs];
+  uint64_t q_empty[kQBufs];
   uint64_t kv_full[kStages];     // pair {V_j, K_j+1} (or K_0 alone / V_last alone) has landed
   uint64_t kv_empty[kStages];    // ... has been consumed by the MMAs
   uint64_t s_full[kSlots];
   uint64_t p_ready[kSlots];
   uint64_t o_done[kSlots];
-  uint64_t o_free[kSlots];
   uint64_t sched_full[2];
   uint64_t sched_empty[2];
   int sched_item[2];
@@ -105,9 +105,10 @@ struct SmemPlan {
   static constexpr int kChunkBytes = kBN * 128;            // one column block of a 128-row tile
   static constexpr int kTileBytes = kChunks * kChunkBytes; // 128 x D 16-bit tile
   static constexpr int kQOff = 0;
-  static constexpr int kRingOff = kSlots * kTileBytes;
+  static constexpr int kRingOff = kQBufs * kTileBytes;
   static constexpr int kCtrlOff = kRingOff + kRing * kTileBytes;
   static constexpr int kTotal = kCtrlOff + static_cast<int>(sizeof(Control));
+  static_assert(kTotal + 1024 <= 227 * 1024, "shared memory of an SM (1 KiB for the alignment of the tiles)");
 };
 
 // bounded mbarrier wait whose verdict is uniform over the (converged) warp
@@ -267,14 +268,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // allocation of the MMA warp (it never touches tensor memory).  Everybody else waits until both are done.
   if (warp == kProducerWarp) {
     if (lane == 0) {
-      mbar_init(smem_u32(&ctrl->q_full), 1);
-      mbar_init(smem_u32(&ctrl->q_empty), 1);
+      for (int i = 0; i < kQBufs; ++i) { mbar_init(smem_u32(&ctrl->q_full[i]), 1); mbar_init(smem_u32(&ctrl->q_empty[i]), 1); }
       for (int i = 0; i < kStages; ++i) { mbar_init(smem_u32(&ctrl->kv_full[i]), 1); mbar_init(smem_u32(&ctrl->kv_empty[i]), 1); }
       for (int s = 0; s < kSlots; ++s) {
         mbar_init(smem_u32(&ctrl->s_full[s]), 1);
         mbar_init(smem_u32(&ctrl->p_ready[s]), 8);         // one arrival per softmax warp of the slot
         mbar_init(smem_u32(&ctrl->o_done[s]), 1);
-        mbar_init(smem_u32(&ctrl->o_free[s]), 8);          // one arrival per softmax warp of the slot
       }
       for (int i = 0; i < 2; ++i) {
         mbar_init(smem_u32(&ctrl->sched_full[i]), 1);
@@ -321,6 +320,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int page_shift = 31 - __clz(p.page_size);
     int pg_k = kNoPage, pg_v = kNoPage, pg_k_next = kNoPage, pg_v_next = kNoPage;
     int pair_e = 0;       // K/V pairs issued so far, across items
+    int q_uses = 0;       // Q tiles issued (or skipped) so far
     int pair_lo = 0;      // first pair of the current item
     for (int k = 0; ok; ++k) {
       if (k >= 2) {
@@ -358,40 +358,36 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           pg_v_next = read_page(vtab, 32);
         }
       }
-      if (k >= 1 && lane == 0) {
-        // the previous item is still running: pull this item's Q tiles and first K/V tiles into L2 now, so the
-        // copies issued once the Q buffer is free only pay an L2 round trip
-        for (int s = 0; s < kSlots; ++s) {
-          if (w.nkv[s] == 0) continue;
-          for (int c = 0; c < Plan::kChunks; ++c)
-            tma_prefetch_3d(&tm_q, c * 64, w.q_head_coord[s], static_cast<int>(w.q_row0[s] + w.m0[s]));
-        }
-        if (p.layout != B200ATTN_PAGED && w.nkv_max > 0) {
-          for (int c = 0; c < Plan::kChunks; ++c) {
-            tma_prefetch_3d(&tm_k, c * 64, w.kv_head_coord, static_cast<int>(w.kv_row0));
-            tma_prefetch_3d(&tm_v, c * 64, w.kv_head_coord, static_cast<int>(w.kv_row0));
-          }
-        }
-      }
-      // Q may be overwritten once every S MMA of the previous item has completed
-      if (k >= 1) {
-        ok = warp_wait(smem_u32(&ctrl->q_empty), (k - 1) & 1);
-        if (!ok || *abort_flag) { ok = false; break; }
-      }
-      if (lane == 0) {
-        uint32_t bytes = 0;
-        for (int s = 0; s < kSlots; ++s) if (w.nkv[s] > 0) bytes += Plan::kTileBytes;
-        if (bytes > 0) {
-          mbar_arrive_expect_tx(smem_u32(&ctrl->q_full), bytes);
-          for (int s = 0; s < kSlots; ++s) {
-            if (w.nkv[s] == 0) continue;
+      // Q tile of slot s: use 2 k + s of the three Q buffers, so the first tile of an item never waits for the item before
+      // it, and the second only for that item's first slot
+      auto load_q = [&](int s) -> bool {
+        const int use = 2 * k + s, buf = use % kQBufs, n = use / kQBufs;
+        if (n > 0 && (!warp_wait(smem_u32(&ctrl->q_empty[buf]), (n - 1) & 1) || *abort_flag)) return false;
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(&ctrl->q_full[buf]);
+          if (w.nkv[s] > 0) {
+            mbar_arrive_expect_tx(bar, Plan::kTileBytes);
             for (int c = 0; c < Plan::kChunks; ++c)
-              tma_load_3d(smem_base + Plan::kQOff + s * Plan::kTileBytes + c * Plan::kChunkBytes, &tm_q,
-                          smem_u32(&ctrl->q_full), c * 64, w.q_head_coord[s], static_cast<int>(w.q_row0[s] + w.m0[s]));
+              tma_load_3d(smem_base + Plan::kQOff + buf * Plan::kTileBytes + c * Plan::kChunkBytes, &tm_q, bar, c * 64,
+                          w.q_head_coord[s], static_cast<int>(w.q_row0[s] + w.m0[s]));
+          } else {
+            mbar_arrive(bar);   // keeps one q_full phase per use
           }
-        } else {
-          mbar_arrive(smem_u32(&ctrl->q_full));   // keeps one q_full phase per item
         }
+        q_uses = use + 1;
+        __syncwarp();
+        return true;
+      };
+      if (k >= 1 && lane == 0 && w.nkv[1] > 0) {
+        // pull the second slot's Q into L2 now, so the copies issued once its buffer is free only pay an L2 round trip
+        for (int c = 0; c < Plan::kChunks; ++c)
+          tma_prefetch_3d(&tm_q, c * 64, w.q_head_coord[1], static_cast<int>(w.q_row0[1] + w.m0[1]));
+      }
+      ok = load_q(0);
+      if (!ok) break;
+      if (w.nkv_max == 0) {
+        ok = load_q(1);
+        if (!ok) break;
       }
       // K/V tiles travel in pairs that share one barrier: pair 0 of an item is K_0 alone, pair j + 1 is {V_j, K_j+1}
       // (the last one V alone).  Stage = pair % 2; its V buffer is ring buffer 2 * stage, its K buffer 2 * stage + 1.
@@ -490,12 +486,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
           }
         }
+        if (pi == 0) ok = load_q(1);
       }
     }
     if (!ok) {
       if (lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
       // drain: wait (bounded) for the copies still in flight before the CTA may exit
       for (int e = max(pair_lo, pair_e - kStages); e < pair_e; ++e) mbar_wait(smem_u32(&ctrl->kv_full[e % kStages]), (e / kStages) & 1);
+      for (int u = max(0, q_uses - kQBufs); u < q_uses; ++u) mbar_wait(smem_u32(&ctrl->q_full[u % kQBufs]), (u / kQBufs) & 1);
     }
     if (lane == 0) {
       // This CTA draws no more items.  The last CTA to get here puts both counters back to zero for the next
@@ -528,16 +526,22 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // The warp stays converged while it issues: every lane runs the descriptor arithmetic, one elected lane
     // issues the tensor-core instructions and their commits.
     const uint32_t lead = elect_one();
+    auto uniform = [](uint64_t x) -> uint64_t {
+      const uint32_t lo = __shfl_sync(0xffffffffu, static_cast<uint32_t>(x), 0), hi = __shfl_sync(0xffffffffu, static_cast<uint32_t>(x >> 32), 0);
+      return (static_cast<uint64_t>(hi) << 32) | lo;
+    };
     // operand descriptors of the K and the V buffer of a pair's stage
     auto k_desc_of = [&](int pr) -> uint64_t {
-      return kdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages) + 1) * Plan::kTileBytes) >> 4);
+      return uniform(kdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages) + 1) * Plan::kTileBytes) >> 4));
     };
     auto v_desc_of = [&](int pr) -> uint64_t {
-      return vdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages)) * Plan::kTileBytes) >> 4);
+      return uniform(vdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages)) * Plan::kTileBytes) >> 4));
     };
-    auto issue_s = [&](int s, uint64_t kb) {
+    auto q_desc_of = [&](int buf) -> uint64_t {
+      return uniform(kdesc + static_cast<uint64_t>((Plan::kQOff + buf * Plan::kTileBytes) >> 4));
+    };
+    auto issue_s = [&](int s, uint64_t qa, uint64_t kb) {
       // S_s = Q_s K^T : K-major A and B, D/16 k-steps
-      const uint64_t qa = kdesc + static_cast<uint64_t>((Plan::kQOff + s * Plan::kTileBytes) >> 4);
       mma_ss_batch<D / 16>(tmem_S[s], qa, kb, idesc_s, 0u, lead);
       mma_commit_lead(smem_u32(&ctrl->s_full[s]), lead);
     };
@@ -548,6 +552,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       mma_commit_lead(smem_u32(&ctrl->o_done[s]), lead);
     };
 
+    // First score tile of slot s of item kk, whose K_0 is pair `pr`: once its Q tile and K_0 have landed.  A slot without
+    // tiles only takes its turn at the Q buffer.
+    auto start_slot = [&](int s, int kk, int nkv_s, int pr) -> bool {
+      const int use = 2 * kk + s, buf = use % kQBufs;
+      if (!warp_wait(smem_u32(&ctrl->q_full[buf]), (use / kQBufs) & 1)) return false;
+      if (nkv_s > 0) {
+        if (!pair_full_wait(pr)) return false;
+        tc_fence_after();
+        issue_s(s, q_desc_of(buf), k_desc_of(pr));
+        if (nkv_s == 1) mma_commit_lead(smem_u32(&ctrl->q_empty[buf]), lead);    // the slot's last use of its Q tile
+      } else if (lane == 0) {
+        mbar_arrive(smem_u32(&ctrl->q_empty[buf]));
+      }
+      __syncwarp();
+      return true;
+    };
+
     for (int k = 0; ok; ++k) {
       ok = warp_wait(smem_u32(&ctrl->sched_full[k & 1]), (k >> 1) & 1);
       if (!ok || *abort_flag) { ok = false; break; }
@@ -555,47 +576,20 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (item < 0) break;
       const ItemWork& wr = ctrl->sched_work[k & 1];
       const int nkv0 = wr.nkv[0], nkv1 = wr.nkv[1], nkv_max = wr.nkv_max, len_k = wr.len_k;
-      ok = warp_wait(smem_u32(&ctrl->q_full), k & 1);
+      const int qbuf0 = (2 * k) % kQBufs, qbuf1 = (2 * k + 1) % kQBufs;
+      const uint64_t qd0 = q_desc_of(qbuf0), qd1 = q_desc_of(qbuf1);
+      // (slots whose first score tile was already issued while the previous item finished are skipped)
+      if (!pre_issued0) ok = start_slot(0, k, nkv0, pair_base);
+      if (ok && !pre_issued1) ok = start_slot(1, k, nkv1, pair_base);
       if (!ok) break;
-      if (nkv_max > 0) {
-        ok = pair_full_wait(pair_base);
-        if (!ok) break;
-        tc_fence_after();
-        // (slots whose first score tile was already issued while the previous item finished are skipped)
-        if (nkv0 > 0 && !pre_issued0) issue_s(0, k_desc_of(pair_base));
-        if (nkv1 > 0 && !pre_issued1) issue_s(1, k_desc_of(pair_base));
-        mma_commit_lead(smem_u32(&ctrl->kv_empty[pair_base % kStages]), lead);
-        if (nkv_max == 1) mma_commit_lead(smem_u32(&ctrl->q_empty), lead);
-      } else {
-        mma_commit_lead(smem_u32(&ctrl->q_empty), lead);
-      }
+      if (nkv_max > 0) mma_commit_lead(smem_u32(&ctrl->kv_empty[pair_base % kStages]), lead);
       pre_issued0 = pre_issued1 = false;
       for (int j = 0; j < nkv_max && ok; ++j) {
         const int pr = pair_base + 1 + j;     // the pair {V_j, K_j+1}
         const bool last_iter = j + 1 == nkv_max;
-        // On the last tile of the item the first score tile of the next item is issued right behind each slot's
-        // final PV, so the softmax warps can carry straight on.  Everything waited
-        // for here (next item published, its Q and first K tile loaded) depends only on work this warp has
-        // already issued: Q may be replaced once the last score MMAs of this item, issued one tile ago, complete.
-        int next_state = 0;            // 0 = not looked at yet, 1 = ready, -1 = nothing to issue ahead
-        int next_nkv0 = 0, next_nkv1 = 0;   // tiles per slot of the next item
-        auto prepare_next = [&]() -> bool {
-          if (next_state != 0) return true;
-          next_state = -1;
-          if (!warp_wait(smem_u32(&ctrl->sched_full[(k + 1) & 1]), ((k + 1) >> 1) & 1)) return false;
-          if (ctrl->sched_item[(k + 1) & 1] < 0) return true;
-          const ItemWork& wn = ctrl->sched_work[(k + 1) & 1];
-          if (wn.nkv_max == 0) return true;
-          next_nkv0 = wn.nkv[0];
-          next_nkv1 = wn.nkv[1];
-          if (!warp_wait(smem_u32(&ctrl->q_full), (k + 1) & 1)) return false;
-          if (!pair_full_wait(pair_base + nkv_max + 1)) return false;
-          next_state = 1;
-          return true;
-        };
         // Everything that does not depend on the softmax warps is waited for and computed before their P is: the
-        // pair {V_j, K_j+1} (one barrier; in steady state loaded long ago), the operand descriptors, and on the last
-        // tile the next item.  Between a slot's P and its two batches of MMAs the warp then only runs the issue.
+        // pair {V_j, K_j+1} (one barrier; in steady state loaded long ago) and the operand descriptors.  Between a slot's
+        // P and its two batches of MMAs the warp then only runs the issue.
         ok = pair_full_wait(pr);
         if (!ok) break;
         {
@@ -614,48 +608,50 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             __syncwarp();
           }
         }
-        int pr_k = pr;                // pair whose K buffer the score MMAs issued in this iteration read
-        if (last_iter) {
-          ok = prepare_next();
-          if (!ok) break;
-          pr_k = pair_base + nkv_max + 1;       // K_0 of the next item (read only when next_state == 1)
-        }
         const uint64_t vb = v_desc_of(pr);
-        const uint64_t kb = k_desc_of(pr_k);
-        auto slot_step = [&](const int s, const int nkv_s, const int next_nkv_s, int& tiles_done, bool& pre_issued) -> bool {
+        const uint64_t kb = k_desc_of(pr);
+        auto slot_step = [&](const int s, const int nkv_s, const int qbuf, const uint64_t qd, int& tiles_done) -> bool {
           if (j >= nkv_s) return true;
-          const bool s_next = last_iter ? (next_state == 1 && next_nkv_s > 0) : (j + 1 < nkv_s);
-          if (j == 0 && k > 0) {
-            // the first PV of an item overwrites O: the epilogue of the previous item must have read it out
-            // (the softmax warps do that just before they hand over this tile's P)
-            if (!warp_wait(smem_u32(&ctrl->o_free[s]), (k - 1) & 1)) return false;
-          }
+          // (P of an item's first tile also says that the previous item's O has been read out: the softmax warps hand it
+          // over after that)
           if (!warp_wait(smem_u32(&ctrl->p_ready[s]), tiles_done & 1)) return false;
           tc_fence_after();
           issue_pv(s, vb, j == 0);
-          if (s_next) {
-            issue_s(s, kb);
-            if (last_iter) pre_issued = true;
+          if (j + 1 < nkv_s) {
+            issue_s(s, qd, kb);
+            if (j + 2 == nkv_s) mma_commit_lead(smem_u32(&ctrl->q_empty[qbuf]), lead);   // the slot's last use of its Q tile
           }
           ++tiles_done;
           return true;
         };
-        ok = slot_step(0, nkv0, next_nkv0, tiles_done0, pre_issued0);
-        if (ok) ok = slot_step(1, nkv1, next_nkv1, tiles_done1, pre_issued1);
-        if (!ok) break;
-        if (last_iter) {
-          // a slot that ran out of tiles earlier in this item gets its head start here
-          ok = prepare_next();
+        if (!last_iter) {
+          ok = slot_step(0, nkv0, qbuf0, qd0, tiles_done0) && slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
           if (!ok) break;
-          if (next_state == 1) {
-            if (!pre_issued0 && next_nkv0 > 0) { tc_fence_after(); issue_s(0, kb); pre_issued0 = true; }
-            if (!pre_issued1 && next_nkv1 > 0) { tc_fence_after(); issue_s(1, kb); pre_issued1 = true; }
+          // V_j and K_j+1 have been read by everything that will read them: one commit releases the stage
+          mma_commit_lead(smem_u32(&ctrl->kv_empty[pr % kStages]), lead);
+        } else {
+          // The item's last tile: each slot's first score tile of the next item is issued right behind its final PV, so
+          // that the tensor cores have work while the softmax warps read O out.  What is waited for here (the next item
+          // published, its Q tiles and its first K tile) depends only on work this warp has already issued: the first
+          // slot's Q has a buffer of its own, the second's takes the one this item's first slot gave back a tile ago.
+          ok = slot_step(0, nkv0, qbuf0, qd0, tiles_done0) &&
+               warp_wait(smem_u32(&ctrl->sched_full[(k + 1) & 1]), ((k + 1) >> 1) & 1);
+          if (!ok) break;
+          const bool more = ctrl->sched_item[(k + 1) & 1] >= 0;
+          const ItemWork& wn = ctrl->sched_work[(k + 1) & 1];
+          if (more) {
+            ok = start_slot(0, k + 1, wn.nkv[0], pair_base + nkv_max + 1);
+            if (!ok) break;
           }
+          ok = slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
+          if (!ok) break;
+          mma_commit_lead(smem_u32(&ctrl->kv_empty[pr % kStages]), lead);
+          if (more) {
+            ok = start_slot(1, k + 1, wn.nkv[1], pair_base + nkv_max + 1);
+            if (!ok) break;
+          }
+          pre_issued0 = pre_issued1 = more;
         }
-        // V_j and K_j+1 have been read by everything that will read them: one commit releases the stage
-        mma_commit_lead(smem_u32(&ctrl->kv_empty[pr % kStages]), lead);
-        // the last score MMAs of the item have been issued: Q may be replaced once they complete
-        if (j + 2 == nkv_max) mma_commit_lead(smem_u32(&ctrl->q_empty), lead);
       }
       if (nkv_max > 0) pair_base += nkv_max + 1;
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));
@@ -728,12 +724,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       tc_fence_after();
       const float inv_a = out_la > 0.f ? 1.f / out_la : 0.f;
       const float inv_b = out_lb > 0.f ? 1.f / out_lb : 0.f;
-      auto o_is_read = [&]() {
-        // O has been read out: the MMA warp may start the next item's PV into it
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&ctrl->o_free[s]));
-      };
       constexpr int kChunksO = D / 64;
       if constexpr (k16) {
         // 16-bit output: 64 columns of a row are one 128-byte line.  A quad holds 8 consecutive columns per group;
@@ -750,7 +740,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
-          if (c == kChunksO - 1) o_is_read();
           uint32_t a[8], b[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -794,7 +783,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
-          if (c == kChunksO - 1) o_is_read();
           float* out = static_cast<float*>(p.out) + out_off + c * 64 + q * 2;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
