@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   __shared__ int s_warp[32];
   __shared__ int s_carry;
   __shared__ int s_chunk;
-  __shared__ int s_cand_chunk[kPlanThreads / 32], s_cand_items[kPlanThreads / 32], s_cand_max[kPlanThreads / 32];
-  __shared__ int s_pick_items;
+  // per candidate, of several waves [0] and of a single one [1]: chunk, items; largest item of a single wave
+  __shared__ int s_cand_chunk[2][kPlanThreads / 32], s_cand_items[2][kPlanThreads / 32], s_cand_max[kPlanThreads / 32];
   __shared__ int s_slots;                            // > 0: the batch is dealt out to that many slots
   __shared__ int s_rank[kPlanMaxSlots];              // cuts inside sequences among the slot boundaries 1 .. i
   __shared__ int s_cut[kPlanMaxSlots];               // their keys, in order
@@ -397,15 +397,18 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();      // (the call before may still be using the records and tickets that are written below)
   if (tid < kPlanBuckets) { s_hist[tid] = 0; s_cursor[tid] = 0; }
-  if (tid == 0) s_slots = 0;
   const bool cached = p.batch <= kPlanLenCache;
   auto len_of = [&](int b) -> int { return cached ? s_len[b] : seq_info(p, b).len; };
 
   long long tot = 0;
+  SeqInfo mine;                             // of sequence tid: kept, the records need it again
+  mine.start = 0;
+  mine.len = 0;
   for (int b = tid; b < p.batch; b += kPlanThreads) {
-    const int len = seq_info(p, b).len;
-    if (cached) s_len[b] = len;
-    tot += len;
+    const SeqInfo si = seq_info(p, b);
+    if (b == tid) mine = si;
+    if (cached) s_len[b] = si.len;
+    tot += si.len;
   }
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   if (lane == 0) s_tot[warp] = tot;
@@ -423,80 +426,78 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   for (int w = 0; w < kPlanThreads / 32; ++w) t += s_tot[w];
   // (the two divisions per sequence go through a float reciprocal, corrected to the exact quotient: a pass over 256
   // lengths with integer divisions cost 2 us, and the pass runs once or twice per call)
-  auto evaluate = [&](int target, bool with_largest) {
-    long long base = (t + target - 1) / target;
+  // Both kinds of candidate are evaluated in one pass, and what one thread used to decide in loops over shared memory
+  // warp 0 decides in ballots; with that, 32-bit divisions and the lengths kept in registers a call of 16 fp32 sequences of
+  // 100 to 4 096 keys, 8 heads, takes 35.1 us instead of 36.3.
+  auto candidate = [&](int target) -> int {
+    long long base = t <= 0x7fffffff ? (static_cast<unsigned>(t) + target - 1) / static_cast<unsigned>(target) : (t + target - 1) / target;
     base = ((base + kTileN - 1) / kTileN) * kTileN;
     if (base < p.min_chunk) base = p.min_chunk;
     if (base > (1 << 29)) base = 1 << 29;
-    long long cand = base + (base * warp) / 32;
-    cand = ((cand + kTileN - 1) / kTileN) * kTileN;
-    const int ck = static_cast<int>(cand);
-    const float inv_ck = 1.f / static_cast<float>(ck);
-    long long n = 0;
+    const long long cand = base + (base * warp) / 32;
+    return static_cast<int>(((cand + kTileN - 1) / kTileN) * kTileN);
+  };
+  // (a batch of more sequences than a wave has CTAs cannot fit one: every sequence is at least one item)
+  const bool try_wave = p.wave_items > 0 && p.wave_items < p.target_items && p.batch <= p.wave_items;
+  {
+    const int ck0 = candidate(p.target_items), ck1 = try_wave ? candidate(p.wave_items) : ck0;
+    const float inv0 = 1.f / static_cast<float>(ck0), inv1 = 1.f / static_cast<float>(ck1);
+    long long n0 = 0, n1 = 0;
     int biggest = 0;
     for (int b = lane; b < p.batch; b += 32) {
       const int len = len_of(b);
-      int v = ceil_div_fast(len, ck, inv_ck);
-      if (v < 1) v = 1;
-      n += v;
-      if (with_largest) {
-        int per = ((ceil_div_fast(len, v, __frcp_rn(static_cast<float>(v))) + kTileN - 1) / kTileN) * kTileN;
-        if (per < kTileN) per = kTileN;
-        biggest = max(biggest, min(len, per));
+      n0 += max(1, ceil_div_fast(len, ck0, inv0));
+      if (try_wave) {
+        const int v = max(1, ceil_div_fast(len, ck1, inv1));
+        n1 += v;
+        const int per = ((ceil_div_fast(len, v, __frcp_rn(static_cast<float>(v))) + kTileN - 1) / kTileN) * kTileN;
+        biggest = max(biggest, min(len, max(per, kTileN)));
       }
     }
     for (int o = 16; o > 0; o >>= 1) {
-      n += __shfl_xor_sync(0xffffffffu, n, o);
-      biggest = max(biggest, __shfl_xor_sync(0xffffffffu, biggest, o));
+      n0 += __shfl_xor_sync(0xffffffffu, n0, o);
+      if (try_wave) {
+        n1 += __shfl_xor_sync(0xffffffffu, n1, o);
+        biggest = max(biggest, __shfl_xor_sync(0xffffffffu, biggest, o));
+      }
     }
     if (lane == 0) {
-      s_cand_chunk[warp] = ck;
-      s_cand_items[warp] = n > 0x7fffffff ? 0x7fffffff : static_cast<int>(n);
+      s_cand_chunk[0][warp] = ck0;
+      s_cand_chunk[1][warp] = ck1;
+      s_cand_items[0][warp] = n0 > 0x7fffffff ? 0x7fffffff : static_cast<int>(n0);
+      s_cand_items[1][warp] = n1 > 0x7fffffff ? 0x7fffffff : static_cast<int>(n1);
       s_cand_max[warp] = biggest;
     }
-  };
-  evaluate(p.target_items, false);
-  __syncthreads();
-  if (tid == 0) {
-    int pick = kPlanThreads / 32 - 1;
-    for (int k = 0; k < kPlanThreads / 32; ++k) {
-      if (s_cand_items[k] <= p.target_items) { pick = k; break; }
-    }
-    s_chunk = s_cand_chunk[pick];
-    s_pick_items = s_cand_items[pick];
-    s_carry = 0;
   }
   __syncthreads();
-  // Estimated run time of a plan in several waves, in keys: the average load of a resident CTA plus half an item.
-  const float ovh = static_cast<float>(p.item_overhead);
-  auto several_cost = [&]() -> float {
-    const float n = static_cast<float>(s_pick_items);
-    return (static_cast<float>(t) + n * ovh) / static_cast<float>(p.wave_items) + 0.5f * (static_cast<float>(t) / n + ovh);
-  };
-  float best = p.wave_items > 0 ? several_cost() : 0.f;   // (read by thread 0 only)
-  // (a batch of more sequences than a wave has CTAs cannot fit one: every sequence is at least one item)
-  if (p.wave_items > 0 && p.wave_items < p.target_items && s_pick_items > p.wave_items && p.batch <= p.wave_items) {
-    evaluate(p.wave_items, true);
-    __syncthreads();
-    if (tid == 0) {
-      int pick = -1;
-      for (int k = 0; k < kPlanThreads / 32; ++k) {
-        if (s_cand_items[k] <= p.wave_items) { pick = k; break; }
-      }
-      if (pick >= 0) {
-        const float one = static_cast<float>(s_cand_max[pick]) + ovh;
-        if (one < best) { best = one; s_chunk = s_cand_chunk[pick]; }
-      }
-    }
-  }
   // Dealing out: the persistent kernel's CTAs of a KV head ("slots") each take one stretch of the sequences laid end to
   // end, all of the same length with item_overhead keys added per item, cutting sequences where a stretch ends.  That is
   // about one item per sequence and one per slot instead of three per slot, and no slot ends later than another.
   const long long line = t + static_cast<long long>(p.batch + p.slots - 1) * p.item_overhead;
-  if (tid == 0 && p.slots > 1 && p.slots <= kPlanMaxSlots && cached && line < (1 << 30) && s_pick_items > p.wave_items) {
-    // (a cut moved to the end of a sequence makes a stretch up to min_chunk longer: without that in the estimate 47
-    // sequences of 350 to 5 600 keys on one KV head were dealt out and took 48 us instead of 45)
-    if (static_cast<float>(line) / static_cast<float>(p.slots) + static_cast<float>(p.min_chunk) < best) s_slots = p.slots;
+  if (warp == 0) {
+    const unsigned fit0 = __ballot_sync(0xffffffffu, s_cand_items[0][lane] <= p.target_items);
+    const unsigned fit1 = __ballot_sync(0xffffffffu, s_cand_items[1][lane] <= p.wave_items);
+    if (lane == 0) {
+      const int pick0 = fit0 ? __ffs(fit0) - 1 : kPlanThreads / 32 - 1, items0 = s_cand_items[0][pick0];
+      int pick_chunk = s_cand_chunk[0][pick0];
+      // Estimated run time of a plan in several waves, in keys: the average load of a resident CTA plus half an item.
+      const float ovh = static_cast<float>(p.item_overhead), n = static_cast<float>(items0);
+      float best = p.wave_items > 0 ? (static_cast<float>(t) + n * ovh) / static_cast<float>(p.wave_items) +
+                                          0.5f * (static_cast<float>(t) / n + ovh)
+                                    : 0.f;
+      if (try_wave && items0 > p.wave_items && fit1) {
+        const int pick1 = __ffs(fit1) - 1;
+        const float one = static_cast<float>(s_cand_max[pick1]) + ovh;
+        if (one < best) { best = one; pick_chunk = s_cand_chunk[1][pick1]; }
+      }
+      s_chunk = pick_chunk;
+      s_carry = 0;
+      // (a cut moved to the end of a sequence makes a stretch up to min_chunk longer: without that in the estimate 47
+      // sequences of 350 to 5 600 keys on one KV head were dealt out and took 48 us instead of 45)
+      const bool deal = p.slots > 1 && p.slots <= kPlanMaxSlots && cached && line < (1 << 30) && items0 > p.wave_items &&
+                        static_cast<float>(line) / static_cast<float>(p.slots) + static_cast<float>(p.min_chunk) < best;
+      s_slots = deal ? p.slots : 0;
+    }
   }
   for (int i = tid; i < p.batch * p.kv_heads; i += kPlanThreads) p.counters[i] = 0;
   __syncthreads();
@@ -527,13 +528,14 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
       if (b < n) put(b, carry + before + incl);
       __syncthreads();
       if (tid == 0) s_carry = carry + s_warp[31];
-      __syncthreads();
+      if (base + kPlanThreads < n) __syncthreads();      // (the last pass: the caller's next barrier)
     }
   };
   const int slots = s_slots;
   if (slots > 0) {
     // s_first[b]: where sequence b starts on the line
     prefix(p.batch, [&](int b) { return s_len[b] + p.item_overhead; }, [&](int b, int incl) { s_first[b + 1] = incl; });
+    __syncthreads();
     if (tid == 0) { s_first[0] = 0; s_carry = 0; }
     __syncthreads();
     const int end = s_first[p.batch];
@@ -559,6 +561,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
       s_rank[i] = incl;
       if (cut_t > 0) s_cut[incl - 1] = cut_t;
     });
+    __syncthreads();
     int* slot_first = reinterpret_cast<int*>(p.item_info + 2 * static_cast<long long>(p.max_items)) - (slots + 1);   // behind the records in use
     if (tid < slots) slot_first[tid] = cut_b + s_rank[tid];
     // cuts before sequence b, i.e. at boundaries that lie before its start
@@ -568,7 +571,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
       return k > 0 ? s_rank[k] : 0;
     };
     for (int b = tid; b < p.batch; b += kPlanThreads) {
-      const SeqInfo si = seq_info(p, b);
+      const SeqInfo si = b == tid ? mine : seq_info(p, b);
       const int r = cuts_before(b), first = b + r, n = cuts_before(b + 1) - r + 1;
       p.item_start[b + 1] = first + n;
       for (int c = 0; c < n && first + c < p.max_items; ++c) {
@@ -593,12 +596,14 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     p.item_start[b + 1] = incl;
     if (cached) s_first[b + 1] = incl;
   });
+  __syncthreads();
   // Per-item records, so that a CTA learns everything about its work item from one 32-byte read.  Records are laid
   // out in execution order: longest items first (by size class), so that the CTAs still running when the grid
   // drains are the short ones.  item_start keeps the per-sequence (logical) numbering, which is what the partial
   // results and the merge use.
+  const float class_of_key = static_cast<float>(kPlanBuckets) / static_cast<float>(chunk + 1);
   auto size_class = [&](int item_len) -> int {
-    int q = kPlanBuckets - 1 - static_cast<int>((static_cast<long long>(item_len) * kPlanBuckets) / (chunk + 1));
+    const int q = kPlanBuckets - 1 - static_cast<int>(static_cast<float>(item_len) * class_of_key);
     return q < 0 ? 0 : (q > kPlanBuckets - 1 ? kPlanBuckets - 1 : q);
   };
   // (a sequence's first n - 1 items have the same size, its last one takes the remainder: two size classes)
@@ -612,13 +617,19 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     atomicAdd(&s_hist[size_class(rem)], 1);
   }
   __syncthreads();
-  if (tid == 0) {
-    int run = 0;
-    for (int q = 0; q < kPlanBuckets; ++q) { const int c = s_hist[q]; s_hist[q] = run; run += c; }
+  if (warp == 0) {
+    static_assert(kPlanBuckets == 32, "one class per lane");
+    const int c = s_hist[lane];
+    int incl = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    s_hist[lane] = incl - c;
   }
   __syncthreads();
   for (int b = tid; b < p.batch; b += kPlanThreads) {
-    const SeqInfo si = seq_info(p, b);
+    const SeqInfo si = b == tid ? mine : seq_info(p, b);
     const int first = b == 0 ? 0 : (cached ? s_first[b] : p.item_start[b]);
     const int n = (cached ? s_first[b + 1] : p.item_start[b + 1]) - first;
     const int per = seq_chunk(si.len, n);
