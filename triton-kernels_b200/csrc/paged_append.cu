@@ -11,27 +11,45 @@ namespace b200attn {
 
 namespace {
 
+// What bounds it at the sizes it runs at (a token, a chunk) is its chain of dependent reads, each an L2 round trip: the owner
+// of a row is looked for by the whole warp, 32 prefix sums per step, together with the sequence's position and while the row
+// itself is on its way, which leaves two round trips, those and the table's, where a binary search by every lane made seven
+// of them at sixteen sequences.  APPENDUS
 __global__ void __launch_bounds__(256) paged_append_kernel(const PagedAppendParams p) {
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   const int pieces = p.row_bytes >> 4;
+  constexpr int kHeld = 4;                  // 16-byte pieces of the row that a lane holds before it knows where they go
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();
   for (long long row = warp; row < p.total_rows; row += nwarps) {
-    // sequence that owns this source row: last b with indptr[b] <= row
-    int lo = 0, hi = p.batch;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (load_index(p.src_indptr, p.indptr_is_i64, mid) <= row) lo = mid; else hi = mid;
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.src) + row * p.row_bytes);
+    uint4 held[kHeld];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i)
+      if (lane + 32 * i < pieces) held[i] = __ldcg(src + lane + 32 * i);
+    // sequence that owns this source row: the last b with indptr[b] <= row, among [lo, lo + n)
+    int lo = 0, n = p.batch;
+    while (n > 32) {
+      const int step = (n + 31) >> 5, at = lane * step;
+      const unsigned below = __ballot_sync(0xffffffffu, at < n && load_index(p.src_indptr, p.indptr_is_i64, lo + at) <= row);
+      const int k = below ? 31 - __clz(below) : 0;
+      lo += k * step;
+      n = min(step, n - k * step);
     }
-    const int b = lo;
-    const long long first = load_index(p.src_indptr, p.indptr_is_i64, b);
-    const long long end = load_index(p.src_indptr, p.indptr_is_i64, b + 1);
-    if (row < first || row >= end) continue;  // malformed prefix sums: nothing is written
-    long long pos = row - first;
-    if (p.dst_pos) pos += load_index(p.dst_pos, p.indptr_is_i64, b);
-    const long long lp = pos / p.page_size;
+    long long first = 0, end = 0, pos0 = 0;
+    if (lane < n) {
+      first = load_index(p.src_indptr, p.indptr_is_i64, lo + lane);
+      end = load_index(p.src_indptr, p.indptr_is_i64, lo + lane + 1);
+      if (p.dst_pos) pos0 = load_index(p.dst_pos, p.indptr_is_i64, lo + lane);
+    }
+    const unsigned owner = __ballot_sync(0xffffffffu, first <= row && row < end);
+    if (owner == 0) continue;                 // malformed prefix sums: nothing is written
+    const int o = 31 - __clz(owner), b = lo + o;
+    const long long pos = row - __shfl_sync(0xffffffffu, first, o) + __shfl_sync(0xffffffffu, pos0, o);
+    const long long lp = (static_cast<unsigned long long>(pos) >> 31) == 0
+                             ? static_cast<long long>(static_cast<unsigned>(pos) / static_cast<unsigned>(p.page_size)) : pos / p.page_size;
     if (pos < 0 || lp >= p.table_stride) {
       if (lane == 0) p.header[0] = DEV_ERR_PAGE_RANGE;
       continue;
@@ -42,9 +60,11 @@ __global__ void __launch_bounds__(256) paged_append_kernel(const PagedAppendPara
       continue;
     }
     const long long dst_row = static_cast<long long>(page) * p.page_size + (pos - lp * p.page_size);
-    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(p.src) + row * p.row_bytes);
     uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(p.cache) + dst_row * p.row_bytes);
-    for (int i = lane; i < pieces; i += 32) dst[i] = __ldcg(src + i);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i)
+      if (lane + 32 * i < pieces) dst[lane + 32 * i] = held[i];
+    for (int i = lane + 32 * kHeld; i < pieces; i += 32) dst[i] = __ldcg(src + i);
   }
 }
 
