@@ -920,12 +920,41 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
   constexpr int STAGE_BYTES = 2 * TILE_BYTES;
   constexpr int KSTEPS = D / 16;
 
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int NMT = p.n_mtiles;
+  const int n_cwarps = (blockDim.x >> 5) - 1;   // consumer warps
+  const int KS = n_cwarps / NMT;
+  const int mt = warp % NMT, ks = warp / NMT;   // meaningful for consumer warps only
+  const int rows_pad = NMT * 16;
+  const bool is_producer = warp == n_cwarps;
+  // (a part of a few tiles: the ring is as long as they are, or as shared memory allows)
+  const int n_stages = kCluster ? p.stages : kStages;
+
+  // smem: [stages (1024-byte aligned)] [Q rows] [control]
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* stage_base = smem;
+  unsigned char* q_smem = smem + n_stages * STAGE_BYTES;
+  DecodeCtrl* ctrl = reinterpret_cast<DecodeCtrl*>(q_smem + rows_pad * ROW_BYTES);
+  const uint32_t stage_s = smem_u32(stage_base);
+  const uint32_t q_s = smem_u32(q_smem);
+
+  // Everything that needs nothing from earlier launches comes before the wait for them.
+  if (tid == 0) {
+    for (int i = 0; i < n_stages; ++i) {
+      ptx::mbar_init(smem_u32(&ctrl->full[i]), 1);
+      ptx::mbar_init(smem_u32(&ctrl->empty[i]), n_cwarps);
+    }
+    ctrl->abort_flag = 0;
+    ptx::mbar_fence_init();
+  }
+  if (is_producer && lane == 0) { ptx::prefetch_tensormap(&tm_k); ptx::prefetch_tensormap(&tm_v); }
   ClusterPart part = {};
   __shared__ uint64_t recv_bar;
   if constexpr (kCluster) {
     part = cluster_part<D>(p);
     if (part.size > 1) cluster_begin<D>(p, part, &recv_bar);
   }
+  __syncthreads();
   ptx::grid_dep_launch_dependents();
   ptx::grid_dep_wait();      // what earlier launches wrote (the planner's records among it) is visible from here on
   // heads vary fastest across CTAs: the CTAs that run side by side walk the same pages and read
@@ -942,47 +971,10 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     if (!decode_item(p, item, s_plan, it)) return;
     h = blockIdx.x - item * p.kv_heads;
   }
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int NMT = p.n_mtiles;
-  const int n_cwarps = (blockDim.x >> 5) - 1;   // consumer warps
-  const int KS = n_cwarps / NMT;
-  const int mt = warp % NMT, ks = warp / NMT;   // meaningful for consumer warps only
-  const int rows_pad = NMT * 16;
-  const bool is_producer = warp == n_cwarps;
-
   const int b = it.b, c = it.c, n_chunks = it.n_chunks, item0 = it.item0;
   const int len = it.len;
   const int t_begin = it.t_begin, t_end = it.t_end;
   const int ntiles = t_end > t_begin ? (t_end - t_begin + kTileN - 1) / kTileN : 0;
-
-  // smem: [stages (1024-byte aligned)] [Q rows] [control]
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* stage_base = smem;
-  unsigned char* q_smem = smem + kStages * STAGE_BYTES;
-  DecodeCtrl* ctrl = reinterpret_cast<DecodeCtrl*>(q_smem + rows_pad * ROW_BYTES);
-  const uint32_t stage_s = smem_u32(stage_base);
-  const uint32_t q_s = smem_u32(q_smem);
-
-  if (tid == 0) {
-    for (int i = 0; i < kStages; ++i) {
-      ptx::mbar_init(smem_u32(&ctrl->full[i]), 1);
-      ptx::mbar_init(smem_u32(&ctrl->empty[i]), n_cwarps);
-    }
-    ctrl->abort_flag = 0;
-    ptx::mbar_fence_init();
-  }
-  // Q rows (group x drafts, contiguous in memory) -> smem, zero padded to 16-row tiles
-  {
-    const T* qg = static_cast<const T*>(p.q) +
-                  ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
-    for (int idx = tid; idx < rows_pad * CPR; idx += blockDim.x) {
-      const int row = idx / CPR, ch = idx % CPR;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (row < p.rows) val = *reinterpret_cast<const uint4*>(qg + static_cast<long long>(row) * D + ch * 8);
-      *reinterpret_cast<uint4*>(q_smem + row * ROW_BYTES + ((ch ^ (row & 7)) << 4)) = val;
-    }
-  }
-  __syncthreads();
 
   float m_used[2] = {-INFINITY, -INFINITY};  // exponent reference baked into o[] and l_run[]
   float l_run[2] = {0.f, 0.f};
@@ -994,7 +986,6 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
 
   if (is_producer) {
     // =========================== TMA producer ===========================
-    if (lane == 0) { ptx::prefetch_tensormap(&tm_k); ptx::prefetch_tensormap(&tm_v); }
     int h_coord = h;
     long long row0 = it.start;               // ragged
     if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(b) * p.kv_heads + h) * p.max_kv; }
@@ -1002,8 +993,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     int issued = 0;
     PageAhead ahead(p, lane);
     ahead.start(p, b, t_begin, t_end);
-    for (int tile = 0; tile < ntiles; ++tile) {
-      const int stage = tile % kStages, use = tile / kStages;
+    int stage = 0, use = 0;
+    for (int tile = 0; tile < ntiles; ++tile, stage = stage + 1 < n_stages ? stage + 1 : 0, use += stage == 0) {
       if (use > 0) {
         ok = warp_wait(smem_u32(&ctrl->empty[stage]), (use - 1) & 1);
         if (!ok) break;
@@ -1070,11 +1061,23 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     if (!ok) {
       if (lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; ctrl->abort_flag = 1; }
       // bounded drain of the copies still in flight before the CTA may exit
-      for (int t = max(0, issued - kStages); t < issued; ++t)
-        ptx::mbar_wait(smem_u32(&ctrl->full[t % kStages]), (t / kStages) & 1);
+      for (int t = max(0, issued - n_stages); t < issued; ++t)
+        ptx::mbar_wait(smem_u32(&ctrl->full[t % n_stages]), (t / n_stages) & 1);
     }
   } else {
     // =========================== consumers ===========================
+    // Q rows (group x drafts, contiguous in memory) -> smem, zero padded to 16-row tiles (the producer does not wait for them)
+    {
+      const T* qg = static_cast<const T*>(p.q) +
+                    ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
+      for (int idx = tid; idx < rows_pad * CPR; idx += n_cwarps * 32) {
+        const int row = idx / CPR, ch = idx % CPR;
+        uint4 val = make_uint4(0u, 0u, 0u, 0u);
+        if (row < p.rows) val = *reinterpret_cast<const uint4*>(qg + static_cast<long long>(row) * D + ch * 8);
+        *reinterpret_cast<uint4*>(q_smem + row * ROW_BYTES + ((ch ^ (row & 7)) << 4)) = val;
+      }
+      ptx::named_bar_sync(1, n_cwarps * 32);
+    }
     uint32_t qf[4];
     const int q_row = mt * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);
     const uint32_t q_rbase = q_s + q_row * ROW_BYTES;
@@ -1087,8 +1090,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
     const float sl2 = p.scale_log2;
     bool ok = true;
 
-    for (int tile = 0; tile < ntiles; ++tile) {
-      const int stage = tile % kStages, use = tile / kStages;
+    int stage = 0, use = 0;
+    for (int tile = 0; tile < ntiles; ++tile, stage = stage + 1 < n_stages ? stage + 1 : 0, use += stage == 0) {
       ok = warp_wait(smem_u32(&ctrl->full[stage]), use & 1);
       if (!ok) break;
       const uint32_t ks_base = stage_s + stage * STAGE_BYTES;
@@ -2502,9 +2505,18 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     const int threads = 32 * (nmt * ksl + 1);
     // measured on B200 (paged decode, 32/8 heads): 2 stages with Q re-read from shared memory lets three CTAs share an
     // SM and hides each CTA's start-up and merge behind its neighbours
-    const int stages = 2;
-    const size_t stage_bytes = static_cast<size_t>(stages) * 2 * kTileN * D * 2;
+    int stages = 2;
     const size_t comb_bytes = sizeof(float) * static_cast<size_t>(ksl) * nmt * 16 * (D + 2);
+    if (p.cluster) {
+      // The parts are a few tiles long: as many stages as fit with all CTAs resident, so that a part's copies are under way
+      // at once (two stages made every second tile wait for its copy; with that, and a producer that does not wait for the Q rows,
+      // 16 x 2 048 keys of two heads, D 64, take 7.5 us instead of 8.0, one sequence of 1 500 in pages, D 128, 7.5 instead of 8.8)
+      const int per_sm = static_cast<int>(std::min<long long>(3, (pairs * p.cluster + sm_count - 1) / sm_count));
+      const size_t rest = 1024 + static_cast<size_t>(nmt) * 16 * D * 2 + sizeof(DecodeCtrl) + recv_bytes + 2048;
+      while (stages < kMaxStages && (rest + static_cast<size_t>(stages + 1) * 2 * kTileN * D * 2) * per_sm <= 227u * 1024) ++stages;
+    }
+    p.stages = stages;
+    const size_t stage_bytes = static_cast<size_t>(stages) * 2 * kTileN * D * 2;
     const size_t smem = 1024 + std::max(stage_bytes, comb_bytes) + static_cast<size_t>(nmt) * 16 * D * 2 + sizeof(DecodeCtrl) + recv_bytes;
     // tensor maps over K and V: (D, heads, tokens), one box = 64 elements x 1 head x box_rows keys
     CUtensorMap tk, tv;

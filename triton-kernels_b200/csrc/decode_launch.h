@@ -55,6 +55,7 @@ struct DecodeParams {
   int slots;         // persistent kernel: CTAs per KV head that the planner may deal the batch out to; 0: none
   int inline_plan;   // 1: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs)
   int cluster;       // CTAs that share a (sequence, KV head) pair in the kernels without a plan; 0: items are planned
+  int stages;        // K/V stages of a CTA of the warp-level kernel in a cluster
   float scale_log2;  // sm_scale * log2(e)
 };
 
