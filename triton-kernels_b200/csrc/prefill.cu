@@ -150,51 +150,82 @@ __device__ __forceinline__ bool find_ragged_work(const PrefillParams& p, int x, 
   return false;
 }
 
-__device__ __forceinline__ ItemWork decode_item(const PrefillParams& p, int item, int lane) {
+// An item is decoded in two steps.  locate_item is arithmetic on the launch's sizes and reads no memory, so that a CTA does
+// it for its first item before it waits for earlier launches (a microsecond, most of it the first fetch of the code);
+// finish_item reads the lengths, and for packed sequences, whose row blocks cannot be placed without them, does all of it.
+__device__ __forceinline__ void place_heads(const PrefillParams& p, ItemWork& w, int wblock, int wunit) {
+#pragma unroll
+  for (int s = 0; s < kSlots; ++s) {
+    w.q_head[s] = p.head_pair ? wunit * 2 + s : wunit;
+    w.m0[s] = p.head_pair ? wblock * kBM : (wblock * kSlots + s) * kBM;
+  }
+}
+
+__device__ __forceinline__ ItemWork locate_item(const PrefillParams& p, int item) {
   ItemWork w;
+  w.valid = false;
+  w.len_q = w.len_k = 0;
+  w.kv_row0 = 0;
+  w.kv_tok0 = 0;
+  w.kv_head_coord = 0;
+  w.b = 0;
+  w.nkv_max = 0;
+#pragma unroll
+  for (int s = 0; s < kSlots; ++s) {
+    w.q_row0[s] = w.out_row0[s] = 0;
+    w.q_head[s] = w.q_head_coord[s] = w.m0[s] = w.nkv[s] = 0;
+  }
+  if (p.layout == B200ATTN_RAGGED) return w;
   const int heads_per_item = p.head_pair ? 2 : 1;
   const int head_units = p.q_heads / heads_per_item;
   const int rows = p.head_pair ? kBM : 2 * kBM;      // query rows an item covers
-  int wb = -1, wblock = 0, wunit = 0;
+  // row blocks are the slowest-varying index and, under a causal mask, are handed out heaviest first;
+  // the q heads of one KV head are neighbours and share its K/V in L2
+  // with a split KV range every (sequence, KV part) pair is a sequence of its own here ("virtual" batch index)
+  const int per_block = head_units * p.batch * p.kv_split;
+  const int nblocks = blocks_of(p.max_q, rows);
+  const int blk = item / per_block, rest = item - blk * per_block;
+  const int wblock = p.is_causal ? (nblocks - 1 - blk) : blk;
+  const int wunit = rest % head_units;
+  const int vb = rest / head_units;                    // virtual batch index: rows of the partial buffer
+  int part = 0;
+  w.valid = true;
+  w.b = vb;
+  if (p.kv_split > 1) { part = vb % p.kv_split; w.b = vb / p.kv_split; }
+  w.kv_tok0 = part * p.kv_split_len;
+  place_heads(p, w, wblock, wunit);
+  const int kv_head = w.q_head[0] / p.group;
+  w.len_q = p.max_q;
+#pragma unroll
+  for (int s = 0; s < kSlots; ++s) {
+    w.q_row0[s] = (static_cast<long long>(w.b) * p.q_heads + w.q_head[s]) * p.max_q;
+    w.out_row0[s] = (static_cast<long long>(vb) * p.q_heads + w.q_head[s]) * p.max_q;
+  }
+  if (p.layout == B200ATTN_DENSE) {
+    w.len_k = p.max_kv;
+    w.kv_row0 = (static_cast<long long>(w.b) * p.kv_heads + kv_head) * p.max_kv + w.kv_tok0;
+  } else {
+    w.kv_head_coord = kv_head;
+  }
+  return w;
+}
+
+__device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
   if (p.layout == B200ATTN_RAGGED) {
-    wunit = item % head_units;
+    const int heads_per_item = p.head_pair ? 2 : 1;
+    const int head_units = p.q_heads / heads_per_item;
+    const int rows = p.head_pair ? kBM : 2 * kBM;
+    int wb = -1, wblock = 0;
+    const int wunit = item % head_units;
     // Under a causal mask the row blocks are handed out from the end of the packed tensor backwards: the later
     // blocks of a sequence are the heavier ones, and the blocks left for the drain of the grid are then the first,
     // light ones of the first sequences (the sizes are not known on the host, so there is no global order by weight).
     const int nflat = p.total_items / head_units;
     const int flat = item / head_units;
-    if (!find_ragged_work(p, p.is_causal ? nflat - 1 - flat : flat, rows, lane, &wb, &wblock)) wb = -1;
-  } else {
-    // row blocks are the slowest-varying index and, under a causal mask, are handed out heaviest first;
-    // the q heads of one KV head are neighbours and share its K/V in L2
-    // with a split KV range every (sequence, KV part) pair is a sequence of its own here ("virtual" batch index)
-    const int per_block = head_units * p.batch * p.kv_split;
-    const int nblocks = blocks_of(p.max_q, rows);
-    const int blk = item / per_block, rest = item - blk * per_block;
-    wblock = p.is_causal ? (nblocks - 1 - blk) : blk;
-    wunit = rest % head_units;
-    wb = rest / head_units;
-  }
-  w.valid = wb >= 0;
-  const int vb = wb;                                   // virtual batch index: rows of the partial buffer
-  int part = 0;
-  if (p.kv_split > 1 && wb >= 0) { part = wb % p.kv_split; wb /= p.kv_split; }
-  w.b = wb;
-  w.kv_tok0 = part * p.kv_split_len;
-  w.len_q = w.len_k = 0;
-  w.kv_row0 = 0;
-  w.kv_head_coord = 0;
-#pragma unroll
-  for (int s = 0; s < kSlots; ++s) {
-    w.q_head[s] = p.head_pair ? wunit * 2 + s : wunit;
-    w.m0[s] = p.head_pair ? wblock * kBM : (wblock * kSlots + s) * kBM;
-    w.q_row0[s] = 0;
-    w.out_row0[s] = 0;
-    w.q_head_coord[s] = 0;
-  }
-  if (w.valid) {
-    const int kv_head = w.q_head[0] / p.group;
-    if (p.layout == B200ATTN_RAGGED) {
+    w.valid = find_ragged_work(p, p.is_causal ? nflat - 1 - flat : flat, rows, lane, &wb, &wblock);
+    place_heads(p, w, wblock, wunit);
+    if (w.valid) {
+      w.b = wb;
       const long long qa = load_index(p.q_indptr, p.indptr_is_i64, wb);
       const long long qe = load_index(p.q_indptr, p.indptr_is_i64, wb + 1);
       const long long ka = load_index(p.kv_indptr, p.indptr_is_i64, wb);
@@ -202,32 +233,22 @@ __device__ __forceinline__ ItemWork decode_item(const PrefillParams& p, int item
       w.len_q = static_cast<int>(qe > qa ? qe - qa : 0);
       w.len_k = static_cast<int>(ke > ka ? ke - ka : 0);
       w.kv_row0 = ka;
-      w.kv_head_coord = kv_head;
+      w.kv_head_coord = w.q_head[0] / p.group;
 #pragma unroll
       for (int s = 0; s < kSlots; ++s) { w.q_row0[s] = qa; w.out_row0[s] = qa; w.q_head_coord[s] = w.q_head[s]; }
-    } else {
-      w.len_q = p.max_q;
-#pragma unroll
-      for (int s = 0; s < kSlots; ++s) {
-        w.q_row0[s] = (static_cast<long long>(wb) * p.q_heads + w.q_head[s]) * p.max_q;
-        w.out_row0[s] = (static_cast<long long>(vb) * p.q_heads + w.q_head[s]) * p.max_q;
-      }
-      if (p.layout == B200ATTN_DENSE) {
-        w.len_k = p.max_kv;
-        w.kv_row0 = (static_cast<long long>(wb) * p.kv_heads + kv_head) * p.max_kv + w.kv_tok0;
-      } else {
-        long long n = load_index(p.kv_indptr, p.indptr_is_i64, wb);
-        const long long cap = p.table_stride * static_cast<long long>(p.page_size);
-        n = n < 0 ? 0 : (n > cap ? cap : n);
-        w.len_k = static_cast<int>(n);
-        w.kv_head_coord = kv_head;
-      }
-      if (p.kv_split > 1) {
-        // this item sees the keys [kv_tok0, kv_tok0 + kv_split_len) of the sequence only
-        int local = w.len_k - w.kv_tok0;
-        local = local < 0 ? 0 : (local > p.kv_split_len ? p.kv_split_len : local);
-        w.len_k = local;
-      }
+    }
+  } else {
+    if (p.layout == B200ATTN_PAGED) {
+      long long n = load_index(p.kv_indptr, p.indptr_is_i64, w.b);
+      const long long cap = p.table_stride * static_cast<long long>(p.page_size);
+      n = n < 0 ? 0 : (n > cap ? cap : n);
+      w.len_k = static_cast<int>(n);
+    }
+    if (p.kv_split > 1) {
+      // this item sees the keys [kv_tok0, kv_tok0 + kv_split_len) of the sequence only
+      int local = w.len_k - w.kv_tok0;
+      local = local < 0 ? 0 : (local > p.kv_split_len ? p.kv_split_len : local);
+      w.len_k = local;
     }
   }
   w.nkv_max = 0;
@@ -242,7 +263,6 @@ __device__ __forceinline__ ItemWork decode_item(const PrefillParams& p, int item
     w.nkv[s] = n;
     w.nkv_max = max(w.nkv_max, n);
   }
-  return w;
 }
 
 // Persistent kernel: one CTA per SM; work items are drawn from a global counter (heaviest first).
@@ -303,6 +323,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   if (warp == kProducerWarp) {
     // =========================== scheduler + TMA producer ===========================
     if (lane == 0) { prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); }
+    // the first item of a CTA is its own index (the grid never exceeds the item count); later ones are drawn
+    ItemWork w = locate_item(p, static_cast<int>(blockIdx.x));
     // everything the other warps read or write outside this CTA follows an item published or a tile loaded below
     ptx::grid_dep_wait();
     bool ok = true;
@@ -322,6 +344,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     int pair_e = 0;       // K/V pairs issued so far, across items
     int q_uses = 0;       // Q tiles issued (or skipped) so far
     int pair_lo = 0;      // first pair of the current item
+    auto first_pages = [&](const int* table, const ItemWork& it) -> int {
+      const long long tg = static_cast<long long>(lane << box_shift) + it.kv_tok0;
+      const long long lp = page_pow2 ? tg >> page_shift : tg / p.page_size;
+      return lp < p.table_stride ? __ldcg(table + static_cast<long long>(it.b) * p.table_stride + lp) : kNoPage;
+    };
     for (int k = 0; ok; ++k) {
       if (k >= 2) {
         ok = warp_wait(smem_u32(&ctrl->sched_empty[k & 1]), ((k >> 1) - 1) & 1);
@@ -329,13 +356,19 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       int item = -1;
       if (lane == 0) {
-        // the first item of a CTA is its own index (the grid never exceeds the item count); later ones are drawn
         item = k == 0 ? static_cast<int>(blockIdx.x) : static_cast<int>(gridDim.x) + atomicAdd(p.work_counter, 1);
         if (item >= p.total_items) item = -1;
       }
       item = __shfl_sync(0xffffffffu, item, 0);
-      ItemWork w;
-      if (item >= 0) w = decode_item(p, item, lane);
+      if (item >= 0) {
+        if (k > 0) w = locate_item(p, item);
+        // (the entries of a table row may be read before the sequence's length is known: which of them count is decided later)
+        if (pf) {
+          pg_k = first_pages(p.k_table, w);
+          pg_v = first_pages(p.v_table, w);
+        }
+        finish_item(p, w, item, lane);
+      }
       if (lane == 0) {
         if (item >= 0) ctrl->sched_work[k & 1] = w;
         ctrl->sched_item[k & 1] = item;
@@ -351,8 +384,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // (a cache without a whole page: no entry can be right, and the tiles have no boxes whose entries would be checked)
       if (pf && p.num_pages <= 0 && w.nkv_max > 0 && lane == 0) p.header[0] = DEV_ERR_PAGE_RANGE;
       if (pf && w.nkv_max > 0) {
-        pg_k = read_page(ktab, 0);
-        pg_v = read_page(vtab, 0);
         if (w.len_k > (32 << box_shift)) {
           pg_k_next = read_page(ktab, 32);
           pg_v_next = read_page(vtab, 32);
