@@ -868,27 +868,41 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             pq[2 * i + 1] = exp_pair(v[4 * i + 2], v[4 * i + 3], negb_2, rs_b);
           }
         };
+        float mx_a = -INFINITY, mx_b = -INFINITY;       // maxima over this thread's columns
+        auto max_quarter = [&](const uint32_t (&v)[16]) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            mx_a = max3(mx_a, __uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]));
+            mx_b = max3(mx_b, __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+          }
+        };
         float sum_a, sum_b;     // row sums over this thread's columns
         auto pair_sum = [](uint64_t v) {
           float x, y;
           unpack_f2(v, x, y);
           return x + y;
         };
-        // One pass where no row's exponent reference has to move, which is nearly every tile but an item's first: the
+        // One pass where no row's exponent reference has to move, which is nearly every tile: the
         // scores are exponentiated, as they arrive, against the reference that stands, and the sums, needed anyhow, tell
         // afterwards whether it could stand: no maximum is computed, no exponential waits for one, nothing is exchanged
         // between threads, and the tile is read from tensor memory once.  P stays in registers until the verdict: if a row
         // has to move, the scores are still there for the two passes below.
+        // An item's first tile takes the maximum of its first 32 columns for a reference.
         bool done = false;
-        if (j > 0 && lo >= kBN - 1) {
-          // (a row without a reference yet has -inf here: its sum is then no number and the verdict is no)
-          nega_2 = pack_f2(-m_a, -m_a);
-          negb_2 = pack_f2(-m_b, -m_b);
+        if (lo >= kBN - 1) {
           uint32_t pk[2][16];
           uint32_t v0[16], v1[16];
           tmem_ld_16x256b_x4(tS, v0);
           tmem_wait_ld_regs(v0);
           tmem_ld_16x256b_x4(tS + 32, v1);
+          if (j == 0) {
+            max_quarter(v0);
+            m_a = quad_max(mx_a) * sl2;
+            m_b = quad_max(mx_b) * sl2;
+          }
+          // (a row without a reference yet has -inf here: its sum is then no number and the verdict is no)
+          nega_2 = pack_f2(-m_a, -m_a);
+          negb_2 = pack_f2(-m_b, -m_b);
           exp_quarter(v0, pk[0]);
           tmem_wait_ld_regs(v1);
           tmem_ld_16x256b_x4(tS + 64, v0);
@@ -907,7 +921,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
         }
         if (!done) {
-          // Two passes, 32 columns at a time: an item's first tile, a tile with hidden columns, a row whose reference moves.
+          // Two passes, 32 columns at a time: a tile with hidden columns, a row whose reference moves.
           // Columns hidden from all sixteen rows are neither read nor exponentiated.
           auto mask_quarter = [&](uint32_t (&v)[16], int c) {
             const int ta = min(len_k - 1, p.is_causal ? row0_abs + (lane >> 2) : 0x7fffffff) - j * kBN - c * 32 - 2 * q;
@@ -921,7 +935,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
               }
             }
           };
-          float mx_a = -INFINITY, mx_b = -INFINITY;       // maxima over this thread's columns
+          mx_a = mx_b = -INFINITY;
           rs_a = rs_b = pack_f2(0.f, 0.f);
 #pragma unroll 1
           for (int c = 0; c < 4 && c * 32 <= hi; ++c) {
@@ -929,11 +943,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             tmem_ld_16x256b_x4(tS + c * 32, v);
             tmem_wait_ld_regs(v);
             if (lo < c * 32 + 31) mask_quarter(v, c);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              mx_a = max3(mx_a, __uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]));
-              mx_b = max3(mx_b, __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-            }
+            max_quarter(v);
           }
           mx_a = quad_max(mx_a);
           mx_b = quad_max(mx_b);
