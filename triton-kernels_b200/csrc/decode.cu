@@ -1765,15 +1765,22 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         };
         float sum;
         bool done = false;
-        // One pass where no row's exponent reference has to move, which is nearly every tile but a unit's first: against the
-        // reference that stands, with the sum to tell whether it could (see kMaxRowSum); P stays in registers until then.
-        if (tile > 0 && first_lim - t0 >= kTileN - 1) {
+        // One pass where no row's exponent reference has to move, which is nearly every tile: against the reference that
+        // stands, with the sum to tell whether it could (see kMaxRowSum); P stays in registers until then.  A unit's first
+        // tile takes the maximum of its first 16 columns for a reference.
+        if (first_lim - t0 >= kTileN - 1) {
           uint32_t va[16], vb[16], pk[32];
           rs = pack_f2(0.f, 0.f);
-          neg_m = -m_used;             // (+inf for a row without a reference yet: the sum is then no number)
           tmem_ld16(tS, va);
           tmem_wait_ld_regs(va);
           tmem_ld16(tS + 16, vb);
+          if (tile == 0) {
+            float mx = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) mx = max3(mx, __uint_as_float(va[i]), __uint_as_float(va[i + 1]));
+            m_used = mx * sl2;
+          }
+          neg_m = -m_used;             // (+inf for a row without a reference yet: the sum is then no number)
           exp_part(va, pk);
           tmem_wait_ld_regs(vb);
           tmem_ld16(tS + 32, va);
@@ -1788,7 +1795,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
           if (done) tmem_st32(tS, pk);
         }
         if (!done) {
-          // two passes, 16 columns at a time: a unit's first tile, hidden columns, a reference that moves
+          // two passes, 16 columns at a time: hidden columns, a reference that moves
           auto load_part = [&](uint32_t (&v)[16], int c) {
             tmem_ld16(tS + c * 16, v);
             tmem_wait_ld_regs(v);
