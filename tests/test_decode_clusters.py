@@ -82,3 +82,14 @@ def test_calls_in_a_row_and_in_a_graph():
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, first)
+
+
+@pytest.mark.parametrize("qh,kvh", [(16, 1), (17, 1), (64, 1), (128, 1), (96, 2)])
+def test_fp32_rows_either_side_of_the_line(qh, kvh):
+    """fp32 decode takes any number of q rows per KV head; up to sixteen of them share a cluster."""
+    gen = torch.Generator().manual_seed(qh)
+    for d in (64, 128):
+        lens = [300, 40]
+        qs, ks, vs = _problem(gen, lens, qh, kvh, d, torch.float32)
+        out = _call(qs, ks, vs, "ragged", 0)
+        assert_close_both(out, _reference(qs, ks, vs, qh, kvh, 0), torch.float32, 300, f"fp32 {qh}/{kvh} d{d}")

@@ -25,10 +25,18 @@ static __global__ void __launch_bounds__(256) cast_f32_to_f16_kernel(const CastJ
   const float4* src = t == 0 ? job.src[0] : (t == 1 ? job.src[1] : job.src[2]);
   uint2* dst = t == 0 ? job.dst[0] : (t == 1 ? job.dst[1] : job.dst[2]);
   const long long n4 = t == 0 ? job.n4[0] : (t == 1 ? job.n4[1] : job.n4[2]);
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float4 x = __ldcg(src + i);
-    dst[i] = make_uint2(ElemTraits<__half>::pack2(x.x, x.y), ElemTraits<__half>::pack2(x.z, x.w));
+  // (four loads in flight per thread: one left an SM with 32 KB on the way.  One prompt of 512: 14.2 -> 13.8 us
+  // a call; 4 x 4 096, 8 heads, D 64: 217 -> 213)
+  constexpr int kLoads = 4;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n4; i += kLoads * step) {
+    float4 x[kLoads];
+#pragma unroll
+    for (int j = 0; j < kLoads; ++j)
+      if (i + j * step < n4) x[j] = __ldcg(src + i + j * step);
+#pragma unroll
+    for (int j = 0; j < kLoads; ++j)
+      if (i + j * step < n4) dst[i + j * step] = make_uint2(ElemTraits<__half>::pack2(x[j].x, x[j].y), ElemTraits<__half>::pack2(x[j].z, x[j].w));
   }
 }
 

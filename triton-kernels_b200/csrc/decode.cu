@@ -2431,7 +2431,8 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   // the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
   // in every call.
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
-  p.cluster = a.dtype == B200ATTN_F32 || p.rows <= 16 ? cluster_size(a, sm_count) : 0;
+  // (fp32 rows beyond sixteen: what the CTAs send one another would not fit beside the copy ring)
+  p.cluster = p.rows <= 16 ? cluster_size(a, sm_count) : 0;
   p.inline_plan = !built_in && !p.cluster && (a.dtype == B200ATTN_F32 || p.rows <= 16) && pairs <= kInlinePairs ? 1 : 0;
   unsigned grid_items = static_cast<unsigned>(w.max_items);
   cudaError_t e = cudaSuccess;

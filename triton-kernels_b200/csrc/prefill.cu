@@ -1052,7 +1052,9 @@ namespace {
 // Merge of the parts of a split KV range.  part[(b * parts + s)][h][r][:] holds the normalised output of part s and
 // lse[...] its log-sum-exp (log2 domain): out = sum_s 2^(lse_s - max) part_s / sum_s 2^(lse_s - max)
 // (the reference's merge kernel, kernels/attention.py:659-746, on normalised instead of raw accumulators).
-template <typename OutT, int D>
+constexpr int kMaxParts = 8;       // split_plan cuts no finer
+// kParts: parts that registers are held for (two parts in the form for eight are 1 % slower: 70 registers a thread)
+template <typename OutT, int D, int kParts>
 __global__ void __launch_bounds__(256) prefill_merge_kernel(const OutT* part, const float* lse, OutT* out,
                                                             long long rows_per_batch, int batch, int parts) {
   ptx::grid_dep_launch_dependents();
@@ -1065,21 +1067,35 @@ __global__ void __launch_bounds__(256) prefill_merge_kernel(const OutT* part, co
     const int piece = static_cast<int>(idx % PIECES);
     const long long row = idx / PIECES;                    // (b, h, r) flattened
     const long long b = row / rows_per_batch, hr = row - b * rows_per_batch;
+    // (all reads of a piece are on their way at once: a loop over the parts was a chain of L2 round trips.  128 queries over
+    // 8 192 keys, eight parts: 23.1 -> 21.7 us)
+    float l[kParts];
+    uint4 u[kParts];
+#pragma unroll
+    for (int sp = 0; sp < kParts; ++sp) {
+      if (sp < parts) {
+        const long long prow = (b * parts + sp) * rows_per_batch + hr;
+        l[sp] = __ldcg(lse + prow);
+        u[sp] = __ldcg(reinterpret_cast<const uint4*>(part + prow * D) + piece);
+      }
+    }
     float mx = -INFINITY;
-    for (int sp = 0; sp < parts; ++sp) mx = fmaxf(mx, __ldcg(lse + (b * parts + sp) * rows_per_batch + hr));
+#pragma unroll
+    for (int sp = 0; sp < kParts; ++sp)
+      if (sp < parts) mx = fmaxf(mx, l[sp]);
     float acc[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; ++i) acc[i] = 0.f;
     float wsum = 0.f;
-    for (int sp = 0; sp < parts; ++sp) {
-      const long long prow = (b * parts + sp) * rows_per_batch + hr;
-      const float l = __ldcg(lse + prow);
-      const float w = (l == -INFINITY) ? 0.f : fast_exp2(l - mx);
-      wsum += w;
-      const uint4 u = __ldcg(reinterpret_cast<const uint4*>(part + prow * D) + piece);
-      const OutT* e = reinterpret_cast<const OutT*>(&u);
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) acc[i] += w * ElemTraits<OutT>::to_float(e[i]);
+    for (int sp = 0; sp < kParts; ++sp) {
+      if (sp < parts) {
+        const float w = (l[sp] == -INFINITY) ? 0.f : fast_exp2(l[sp] - mx);
+        wsum += w;
+        const OutT* e = reinterpret_cast<const OutT*>(&u[sp]);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) acc[i] += w * ElemTraits<OutT>::to_float(e[i]);
+      }
     }
     const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
     uint4 o;
@@ -1127,7 +1143,7 @@ SplitPlan split_plan(const b200attn_prefill_args_t& a, int sm_count) {
   };
   long long best = 1;
   double best_cost = cost(1);
-  for (long long parts = 2; parts <= 8 && tiles / parts >= 4; parts *= 2) {
+  for (long long parts = 2; parts <= kMaxParts && tiles / parts >= 4; parts *= 2) {
     const double c = cost(parts);
     if (c < 0.85 * cost(1) && c < best_cost) { best = parts; best_cost = c; }
   }
@@ -1300,7 +1316,8 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
     const long long pieces = static_cast<long long>(a.batch) * rows_per_batch * (D / (f32 ? 4 : 8));
     const int blocks = static_cast<int>(std::min<long long>((pieces + 255) / 256, static_cast<long long>(sm_count) * 8));
 #define B200ATTN_LAUNCH_MERGE(OUT, DIM)                                                                              \
-    launch_dependent(prefill_merge_kernel<OUT, DIM>, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1,          \
+    launch_dependent(p.kv_split <= 2 ? prefill_merge_kernel<OUT, DIM, 2> : prefill_merge_kernel<OUT, DIM, kMaxParts>, \
+                     dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1,                                          \
                      static_cast<const OUT*>(p.out), static_cast<const float*>(p.lse), static_cast<OUT*>(a_in.out),   \
                      rows_per_batch, a.batch, p.kv_split)
     if (f32) { if (D == 128) B200ATTN_LAUNCH_MERGE(float, 128); else B200ATTN_LAUNCH_MERGE(float, 64); }
