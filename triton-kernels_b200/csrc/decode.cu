@@ -1768,12 +1768,22 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         // One pass where no row's exponent reference has to move, which is nearly every tile: against the reference that
         // stands, with the sum to tell whether it could (see kMaxRowSum); P stays in registers until then.  A unit's first
         // tile takes the maximum of its first 16 columns for a reference.
-        if (first_lim - t0 >= kTileN - 1) {
+        // Hidden columns (the draft-causal tail, the sequence's end) are -inf on the way: a row that sees nothing yet has no
+        // reference, and its sum no number.
+        {
+          const bool full = first_lim - t0 >= kTileN - 1;
+          auto hide = [&](uint32_t (&v)[16], int c) {
+            if (full) return;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (c * 16 + i > limit) v[i] = 0xff800000u;          // -inf
+          };
           uint32_t va[16], vb[16], pk[32];
           rs = pack_f2(0.f, 0.f);
           tmem_ld16(tS, va);
           tmem_wait_ld_regs(va);
           tmem_ld16(tS + 16, vb);
+          hide(va, 0);
           if (tile == 0) {
             float mx = -INFINITY;
 #pragma unroll
@@ -1784,18 +1794,21 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
           exp_part(va, pk);
           tmem_wait_ld_regs(vb);
           tmem_ld16(tS + 32, va);
+          hide(vb, 1);
           exp_part(vb, pk + 8);
           tmem_wait_ld_regs(va);
           tmem_ld16(tS + 48, vb);
+          hide(va, 2);
           exp_part(va, pk + 16);
           tmem_wait_ld_regs(vb);
+          hide(vb, 3);
           exp_part(vb, pk + 24);
           sum = row_sum();
           done = __all_sync(0xffffffffu, sum <= kMaxRowSum);
           if (done) tmem_st32(tS, pk);
         }
         if (!done) {
-          // two passes, 16 columns at a time: hidden columns, a reference that moves
+          // two passes, 16 columns at a time: a reference that moves
           auto load_part = [&](uint32_t (&v)[16], int c) {
             tmem_ld16(tS + c * 16, v);
             tmem_wait_ld_regs(v);
@@ -2373,7 +2386,9 @@ namespace {
 //   paged: the longest sequence is known (the table's width), the others may be shorter, and a plan would make use of that:
 //     a quarter of the dense limit, where the worst case, half of the keys not there, still breaks even.
 //   ragged: the average is known; half of that again, and no part longer than 1 MiB whatever the lengths.
-int cluster_size(const b200attn_decode_args_t& a, int sm_count) {
+//   fp32: the FMA kernel's time goes with the rows as well; beyond two rows (four where the CTAs fill the GPU) the limit shrinks
+//     with them (8/1 heads, D 64, 1 x 1 024 14.6 -> 11.0 us, but 1 x 2 048 15.8 -> 17.0 and 1 x 4 096 18.0 -> 29.0).
+int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
   if (pairs <= 0) return 0;
   const bool ragged = a.layout == B200ATTN_RAGGED, dense = a.layout == B200ATTN_DENSE;
@@ -2384,7 +2399,8 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count) {
   long long c = 8;
   while (c > 1 && (pairs * c > 3ll * sm_count || tiles <= c / 2)) c /= 2;
   const bool full = pairs * c >= 2ll * sm_count;
-  const long long limit = (dense ? (full ? 512 : 256) : ragged ? (full ? 64 : 128) : (full ? 128 : 256)) * 1024ll;
+  long long limit = (dense ? (full ? 512 : 256) : ragged ? (full ? 64 : 128) : (full ? 128 : 256)) * 1024ll;
+  if (a.dtype == B200ATTN_F32) limit = limit * (full ? 4 : 2) / std::max(rows, full ? 4 : 2);
   if ((tiles + c - 1) / c * tile_bytes > limit) return 0;
   if (ragged && a.total_kv / kTileN * tile_bytes > c * (1ll << 20)) return 0;
   return static_cast<int>(c);
@@ -2432,7 +2448,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   // in every call.
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
   // (fp32 rows beyond sixteen: what the CTAs send one another would not fit beside the copy ring)
-  p.cluster = p.rows <= 16 ? cluster_size(a, sm_count) : 0;
+  p.cluster = p.rows <= 16 ? cluster_size(a, sm_count, p.rows) : 0;
   p.inline_plan = !built_in && !p.cluster && (a.dtype == B200ATTN_F32 || p.rows <= 16) && pairs <= kInlinePairs ? 1 : 0;
   unsigned grid_items = static_cast<unsigned>(w.max_items);
   cudaError_t e = cudaSuccess;
