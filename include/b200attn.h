@@ -212,6 +212,14 @@ int b200attn_decode_static_check(int device, void* cuda_stream, int32_t* code);
 int b200attn_selftest_wait_expiry(int device, void* workspace, uint32_t tries, void* cuda_stream);
 
 /*
+ * Self-test of a decode cluster whose second CTA (of two) is late: with `late` != 0 it sends its part only after the
+ * first CTA's wait for it, `tries` attempts (1..2^14) four times over, has run out.  out (65 floats, device): the merged
+ * row of 64, of which the first CTA then writes its half as NaN, and 1 where everything sent to the first CTA had landed
+ * before it left.  Code 1 in word 0 of `workspace` (>= 256 bytes, zeroed) as above.  No counterpart in the reference.
+ */
+int b200attn_selftest_cluster_expiry(int device, void* workspace, float* out, uint32_t tries, int late, void* cuda_stream);
+
+/*
  * Paged KV-cache append: copies the new rows of every sequence into the pages its block table names.
  *   src        [total_rows, heads, head_dim]  new K (or V) rows of all sequences, packed
  *   src_indptr [B+1] prefix sums over src rows;  dst_pos [B] position in each sequence of its first new row

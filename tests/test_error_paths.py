@@ -43,3 +43,34 @@ def test_wait_expiry_selftest_rejects_unbounded_limits():
     assert lib.b200attn_selftest_wait_expiry(torch.cuda.current_device(), C.c_void_p(ws.data_ptr()), 0, stream) == -1
     assert lib.b200attn_selftest_wait_expiry(torch.cuda.current_device(), C.c_void_p(ws.data_ptr()), (1 << 20) + 1, stream) == -1
     assert lib.b200attn_selftest_wait_expiry(torch.cuda.current_device(), None, 16, stream) == -1
+
+
+@pytest.mark.parametrize("late", [0, 1])
+def test_cluster_waits_for_a_late_cta_before_it_leaves(late):
+    """A decode CTA that gave up on a peer's part reports it, and is still there when the part arrives."""
+    from kernels import _native
+
+    lib = _native.lib()
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    ws = torch.zeros(256, dtype=torch.uint8, device="cuda")
+    out = torch.full((65,), -1.0, device="cuda")
+    _native.check(lib.b200attn_selftest_cluster_expiry(torch.cuda.current_device(), C.c_void_p(ws.data_ptr()),
+                                                       C.c_void_p(out.data_ptr()), 1 << 10, late, stream),
+                  "b200attn_selftest_cluster_expiry")
+    code = C.c_int32(0)
+    rc = lib.b200attn_check_workspace(C.c_void_p(ws.data_ptr()), stream, C.byref(code))
+    assert (rc, code.value) == ((-6, 1) if late else (0, 0))
+    assert out[64] == 1, "the first CTA left while the second still had stores on the way to it"
+    assert (out[32:64] == 1.5).all()                 # the second CTA's half: the mean of 1 and 2
+    assert torch.isnan(out[:32]).all() if late else (out[:32] == 1.5).all()
+
+
+def test_cluster_selftest_rejects_what_it_cannot_bound():
+    from kernels import _native
+
+    lib = _native.lib()
+    stream, dev = C.c_void_p(torch.cuda.current_stream().cuda_stream), torch.cuda.current_device()
+    ws, out = torch.zeros(256, dtype=torch.uint8, device="cuda"), torch.zeros(65, device="cuda")
+    w, o = C.c_void_p(ws.data_ptr()), C.c_void_p(out.data_ptr())
+    for args in ((w, o, 0), (w, o, (1 << 14) + 1), (None, o, 16), (w, None, 16)):
+        assert lib.b200attn_selftest_cluster_expiry(dev, *args, 1, stream) == -1

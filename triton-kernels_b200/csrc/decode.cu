@@ -294,9 +294,11 @@ __device__ __forceinline__ void cluster_item(const DecodeParams& p, const Cluste
 }
 
 // `recv`: shared memory for the pieces ([CTA][share] of 16 bytes) and the rows' (m, l) ([CTA][row]) sent to this CTA.
+// Every CTA of the cluster comes here, also one that gave up on a copy: it sends its rows as NaN.  `tries`: limit of a wait.
 template <typename T, int D>
 __device__ __forceinline__ void cluster_emit(const DecodeParams& p, const ClusterPart& cp, int b, int h, const float* comb_o,
-                                             const float* comb_ml, int KS, int rows_pad, unsigned char* recv, uint64_t* bar) {
+                                             const float* comb_ml, int KS, int rows_pad, unsigned char* recv, uint64_t* bar,
+                                             uint32_t tries = ptx::kWaitTries) {
   constexpr int D4 = D / 4;
   const int R = p.rows;
   const uint32_t bar_s = smem_u32(bar), recv_o = smem_u32(recv), recv_ml = recv_o + cp.size * cp.share * 16;
@@ -322,10 +324,17 @@ __device__ __forceinline__ void cluster_emit(const DecodeParams& p, const Cluste
   }
   const int first = cp.rank * cp.share, n = min(cp.share, cp.total - first);
   if (n <= 0) return;                    // (nothing is sent to this CTA)
-  // (four times a wait of its own: a CTA of the cluster that gave up on a copy still sends its rows, as NaN)
-  bool ok = false;
-  for (int i = 0; i < 4 && !ok; ++i) ok = ptx::mbar_wait(bar_s, 0);
-  if (!ok) p.header[0] = DEV_ERR_WAIT_EXPIRED;
+  const bool ok = __all_sync(0xffffffffu, ptx::mbar_wait_limit(bar_s, 0, 4 * tries));
+  if (!ok) {
+    // A peer is late by more than that (one that gives up on a copy first drains its others, a limit each, and limits of
+    // different CTAs do not compare).  This CTA may not leave: the peer still stores into its shared memory.  Each peer either
+    // comes to the cluster's barrier here, having sent everything, or has left after doing so, and every wait on its way
+    // has a limit; what has been sent then only has to land.
+    p.header[0] = DEV_ERR_WAIT_EXPIRED;
+    ptx::cluster_arrive();
+    ptx::cluster_wait();
+    ptx::mbar_wait_limit(bar_s, 0, tries);
+  }
   T* out = static_cast<T*>(p.out) +
            ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
   const float4* po = reinterpret_cast<const float4*>(recv);
@@ -2673,6 +2682,46 @@ int check_decode_static(int device, cudaStream_t stream, int32_t* code) {
   set_error("a decode_static kernel reported device error code %d (1 = bounded wait expired, 2 = block-table entry "
             "out of range, 3 = planner overflow)", word);
   return B200ATTN_E_DEVICE;
+}
+
+// ---------------------------------------------------------------------------
+// Self-test of a cluster in which one CTA is late: of two CTAs that share a row the second sends its part only after the
+// first has run out of patience (a bounded wait on a barrier that nothing completes, much longer than the first's).
+// out[0 .. 63]: the row, out[64]: 1 when everything sent to the first CTA had landed by the time it left cluster_emit.
+// ---------------------------------------------------------------------------
+namespace {
+__global__ void __launch_bounds__(64) cluster_expiry_selftest_kernel(const DecodeParams p, uint32_t tries, int late) {
+  constexpr int D = 64;
+  __shared__ __align__(16) float comb_o[D];
+  __shared__ float comb_ml[2];
+  __shared__ __align__(16) unsigned char recv[2 * (D / 8) * 16 + 2 * 8];
+  __shared__ uint64_t recv_bar, dead_bar;
+  const ClusterPart part = cluster_part<D>(p);
+  cluster_begin<D>(p, part, &recv_bar);
+  ptx::grid_dep_wait();      // (the caller's zero fill of the header)
+  comb_o[threadIdx.x] = static_cast<float>(part.rank + 1);
+  if (threadIdx.x == 0) {
+    comb_ml[0] = 0.f;
+    comb_ml[1] = 1.f;
+    ptx::mbar_init(smem_u32(&dead_bar), 1);
+    ptx::mbar_fence_init();
+  }
+  __syncthreads();
+  if (late && part.rank == 1) ptx::mbar_wait_limit(smem_u32(&dead_bar), 0, 64 * tries);
+  __syncthreads();
+  cluster_emit<float, D>(p, part, 0, 0, comb_o, comb_ml, 1, 1, recv, &recv_bar, tries);
+  if (part.rank == 0 && threadIdx.x == 0) static_cast<float*>(p.out)[D] = ptx::mbar_try_wait(smem_u32(&recv_bar), 0) ? 1.f : 0.f;
+}
+}  // namespace
+
+int launch_cluster_selftest(int* header, float* out, uint32_t tries, int late, cudaStream_t stream) {
+  DecodeParams p = {};
+  p.header = header;
+  p.out = out;
+  p.cluster = 2;
+  p.batch = p.q_heads = p.kv_heads = p.group = p.head_stride = p.q_len = p.rows = 1;
+  const cudaError_t e = launch_dependent(cluster_expiry_selftest_kernel, dim3(2), 64, 0, stream, 2, p, tries, late);
+  return e == cudaSuccess ? B200ATTN_OK : cuda_fail(e, "cluster selftest kernel launch");
 }
 
 }  // namespace b200attn

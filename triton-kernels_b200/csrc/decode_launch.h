@@ -84,5 +84,6 @@ DecodeWsLayout decode_ws_layout(const b200attn_decode_args_t& a, int sm_count, b
 int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, bool built_in = false);
 int launch_decode_static(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream);
 int check_decode_static(int device, cudaStream_t stream, int32_t* code);
+int launch_cluster_selftest(int* header, float* out, uint32_t tries, int late, cudaStream_t stream);
 
 }  // namespace b200attn
