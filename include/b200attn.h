@@ -41,6 +41,9 @@ enum { B200ATTN_F16 = 0, B200ATTN_BF16 = 1, B200ATTN_F32 = 2 };
 /* K/V layout (reference "TYPE" 0/1/2: kernels/attention.py:785,810,832) */
 enum { B200ATTN_DENSE = 0, B200ATTN_RAGGED = 1, B200ATTN_PAGED = 2 };
 
+/* b200attn_decode_route: 1 .. 8 are CTAs per (sequence, KV head) pair of a call in clusters */
+enum { B200ATTN_ROUTE_PLANNER = 0, B200ATTN_ROUTE_INLINE = 16 };
+
 /* status codes */
 enum {
   B200ATTN_OK = 0,
@@ -162,6 +165,14 @@ int b200attn_device_info(int device, b200attn_device_info_t* info);
  */
 size_t b200attn_prefill_workspace_bytes(const b200attn_prefill_args_t* args);
 size_t b200attn_decode_workspace_bytes(const b200attn_decode_args_t* args);
+
+/*
+ * Which way b200attn_decode (`is_static`: b200attn_decode_static) takes a call on a GPU of `sm_count` SMs: in clusters of 1, 2, 4
+ * or 8 CTAs per (sequence, KV head) pair, in items that the CTAs plan for themselves (B200ATTN_ROUTE_INLINE) or behind the
+ * planner's launch (B200ATTN_ROUTE_PLANNER).  Host arithmetic on the sizes; needs no GPU, reads no pointer.  No counterpart in
+ * the reference.
+ */
+int b200attn_decode_route(const b200attn_decode_args_t* args, int sm_count, int is_static);
 
 int b200attn_prefill(const b200attn_prefill_args_t* args, void* cuda_stream);
 int b200attn_decode(const b200attn_decode_args_t* args, void* cuda_stream);

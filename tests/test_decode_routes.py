@@ -1,0 +1,86 @@
+"""Which way a decode call goes: clusters, items that the CTAs plan for themselves, or items behind the planner.  The rule is
+host arithmetic of the library; what it may not do is checked without a GPU."""
+import ctypes as C
+
+import pytest
+
+PLANNER, INLINE = 0, 16           # include/b200attn.h
+SMS = 148
+
+
+def route(layout, dtype, batch, qh, kvh, d, keys, m=1, total=None, static=False, page=16, sms=SMS):
+    """``keys``: per sequence (dense), on average (ragged), of the block table (paged)."""
+    from kernels import _native
+
+    a = _native.DecodeArgs()
+    a.layout = {"dense": _native.DENSE, "ragged": _native.RAGGED, "paged": _native.PAGED}[layout]
+    a.dtype = {"fp16": _native.F16, "bf16": _native.BF16, "fp32": _native.F32}[dtype]
+    a.batch, a.q_heads, a.kv_heads, a.head_dim, a.q_len = batch, qh, kvh, d, m
+    a.max_kv = keys
+    a.page_size, a.table_stride = page, -(-keys // page)
+    a.total_kv = total if total is not None else batch * keys
+    return _native.lib().b200attn_decode_route(C.byref(a), sms, int(static))
+
+
+def test_arguments_that_mean_nothing_are_refused():
+    assert route("dense", "bf16", 1, 8, 0, 64, 100) < 0
+    assert route("dense", "bf16", 1, 7, 2, 64, 100) < 0
+    assert route("dense", "bf16", 1, 8, 2, 64, 100, sms=0) < 0
+    assert route("dense", "bf16", 0, 8, 2, 64, 100) in (PLANNER, INLINE)
+
+
+# A CTA takes about 0.5 us per tile of 64 keys and 64 elements of a head in 16 bits; in fp32 0.8, 1.5, 3 and 6 us at 1, 4, 8 and 16
+# rows.  A call behind the planner takes some 15 us with one long sequence, one without a planner launch 10 to 12, and its
+# shortest items are two tiles.
+def _tile_us(dtype, d, rows):
+    if dtype != "fp32":
+        return 0.46 if d == 64 else 0.8
+    return (0.83 if rows == 1 else 1.1 if rows == 2 else 1.5 if rows <= 4 else 3.0 if rows <= 8 else 6.0) * d / 64
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp32"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("rows", [1, 2, 4, 8, 16])
+def test_no_part_of_a_cluster_outlasts_a_planned_call(dtype, d, rows):
+    """Also where one packed sequence holds all keys, or one of a paged batch fills the table."""
+    for batch, kvh in ((1, 1), (2, 1), (4, 1), (16, 1), (4, 2), (16, 2), (4, 8), (13, 8), (32, 8), (100, 8)):
+        for keys in (1, 20, 64, 100, 128, 250, 500, 1000, 2000, 4000, 8000):
+            own = 2 * _tile_us(dtype, d, rows) if dtype == "fp32" else 0
+            for layout, longest in (("ragged", batch * keys), ("paged", keys)):
+                c = route(layout, dtype, batch, rows * kvh, kvh, d, keys)
+                if 1 <= c <= 8:
+                    part = -(--(-longest // 64) // c) * _tile_us(dtype, d, rows)
+                    assert part <= (15 if batch * kvh > 96 else 8) + own, (layout, batch, kvh, keys, c, part)
+
+
+def test_one_long_sequence_among_short_ones_is_planned():
+    # 16 packed fp32 sequences, 8 rows per KV head, 8 000 keys in all: eight CTAs would take 50 us for the one that may have them all
+    for total in (2000, 4000, 8000):
+        assert route("ragged", "fp32", 16, 8, 1, 64, 0, total=total) in (PLANNER, INLINE)
+        assert route("ragged", "fp32", 16, 8, 2, 128, 0, total=total) in (PLANNER, INLINE)
+    assert route("ragged", "fp16", 16, 8, 8, 128, 0, total=8000) in (PLANNER, INLINE)
+    # ... and short ones still share clusters
+    assert 1 <= route("ragged", "fp16", 16, 8, 2, 64, 0, m=4, total=8300) <= 8
+    assert 1 <= route("ragged", "fp32", 16, 8, 1, 64, 0, total=500) <= 8
+
+
+@pytest.mark.parametrize("sms", [1, 108, 132, 148, 160])
+def test_clusters_take_what_they_can_hold(sms):
+    """More than sixteen rows never share a cluster; the library's own array never brings tickets along."""
+    for layout in ("dense", "ragged", "paged"):
+        for batch in (1, 3, 50, 97):
+            for keys in (0, 1, 100, 3000):
+                for qh, m in ((8, 1), (16, 1), (24, 1), (8, 4), (8, 16)):
+                    for dtype in ("bf16", "fp32"):
+                        c = route(layout, dtype, batch, qh, 1, 64, keys, m=m, sms=sms)
+                        assert c in (PLANNER, INLINE, 1, 2, 4, 8)
+                        if keys and qh * m > 16 and (dtype == "bf16" or m > 1):
+                            assert c == PLANNER
+                        if batch > 96:
+                            assert c != INLINE
+                        if 1 < c <= 8:
+                            assert batch * c <= 3 * sms
+                        s = route(layout, dtype, batch, qh, 1, 64, keys, m=m, static=True, sms=sms)
+                        assert s != INLINE
+                        if m == 1:
+                            assert s == (PLANNER if c == INLINE else c)

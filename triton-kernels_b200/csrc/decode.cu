@@ -2385,36 +2385,85 @@ int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t st
 }
 
 namespace {
-// `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
+// What one CTA takes for a tile of 64 keys, alone on its SM, in ns.  (The fp32 kernel multiplies blocks of 1, 2 or 4 rows, each
+// block's keys split over the warps that the blocks leave it: see there.)
+int tile_ns(const b200attn_decode_args_t& a, int rows) {
+  if (a.dtype != B200ATTN_F32) return a.head_dim == 128 ? 800 : 460;
+  return (rows == 1 ? 830 : rows == 2 ? 1100 : rows <= 4 ? 1500 : rows <= 8 ? 3000 : 6000) * a.head_dim / 64;
+}
+
 // CTAs per (sequence, KV head) pair when the call runs without a plan, 0 when it is planned.  Up to eight CTAs share a pair,
-// as long as all of them are resident at once (three on an SM).  The line is drawn by the bytes of K and V in a part, from
-// the lengths that the host can know of, and by what a plan is there for:
-//   dense: every part is as long as any other, there is nothing to plan.  bf16, 32/8 heads, D 128, planned -> not, us: 1 x
-//     2 048 13.9 -> 9.0, 6 x 2 048 18.0 -> 14.5, 6 x 8 192 42.2 -> 38.2, 25 x 2 048 48.5 -> 39.2; fp32, D 64, 13 x 2 048
-//     29.9 -> 25.8.  With few pairs a plan cuts finer (1 x 8 192 19.3 -> 19.2, fp32, D 128 1 x 4 096 22.4 -> 32.2).
-//   paged: the longest sequence is known (the table's width), the others may be shorter, and a plan would make use of that:
-//     a quarter of the dense limit, where the worst case, half of the keys not there, still breaks even.
-//   ragged: the average is known; half of that again, and no part longer than 1 MiB whatever the lengths.
-//   fp32: the FMA kernel's time goes with the rows as well; beyond two rows (four where the CTAs fill the GPU) the limit shrinks
-//     with them (8/1 heads, D 64, 1 x 1 024 14.6 -> 11.0 us, but 1 x 2 048 15.8 -> 17.0 and 1 x 4 096 18.0 -> 29.0).
+// as long as all of them are resident at once.  A planned call takes 9 to 12 us before its items' length counts, some 5 more when
+// the planner has a launch of its own (more pairs than kInlinePairs), and cuts the keys evenly over the GPU whatever the lengths are;
+// a call in clusters takes 3 us and its longest part.  So the line is drawn by the time of a part (tile_ns), of one as long as the
+// host can tell: dense, the length of all; paged, the table's width; ragged, the average, and the longest that there can be,
+// a sequence that holds all keys, has a line of its own.  The lines are where the sweep below found the last call that was not faster
+// planned: 16-bit and fp32, D 64 and 128, 1 to 16 rows, 1 to 768 pairs, 64 to 16 000 keys; equal lengths, lengths from
+// nothing to twice the average, and one sequence with nearly all keys among 2 to 32.  Planned -> in clusters, us:
+//   dense: more CTAs than SMs share the bandwidth either way, and parts up to 15 us are worth it (32/8 heads, D 128, 16 x 2 048
+//     36 -> 27; 4 x 8 192 32 -> 27), below that up to 7.5 (1 x 4 096 16.1 -> 10.6, but in clusters of two 30).
+//   paged: the same without the first: the other sequences may be shorter (4 x 8 pairs, a table of 4 096 keys, D 64: 13.6 -> 11.0 with
+//     lengths anywhere up to that, 10.7 with one of them that long).
+//   ragged: 16 sequences of 125 keys on average, 8/8 heads, D 128: 12.9 -> 6.4, and when one has nearly all of them 17.9 -> 17.2;
+//     of 250 keys 16.1 -> 7.5 and 21 -> 30: the first is let through, the second not.
+//   fp32: the plan's shortest items, 128 keys, are in the planned time, so two tiles are added to the line: 8/1 heads, D 64, 1 x 1 024
+//     14.6 -> 11.1, 1 x 2 048 15.8 -> 17.2; 16 packed sequences, one with 1 900 keys, 8/1 heads: 17 in clusters of eight, 50 in those
+//     of two.  With more than two rows the CTAs of an SM hold one another up: a part takes half as long again where there are
+//     more CTAs than SMs (4 x 1 024, 64/8 heads, D 128: 27.8 -> 30.4).
 int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
   if (pairs <= 0) return 0;
-  const bool ragged = a.layout == B200ATTN_RAGGED, dense = a.layout == B200ATTN_DENSE;
-  const long long keys = ragged ? (a.total_kv + a.batch - 1) / a.batch
-                         : dense ? a.max_kv : a.table_stride * static_cast<long long>(a.page_size);
-  const long long tiles = (keys + kTileN - 1) / kTileN;
-  const long long tile_bytes = 2ll * kTileN * a.head_dim * (a.dtype == B200ATTN_F32 ? 4 : 2);
-  long long c = 8;
-  while (c > 1 && (pairs * c > 3ll * sm_count || tiles <= c / 2)) c /= 2;
-  const bool full = pairs * c >= 2ll * sm_count;
-  long long limit = (dense ? (full ? 512 : 256) : ragged ? (full ? 64 : 128) : (full ? 128 : 256)) * 1024ll;
-  if (a.dtype == B200ATTN_F32) limit = limit * (full ? 4 : 2) / std::max(rows, full ? 4 : 2);
-  if ((tiles + c - 1) / c * tile_bytes > limit) return 0;
-  if (ragged && a.total_kv / kTileN * tile_bytes > c * (1ll << 20)) return 0;
-  return static_cast<int>(c);
+  const bool ragged = a.layout == B200ATTN_RAGGED, dense = a.layout == B200ATTN_DENSE, fp32 = a.dtype == B200ATTN_F32;
+  const bool planner = pairs > kInlinePairs;
+  auto tiles_of = [](long long keys) { return (keys + kTileN - 1) / kTileN; };
+  const long long tiles = tiles_of(ragged ? (a.total_kv + a.batch - 1) / a.batch
+                                   : dense ? a.max_kv : a.table_stride * static_cast<long long>(a.page_size));
+  const long long longest = ragged ? tiles_of(a.total_kv) : tiles;
+  const long long ns = tile_ns(a, rows);
+  const long long resident = 3ll * sm_count;
+  long long most = 8;
+  while (most > 1 && pairs * most > resident) most /= 2;
+  long long c = most;
+  while (c > 1 && tiles <= c / 2) c /= 2;
+  for (; c <= most; c *= 2) {
+    const long long ctas = pairs * c;
+    long long near, far;
+    if (dense && fp32) near = far = ctas >= 2ll * sm_count ? 16000 : 5500 + 2 * ns;
+    else if (dense) near = far = ctas > sm_count ? 15000 : c == 8 ? 7500 : 5000;
+    else if (fp32) near = (planner ? 4500 : 3200) + 2 * ns, far = ragged ? (planner ? 13000 : 5500) + 2 * ns : near;
+    else near = c == 8 || planner ? 7500 : 5000, far = !ragged ? near : planner ? 15000 : c == 8 ? 8000 : 6500;
+    // (time of a part: with more CTAs than an SM each, and of the waves when a pair's only CTA has to wait for its turn)
+    double part = static_cast<double>(ns);
+    if (fp32 && rows > 2) {
+      if (ctas > sm_count) part *= 1.5;
+      if (ctas > resident) part *= static_cast<double>((ctas + resident - 1) / resident) * resident / ctas;
+    }
+    if ((tiles + c - 1) / c * part <= near && (longest + c - 1) / c * part <= far) return static_cast<int>(c);
+  }
+  return 0;
 }
 
+// Which way a pass of `rows` q rows per KV head goes: clusters (CTAs per pair), or items that the CTAs plan for themselves, or
+// (neither) items behind the planner.  More than sixteen rows of 16-bit elements always go to the tcgen05 kernel.
+//
+// Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's
+// launch, 4 to 5 us in front of the kernel, goes.  The line is the number of merge tickets that fit into the header,
+// the only part of a workspace that may be relied on to be zero without a launch; beyond it a call streams for longer
+// and the planner is a smaller part of it.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
+// keys of two heads 17.2 -> 13.0, four drafts for 16 short sequences 15.1 -> 12.9, 7 x 30 201 keys at 0.98 of the copy
+// bandwidth.  Not in the library's own array (`built_in`): nobody can zero that again after two calls have overlapped on it against
+// the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
+// in every call.
+struct Route { int cluster, inline_plan; };
+Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in) {
+  Route r;
+  r.cluster = rows <= 16 ? cluster_size(a, sm_count, rows) : 0;
+  r.inline_plan = !built_in && !r.cluster && (a.dtype == B200ATTN_F32 || rows <= 16) &&
+                          static_cast<long long>(a.batch) * a.kv_heads <= kInlinePairs ? 1 : 0;
+  return r;
+}
+
+// `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
 int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, const DecodeWsLayout& w,
                        int pass_group, int head0, bool f32_out, bool built_in) {
   DecodeParams p;
@@ -2447,18 +2496,10 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   p.slots = a.dtype != B200ATTN_F32 && p.rows > 16 ? 2 * sm_count / a.kv_heads : 0;
   p.scale_log2 = a.sm_scale * 1.4426950408889634f;
 
-  // Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's
-  // launch, 4 to 5 us in front of the kernel, goes.  The line is the number of merge tickets that fit into the header,
-  // the only part of a workspace that may be relied on to be zero without a launch; beyond it a call streams for longer
-  // and the planner is a smaller part of it.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
-  // keys of two heads 17.2 -> 13.0, four drafts for 16 short sequences 15.1 -> 12.9, 7 x 30 201 keys at 0.98 of the copy
-  // bandwidth.  Not in the library's own array: nobody can zero that again after two calls have overlapped on it against
-  // the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
-  // in every call.
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
-  // (fp32 rows beyond sixteen: what the CTAs send one another would not fit beside the copy ring)
-  p.cluster = p.rows <= 16 ? cluster_size(a, sm_count, p.rows) : 0;
-  p.inline_plan = !built_in && !p.cluster && (a.dtype == B200ATTN_F32 || p.rows <= 16) && pairs <= kInlinePairs ? 1 : 0;
+  const Route route = route_of(a, sm_count, p.rows, built_in);
+  p.cluster = route.cluster;
+  p.inline_plan = route.inline_plan;
   unsigned grid_items = static_cast<unsigned>(w.max_items);
   cudaError_t e = cudaSuccess;
   if (p.inline_plan) {
@@ -2596,6 +2637,13 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   return B200ATTN_OK;
 }
 }  // namespace
+
+int decode_route(const b200attn_decode_args_t& a, int sm_count, bool built_in) {
+  b200attn_decode_args_t b = a;
+  if (decode_ws_layout(a, sm_count, /*allow_cast=*/!built_in).cast_kv_elems > 0) b.dtype = B200ATTN_F16;
+  const Route r = route_of(b, sm_count, decode_pass_group(a.q_heads / a.kv_heads, a.q_len) * a.q_len, built_in);
+  return r.cluster ? r.cluster : r.inline_plan ? B200ATTN_ROUTE_INLINE : B200ATTN_ROUTE_PLANNER;
+}
 
 // ---------------------------------------------------------------------------
 // Decode without any caller-provided or allocated scratch memory.
