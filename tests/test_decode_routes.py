@@ -84,3 +84,18 @@ def test_clusters_take_what_they_can_hold(sms):
                         assert s != INLINE
                         if m == 1:
                             assert s == (PLANNER if c == INLINE else c)
+
+
+# From shared memory: 16-bit calls at D 128 fit three CTAs to an SM up to ten rows per KV head, fp32 calls up to seven; of 148 SMs,
+# clusters of eight leave SMs over in every processing cluster: 15, 33 and 48 are resident at one, two and three CTAs per SM.
+@pytest.mark.parametrize("dtype,rows,per_sm", [("bf16", 4, 3), ("bf16", 10, 3), ("bf16", 12, 2), ("bf16", 16, 2), ("fp32", 4, 3),
+                                               ("fp32", 8, 2), ("fp32", 16, 2)])
+def test_all_clusters_of_a_call_are_resident(dtype, rows, per_sm):
+    held = {2: (74, 148, 222), 4: (33, 71, 104), 8: (15, 33, 48)}
+    for pairs in range(1, 230):
+        for layout in ("dense", "paged"):
+            for keys in (200, 500):
+                c = route(layout, dtype, pairs, rows, 1, 128, keys)
+                if 1 < c <= 8:
+                    assert pairs <= held[c][per_sm - 1], (pairs, c)
+    assert route("dense", dtype, held[8][per_sm - 1], rows, 1, 128, 500) == 8

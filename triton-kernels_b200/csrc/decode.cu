@@ -28,6 +28,7 @@
 //       CTAs of the warp-level or the fp32 kernel shares a (sequence, kv head) pair and merges through distributed shared
 //       memory; there, and only there, a CTA waits (with a limit) for the others of its cluster.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -2385,6 +2386,62 @@ int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t st
 }
 
 namespace {
+// Dynamic shared memory of a CTA.  `cluster`: CTAs that share a pair, 0 behind a plan; what they send to one of them, pieces and rows'
+// (m, l), comes behind the rest, with up to 32 bytes of alignment.
+size_t recv_bytes(int cluster, int rows, int D) {
+  return cluster ? static_cast<size_t>(cluster) * ((rows * (D / 4) + cluster - 1) / cluster * 16 + rows * 8) + 32 : 0;
+}
+constexpr int kMmaSlices = 4;              // consumer warps of the warp-level kernel, which split the keys of a tile
+size_t mma_smem(int stages, int cluster, int rows, int D) {
+  const size_t stage_bytes = static_cast<size_t>(stages) * 2 * kTileN * D * 2;
+  const size_t comb_bytes = sizeof(float) * static_cast<size_t>(kMmaSlices) * 16 * (D + 2);
+  return 1024 + std::max(stage_bytes, comb_bytes) + static_cast<size_t>(16) * D * 2 + sizeof(DecodeCtrl) + recv_bytes(cluster, rows, D);
+}
+size_t simt_smem(int cluster, int rows, int D) {
+  // (four warps leave at most 4 / blocks-of-rows partials per row: see the kernel)
+  const int rb = rows >= 3 ? 4 : rows;
+  return kSimtRingBytes + sizeof(float) * static_cast<size_t>(std::max(rows, 4 * rb)) * (D + 2) + recv_bytes(cluster, rows, D);
+}
+
+// CTAs of either kernel that an SM holds: by their registers three, by shared memory maybe fewer (at D 128 the 16-bit kernel's
+// fit three times up to ten rows, the fp32 kernel's up to seven).
+int ctas_per_sm(size_t smem) {
+  return static_cast<int>(std::min<size_t>(3, 228 * 1024 / (smem + 1024 + 64)));
+}
+
+// Clusters of `c` CTAs, `per_sm` of them to an SM, that the GPU holds at once.  Those of four and eight leave SMs over in each of its
+// processing clusters: a call of 16 clusters of eight at one CTA per SM went in two waves and took 20.4 us instead of 15.4 planned
+// (two sequences of 4 096 keys, 32/8 heads, D 128).  The driver is asked once (`ask`; the answer depends on the device model
+// only); without a GPU the figures are those it gave for a B200.
+int clusters_held(int c, int per_sm, int sm_count, bool ask) {
+  if (c == 1) return per_sm * sm_count;
+  const int log_c = c == 2 ? 0 : c == 4 ? 1 : 2;
+  static std::atomic<int> known[3][3];
+  int n = ask ? known[log_c][per_sm - 1].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  static const int b200[3][3] = {{74, 148, 222}, {33, 71, 104}, {15, 33, 48}};
+  n = b200[log_c][per_sm - 1] * sm_count / 148;
+  if (!ask) return n;
+  auto kernel = decode_mma_kernel<__nv_bfloat16, 64, 2, 1, 160, 3, __nv_bfloat16, true>;
+  const size_t smem = (per_sm == 1 ? 120 : per_sm == 2 ? 80 : 60) * 1024;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(sm_count * 3 / c * c), 1, 1);
+  cfg.blockDim = dim3(32 * (kMmaSlices + 1), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = c;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int got = 0;
+  if (set_smem(kernel, smem) == 0 && cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) == cudaSuccess && got > 0) n = got;
+  else cudaGetLastError();                 // (no answer: the figures above stand)
+  known[log_c][per_sm - 1].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 // What one CTA takes for a tile of 64 keys, alone on its SM, in ns.  (The fp32 kernel multiplies blocks of 1, 2 or 4 rows, each
 // block's keys split over the warps that the blocks leave it: see there.)
 int tile_ns(const b200attn_decode_args_t& a, int rows) {
@@ -2410,7 +2467,7 @@ int tile_ns(const b200attn_decode_args_t& a, int rows) {
 //     14.6 -> 11.1, 1 x 2 048 15.8 -> 17.2; 16 packed sequences, one with 1 900 keys, 8/1 heads: 17 in clusters of eight, 50 in those
 //     of two.  With more than two rows the CTAs of an SM hold one another up: a part takes half as long again where there are
 //     more CTAs than SMs (4 x 1 024, 64/8 heads, D 128: 27.8 -> 30.4).
-int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
+int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows, bool ask) {
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
   if (pairs <= 0) return 0;
   const bool ragged = a.layout == B200ATTN_RAGGED, dense = a.layout == B200ATTN_DENSE, fp32 = a.dtype == B200ATTN_F32;
@@ -2420,9 +2477,13 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
                                    : dense ? a.max_kv : a.table_stride * static_cast<long long>(a.page_size));
   const long long longest = ragged ? tiles_of(a.total_kv) : tiles;
   const long long ns = tile_ns(a, rows);
-  const long long resident = 3ll * sm_count;
+  auto held = [&](long long c) -> long long {
+    const int n = static_cast<int>(c);
+    const int per_sm = ctas_per_sm(fp32 ? simt_smem(n, rows, a.head_dim) : mma_smem(2, n, rows, a.head_dim));
+    return clusters_held(n, per_sm, sm_count, ask);
+  };
   long long most = 8;
-  while (most > 1 && pairs * most > resident) most /= 2;
+  while (most > 1 && pairs > held(most)) most /= 2;
   long long c = most;
   while (c > 1 && tiles <= c / 2) c /= 2;
   for (; c <= most; c *= 2) {
@@ -2436,7 +2497,7 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
     double part = static_cast<double>(ns);
     if (fp32 && rows > 2) {
       if (ctas > sm_count) part *= 1.5;
-      if (ctas > resident) part *= static_cast<double>((ctas + resident - 1) / resident) * resident / ctas;
+      if (const long long n = held(c); pairs > n) part *= static_cast<double>((pairs + n - 1) / n) * n / pairs;
     }
     if ((tiles + c - 1) / c * part <= near && (longest + c - 1) / c * part <= far) return static_cast<int>(c);
   }
@@ -2444,7 +2505,8 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
 }
 
 // Which way a pass of `rows` q rows per KV head goes: clusters (CTAs per pair), or items that the CTAs plan for themselves, or
-// (neither) items behind the planner.  More than sixteen rows of 16-bit elements always go to the tcgen05 kernel.
+// (neither) items behind the planner.  More than sixteen rows of 16-bit elements always go to the tcgen05 kernel; those of fp32 are
+// planned (at six microseconds a tile and more a part is rarely short enough, and none was measured).
 //
 // Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's
 // launch, 4 to 5 us in front of the kernel, goes.  The line is the number of merge tickets that fit into the header,
@@ -2455,9 +2517,10 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows) {
 // the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
 // in every call.
 struct Route { int cluster, inline_plan; };
-Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in) {
+// `ask`: see clusters_held.
+Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in, bool ask) {
   Route r;
-  r.cluster = rows <= 16 ? cluster_size(a, sm_count, rows) : 0;
+  r.cluster = rows <= 16 ? cluster_size(a, sm_count, rows, ask) : 0;
   r.inline_plan = !built_in && !r.cluster && (a.dtype == B200ATTN_F32 || rows <= 16) &&
                           static_cast<long long>(a.batch) * a.kv_heads <= kInlinePairs ? 1 : 0;
   return r;
@@ -2497,7 +2560,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   p.scale_log2 = a.sm_scale * 1.4426950408889634f;
 
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
-  const Route route = route_of(a, sm_count, p.rows, built_in);
+  const Route route = route_of(a, sm_count, p.rows, built_in, /*ask=*/true);
   p.cluster = route.cluster;
   p.inline_plan = route.inline_plan;
   unsigned grid_items = static_cast<unsigned>(w.max_items);
@@ -2514,12 +2577,9 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
 
   const dim3 grid(p.cluster ? static_cast<unsigned>(pairs * p.cluster) : grid_items * a.kv_heads, 1);
   const int D = a.head_dim;
-  // shared memory of the pieces and the rows' (m, l) that the CTAs of a cluster send to one another, and their alignment
-  const size_t recv_bytes = p.cluster ? static_cast<size_t>(p.cluster) * ((p.rows * (D / 4) + p.cluster - 1) / p.cluster * 16 + p.rows * 8) + 32 : 0;
   if (a.dtype == B200ATTN_F32) {
-    // (four warps leave at most 4 / blocks-of-rows partials per row: see the kernel)
     const int rb = p.rows >= 3 ? 4 : p.rows;
-    const size_t smem = kSimtRingBytes + sizeof(float) * static_cast<size_t>(std::max(p.rows, 4 * rb)) * (D + 2) + recv_bytes;
+    const size_t smem = simt_smem(p.cluster, p.rows, D);
     int rc = 0;
 #define B200ATTN_LAUNCH_SIMT(DIM, RB)                                                                 \
     do {                                                                                              \
@@ -2575,23 +2635,23 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     // consumer warps that split every K/V tile by key slice, and the producer warp
     const int nmt = p.n_mtiles;
     if (nmt != 1) { set_error("decode: %d row tiles per KV head in the warp-level kernel", nmt); return B200ATTN_E_UNSUPPORTED; }
-    const int ksl = 4;
-    const int threads = 32 * (nmt * ksl + 1);
+    const int threads = 32 * (kMmaSlices + 1);
     // measured on B200 (paged decode, 32/8 heads): 2 stages with Q re-read from shared memory lets three CTAs share an
     // SM and hides each CTA's start-up and merge behind its neighbours
     int stages = 2;
-    const size_t comb_bytes = sizeof(float) * static_cast<size_t>(ksl) * nmt * 16 * (D + 2);
     if (p.cluster) {
-      // The parts are a few tiles long: as many stages as fit with all CTAs resident, so that a part's copies are under way
+      // The parts are a few tiles long: as many stages as fit with all clusters resident, so that a part's copies are under way
       // at once (two stages made every second tile wait for its copy; with that, and a producer that does not wait for the Q rows,
       // 16 x 2 048 keys of two heads, D 64, take 7.5 us instead of 8.0, one sequence of 1 500 in pages, D 128, 7.5 instead of 8.8)
-      const int per_sm = static_cast<int>(std::min<long long>(3, (pairs * p.cluster + sm_count - 1) / sm_count));
-      const size_t rest = 1024 + static_cast<size_t>(nmt) * 16 * D * 2 + sizeof(DecodeCtrl) + recv_bytes + 2048;
-      while (stages < kMaxStages && (rest + static_cast<size_t>(stages + 1) * 2 * kTileN * D * 2) * per_sm <= 227u * 1024) ++stages;
+      auto fits = [&](int n) {
+        const int per_sm = ctas_per_sm(mma_smem(n, p.cluster, p.rows, D));
+        const int held = per_sm > 0 ? clusters_held(p.cluster, per_sm, sm_count, /*ask=*/true) : 0;
+        return pairs <= held + held / 16;
+      };
+      while (stages < kMaxStages && fits(stages + 1)) ++stages;
     }
     p.stages = stages;
-    const size_t stage_bytes = static_cast<size_t>(stages) * 2 * kTileN * D * 2;
-    const size_t smem = 1024 + std::max(stage_bytes, comb_bytes) + static_cast<size_t>(nmt) * 16 * D * 2 + sizeof(DecodeCtrl) + recv_bytes;
+    const size_t smem = mma_smem(stages, p.cluster, p.rows, D);
     // tensor maps over K and V: (D, heads, tokens), one box = 64 elements x 1 head x box_rows keys
     CUtensorMap tk, tv;
     int rc = 0;
@@ -2641,7 +2701,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
 int decode_route(const b200attn_decode_args_t& a, int sm_count, bool built_in) {
   b200attn_decode_args_t b = a;
   if (decode_ws_layout(a, sm_count, /*allow_cast=*/!built_in).cast_kv_elems > 0) b.dtype = B200ATTN_F16;
-  const Route r = route_of(b, sm_count, decode_pass_group(a.q_heads / a.kv_heads, a.q_len) * a.q_len, built_in);
+  const Route r = route_of(b, sm_count, decode_pass_group(a.q_heads / a.kv_heads, a.q_len) * a.q_len, built_in, /*ask=*/false);
   return r.cluster ? r.cluster : r.inline_plan ? B200ATTN_ROUTE_INLINE : B200ATTN_ROUTE_PLANNER;
 }
 
