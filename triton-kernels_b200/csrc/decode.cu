@@ -2460,12 +2460,16 @@ int tile_ns(const b200attn_decode_args_t& a, int rows) {
 //   dense: more CTAs than SMs share the bandwidth either way, and parts up to 15 us are worth it (32/8 heads, D 128, 16 x 2 048
 //     36 -> 27; 4 x 8 192 32 -> 27), below that up to 7.5 (1 x 4 096 16.1 -> 10.6, but in clusters of two 30).
 //   paged: the same without the first: the other sequences may be shorter (4 x 8 pairs, a table of 4 096 keys, D 64: 13.6 -> 11.0 with
-//     lengths anywhere up to that, 10.7 with one of them that long).
+//     lengths anywhere up to that, 10.7 with one of them that long; but 8 x 8 pairs in clusters of four 23 -> 18.6 if all are that
+//     long, a fifth slower than planned if one is).
 //   ragged: 16 sequences of 125 keys on average, 8/8 heads, D 128: 12.9 -> 6.4, and when one has nearly all of them 17.9 -> 17.2;
-//     of 250 keys 16.1 -> 7.5 and 21 -> 30: the first is let through, the second not.
+//     of 250 keys 16.1 -> 7.5 and 21 -> 30.  A pair gets as many CTAs as make the second case a gain too, or else the most there
+//     are, and the call is planned when that would take it half as long again as the plan (26 us for the part): over the
+//     sweep clusters give 0.65 of the planned time to equal and to evenly spread lengths, 0.78 to batches of one long sequence,
+//     1.5 to the worst of them.
 //   fp32: the plan's shortest items, 128 keys, are in the planned time, so two tiles are added to the line: 8/1 heads, D 64, 1 x 1 024
-//     14.6 -> 11.1, 1 x 2 048 15.8 -> 17.2; 16 packed sequences, one with 1 900 keys, 8/1 heads: 17 in clusters of eight, 50 in those
-//     of two.  With more than two rows the CTAs of an SM hold one another up: a part takes half as long again where there are
+//     14.6 -> 11.1, 1 x 2 048 15.8 -> 17.2; 16 packed sequences, one with 1 900 keys, 8/1 heads: 17 planned and in clusters of eight,
+//     50 in those of two; one with 7 900: 26 and 53.  With more than two rows the CTAs of an SM hold one another up: a part takes half as long again where there are
 //     more CTAs than SMs (4 x 1 024, 64/8 heads, D 128: 27.8 -> 30.4).
 int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows, bool ask) {
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
@@ -2486,22 +2490,25 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows, bool a
   while (most > 1 && pairs > held(most)) most /= 2;
   long long c = most;
   while (c > 1 && tiles <= c / 2) c /= 2;
-  for (; c <= most; c *= 2) {
+  for (;; c *= 2) {
     const long long ctas = pairs * c;
-    long long near, far;
-    if (dense && fp32) near = far = ctas >= 2ll * sm_count ? 16000 : 5500 + 2 * ns;
-    else if (dense) near = far = ctas > sm_count ? 15000 : c == 8 ? 7500 : 5000;
-    else if (fp32) near = (planner ? 4500 : 3200) + 2 * ns, far = ragged ? (planner ? 13000 : 5500) + 2 * ns : near;
-    else near = c == 8 || planner ? 7500 : 5000, far = !ragged ? near : planner ? 15000 : c == 8 ? 8000 : 6500;
+    long long near, far, last;
+    if (dense && fp32) near = ctas >= 2ll * sm_count ? 16000 : 5500 + 2 * ns;
+    else if (dense) near = ctas > sm_count ? 15000 : c == 8 ? 7500 : 5000;
+    else if (fp32) near = (planner ? 4500 : 3200) + 2 * ns;
+    else near = !ragged && (c == most || planner) ? 7500 : 5000;
+    far = last = near;
+    if (ragged && fp32) far = (planner ? 13000 : 5500) + 2 * ns, last = (planner ? 22000 : 9000) + 2 * ns;
+    else if (ragged) far = planner ? 15000 : c == 8 ? 8000 : 6500, last = planner ? 26000 : 15000;
     // (time of a part: with more CTAs than an SM each, and of the waves when a pair's only CTA has to wait for its turn)
     double part = static_cast<double>(ns);
     if (fp32 && rows > 2) {
       if (ctas > sm_count) part *= 1.5;
       if (const long long n = held(c); pairs > n) part *= static_cast<double>((pairs + n - 1) / n) * n / pairs;
     }
-    if ((tiles + c - 1) / c * part <= near && (longest + c - 1) / c * part <= far) return static_cast<int>(c);
+    if ((tiles + c - 1) / c * part <= near && (longest + c - 1) / c * part <= (c == most ? last : far)) return static_cast<int>(c);
+    if (c == most) return 0;
   }
-  return 0;
 }
 
 // Which way a pass of `rows` q rows per KV head goes: clusters (CTAs per pair), or items that the CTAs plan for themselves, or
