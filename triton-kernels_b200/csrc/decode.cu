@@ -2647,13 +2647,18 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     // SM and hides each CTA's start-up and merge behind its neighbours
     int stages = 2;
     if (p.cluster) {
-      // The parts are a few tiles long: as many stages as fit with all clusters resident, so that a part's copies are under way
-      // at once (two stages made every second tile wait for its copy; with that, and a producer that does not wait for the Q rows,
-      // 16 x 2 048 keys of two heads, D 64, take 7.5 us instead of 8.0, one sequence of 1 500 in pages, D 128, 7.5 instead of 8.8)
+      // The parts are a few tiles long: as many stages as fit, so that a part's copies are under way at once (two stages made every
+      // second tile wait for its copy; with that, and a producer that does not wait for the Q rows, 16 x 2 048 keys of two heads,
+      // D 64, take 7.5 us instead of 8.0, one sequence of 1 500 in pages, D 128, 7.5 instead of 8.8).  Stages that cost an SM
+      // a CTA are taken only where the clusters then leave a sixteenth of the GPU free: the next call's set up
+      // beside them (4 x 300 keys, 32/8 heads, D 128, 32 clusters of 33: 8.2 us with three stages, 7.2 with two, 2 048 keys in
+      // pages 12.6 and 11.5; 8 x 300, 64 of 71: 7.2 and 8.2).
+      const int most = ctas_per_sm(mma_smem(2, p.cluster, p.rows, D));
       auto fits = [&](int n) {
         const int per_sm = ctas_per_sm(mma_smem(n, p.cluster, p.rows, D));
+        if (per_sm == most) return true;
         const int held = per_sm > 0 ? clusters_held(p.cluster, per_sm, sm_count, /*ask=*/true) : 0;
-        return pairs <= held + held / 16;
+        return pairs <= held - held / 16;
       };
       while (stages < kMaxStages && fits(stages + 1)) ++stages;
     }
