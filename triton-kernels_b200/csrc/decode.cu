@@ -1306,7 +1306,7 @@ constexpr int kUmmaTmemCols = 256;
 constexpr float kMaxRowSum = 1024.0f;
 constexpr float kMoveThreshold = 3.0f;   // log2 units
 constexpr int kUmmaThreads = 256;     // four softmax warps, three that issue copies, the MMA warp
-constexpr int kUmmaIssuers = 3;       // warps that share the copies of a stage
+constexpr int kUmmaIssuers = 3;       // warps that share the copies of a stage of pages
 constexpr int kUmmaUnitRing = 4;      // units the producer may be ahead of the slowest consumer
 constexpr int kUmmaMaxClaims = 1;     // merges a CTA takes per sweep of the ticket counters in its teardown
 constexpr int kMergeClaimed = 1 << 30; // added to a pair's ticket counter by the CTA that merges it
@@ -1380,9 +1380,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
   const int n_softmax = active_warps * 32;
   // A warp issues a box every 95 to 130 cycles, whatever the box's size, and different warps do not hold one another up: the
   // sixteen boxes of a stage of 16-key pages took one warp 1 580 of the 2 540 cycles that a CTA had for a tile.  (Pages that
-  // are cut into more boxes than a warp has lanes are left to the producer.)
+  // are cut into more boxes than a warp has lanes are left to the producer.)  The two or four boxes of a dense or packed tile
+  // are the producer's alone: what a further warp saves there is less than its way to the unit's record and the arrivals cost
+  // (64 sequences of 20 keys, 64/8 heads, D 128, 16.0 -> 15.4 us, of 600 41.5 -> 41.2; 16 of 20 to 60 13.1 -> 12.6).
   const int boxes_log2 = p.layout == B200ATTN_PAGED ? 6 - p.box_shift : 0;
   const bool shared_issue = boxes_log2 <= 5;
+  const int issuers = p.layout == B200ATTN_PAGED && shared_issue ? kUmmaIssuers : 1;
 
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   UmmaCtrl* ctrl = reinterpret_cast<UmmaCtrl*>(smem + kUmmaStages * STAGE_BYTES);
@@ -1390,7 +1393,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
 
   if (tid == 0) {
     for (int i = 0; i < kUmmaStages; ++i) {
-      mbar_init(smem_u32(&ctrl->full[i]), shared_issue ? kUmmaIssuers : 1);
+      mbar_init(smem_u32(&ctrl->full[i]), issuers);
       mbar_init(smem_u32(&ctrl->empty[i]), 1);
     }
     mbar_init(smem_u32(&ctrl->q_ready), n_softmax);
@@ -1401,7 +1404,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     mbar_init(smem_u32(&ctrl->rows_out), n_softmax);
     for (int i = 0; i < kUmmaUnitRing; ++i) {
       mbar_init(smem_u32(&ctrl->unit_full[i]), 1);
-      mbar_init(smem_u32(&ctrl->unit_empty[i]), 1 + active_warps + (shared_issue ? kUmmaIssuers - 1 : 0));
+      mbar_init(smem_u32(&ctrl->unit_empty[i]), active_warps + issuers);
     }
     ctrl->published = 0;
     ctrl->abort_flag = 0;
@@ -1437,7 +1440,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     if (lane == 0) mbar_arrive(smem_u32(&ctrl->unit_empty[r % kUmmaUnitRing]));
   };
 
-  // Issuing warp `part`'s share of a stage: every kUmmaIssuers-th (box, operand, column block) of the tile.
+  // Issuing warp `part`'s share of a stage: of the tile's (box, operand, column block) every `issuers`-th.
   auto issue_share = [&](const UmmaUnit& w, PageAhead& ahead, int tile, int stage, int part) {
     const bool paged = p.layout == B200ATTN_PAGED;
     const int t0 = w.t_begin + tile * kTileN;
@@ -1448,10 +1451,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     int h_coord = w.h;
     long long row0 = w.seq_start;
     if (p.layout == B200ATTN_DENSE) { h_coord = 0; row0 = (static_cast<long long>(w.b) * p.kv_heads + w.h) * p.max_kv; }
-    // boxes of the share in this tile: the indices part, part + kUmmaIssuers, ... whose box is one of the first n
+    // boxes of the share in this tile: the indices part, part + issuers, ... whose box is one of the first n
     int count = 0;
-    for (int base = 0; base < total; base += 32 * kUmmaIssuers) {
-      const int idx = base + lane * kUmmaIssuers + part;
+    for (int base = 0; base < total; base += 32 * issuers) {
+      const int idx = base + lane * issuers + part;
       count += __popc(__ballot_sync(0xffffffffu, idx < total && (idx & (boxes - 1)) < n));
     }
     if (lane == 0) {
@@ -1459,8 +1462,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
       else mbar_arrive(bar);
     }
     __syncwarp();
-    for (int base = 0; base < total; base += 32 * kUmmaIssuers) {
-      const int idx = base + lane * kUmmaIssuers + part;
+    for (int base = 0; base < total; base += 32 * issuers) {
+      const int idx = base + lane * issuers + part;
       const int box = idx & (boxes - 1), rest = idx >> boxes_log2, op = rest & 1, cc = rest >> 1;
       const int row = paged ? ahead.box_row(p, tile, n, box, idx < total ? op : 2) : (idx < total ? static_cast<int>(row0 + t0) : -1);
       const uint32_t dst = smem_base + stage * STAGE_BYTES + op * TILE_BYTES + cc * CHUNK_BYTES + box * box_bytes;
@@ -1582,7 +1585,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     }
   } else if (warp >= kHelper && warp < kHelper + kUmmaIssuers - 1) {
     // =========================== further issuing warps ===========================
-    if (shared_issue) {
+    if (issuers > 1) {
       bool ok = true;
       int g = 0;
       PageAhead ahead(p, lane);
