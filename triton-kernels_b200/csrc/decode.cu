@@ -388,7 +388,7 @@ __device__ __forceinline__ int ceil_div_fast(int a, int b, float inv_b) {
 }
 
 __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeParams p) {
-  __shared__ long long s_tot[32];
+  __shared__ unsigned long long s_tot[32];
   __shared__ int s_warp[32];
   __shared__ int s_carry;
   __shared__ int s_chunk;
@@ -410,7 +410,10 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   const bool cached = p.batch <= kPlanLenCache;
   auto len_of = [&](int b) -> int { return cached ? s_len[b] : seq_info(p, b).len; };
 
-  long long tot = 0;
+  // keys, and above kKeyBits the items that the smallest chunk would make (more than a wave's only matter, see try_wave)
+  constexpr int kKeyBits = 44;
+  const float inv_min = 1.f / static_cast<float>(p.min_chunk);
+  unsigned long long tot = 0;
   SeqInfo mine;                             // of sequence tid: kept, the records need it again
   mine.start = 0;
   mine.len = 0;
@@ -418,7 +421,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     const SeqInfo si = seq_info(p, b);
     if (b == tid) mine = si;
     if (cached) s_len[b] = si.len;
-    tot += si.len;
+    tot += static_cast<unsigned long long>(si.len) +
+           (static_cast<unsigned long long>(max(1, ceil_div_fast(si.len, p.min_chunk, inv_min))) << kKeyBits);
   }
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   if (lane == 0) s_tot[warp] = tot;
@@ -432,13 +436,18 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   // against 245 us; one KV head of that batch: 91 us against 159 us).  The two plans are compared by an estimate
   // of their run time in keys: the largest item plus the per-item overhead for one wave, the average load of a
   // resident CTA plus half an item for several.
-  long long t = 0;
-  for (int w = 0; w < kPlanThreads / 32; ++w) t += s_tot[w];
+  unsigned long long sum = 0;
+  for (int w = 0; w < kPlanThreads / 32; ++w) sum += s_tot[w];
+  const long long t = static_cast<long long>(sum & ((1ull << kKeyBits) - 1));
+  const int at_most = static_cast<int>(sum >> kKeyBits);
   // (the two divisions per sequence go through a float reciprocal, corrected to the exact quotient: a pass over 256
   // lengths with integer divisions cost 2 us, and the pass runs once or twice per call)
   // Both kinds of candidate are evaluated in one pass, and what one thread used to decide in loops over shared memory
   // warp 0 decides in ballots; with that, 32-bit divisions and the lengths kept in registers a call of 16 fp32 sequences of
-  // 100 to 4 096 keys, 8 heads, takes 35.1 us instead of 36.3.
+  // 100 to 4 096 keys, 8 heads, takes 35.1 us instead of 36.3 (in two passes, the second where it is needed, 37.1).  But 32 warps
+  // that look at every length keep the SM busy: the second kind is left out where even the smallest chunk makes no more items
+  // than a wave has CTAs, and of a dense batch one length is looked at.  Without that 200 fp32 sequences of 250 keys, 8/1
+  // heads, D 128, took 35.1 us instead of 32.5, 64 of 20 keys with 8 drafts, 8/1 heads, D 64 in 16 bits, 12.5 instead of 11.2.
   auto candidate = [&](int target) -> int {
     long long base = t <= 0x7fffffff ? (static_cast<unsigned>(t) + target - 1) / static_cast<unsigned>(target) : (t + target - 1) / target;
     base = ((base + kTileN - 1) / kTileN) * kTileN;
@@ -448,18 +457,22 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     return static_cast<int>(((cand + kTileN - 1) / kTileN) * kTileN);
   };
   // (a batch of more sequences than a wave has CTAs cannot fit one: every sequence is at least one item)
-  const bool try_wave = p.wave_items > 0 && p.wave_items < p.target_items && p.batch <= p.wave_items;
+  const bool try_wave = p.wave_items > 0 && p.wave_items < p.target_items && p.batch <= p.wave_items &&
+                        at_most > p.wave_items;
   {
     const int ck0 = candidate(p.target_items), ck1 = try_wave ? candidate(p.wave_items) : ck0;
     const float inv0 = 1.f / static_cast<float>(ck0), inv1 = 1.f / static_cast<float>(ck1);
     long long n0 = 0, n1 = 0;
     int biggest = 0;
-    for (int b = lane; b < p.batch; b += 32) {
+    // (sequences of a dense batch are all alike)
+    const bool dense = p.layout == B200ATTN_DENSE;
+    const int looked_at = dense ? 1 : p.batch, weight = dense ? p.batch : 1;
+    for (int b = lane; b < looked_at; b += 32) {
       const int len = len_of(b);
-      n0 += max(1, ceil_div_fast(len, ck0, inv0));
+      n0 += max(1, ceil_div_fast(len, ck0, inv0)) * weight;
       if (try_wave) {
         const int v = max(1, ceil_div_fast(len, ck1, inv1));
-        n1 += v;
+        n1 += v * weight;
         const int per = ((ceil_div_fast(len, v, __frcp_rn(static_cast<float>(v))) + kTileN - 1) / kTileN) * kTileN;
         biggest = max(biggest, min(len, max(per, kTileN)));
       }
