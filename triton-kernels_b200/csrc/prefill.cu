@@ -887,19 +887,28 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // afterwards whether it could stand: no maximum is computed, no exponential waits for one, nothing is exchanged
         // between threads, and the tile is read from tensor memory once.  P stays in registers until the verdict: if a row
         // has to move, the scores are still there for the two passes below.
-        // An item's first tile takes the maximum of its first 32 columns for a reference.
+        // An item's first tile is read once more for its maximum: the largest weight is then exactly one.  (Against the maximum of
+        // the first 32 columns it was rounded like all others, and outputs came out up to 1 % further from 64 bits.)
         bool done = false;
         if (lo >= kBN - 1) {
           uint32_t pk[2][16];
           uint32_t v0[16], v1[16];
-          tmem_ld_16x256b_x4(tS, v0);
-          tmem_wait_ld_regs(v0);
-          tmem_ld_16x256b_x4(tS + 32, v1);
           if (j == 0) {
-            max_quarter(v0);
+#pragma unroll 1
+            for (int c = 0; c < 4; c += 2) {
+              tmem_ld_16x256b_x4(tS + c * 32, v0);
+              tmem_ld_16x256b_x4(tS + c * 32 + 32, v1);
+              tmem_wait_ld_regs(v0);
+              tmem_wait_ld_regs(v1);
+              max_quarter(v0);
+              max_quarter(v1);
+            }
             m_a = quad_max(mx_a) * sl2;
             m_b = quad_max(mx_b) * sl2;
           }
+          tmem_ld_16x256b_x4(tS, v0);
+          tmem_wait_ld_regs(v0);
+          tmem_ld_16x256b_x4(tS + 32, v1);
           // (a row without a reference yet has -inf here: its sum is then no number and the verdict is no)
           nega_2 = pack_f2(-m_a, -m_a);
           negb_2 = pack_f2(-m_b, -m_b);
