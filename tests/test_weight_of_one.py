@@ -26,6 +26,15 @@ def _inputs(qh, m, n, key, above):
 
 # (the weight of key 0 is 2^-above, rounded to 2^-12 of itself: 2^-12 / 2^above of the sum; the sums' own rounding is 2^-23)
 @pytest.mark.parametrize("above", [5.3, 7.7, 9.1, 9.4])
+@pytest.mark.parametrize("qh,m", [(5, 8), (8, 16)])
+@pytest.mark.parametrize("key", [17, 40, 63])
+def test_speculative_decode(above, qh, m, key):
+    for n in (64, 300):
+        out = speculative_decode_attention(*_inputs(qh, m, n, key, above))
+        assert (out - 1).abs().max().item() <= 2.0 ** -(12 + above) * 1.1 + 2e-6
+
+
+@pytest.mark.parametrize("above", [5.3, 7.7, 9.1, 9.4])
 @pytest.mark.parametrize("key", [33, 70, 127])
 def test_prefill(above, key):
     for n in (128, 500):
