@@ -40,3 +40,12 @@ def test_prefill(above, key):
     for n in (128, 500):
         out = flash_attention_v2(*_inputs(2, 100, n, key, above))
         assert (out - 1).abs().max().item() <= 2.0 ** -(12 + above) * 1.1 + 2e-6
+
+
+@pytest.mark.parametrize("above", [2.3, 5.3, 7.7])
+@pytest.mark.parametrize("key", [64, 70, 130])
+def test_decode_cluster(above, key):
+    """Key 0's warp meets the other key in a later tile."""
+    q, k, v = _inputs(2, 4, 400, key, above)
+    out = speculative_decode_attention(q[:1], k[:1], v[:1])
+    assert (out - 1).abs().max().item() <= 2.0 ** -(12 + above) * 1.1 + 2e-6

@@ -1193,8 +1193,12 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) decode_mma_kernel(con
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
         // the accumulators are rescaled only when a row's max grew by more than 2^8; until then the
-        // older reference keeps being used (exact: the same reference normalises the row at the end)
-        const bool need0 = (mx0 - m_used[0]) > 8.f, need1 = (mx1 - m_used[1]) > 8.f;
+        // older reference keeps being used (exact: the same reference normalises the row at the end).  In a cluster a row has
+        // fewer warps than a plan's shortest items give it, with more keys each, and fewer weights that are exactly one: there a
+        // warp follows its maximum more closely.  Error against 64 bits of one user of 1 500 keys, over that of its planned call:
+        // 1.03 at eight powers of two, 1.02 at three, 0.96 at one, 0.93 at none; the last costs up to a tenth of a short call.
+        constexpr float kMove = kCluster ? 1.f : 8.f;
+        const bool need0 = (mx0 - m_used[0]) > kMove, need1 = (mx1 - m_used[1]) > kMove;
         if (__any_sync(0xffffffffu, need0 || need1)) {
           float a0 = 1.f, a1 = 1.f;
           if (need0) { a0 = fast_exp2(m_used[0] - mx0); m_used[0] = mx0; }
