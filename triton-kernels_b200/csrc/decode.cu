@@ -76,6 +76,7 @@ __device__ __forceinline__ SeqInfo seq_info(const DecodeParams& p, int b) {
   return s;
 }
 
+// A CTA's work item: from the planner's records, worked out by the CTA itself, or its part of a pair in a cluster.
 struct DecodeItem {
   long long start;            // ragged: first row of the sequence
   int b, c, n_chunks, item0;  // sequence, chunk, chunks of the sequence, item number of its first chunk
@@ -687,8 +688,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   }
 }
 
-// A CTA's work item, from the planner's records or worked out by the CTA itself.
-
+// What the CTAs of a call without a planner launch work their items out in.
 struct InlinePlan {
   long long tot[kInlinePairs / 32];
   int len[kInlinePairs], n[kInlinePairs], per[kInlinePairs];

@@ -313,7 +313,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tc_fence_before();
     named_bar_sync(1, kThreads);
     tc_fence_after();
-    // (by one thread, once this CTA holds its tensor memory: a later kernel's CTA that took it first would wait for this
+    // (by the MMA warp, once this CTA holds its tensor memory: a later kernel's CTA that took it first would wait for this
     // grid while this grid waits for it)
     if (warp == kMmaWarp) ptx::grid_dep_launch_dependents();
   }
