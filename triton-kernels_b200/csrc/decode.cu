@@ -2506,8 +2506,8 @@ int tile_ns(const b200attn_decode_args_t& a, int rows) {
 //   ragged: 16 sequences of 125 keys on average, 8/8 heads, D 128: 12.9 -> 6.4, and when one has nearly all of them 17.9 -> 17.2;
 //     of 250 keys 16.1 -> 7.5 and 21 -> 30.  A pair gets as many CTAs as make the second case a gain too, or else the most there
 //     are, and the call is planned when that would take it half as long again as the plan (26 us for the part): over the
-//     sweep clusters give 0.65 of the planned time to equal and to evenly spread lengths, 0.78 to batches of one long sequence,
-//     1.5 to the worst of them.
+//     sweep clusters give 0.66 of the planned time to equal and to evenly spread lengths, 0.78 to batches of one long sequence,
+//     1.5 to the worst of them (fp32 0.86, 0.94 and 1.1).
 //   fp32: the plan's shortest items, 128 keys, are in the planned time, so two tiles are added to the line: 8/1 heads, D 64, 1 x 1 024
 //     14.6 -> 11.1, 1 x 2 048 15.8 -> 17.2; 16 packed sequences, one with 1 900 keys, 8/1 heads: 17 planned and in clusters of eight,
 //     50 in those of two; one with 7 900: 26 and 53.  With more than two rows the CTAs of an SM hold one another up: a part takes half as long again where there are
