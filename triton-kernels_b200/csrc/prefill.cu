@@ -91,6 +91,7 @@ struct __align__(8) Control {
   uint64_t s_full[kSlots];
   uint64_t p_ready[kSlots];
   uint64_t o_done[kSlots];
+  uint64_t drained;              // the MMAs of an issuer that gave up
   uint64_t sched_full[2];
   uint64_t sched_empty[2];
   int sched_item[2];
@@ -110,6 +111,14 @@ struct SmemPlan {
   static constexpr int kTotal = kCtrlOff + static_cast<int>(sizeof(Control));
   static_assert(kTotal + 1024 <= 227 * 1024, "shared memory of an SM (1 KiB for the alignment of the tiles)");
 };
+
+// The waits of a tile.  At head_dim 128 the first look is straight-line code (8 x 2 048 without a mask 522.3 -> 520.7 us, 8 x 4 096
+// causal 1 082 -> 1 079); at 64 the softmax, not the chain of waits, is what a step takes, and that costs (4 x 4 096 causal
+// 362 -> 368).
+template <int D> __device__ __forceinline__ bool tile_wait(uint32_t bar, uint32_t parity) {
+  if constexpr (D == 128) return mbar_wait_ready(bar, parity);
+  else return mbar_wait(bar, parity);
+}
 
 // bounded mbarrier wait whose verdict is uniform over the (converged) warp
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
@@ -295,6 +304,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         mbar_init(smem_u32(&ctrl->p_ready[s]), 8);         // one arrival per softmax warp of the slot
         mbar_init(smem_u32(&ctrl->o_done[s]), 1);
       }
+      mbar_init(smem_u32(&ctrl->drained), 1);
       for (int i = 0; i < 2; ++i) {
         mbar_init(smem_u32(&ctrl->sched_full[i]), 1);
         mbar_init(smem_u32(&ctrl->sched_empty[i]), kSoftmaxWarps + 1);
@@ -540,17 +550,24 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     constexpr uint32_t idesc_s = make_idesc_f16(kBM, kBN, kFmt, 0);
     constexpr uint32_t idesc_o = make_idesc_f16(kBM, D, kFmt, 1);
-    const uint32_t tmem_S[kSlots] = {tmem, tmem + kBN};
-    const uint32_t tmem_O[kSlots] = {tmem + 2 * kBN, tmem + 2 * kBN + D};
+    // This warp's instructions between P and the commit of the next scores are part of every step's chain.  The operands of an
+    // MMA are uniform registers: so that little has to be moved into them, addresses are constants added to the start of shared
+    // memory, tensor memory starting at column 0 (all of it is allocated), and the code that issues exists once per stage of
+    // the ring.  With that, fewer votes and the commit of the P V behind that of the scores: cycles per 128 x 128 tile and SM,
+    // 8 x 2 048 without a mask 1 840 -> 1 776, 2 x 2 048 causal 2 145 -> 2 086 (all-zero inputs, so at full clock); at the power
+    // limit 530 -> 521 us and 76.7 -> 75.3.
+    constexpr uint32_t tmem_S[kSlots] = {0, kBN};
+    constexpr uint32_t tmem_O[kSlots] = {2 * kBN, 2 * kBN + D};
     bool ok = true;
-    // Descriptor words are prepared once: the high words never change, the low words are a base
-    // (start address >> 4) plus small constants, so issuing one MMA costs the single thread a few adds.
     const uint64_t kdesc = make_smem_desc_sw128(smem_base, 16);                    // K-major operands (Q, K)
     const uint64_t vdesc = make_smem_desc_sw128(smem_base, Plan::kChunkBytes);     // MN-major operand (V)
     int pair_base = 0;            // pair that holds K_0 of the current item (pair j + 1 holds V_j and K_j+1)
     // per-slot state as scalars (an array indexed by the slot would live in local memory)
     int tiles_done0 = 0, tiles_done1 = 0;       // score tiles issued per slot so far (barrier phases run across items)
     bool pre_issued0 = false, pre_issued1 = false;   // first score tile of the coming item already issued
+    // Inside the tile loop a wait that ran out is noticed after the MMAs behind it have been issued (on whatever is there, into this
+    // CTA's own tensor memory): a vote between P and its MMAs is thirty cycles of every tile.
+    bool good = true;
     auto pair_full_wait = [&](int pr) -> bool {
       return warp_wait(smem_u32(&ctrl->kv_full[pr % kStages]), (pr / kStages) & 1);
     };
@@ -561,26 +578,22 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const uint32_t lo = __shfl_sync(0xffffffffu, static_cast<uint32_t>(x), 0), hi = __shfl_sync(0xffffffffu, static_cast<uint32_t>(x >> 32), 0);
       return (static_cast<uint64_t>(hi) << 32) | lo;
     };
-    // operand descriptors of the K and the V buffer of a pair's stage
-    auto k_desc_of = [&](int pr) -> uint64_t {
-      return uniform(kdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages) + 1) * Plan::kTileBytes) >> 4));
-    };
-    auto v_desc_of = [&](int pr) -> uint64_t {
-      return uniform(vdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages)) * Plan::kTileBytes) >> 4));
-    };
     auto q_desc_of = [&](int buf) -> uint64_t {
       return uniform(kdesc + static_cast<uint64_t>((Plan::kQOff + buf * Plan::kTileBytes) >> 4));
     };
-    auto issue_s = [&](int s, uint64_t qa, uint64_t kb) {
+    using Stage0 = std::integral_constant<int, 0>;
+    using Stage1 = std::integral_constant<int, 1>;
+    auto issue_s = [&](int s, uint64_t qa, auto stage) {
+      const uint64_t kb = kdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * decltype(stage)::value + 1) * Plan::kTileBytes) >> 4);
       // S_s = Q_s K^T : K-major A and B, D/16 k-steps
       mma_ss_batch<D / 16>(tmem_S[s], qa, kb, idesc_s, 0u, lead);
       mma_commit_lead(smem_u32(&ctrl->s_full[s]), lead);
     };
-    auto issue_pv = [&](int s, uint64_t vb, bool first) {
-      // O_s (+)= P_s V : A = packed 16-bit P, 32 TMEM columns at the start of each 64-column half of the S tile;
+    auto issue_pv = [&](int s, auto stage, bool first) {
+      const uint64_t vb = vdesc + static_cast<uint64_t>((Plan::kRingOff + 2 * decltype(stage)::value * Plan::kTileBytes) >> 4);
+      // O_s (+)= P_s V (the caller commits): A = packed 16-bit P, 32 TMEM columns at the start of each 64-column half of the S tile;
       // B = V, MN-major
       mma_ts_batch8(tmem_O[s], tmem_S[s], vb, idesc_o, first ? 0u : 1u, lead);
-      mma_commit_lead(smem_u32(&ctrl->o_done[s]), lead);
     };
 
     // First score tile of slot s of item kk, whose K_0 is pair `pr`: once its Q tile and K_0 have landed.  A slot without
@@ -591,7 +604,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (nkv_s > 0) {
         if (!pair_full_wait(pr)) return false;
         tc_fence_after();
-        issue_s(s, q_desc_of(buf), k_desc_of(pr));
+        if (pr & 1) issue_s(s, q_desc_of(buf), Stage1{});
+        else issue_s(s, q_desc_of(buf), Stage0{});
         if (nkv_s == 1) mma_commit_lead(smem_u32(&ctrl->q_empty[buf]), lead);    // the slot's last use of its Q tile
       } else if (lane == 0) {
         mbar_arrive(smem_u32(&ctrl->q_empty[buf]));
@@ -615,14 +629,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (!ok) break;
       if (nkv_max > 0) mma_commit_lead(smem_u32(&ctrl->kv_empty[pair_base % kStages]), lead);
       pre_issued0 = pre_issued1 = false;
-      for (int j = 0; j < nkv_max && ok; ++j) {
+      auto tile = [&](const int j, auto stage) {
         const int pr = pair_base + 1 + j;     // the pair {V_j, K_j+1}
         const bool last_iter = j + 1 == nkv_max;
         // Everything that does not depend on the softmax warps is waited for and computed before their P is: the
         // pair {V_j, K_j+1} (one barrier; in steady state loaded long ago) and the operand descriptors.  Between a slot's
         // P and its two batches of MMAs the warp then only runs the issue.
-        ok = pair_full_wait(pr);
-        if (!ok) break;
+        good = tile_wait<D>(smem_u32(&ctrl->kv_full[pr % kStages]), (pr / kStages) & 1);
         {
           const int valid = len_k - j * kBN;
           if (valid < kBN) {
@@ -639,56 +652,66 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             __syncwarp();
           }
         }
-        const uint64_t vb = v_desc_of(pr);
-        const uint64_t kb = k_desc_of(pr);
-        auto slot_step = [&](const int s, const int nkv_s, const int qbuf, const uint64_t qd, int& tiles_done) -> bool {
-          if (j >= nkv_s) return true;
+        auto slot_step = [&](const int s, const int nkv_s, const int qbuf, const uint64_t qd, int& tiles_done) {
+          if (j >= nkv_s) return;
           // (P of an item's first tile also says that the previous item's O has been read out: the softmax warps hand it
           // over after that)
-          if (!warp_wait(smem_u32(&ctrl->p_ready[s]), tiles_done & 1)) return false;
+          if (!tile_wait<D>(smem_u32(&ctrl->p_ready[s]), tiles_done & 1)) good = false;
           tc_fence_after();
-          issue_pv(s, vb, j == 0);
+          issue_pv(s, stage, j == 0);
           if (j + 1 < nkv_s) {
-            issue_s(s, qd, kb);
+            issue_s(s, qd, stage);
             if (j + 2 == nkv_s) mma_commit_lead(smem_u32(&ctrl->q_empty[qbuf]), lead);   // the slot's last use of its Q tile
           }
+          // (behind the score tile, which the softmax waits for; of the P V only a reference that moves and an item's end ask)
+          mma_commit_lead(smem_u32(&ctrl->o_done[s]), lead);
           ++tiles_done;
-          return true;
         };
         if (!last_iter) {
-          ok = slot_step(0, nkv0, qbuf0, qd0, tiles_done0) && slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
-          if (!ok) break;
+          slot_step(0, nkv0, qbuf0, qd0, tiles_done0);
+          slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
           // V_j and K_j+1 have been read by everything that will read them: one commit releases the stage
           mma_commit_lead(smem_u32(&ctrl->kv_empty[pr % kStages]), lead);
+          ok = __all_sync(0xffffffffu, good);
         } else {
           // The item's last tile: each slot's first score tile of the next item is issued right behind its final PV, so
           // that the tensor cores have work while the softmax warps read O out.  What is waited for here (the next item
           // published, its Q tiles and its first K tile) depends only on work this warp has already issued: the first
           // slot's Q has a buffer of its own, the second's takes the one this item's first slot gave back a tile ago.
-          ok = slot_step(0, nkv0, qbuf0, qd0, tiles_done0) &&
-               warp_wait(smem_u32(&ctrl->sched_full[(k + 1) & 1]), ((k + 1) >> 1) & 1);
-          if (!ok) break;
+          slot_step(0, nkv0, qbuf0, qd0, tiles_done0);
+          ok = __all_sync(0xffffffffu, good) && warp_wait(smem_u32(&ctrl->sched_full[(k + 1) & 1]), ((k + 1) >> 1) & 1);
+          if (!ok) return;
           const bool more = ctrl->sched_item[(k + 1) & 1] >= 0;
           const ItemWork& wn = ctrl->sched_work[(k + 1) & 1];
           if (more) {
             ok = start_slot(0, k + 1, wn.nkv[0], pair_base + nkv_max + 1);
-            if (!ok) break;
+            if (!ok) return;
           }
-          ok = slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
-          if (!ok) break;
+          slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
+          ok = __all_sync(0xffffffffu, good);
+          if (!ok) return;
           mma_commit_lead(smem_u32(&ctrl->kv_empty[pr % kStages]), lead);
           if (more) {
             ok = start_slot(1, k + 1, wn.nkv[1], pair_base + nkv_max + 1);
-            if (!ok) break;
+            if (!ok) return;
           }
           pre_issued0 = pre_issued1 = more;
         }
+      };
+      for (int j = 0; j < nkv_max && ok; ++j) {
+        if ((pair_base + 1 + j) & 1) tile(j, Stage1{});
+        else tile(j, Stage0{});
       }
       if (nkv_max > 0) pair_base += nkv_max + 1;
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));
       __syncwarp();
     }
-    if (!ok && lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
+    if (!ok) {
+      if (lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
+      // (what has been issued ends before tensor memory is given back)
+      mma_commit_lead(smem_u32(&ctrl->drained), lead);
+      warp_wait(smem_u32(&ctrl->drained), 0);
+    }
   } else if (warp < kSoftmaxWarps) {
     // =========================== softmax warps ===========================
     // Warp w serves slot w / 8, the TMEM lane quadrant w % 4 (the only lanes it may touch) and, inside the quadrant,
@@ -841,8 +864,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       float m_a = -INFINITY, m_b = -INFINITY;   // exponent references currently baked into O and l
       float l_a = 0.f, l_b = 0.f;               // partial row sums over this thread's columns
       for (int j = 0; j < n; ++j, ++tile_cnt) {
-        ok = warp_wait(smem_u32(&ctrl->s_full[s]), tile_cnt & 1);
-        if (!ok) break;
+        // (whether the wait ran out is asked with the verdict on the references: a vote of its own is thirty cycles)
+        const bool here = tile_wait<D>(smem_u32(&ctrl->s_full[s]), tile_cnt & 1);
         tc_fence_after();
         // Last visible column of the tile for the first and for the last of the warp's sixteen rows (the same for all rows
         // without a causal mask): hidden columns exist only on the tile that holds the sequence end or the diagonal.
@@ -923,13 +946,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           exp_quarter(v1, pk[1] + 8);
           sum_a = pair_sum(rs_a);
           sum_b = pair_sum(rs_b);
-          done = __all_sync(0xffffffffu, sum_a <= kMaxPartialSum && sum_b <= kMaxPartialSum);   // (false for NaN)
+          done = __all_sync(0xffffffffu, here && sum_a <= kMaxPartialSum && sum_b <= kMaxPartialSum);   // (false for NaN)
           if (done) {
             tmem_st_16x128b_x8(tS, pk[0]);
             tmem_st_16x128b_x8(tS + ptx::kPHalfStride, pk[1]);
           }
         }
         if (!done) {
+          ok = __all_sync(0xffffffffu, here);
+          if (!ok) break;
           // Two passes, 32 columns at a time: a tile with hidden columns, a row whose reference moves.
           // Columns hidden from all sixteen rows are neither read nor exponentiated.
           auto mask_quarter = [&](uint32_t (&v)[16], int c) {

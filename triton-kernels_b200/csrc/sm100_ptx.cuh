@@ -62,6 +62,11 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, u
   return ok != 0;
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_wait_limit(bar, parity, kWaitTries); }
+// where the phase has nearly always completed: the first look is straight-line code
+__device__ __forceinline__ bool mbar_wait_ready(uint32_t bar, uint32_t parity) {
+  if (__builtin_expect(mbar_try_wait(bar, parity) != 0, 1)) return true;
+  return mbar_wait_limit(bar, parity, kWaitTries);
+}
 
 // Asynchronous 8-byte store of (a, b) to the shared-memory address `slot` of CTA `cta_rank` of this cluster; the
 // receiver's mbarrier at `bar` (same offsets in every CTA) is credited with the 8 bytes when they have landed.
