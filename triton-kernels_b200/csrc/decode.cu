@@ -95,16 +95,22 @@ __device__ __forceinline__ void poison_rows(float* comb_o, float* comb_ml, int r
 // t = 0 .. nt-1 of the CTA that drew the last ticket: g = max m; O = sum 2^(m-g) acc / sum 2^(m-g) l
 // (kernels/decode.py:186-197).  Leaves the ticket counter at zero for the next call.
 // ---------------------------------------------------------------------------
+// Where the header holds a pair's ticket in a call without a planner launch.
+struct TicketPlace { unsigned* word; int shift; };
+__device__ __forceinline__ TicketPlace ticket_place(const DecodeParams& p, int pair) {
+  const int log_per_word = p.inline_plan == 8 ? 2 : 1;
+  return {reinterpret_cast<unsigned*>(p.header) + kTicketWord + (pair >> log_per_word), (pair & ((1 << log_per_word) - 1)) * p.inline_plan};
+}
 // Draws the next merge ticket of a (sequence, kv head) pair.
 __device__ __forceinline__ int draw_ticket(const DecodeParams& p, int pair) {
   if (!p.inline_plan) return atomicAdd(p.counters + pair, 1);
-  const int shift = (pair & 1) * 16;
-  return (atomicAdd(reinterpret_cast<unsigned*>(p.header) + kTicketWord + (pair >> 1), 1u << shift) >> shift) & 0xffff;
+  const TicketPlace t = ticket_place(p, pair);
+  return (atomicAdd(t.word, 1u << t.shift) >> t.shift) & ((1u << p.inline_plan) - 1);
 }
 // Leaves the pair's ticket counter at zero for the next call; `n` tickets were drawn.
 __device__ __forceinline__ void reset_ticket(const DecodeParams& p, int pair, int n) {
   if (!p.inline_plan) p.counters[pair] = 0;
-  else atomicSub(reinterpret_cast<unsigned*>(p.header) + kTicketWord + (pair >> 1), static_cast<unsigned>(n) << ((pair & 1) * 16));
+  else { const TicketPlace t = ticket_place(p, pair); atomicSub(t.word, static_cast<unsigned>(n) << t.shift); }
 }
 
 template <typename T, int D>
@@ -690,14 +696,14 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
 
 // What the CTAs of a call without a planner launch work their items out in.
 struct InlinePlan {
-  long long tot[kInlinePairs / 32];
-  int len[kInlinePairs], n[kInlinePairs], per[kInlinePairs];
+  long long tot[kInlineBatch / 32];
+  int len[kInlineBatch], n[kInlineBatch], per[kInlineBatch];
   int items[2][32], biggest[32];
   DecodeItem mine;
   int found, over;
 };
 
-// The planner's choices (same candidates, same estimate) made by a CTA of at least kInlinePairs threads for itself.
+// The planner's choices (same candidates, same estimate) made by a CTA of at least kInlineBatch threads for itself.
 // Items are numbered sequence by sequence, the sequences with the longest items first.  Returns false when there is no
 // item of that number.
 __device__ __forceinline__ bool plan_inline(const DecodeParams& p, int item, InlinePlan& s, DecodeItem& out) {
@@ -706,7 +712,7 @@ __device__ __forceinline__ bool plan_inline(const DecodeParams& p, int item, Inl
   mine.start = 0;
   mine.len = 0;
   if (tid < p.batch) mine = seq_info(p, tid);
-  if (tid < kInlinePairs) {
+  if (tid < kInlineBatch) {
     s.len[tid] = mine.len;
     long long w = mine.len;
     for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
@@ -717,7 +723,7 @@ __device__ __forceinline__ bool plan_inline(const DecodeParams& p, int item, Inl
   __syncthreads();
   long long t = 0;
 #pragma unroll
-  for (int w = 0; w < kInlinePairs / 32; ++w) t += s.tot[w];
+  for (int w = 0; w < kInlineBatch / 32; ++w) t += s.tot[w];
   // candidate `lane` of either target; the warps share the sequences
   auto candidate = [&](int target) -> int {
     long long base = t <= 0x7fffffff ? (static_cast<unsigned>(t) + target - 1) / static_cast<unsigned>(target) : (t + target - 1) / target;
@@ -2329,6 +2335,16 @@ int decode_pass_group(int group, int q_len) {
   return g < 1 ? 1 : g;
 }
 
+// Six (item, kv head) CTAs per SM: two or three waves of the tensor-core kernels (3 or 2 resident CTAs per SM).
+// Fewer, longer CTAs amortise start-up and merge; the planner keeps the item count at or below this, so the grid
+// is a whole number of waves.  (Measured on B200, paged decode and speculative decode: 4 / 6 / 8 / 12 / 16 per SM
+// give 0.84 / 0.83 / 0.81 / 0.80 / 0.78 and 0.71 / 0.70 / 0.73 / 0.67 / 0.64 of the copy bandwidth without the
+// whole-wave rule, 0.76 for speculative decode with it.)
+static int decode_target_items(int sm_count, int kv_heads) {
+  const int per_sm = 6;
+  return static_cast<int>(std::max<long long>(1, (static_cast<long long>(sm_count) * per_sm) / std::max(1, kv_heads)));
+}
+
 DecodeWsLayout decode_ws_layout(const b200attn_decode_args_t& a, int sm_count, bool allow_cast) {
   DecodeWsLayout w;
   const int group = decode_pass_group(a.kv_heads > 0 ? a.q_heads / a.kv_heads : 1, a.q_len);
@@ -2347,15 +2363,7 @@ DecodeWsLayout decode_ws_layout(const b200attn_decode_args_t& a, int sm_count, b
   const bool cast16 = allow_cast && a.dtype == B200ATTN_F32 && (rows > 16 || a.q_len > 1) &&
                       kv_rows_all * a.head_dim * 4 <= kCastLimitBytes;
   const bool f32_kernel = a.dtype == B200ATTN_F32 && !cast16;
-  // Six (item, kv head) CTAs per SM: two or three waves of the tensor-core kernels (3 or 2 resident CTAs per SM).
-  // Fewer, longer CTAs amortise start-up and merge; the planner keeps the item count at or below this, so the grid
-  // is a whole number of waves.  (Measured on B200, paged decode and speculative decode: 4 / 6 / 8 / 12 / 16 per SM
-  // give 0.84 / 0.83 / 0.81 / 0.80 / 0.78 and 0.71 / 0.70 / 0.73 / 0.67 / 0.64 of the copy bandwidth without the
-  // whole-wave rule, 0.76 for speculative decode with it.)
-  const int per_sm = 6;
-  long long target = (static_cast<long long>(sm_count) * per_sm) / std::max(1, a.kv_heads);
-  if (target < 1) target = 1;
-  w.target_items = static_cast<int>(target);
+  w.target_items = decode_target_items(sm_count, a.kv_heads);
   // one wave: 2 (tcgen05 kernel, more than 16 rows) or 3 resident CTAs per SM; per-item start-up + merge cost in keys of
   // streaming time (from the sweeps quoted in the planner)
   const bool wide = rows > 16 && !f32_kernel;
@@ -2559,18 +2567,33 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows, bool a
 // Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's
 // launch, 4 to 5 us in front of the kernel, goes.  The line is the number of merge tickets that fit into the header,
 // the only part of a workspace that may be relied on to be zero without a launch; beyond it a call streams for longer
-// and the planner is a smaller part of it.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
+// and the planner is a smaller part of it.  fp32, which reads twice the bytes: twice as many pairs, with tickets of eight bits
+// where no pair can be cut into more items than those count, up to 300 MiB of keys and values (the most that there can be).  16
+// packed sequences of 100 to 4 096 keys, 8/8 heads, D 64 36.3 -> 32.4 us, 13 x 1 500 18.9 -> 15.5, 24 x 1 500 at D 128 in pages 43.8 ->
+// 38.7; 20 x 3 000 119 -> 113, but 20 x 10 000 281 -> 290 (64/8 heads, dense): the planner puts the last, shorter item of each
+// sequence behind all others, which is worth more than its launch there.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
 // keys of two heads 17.2 -> 13.0, four drafts for 16 short sequences 15.1 -> 12.9, 7 x 30 201 keys at 0.98 of the copy
 // bandwidth.  Not in the library's own array (`built_in`): nobody can zero that again after two calls have overlapped on it against
 // the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
 // in every call.
-struct Route { int cluster, inline_plan; };
+// keys of all sequences, as many as there can be
+long long most_keys(const b200attn_decode_args_t& a) {
+  if (a.layout == B200ATTN_RAGGED) return a.total_kv;
+  return a.batch * (a.layout == B200ATTN_DENSE ? static_cast<long long>(a.max_kv) : a.table_stride * a.page_size);
+}
+struct Route { int cluster, inline_plan; };      // (inline_plan: the bits of a ticket)
 // `ask`: see clusters_held.
 Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in, bool ask) {
   Route r;
   r.cluster = rows <= 16 ? cluster_size(a, sm_count, rows, ask) : 0;
-  r.inline_plan = !built_in && !r.cluster && (a.dtype == B200ATTN_F32 || rows <= 16) &&
-                          static_cast<long long>(a.batch) * a.kv_heads <= kInlinePairs ? 1 : 0;
+  r.inline_plan = 0;
+  if (built_in || r.cluster || (a.dtype != B200ATTN_F32 && rows > 16)) return r;
+  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
+  if (pairs <= kInlinePairs) r.inline_plan = 16;
+  else if (a.dtype == B200ATTN_F32 && pairs <= kInlinePairs8 && a.batch <= kInlineBatch &&
+           decode_target_items(sm_count, a.kv_heads) + a.batch <= 255 &&
+           2 * most_keys(a) * a.kv_heads * a.head_dim * 4 <= 300ll << 20)
+    r.inline_plan = 8;
   return r;
 }
 
@@ -2615,9 +2638,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   cudaError_t e = cudaSuccess;
   if (p.inline_plan) {
     // no more items than this, whatever the lengths are: an item has min_chunk keys or ends a sequence
-    const long long keys = a.layout == B200ATTN_RAGGED ? a.total_kv
-                           : a.batch * (a.layout == B200ATTN_DENSE ? static_cast<long long>(a.max_kv) : a.table_stride * a.page_size);
-    grid_items = static_cast<unsigned>(std::min<long long>(w.max_items, keys / w.min_chunk + a.batch));
+    grid_items = static_cast<unsigned>(std::min<long long>(w.max_items, most_keys(a) / w.min_chunk + a.batch));
   } else if (!p.cluster) {
     e = launch_dependent(decode_plan_kernel, dim3(1), kPlanThreads, 0, stream, 1, p);
   }

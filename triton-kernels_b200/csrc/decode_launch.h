@@ -9,9 +9,12 @@
 namespace b200attn {
 
 // Merge tickets of calls without a planner launch: 16 bits per (sequence, KV head) pair in the workspace header, the
-// only part of a workspace that keeps its contents between calls (every call leaves them at zero).
+// only part of a workspace that keeps its contents between calls (every call leaves them at zero); 8 bits where a pair cannot be
+// cut into more than 255 items.
 constexpr int kTicketWord = 16;                     // first header word that holds tickets
 constexpr int kInlinePairs = 2 * (64 - kTicketWord);
+constexpr int kInlinePairs8 = 4 * (64 - kTicketWord);
+constexpr int kInlineBatch = kInlinePairs;          // sequences that a CTA plans
 
 // Kernel parameter block (passed by value).
 struct DecodeParams {
@@ -53,7 +56,7 @@ struct DecodeParams {
   int min_chunk;
   int max_items;
   int slots;         // persistent kernel: CTAs per KV head that the planner may deal the batch out to; 0: none
-  int inline_plan;   // 1: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs)
+  int inline_plan;   // not 0: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs); the bits of a merge ticket
   int cluster;       // CTAs that share a (sequence, KV head) pair in the kernels without a plan; 0: items are planned
   int stages;        // K/V stages of a CTA of the warp-level kernel in a cluster
   float scale_log2;  // sm_scale * log2(e)
