@@ -112,9 +112,8 @@ struct SmemPlan {
   static_assert(kTotal + 1024 <= 227 * 1024, "shared memory of an SM (1 KiB for the alignment of the tiles)");
 };
 
-// The waits of a tile.  At head_dim 128 the first look is straight-line code (8 x 2 048 without a mask 522.3 -> 520.7 us, 8 x 4 096
-// causal 1 082 -> 1 079); at 64 the softmax, not the chain of waits, is what a step takes, and that costs (4 x 4 096 causal
-// 362 -> 368).
+// The waits of a tile.  At head_dim 128 the first look is straight-line code (cycles per tile 1 807 -> 1 785); at 64 the softmax,
+// not the chain of waits, is what a step takes, and that costs (4 x 4 096 causal 362 -> 368 us).
 template <int D> __device__ __forceinline__ bool tile_wait(uint32_t bar, uint32_t parity) {
   if constexpr (D == 128) return mbar_wait_ready(bar, parity);
   else return mbar_wait(bar, parity);
@@ -550,23 +549,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     constexpr uint32_t idesc_s = make_idesc_f16(kBM, kBN, kFmt, 0);
     constexpr uint32_t idesc_o = make_idesc_f16(kBM, D, kFmt, 1);
-    // This warp's instructions between P and the commit of the next scores are part of every step's chain.  The operands of an
-    // MMA are uniform registers: so that little has to be moved into them, addresses are constants added to the start of shared
-    // memory, tensor memory starting at column 0 (all of it is allocated), and the code that issues exists once per stage of
-    // the ring.  With that, fewer votes and the commit of the P V behind that of the scores: cycles per 128 x 128 tile and SM,
-    // 8 x 2 048 without a mask 1 840 -> 1 776, 2 x 2 048 causal 2 145 -> 2 086 (all-zero inputs, so at full clock); at the power
-    // limit 530 -> 521 us and 76.7 -> 75.3.
-    constexpr uint32_t tmem_S[kSlots] = {0, kBN};
-    constexpr uint32_t tmem_O[kSlots] = {2 * kBN, 2 * kBN + D};
+    const uint32_t tmem_S[kSlots] = {tmem, tmem + kBN};
+    const uint32_t tmem_O[kSlots] = {tmem + 2 * kBN, tmem + 2 * kBN + D};
     bool ok = true;
+    // Descriptor words are prepared once: the high words never change, the low words are a base
+    // (start address >> 4) plus small constants, so issuing one MMA costs the single thread a few adds.
     const uint64_t kdesc = make_smem_desc_sw128(smem_base, 16);                    // K-major operands (Q, K)
     const uint64_t vdesc = make_smem_desc_sw128(smem_base, Plan::kChunkBytes);     // MN-major operand (V)
     int pair_base = 0;            // pair that holds K_0 of the current item (pair j + 1 holds V_j and K_j+1)
     // per-slot state as scalars (an array indexed by the slot would live in local memory)
     int tiles_done0 = 0, tiles_done1 = 0;       // score tiles issued per slot so far (barrier phases run across items)
     bool pre_issued0 = false, pre_issued1 = false;   // first score tile of the coming item already issued
-    // Inside the tile loop a wait that ran out is noticed after the MMAs behind it have been issued (on whatever is there, into this
-    // CTA's own tensor memory): a vote between P and its MMAs is thirty cycles of every tile.
+    // This warp's instructions between P and the commit of the next scores are part of every step's chain.  Inside the tile loop a
+    // wait that ran out is noticed after the MMAs behind it have been issued (on whatever is there, into this CTA's own tensor
+    // memory), one vote for three waits: cycles per 128 x 128 tile and SM, 8 x 2 048 without a mask 1 840 -> 1 807, 2 x 2 048 causal
+    // 2 144 -> 2 103 (all-zero inputs, so at full clock); at the power limit 74.7 -> 73.9 us.  Tried beside it: the code once per stage
+    // of the ring, so that descriptors are constants in uniform registers (9 cycles, but 64 / 8 heads of 22 tokens took 2 % longer
+    // with it), the commit of the P V behind that of the scores (nothing).
     bool good = true;
     auto pair_full_wait = [&](int pr) -> bool {
       return warp_wait(smem_u32(&ctrl->kv_full[pr % kStages]), (pr / kStages) & 1);
@@ -578,22 +577,26 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const uint32_t lo = __shfl_sync(0xffffffffu, static_cast<uint32_t>(x), 0), hi = __shfl_sync(0xffffffffu, static_cast<uint32_t>(x >> 32), 0);
       return (static_cast<uint64_t>(hi) << 32) | lo;
     };
+    // operand descriptors of the K and the V buffer of a pair's stage
+    auto k_desc_of = [&](int pr) -> uint64_t {
+      return uniform(kdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages) + 1) * Plan::kTileBytes) >> 4));
+    };
+    auto v_desc_of = [&](int pr) -> uint64_t {
+      return uniform(vdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages)) * Plan::kTileBytes) >> 4));
+    };
     auto q_desc_of = [&](int buf) -> uint64_t {
       return uniform(kdesc + static_cast<uint64_t>((Plan::kQOff + buf * Plan::kTileBytes) >> 4));
     };
-    using Stage0 = std::integral_constant<int, 0>;
-    using Stage1 = std::integral_constant<int, 1>;
-    auto issue_s = [&](int s, uint64_t qa, auto stage) {
-      const uint64_t kb = kdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * decltype(stage)::value + 1) * Plan::kTileBytes) >> 4);
+    auto issue_s = [&](int s, uint64_t qa, uint64_t kb) {
       // S_s = Q_s K^T : K-major A and B, D/16 k-steps
       mma_ss_batch<D / 16>(tmem_S[s], qa, kb, idesc_s, 0u, lead);
       mma_commit_lead(smem_u32(&ctrl->s_full[s]), lead);
     };
-    auto issue_pv = [&](int s, auto stage, bool first) {
-      const uint64_t vb = vdesc + static_cast<uint64_t>((Plan::kRingOff + 2 * decltype(stage)::value * Plan::kTileBytes) >> 4);
-      // O_s (+)= P_s V (the caller commits): A = packed 16-bit P, 32 TMEM columns at the start of each 64-column half of the S tile;
+    auto issue_pv = [&](int s, uint64_t vb, bool first) {
+      // O_s (+)= P_s V : A = packed 16-bit P, 32 TMEM columns at the start of each 64-column half of the S tile;
       // B = V, MN-major
       mma_ts_batch8(tmem_O[s], tmem_S[s], vb, idesc_o, first ? 0u : 1u, lead);
+      mma_commit_lead(smem_u32(&ctrl->o_done[s]), lead);
     };
 
     // First score tile of slot s of item kk, whose K_0 is pair `pr`: once its Q tile and K_0 have landed.  A slot without
@@ -604,8 +607,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (nkv_s > 0) {
         if (!pair_full_wait(pr)) return false;
         tc_fence_after();
-        if (pr & 1) issue_s(s, q_desc_of(buf), Stage1{});
-        else issue_s(s, q_desc_of(buf), Stage0{});
+        issue_s(s, q_desc_of(buf), k_desc_of(pr));
         if (nkv_s == 1) mma_commit_lead(smem_u32(&ctrl->q_empty[buf]), lead);    // the slot's last use of its Q tile
       } else if (lane == 0) {
         mbar_arrive(smem_u32(&ctrl->q_empty[buf]));
@@ -629,7 +631,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (!ok) break;
       if (nkv_max > 0) mma_commit_lead(smem_u32(&ctrl->kv_empty[pair_base % kStages]), lead);
       pre_issued0 = pre_issued1 = false;
-      auto tile = [&](const int j, auto stage) {
+      for (int j = 0; j < nkv_max && ok; ++j) {
         const int pr = pair_base + 1 + j;     // the pair {V_j, K_j+1}
         const bool last_iter = j + 1 == nkv_max;
         // Everything that does not depend on the softmax warps is waited for and computed before their P is: the
@@ -652,19 +654,19 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             __syncwarp();
           }
         }
+        const uint64_t vb = v_desc_of(pr);
+        const uint64_t kb = k_desc_of(pr);
         auto slot_step = [&](const int s, const int nkv_s, const int qbuf, const uint64_t qd, int& tiles_done) {
           if (j >= nkv_s) return;
           // (P of an item's first tile also says that the previous item's O has been read out: the softmax warps hand it
           // over after that)
           if (!tile_wait<D>(smem_u32(&ctrl->p_ready[s]), tiles_done & 1)) good = false;
           tc_fence_after();
-          issue_pv(s, stage, j == 0);
+          issue_pv(s, vb, j == 0);
           if (j + 1 < nkv_s) {
-            issue_s(s, qd, stage);
+            issue_s(s, qd, kb);
             if (j + 2 == nkv_s) mma_commit_lead(smem_u32(&ctrl->q_empty[qbuf]), lead);   // the slot's last use of its Q tile
           }
-          // (behind the score tile, which the softmax waits for; of the P V only a reference that moves and an item's end ask)
-          mma_commit_lead(smem_u32(&ctrl->o_done[s]), lead);
           ++tiles_done;
         };
         if (!last_iter) {
@@ -680,27 +682,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           // slot's Q has a buffer of its own, the second's takes the one this item's first slot gave back a tile ago.
           slot_step(0, nkv0, qbuf0, qd0, tiles_done0);
           ok = __all_sync(0xffffffffu, good) && warp_wait(smem_u32(&ctrl->sched_full[(k + 1) & 1]), ((k + 1) >> 1) & 1);
-          if (!ok) return;
+          if (!ok) break;
           const bool more = ctrl->sched_item[(k + 1) & 1] >= 0;
           const ItemWork& wn = ctrl->sched_work[(k + 1) & 1];
           if (more) {
             ok = start_slot(0, k + 1, wn.nkv[0], pair_base + nkv_max + 1);
-            if (!ok) return;
+            if (!ok) break;
           }
           slot_step(1, nkv1, qbuf1, qd1, tiles_done1);
           ok = __all_sync(0xffffffffu, good);
-          if (!ok) return;
+          if (!ok) break;
           mma_commit_lead(smem_u32(&ctrl->kv_empty[pr % kStages]), lead);
           if (more) {
             ok = start_slot(1, k + 1, wn.nkv[1], pair_base + nkv_max + 1);
-            if (!ok) return;
+            if (!ok) break;
           }
           pre_issued0 = pre_issued1 = more;
         }
-      };
-      for (int j = 0; j < nkv_max && ok; ++j) {
-        if ((pair_base + 1 + j) & 1) tile(j, Stage1{});
-        else tile(j, Stage0{});
       }
       if (nkv_max > 0) pair_base += nkv_max + 1;
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));
