@@ -1,0 +1,51 @@
+"""Prefill launches of few work items whose KV range is cut over the CTAs of a cluster: two, four and eight parts, parts that see no key
+(beyond the diagonal, behind a short sequence), rows that no part sees, query blocks that are not full, both element widths."""
+import pytest
+import torch
+
+from helpers import assert_close_both
+from oracle import sdpa_ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# (batch, q heads, kv heads, queries, keys, causal, head_dim); items of one or two q heads x 128 rows: up to 15 for eight parts, 33 for
+# four, 74 for two
+SHAPES = [(1, 8, 2, 100, 600, False, 64), (1, 2, 1, 128, 1024, False, 64), (2, 8, 1, 1, 1500, False, 128), (3, 8, 2, 130, 700, False, 64),
+          (16, 8, 2, 128, 760, False, 64), (1, 8, 2, 512, 512, True, 64), (1, 8, 8, 700, 700, True, 64), (1, 4, 4, 300, 1600, False, 128),
+          (2, 6, 2, 257, 1537, False, 128), (1, 4, 2, 1000, 1000, True, 128)]
+
+
+@pytest.mark.parametrize("layout", ["dense", "paged"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"b{s[0]}-{s[1]}-{s[2]}-q{s[3]}-kv{s[4]}-{'c' if s[5] else 'f'}-d{s[6]}")
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32], ids=["fp16", "fp32"])
+def test_parts(layout, shape, dtype):
+    from test_attention import run_prefill
+
+    b, qh, kvh, lq, lkv, causal, d = shape
+    gen = torch.Generator().manual_seed(lq + 3 * lkv + qh)
+    lens = [lkv] * b if causal or layout == "dense" else [max(1, lkv - 190 * i - 64 * (i % 2)) for i in range(b)]
+    qs = [torch.randn((lq, qh, d), generator=gen).to(dtype).to(DEV) for _ in range(b)]
+    ks = [torch.randn((n, kvh, d), generator=gen).to(dtype).to(DEV) for n in lens]
+    vs = [torch.randn((n, kvh, d), generator=gen).to(dtype).to(DEV) for n in lens]
+    refs = sdpa_ref.prefill_reference(qs, ks, vs, qh, kvh, causal)
+    for _ in range(2):
+        outs = run_prefill(layout, qs, ks, vs, causal, permute=5, pad=-1, poison=float("nan"))
+        for i in range(b):
+            assert_close_both(outs[i], refs[i], dtype, lens[i], f"seq {i}", strict=4e-3 if dtype == torch.float32 else None)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_part_of_nan_shows(d):
+    """One NaN key makes every row NaN, also in a part none of whose scores is a number; values of -inf scores weigh nothing."""
+    from kernels import flash_attention_v2
+
+    gen = torch.Generator().manual_seed(d)
+    q, k, v = (torch.randn((1, 2, n, d), generator=gen).to(torch.bfloat16).to(DEV) for n in (128, 1500, 1500))
+    ref = flash_attention_v2(q, k, v)
+    assert torch.isfinite(ref.float()).all()
+    for lo, hi in ((700, 701), (384, 1500)):
+        bad = k.clone()
+        bad[:, :, lo:hi] = float("nan")
+        assert torch.isnan(flash_attention_v2(q, bad, v).float()).all()

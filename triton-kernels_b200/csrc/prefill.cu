@@ -169,7 +169,7 @@ __device__ __forceinline__ void place_heads(const PrefillParams& p, ItemWork& w,
   }
 }
 
-__device__ __forceinline__ ItemWork locate_item(const PrefillParams& p, int item) {
+template <bool kParts> __device__ __forceinline__ ItemWork locate_item(const PrefillParams& p, int item) {
   ItemWork w;
   w.valid = false;
   w.len_q = w.len_k = 0;
@@ -190,13 +190,15 @@ __device__ __forceinline__ ItemWork locate_item(const PrefillParams& p, int item
   // row blocks are the slowest-varying index and, under a causal mask, are handed out heaviest first;
   // the q heads of one KV head are neighbours and share its K/V in L2
   // with a split KV range every (sequence, KV part) pair is a sequence of its own here ("virtual" batch index)
+  // (in clusters: the parts of an item are the CTAs of one)
+  int part = 0;
+  if constexpr (kParts) { part = item % p.cluster_parts; item /= p.cluster_parts; }
   const int per_block = head_units * p.batch * p.kv_split;
   const int nblocks = blocks_of(p.max_q, rows);
   const int blk = item / per_block, rest = item - blk * per_block;
   const int wblock = p.is_causal ? (nblocks - 1 - blk) : blk;
   const int wunit = rest % head_units;
   const int vb = rest / head_units;                    // virtual batch index: rows of the partial buffer
-  int part = 0;
   w.valid = true;
   w.b = vb;
   if (p.kv_split > 1) { part = vb % p.kv_split; w.b = vb / p.kv_split; }
@@ -252,7 +254,7 @@ __device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w,
       n = n < 0 ? 0 : (n > cap ? cap : n);
       w.len_k = static_cast<int>(n);
     }
-    if (p.kv_split > 1) {
+    if (p.kv_split_len > 0) {
       // this item sees the keys [kv_tok0, kv_tok0 + kv_split_len) of the sequence only
       int local = w.len_k - w.kv_tok0;
       local = local < 0 ? 0 : (local > p.kv_split_len ? p.kv_split_len : local);
@@ -273,13 +275,25 @@ __device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w,
   }
 }
 
+// Parts in clusters: what a CTA sends of a strip of sixteen rows, a 16-byte piece per thread and register group: {references,
+// sums} of its two rows, then its columns.
+template <int D> constexpr int kStripPieces = (1 + D / 8) * 32;
+template <int D> __device__ __forceinline__ uint4* peer_strip(unsigned char* smem, int n) {
+  // (in clusters of eight a CTA owns two strips, of which seven others send it their parts)
+  static_assert(kSoftmaxWarps / 8 * 7 * kStripPieces<D> * 16 <= kRing * SmemPlan<D>::kTileBytes, "the tile buffers hold them");
+  return reinterpret_cast<uint4*>(smem + SmemPlan<D>::kRingOff) + n * kStripPieces<D>;
+}
+// weight of a part whose reference is m beside the largest one (a part that saw no key has -inf)
+__device__ __forceinline__ float part_weight(float m, float largest) { return m == -INFINITY ? 0.f : fast_exp2(m - largest); }
+
 // Persistent kernel: one CTA per SM; work items are drawn from a global counter (heaviest first).
 // The producer warp is also the scheduler: it publishes item indices through a 2-deep ring, so it can fetch Q
 // and the first K/V tiles of the next item while the other roles finish the current one.
 // kPaged: the instantiation launched for paged K/V; only it carries the block-table read-ahead of the producer (in
 // the dense / ragged kernel that code, though never run, cost 1 % on the dense benchmark configuration).  The other
-// layout checks stay run-time checks.
-template <typename T, int D, typename OutT, bool kPaged>
+// layout checks stay run-time checks.  kParts: the one launched in clusters that share an item (its epilogue costs the others
+// registers).
+template <typename T, int D, typename OutT, bool kPaged, bool kParts>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
@@ -333,7 +347,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // =========================== scheduler + TMA producer ===========================
     if (lane == 0) { prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); }
     // the first item of a CTA is its own index (the grid never exceeds the item count); later ones are drawn
-    ItemWork w = locate_item(p, static_cast<int>(blockIdx.x));
+    ItemWork w = locate_item<kParts>(p, static_cast<int>(blockIdx.x));
     // everything the other warps read or write outside this CTA follows an item published or a tile loaded below
     ptx::grid_dep_wait();
     bool ok = true;
@@ -370,7 +384,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       item = __shfl_sync(0xffffffffu, item, 0);
       if (item >= 0) {
-        if (k > 0) w = locate_item(p, item);
+        if (k > 0) w = locate_item<kParts>(p, item);
         // (the entries of a table row may be read before the sequence's length is known: which of them count is decided later)
         if (pf) {
           pg_k = first_pages(p.k_table, w);
@@ -733,6 +747,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     int out_phase = 0;       // o_done phase of its last PV
     int out_rows = 0;        // rows of the tile that exist in the sequence
     float out_la = 0.f, out_lb = 0.f;   // row sums of rows A and B
+    float out_ma = -INFINITY, out_mb = -INFINITY;   // ... and their references (kept for a merge)
     long long out_off = 0;   // element offset of row A's first output column
     long long out_stride = 0;   // elements between consecutive rows of the output
     constexpr bool k16 = !std::is_same<OutT, float>::value;
@@ -769,13 +784,55 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       }
     };
-    auto write_out = [&]() -> bool {
-      if (out_acc) {
+    // kMerge: with the parts that the other CTAs of the cluster have put into this CTA's tile buffers (see the end of the kernel)
+    auto write_out = [&](auto merging) -> bool {
+      constexpr bool kMerge = decltype(merging)::value;
+      if (out_acc && !kMerge) {
         if (!warp_wait(smem_u32(&ctrl->o_done[s]), out_phase)) return false;
       }
       tc_fence_after();
-      const float inv_a = out_la > 0.f ? 1.f / out_la : 0.f;
-      const float inv_b = out_lb > 0.f ? 1.f / out_lb : 0.f;
+      const int n_peers = kMerge ? p.cluster_parts - 1 : 0;
+      const uint4* const strip = kMerge ? peer_strip<D>(smem, warp / p.cluster_parts * n_peers) + lane : nullptr;
+      float self_a = 1.f, self_b = 1.f, ref_a = out_ma, ref_b = out_mb;     // weights of this CTA's part; largest references
+      if constexpr (kMerge) {
+        for (int k = 0; k < n_peers; ++k) {
+          const float4 ml = *reinterpret_cast<const float4*>(strip + k * kStripPieces<D>);
+          ref_a = fmaxf(ref_a, ml.x);
+          ref_b = fmaxf(ref_b, ml.y);
+        }
+        self_a = part_weight(out_ma, ref_a);
+        self_b = part_weight(out_mb, ref_b);
+        out_la *= self_a;
+        out_lb *= self_b;
+        for (int k = 0; k < n_peers; ++k) {
+          const float4 ml = *reinterpret_cast<const float4*>(strip + k * kStripPieces<D>);
+          out_la += ml.z * part_weight(ml.x, ref_a);
+          out_lb += ml.w * part_weight(ml.y, ref_b);
+        }
+      }
+      const float none = kMerge ? 0.f * (out_la + out_lb) : 0.f;      // (the NaN of a part that gave up shows)
+      const float inv_a = out_la > 0.f ? 1.f / out_la : none;
+      const float inv_b = out_lb > 0.f ? 1.f / out_lb : none;
+      // the 64 columns of block c: rows A and B as tmem_ld_16x256b_x8 gives them
+      auto merge_parts = [&](uint32_t (&v)[32], int c) {
+        if constexpr (kMerge) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * (i & 2 ? self_b : self_a));
+          for (int k = 0; k < n_peers; ++k) {
+            const uint4* const piece = strip + k * kStripPieces<D>;
+            const float4 ml = *reinterpret_cast<const float4*>(piece);
+            const float wa = part_weight(ml.x, ref_a), wb = part_weight(ml.y, ref_b);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint4 x = piece[(1 + c * 8 + i) * 32];
+              v[4 * i] = __float_as_uint(fmaf(__uint_as_float(x.x), wa, __uint_as_float(v[4 * i])));
+              v[4 * i + 1] = __float_as_uint(fmaf(__uint_as_float(x.y), wa, __uint_as_float(v[4 * i + 1])));
+              v[4 * i + 2] = __float_as_uint(fmaf(__uint_as_float(x.z), wb, __uint_as_float(v[4 * i + 2])));
+              v[4 * i + 3] = __float_as_uint(fmaf(__uint_as_float(x.w), wb, __uint_as_float(v[4 * i + 3])));
+            }
+          }
+        }
+      };
       constexpr int kChunksO = D / 64;
       if constexpr (k16) {
         // 16-bit output: 64 columns of a row are one 128-byte line.  A quad holds 8 consecutive columns per group;
@@ -792,6 +849,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
+          merge_parts(v, c);
           uint32_t a[8], b[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -835,6 +893,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
+          merge_parts(v, c);
           float* out = static_cast<float*>(p.out) + out_off + c * 64 + q * 2;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -1048,6 +1107,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       out_rows = slot_live ? min(kBM, len_q - m0s) : 0;
       out_la = quad_sum(l_a);
       out_lb = quad_sum(l_b);
+      out_ma = m_a;
+      out_mb = m_b;
       if (p.lse != nullptr && q == 0) {
         // split KV range: the merge needs every row's log-sum-exp (log2 domain; -inf for a row that saw no key)
         float* lse = p.lse + qrow0 + m0s + rowA;
@@ -1063,12 +1124,58 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));
-      ok = write_out();
+      if constexpr (kParts) break;       // (its only item: written when the parts have met)
+      else ok = write_out(std::false_type{});
+    }
+    if constexpr (kParts) {
+      // Parts of a KV range in a cluster: every warp's sixteen rows ("strip") have an owner among the CTAs.  The others send it
+      // their accumulator, row sums and references in fp32 into its tile buffers, register by register as the warp of the same
+      // number there holds its own; one barrier of the cluster says that all tile buffers are done with, a second that the
+      // parts have arrived.  (Every warp of the cluster meets at both; no wait before them is without a limit.)  A part that
+      // gave up sends NaN.
+      if (ok && out_acc) ok = warp_wait(smem_u32(&ctrl->o_done[s]), out_phase);
+      if (!ok) out_la = out_lb = __int_as_float(0x7fc00000);
+      tc_fence_after();
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      const int rank = static_cast<int>(cluster_rank()), parts = p.cluster_parts;
+      const int owner = warp % parts;
+      if (owner != rank) {
+        const int from = rank < owner ? rank : rank - 1;
+        const uint4* const strip = peer_strip<D>(smem, warp / parts * (parts - 1) + from) + lane;
+        const uint32_t to = map_to_rank(smem_u32(strip), static_cast<uint32_t>(owner));
+        st_cluster_v4(to, __float_as_uint(out_ma), __float_as_uint(out_mb), __float_as_uint(out_la), __float_as_uint(out_lb));
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) {
+          uint32_t v[32];
+          if (out_acc) {
+            tmem_ld_16x256b_x8(tO + c * 64, v);
+            tmem_wait_ld();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) st_cluster_v4(to + (1 + c * 8 + i) * 512, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+      }
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      if (owner == rank) write_out(std::true_type{});
     }
     if (!ok && lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
   }
 
   // ---------------- teardown ----------------
+  if (kParts && warp >= kSoftmaxWarps) {
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    cluster_arrive();
+    cluster_wait();
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp) {
@@ -1187,6 +1294,37 @@ SplitPlan split_plan(const b200attn_prefill_args_t& a, int sm_count) {
   return sp;
 }
 
+// The same with the parts of an item in a cluster, merged through distributed shared memory: for launches whose clusters are
+// all resident at once (one CTA to an SM: 74 of two, 33 of four, 15 of eight on a B200).  There is no second launch, and items
+// of four to seven tiles are worth cutting; but what a CTA sends, fp32 accumulators of 64 KB and more at head_dim 128, takes as
+// long as some tiles, so the costs below, in 128-key steps of 1.6 us.  Queries of one block of rows over 4, 6 and 12 tiles, four items,
+// head_dim 64 12.2 -> 11.0, 15.4 -> 12.6, 17.4 -> 13.2 us; at head_dim 128 12 tiles 18.3 -> 16.7 (in eight parts), 16 tiles 15.6 -> 16.8, so
+// those keep their parts in the workspace.
+SplitPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const SplitPlan& other) {
+  SplitPlan sp{1, 0};
+  if (a.layout == B200ATTN_RAGGED || a.batch <= 0 || a.max_q <= 0 || sm_count <= 0) return sp;
+  const bool head_pair = (a.q_heads / a.kv_heads) % 2 == 0;
+  const int item_rows = head_pair ? kBM : 2 * kBM;
+  const long long items = (a.max_q + item_rows - 1ll) / item_rows * (head_pair ? a.q_heads / 2 : a.q_heads) * a.batch;
+  const long long kv_cap = a.layout == B200ATTN_DENSE ? a.max_kv : a.table_stride * static_cast<long long>(a.page_size);
+  long long tiles = (kv_cap + kBN - 1) / kBN;
+  if (a.is_causal) tiles = std::min<long long>(tiles, (a.max_q + kBN - 1ll) / kBN);
+  // steps of the longest item, and what the parts cost beside them
+  static const double cluster_cost[2][3] = {{1.7, 2.3, 2.9}, {2.6, 3.8, 4.5}};
+  constexpr double kLaunchCost = 1.5, kGain = 0.4;
+  const long long whole = (tiles + other.parts - 1) / other.parts;
+  double best = static_cast<double>(whole) + (other.parts > 1 ? kLaunchCost : 0.0) - kGain;
+  static const int held[3] = {74, 33, 15};
+  for (int i = 0; i < 3; ++i) {
+    const int parts = 2 << i;
+    if (items > static_cast<long long>(held[i]) * sm_count / 148 || tiles < parts) break;
+    const long long per = (tiles + parts - 1) / parts;
+    const double cost = static_cast<double>(per) + cluster_cost[a.head_dim == 128][i];
+    if (cost < best) { best = cost; sp.parts = parts; sp.part_len = static_cast<int>(per * kBN); }
+  }
+  return sp;
+}
+
 struct CastPlan {
   size_t q_elems, kv_elems, q_off, k_off, v_off, total;
 };
@@ -1278,6 +1416,12 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
   p.kv_split = wsp.split.parts;
   p.kv_split_len = wsp.split.part_len;
   p.lse = nullptr;
+  p.cluster_parts = 1;
+  if (const SplitPlan cp = cluster_plan(a, sm_count, wsp.split); cp.parts > 1) {
+    p.cluster_parts = cp.parts;
+    p.kv_split = 1;
+    p.kv_split_len = cp.part_len;
+  }
   if (p.kv_split > 1) {
     // the kernel writes every part's normalised output and log-sum-exp into the workspace; a merge kernel follows
     unsigned char* ws = static_cast<unsigned char*>(a_in.workspace);
@@ -1312,25 +1456,32 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
       if ((rc = make_token_map(&tk, a.dtype, a.k, a.total_kv, a.kv_heads, D, box))) return rc;
       if ((rc = make_token_map(&tv, a.dtype, a.v, a.total_kv, a.kv_heads, D, box))) return rc;
     }
-    total_items = static_cast<long long>((a.max_q + item_rows - 1) / item_rows) * head_units * a.batch * p.kv_split;
+    total_items = static_cast<long long>((a.max_q + item_rows - 1) / item_rows) * head_units * a.batch * p.kv_split * p.cluster_parts;
   }
   if (total_items <= 0) return B200ATTN_OK;
   if (total_items > 0x7fffffff) { set_error("prefill: too many work items"); return B200ATTN_E_UNSUPPORTED; }
   p.total_items = static_cast<int>(total_items);
-  grid = dim3(static_cast<unsigned>(std::min<long long>(total_items, sm_count)), 1, 1);
+  grid = dim3(static_cast<unsigned>(p.cluster_parts > 1 ? total_items : std::min<long long>(total_items, sm_count)), 1, 1);
   // The two counters in the header (next item, CTAs finished) are zero here: the workspace starts zeroed and
   // the last CTA of every launch puts them back.
 
   cudaError_t e;
-#define B200ATTN_LAUNCH_PREFILL(TYPE, DIM, OUT)                                                          \
+#define B200ATTN_LAUNCH_PREFILL_AS(TYPE, DIM, OUT, PAGED, PARTS)                                         \
   do {                                                                                                   \
     const size_t smem = std::max<size_t>(SmemPlan<DIM>::kTotal + 1024, 120 * 1024);                      \
+    if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_kernel<TYPE, DIM, OUT, PAGED, PARTS>), smem))) return rc; \
+    launch_dependent(prefill_kernel<TYPE, DIM, OUT, PAGED, PARTS>, grid, kThreads, smem, stream,         \
+                     static_cast<unsigned>(p.cluster_parts), tq, tk, tv, p);                             \
+  } while (0)
+#define B200ATTN_LAUNCH_PREFILL(TYPE, DIM, OUT)                                                          \
+  do {                                                                                                   \
     if (a.layout == B200ATTN_PAGED) {                                                                    \
-      if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_kernel<TYPE, DIM, OUT, true>), smem))) return rc; \
-      launch_dependent(prefill_kernel<TYPE, DIM, OUT, true>, grid, kThreads, smem, stream, 1, tq, tk, tv, p);  \
+      if (p.cluster_parts > 1) B200ATTN_LAUNCH_PREFILL_AS(TYPE, DIM, OUT, true, true);                   \
+      else B200ATTN_LAUNCH_PREFILL_AS(TYPE, DIM, OUT, true, false);                                      \
+    } else if (p.cluster_parts > 1) {                                                                    \
+      B200ATTN_LAUNCH_PREFILL_AS(TYPE, DIM, OUT, false, true);                                           \
     } else {                                                                                             \
-      if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_kernel<TYPE, DIM, OUT, false>), smem))) return rc; \
-      launch_dependent(prefill_kernel<TYPE, DIM, OUT, false>, grid, kThreads, smem, stream, 1, tq, tk, tv, p); \
+      B200ATTN_LAUNCH_PREFILL_AS(TYPE, DIM, OUT, false, false);                                          \
     }                                                                                                    \
   } while (0)
   if (f32) {
@@ -1341,6 +1492,7 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
     if (D == 128) B200ATTN_LAUNCH_PREFILL(__half, 128, __half); else B200ATTN_LAUNCH_PREFILL(__half, 64, __half);
   }
 #undef B200ATTN_LAUNCH_PREFILL
+#undef B200ATTN_LAUNCH_PREFILL_AS
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "prefill kernel launch");
   if (p.kv_split > 1) {
