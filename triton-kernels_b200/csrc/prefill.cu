@@ -20,10 +20,11 @@
 //   O_s += P_s V_j    (TS MMA, A from TMEM, V is the MN-major B operand) -> commit o_done[s]
 // The two slots are interleaved so that one slot's softmax overlaps the other's MMAs.  At the end of an item the
 // MMA warp issues the first score tile of the next item behind the last PVs, and the softmax warps read O out, normalise
-// and store it while that tile is computed.
+// and store it while that tile is computed.  Launches of few items may cut an item's keys over the CTAs of a cluster (kParts,
+// cluster_plan): each runs its part as an item of its own, and the parts meet in the tile buffers at the end.
 //
 // What bounds it.  Long launches run at the board's 1 000 W (1.6 GHz instead of 1.97): there the time is the energy of a
-// tile, and an instruction left out per score counts for more than a shorter chain of waits.  The softmax is therefore as
+// tile, and an instruction left out per score counts in full, a shorter chain of waits half.  The softmax is therefore as
 // few instructions per pair of scores as there can be: one packed FMA, two exponentials, one packed add, one conversion,
 // and no row maximum.  Against a pass for the maximum before them and a quarter of the exponentials as polynomials on the
 // FMA pipes: 2 x 2 048 causal tokens, 32/8 heads, D 128, 86.2 -> 81.1 us; sixteen ragged sequences of 128 to 4 096
