@@ -1379,13 +1379,15 @@ __device__ __forceinline__ UmmaUnit umma_unit(const DecodeParams& p, int u) {
 }
 
 // T: element type of q, k, v as the kernel reads them; OutT: element type of the output rows (T, or float when the
-// inputs are fp16 copies of fp32 tensors).
-template <typename T, int D, typename OutT = T>
+// inputs are fp16 copies of fp32 tensors).  kOwnPlan: no planner has run, and every CTA works out the one unit that is its own.
+template <typename T, int D, typename OutT, bool kOwnPlan>
 __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __grid_constant__ CUtensorMap tm_k,
                                                              const __grid_constant__ CUtensorMap tm_v,
                                                              const DecodeParams p) {
   using namespace ptx;
   extern __shared__ unsigned char smem_raw[];
+  __shared__ InlinePlan s_plan;
+  __shared__ UmmaUnit s_unit;
   constexpr int CHUNKS = D / 64;
   constexpr int CHUNK_BYTES = kTileN * 128;
   constexpr int TILE_BYTES = CHUNKS * CHUNK_BYTES;
@@ -1448,9 +1450,32 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
 
   // (no launch_dependents here: with the next call's planner waiting beside it this kernel ran 3 % slower, 363 us
   // instead of 352 on 32 sequences of 1 to 33 thousand keys)
+  // (Nor without a planner: the next call's CTAs take the SMs that this one leaves empty, and then share some while others
+  // stay empty: one sequence of 8 000 keys, 64/8 heads, 8 drafts 36.0 us instead of 28.4, of 2 000 with 5 drafts 20.8 and 17.6.)
   ptx::grid_dep_wait();      // the planner's records are complete and visible from here on
-  const int n_units = p.header[2] * p.kv_heads;
   const int G = static_cast<int>(gridDim.x), me = static_cast<int>(blockIdx.x);
+  int n_units;
+  if constexpr (kOwnPlan) {
+    // a CTA per unit, which it works out itself: unit `me` is its only one
+    DecodeItem mine;
+    const bool have = plan_inline(p, me / p.kv_heads, s_plan, mine);
+    if (tid == 0 && have) {
+      UmmaUnit w;
+      w.seq_start = mine.start;
+      w.b = mine.b; w.h = me % p.kv_heads; w.c = mine.c; w.n_chunks = mine.n_chunks; w.item0 = mine.item0; w.len = mine.len;
+      w.t_begin = mine.t_begin; w.t_end = mine.t_end;
+      w.ntiles = w.t_end > w.t_begin ? (w.t_end - w.t_begin + kTileN - 1) / kTileN : 0;
+      s_unit = w;
+    }
+    __syncthreads();
+    n_units = have ? me + 1 : 0;
+  } else {
+    n_units = p.header[2] * p.kv_heads;
+  }
+  auto unit_of = [&](int u) -> UmmaUnit {
+    if constexpr (kOwnPlan) return s_unit;
+    else return umma_unit(p, u);
+  };
   // Units are handed out dynamically, longest first: a CTA's first unit is its own index, later ones are drawn from a
   // counter in the workspace header by the producer warp, which publishes them to the other warps through a small
   // ring in shared memory (a static deal cannot follow a batch of a few long and many short sequences: the CTAs that
@@ -1508,7 +1533,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
       mbar_arrive(smem_u32(&ctrl->unit_full[r % kUmmaUnitRing]));
     };
     // Dealt out (slots > 0): the CTA's units are the items of its slot, in order.  Else its first unit is its own index.
-    const int slots = p.header[5];
+    const int slots = kOwnPlan ? 0 : p.header[5];
     int u = me, u_end = n_units;
     if (slots > 0) {
       const int slot = me / p.kv_heads;
@@ -1522,7 +1547,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     if (u >= u_end) u = n_units;
     if (lane == 0) publish(0, u);
     for (int r = 0; ok && u < n_units; ++r) {
-      const UmmaUnit w = umma_unit(p, u);
+      const UmmaUnit w = unit_of(u);
       if (r == 0) ahead.start(p, w.b, w.t_begin, w.t_end);
       for (int tile = 0; tile < w.ntiles; ++tile) {
         const int stage = g % kUmmaStages, use = g / kUmmaStages;
@@ -1588,13 +1613,13 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         if (!ok || *abort_flag) { ok = false; break; }
       }
       if (lane == 0) {
-        u_next = slots > 0 ? u + p.kv_heads : min(G + atomicAdd(p.header + 4, 1), n_units);
+        u_next = kOwnPlan ? n_units : slots > 0 ? u + p.kv_heads : min(G + atomicAdd(p.header + 4, 1), n_units);
         if (u_next >= u_end) u_next = n_units;
         publish(r + 1, u_next);
       }
       u_next = __shfl_sync(0xffffffffu, u_next, 0);
       if (u_next < n_units) {
-        const UmmaUnit w2 = umma_unit(p, u_next);
+        const UmmaUnit w2 = unit_of(u_next);
         ahead.start(p, w2.b, w2.t_begin, w2.t_end);
         const T* q2 = static_cast<const T*>(p.q) +
                       ((static_cast<long long>(w2.b) * p.q_heads + static_cast<long long>(w2.h) * p.head_stride + p.head0) * p.q_len) * D;
@@ -1619,7 +1644,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         if (u < 0) { ok = false; break; }
         unit_done(r);
         if (u >= n_units) break;
-        const UmmaUnit w = umma_unit(p, u);
+        const UmmaUnit w = unit_of(u);
         ahead.start(p, w.b, w.t_begin, w.t_end);
         for (int tile = 0; tile < w.ntiles; ++tile, ++g) {
           const int stage = g % kUmmaStages, use = g / kUmmaStages;
@@ -1659,7 +1684,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
       const int u = unit_at(r);
       if (u < 0) { ok = false; break; }
       if (u >= n_units) break;
-      const UmmaUnit w = umma_unit(p, u);
+      const UmmaUnit w = unit_of(u);
       ok = warp_wait(smem_u32(&ctrl->q_ready), r & 1);
       if (!ok || *abort_flag) { ok = false; break; }
       if (w.ntiles == 0) {
@@ -1771,7 +1796,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     };
     int u = unit_at(0);
     if (u < 0) ok = false;
-    UmmaUnit w = umma_unit(p, min(max(u, 0), max(n_units - 1, 0)));
+    UmmaUnit w = unit_of(min(max(u, 0), max(n_units - 1, 0)));
     if (ok) write_q(u, w);
     for (; ok; ++r) {
       if (u >= n_units) break;
@@ -1931,7 +1956,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
       // way into L2): its Q goes to tensor memory before this unit's rows are written out
       const int u_next = unit_at(r + 1);
       if (u_next < 0) { ok = false; break; }
-      const UmmaUnit w_next = u_next < n_units ? umma_unit(p, u_next) : w;
+      const UmmaUnit w_next = u_next < n_units ? unit_of(u_next) : w;
       write_q(u_next, w_next);
       // ---------------- the unit's rows leave tensor memory ----------------
       if (w.ntiles > 0) {
@@ -1997,7 +2022,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         // mbarrier with a bounded wait, never on bar.sync: a warp that gave up must not hang the rest.
         draw_owed_ticket();
         mbar_arrive(smem_u32(&ctrl->rows_out));
-        owed_pair = w.b * p.kv_heads + w.h;
+        if (!kOwnPlan) owed_pair = w.b * p.kv_heads + w.h;      // (else the teardown draws)
         owed_round = r;
         ++merges;
       }
@@ -2016,12 +2041,34 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
   tc_fence_before();
   __syncthreads();
   if (warp == kMma) { tc_fence_after(); tmem_dealloc(tmem, kUmmaTmemCols); }
+  if constexpr (kOwnPlan) {
+    // One unit: its ticket is drawn here, by every CTA that has one, and the last of a pair's merges it.
+    const UmmaUnit w = s_unit;
+    if (n_units > 0 && w.n_chunks > 1) {
+      const long long slot = (static_cast<long long>(w.item0) + w.c) * p.kv_heads + w.h;
+      if (ctrl->abort_flag) {
+        // (a wait ran out: the rows are unknown, and NaN says so in the merge)
+        for (int i = tid; i < R * D; i += blockDim.x) p.part_o[slot * R * D + i] = __int_as_float(0x7fc00000);
+        for (int i = tid; i < R * 2; i += blockDim.x) p.part_ml[slot * R * 2 + i] = __int_as_float(0x7fc00000);
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) ctrl->ready = draw_ticket(p, w.b * p.kv_heads + w.h);
+      __syncthreads();
+      if (ctrl->ready == w.n_chunks - 1) {
+        OutT* out = static_cast<OutT*>(p.out) +
+                    ((static_cast<long long>(w.b) * p.q_heads + static_cast<long long>(w.h) * p.head_stride + p.head0) * p.q_len) * D;
+        merge_chunks<OutT, D>(p, w.b, w.h, w.n_chunks, w.item0, out, tid, static_cast<int>(blockDim.x));
+      }
+      return;
+    }
+  }
   // Merges.  A (sequence, kv head) pair whose chunks have all drawn their tickets is merged by whichever CTA claims
   // it while sweeping the ticket counters here, with all of its threads: CTAs that finish early take the pairs that
   // are complete, the CTA that draws a pair's last ticket sweeps after it did, so every pair is merged by the time
   // the last CTA leaves, and no CTA waits for another.  A CTA takes one pair per sweep and sweeps again as long as it
   // saw a complete pair; header[3] (tickets drawn and not merged) lets a CTA skip the sweep when there is nothing.
-  if (!ctrl->abort_flag) {
+  if (!ctrl->abort_flag && !kOwnPlan) {
     const int n_pairs = p.batch * p.kv_heads;
     for (int sweep = 0; sweep < n_pairs + 64; ++sweep) {
       if (tid == 0) {
@@ -2065,7 +2112,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     for (int r = ctrl->abort_round; r < ctrl->published; ++r) {
       const int u = ctrl->unit_ring[r % kUmmaUnitRing];
       if (u >= n_units) break;
-      const UmmaUnit w = umma_unit(p, u);
+      const UmmaUnit w = unit_of(u);
       OutT* out = static_cast<OutT*>(p.out) +
                   ((static_cast<long long>(w.b) * p.q_heads + static_cast<long long>(w.h) * p.head_stride + p.head0) * p.q_len) * D;
       for (int i = tid; i < R * D; i += blockDim.x) out[i] = nan_t;
@@ -2605,6 +2652,18 @@ Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool bui
   return r;
 }
 
+// Whether the CTAs of the tcgen05 kernel (16-bit elements, more than sixteen rows; two CTAs to an SM) plan for themselves too.
+//
+// The planner's launch was some 5 us of a call there.  But it deals a batch out to the CTAs by keys, which no CTA can see by itself (a
+// batch cut into equal items leaves some CTAs without one), and a CTA's own plan takes longer the more sequences there are.
+// So: up to 1 024 keys for each CTA, less 8 for every sequence.  40 rows, D 128, with the planner and without, in us: 12 x 300
+// keys of eight heads 15.7, 12.4; 1 x 2 000 22.9, 17.6; 10 x 2 590 39.0, 31.9; 38 x 1 557 of two heads 30.8, 25.7; 60 x 1 973 of one
+// 30.8, 26.8; 90 x 1 315 30.3, 30.0; and beyond the line 60 x 4 933 45.6, 47.9; 75 x 3 946 45.7, 49.8; 90 x 2 302 38.4, 44.3.
+bool wide_plans_itself(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in) {
+  return !built_in && a.dtype != B200ATTN_F32 && rows > 16 && static_cast<long long>(a.batch) * a.kv_heads <= kInlinePairs &&
+         most_keys(a) * a.kv_heads <= (1024 - 8ll * a.batch) * 2 * sm_count;
+}
+
 // `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
 int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, const DecodeWsLayout& w,
                        int pass_group, int head0, bool f32_out, bool built_in) {
@@ -2642,6 +2701,17 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   const Route route = route_of(a, sm_count, p.rows, built_in, /*ask=*/true);
   p.cluster = route.cluster;
   p.inline_plan = route.inline_plan;
+  if (wide_plans_itself(a, sm_count, p.rows, built_in)) {
+    p.inline_plan = 16;
+    // Few sequences: items for one CTA an SM, not two, up to six of the shortest.  A second CTA on some of the SMs holds its neighbour up,
+    // and a merge, one CTA's work, is as long as a sequence has items: 1 x 8 000 keys of eight heads, 40 rows, D 128, 35.8 -> 25.7
+    // us, 3 x 12 000 of two 45.6 -> 28.6, 1 x 30 000 of four, 64 rows, 71.2 -> 50.1.  (With any batch 12 x 1 400 in pages 21.0 ->
+    // 23.6, 4 x 3 000 of eight, D 64, 16.0 -> 19.1.)
+    if (a.batch <= 3 && most_keys(a) * a.kv_heads <= 6ll * w.min_chunk * sm_count) {
+      p.target_items = std::max(1, sm_count / a.kv_heads);
+      p.wave_items = 0;
+    }
+  }
   unsigned grid_items = static_cast<unsigned>(w.max_items);
   cudaError_t e = cudaSuccess;
   if (p.inline_plan) {
@@ -2692,12 +2762,13 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     const size_t smem = 1024 + stage_bytes + sizeof(UmmaCtrl);
     // persistent: one wave of two CTAs per SM walks the unit list (fewer CTAs when the list cannot be longer)
     const unsigned wave = 2u * static_cast<unsigned>(sm_count);
-    const dim3 grid(std::min(static_cast<unsigned>(w.max_items) * a.kv_heads, wave), 1);
-#define B200ATTN_LAUNCH_UMMA(TYPE, DIM, OUT)                             \
-    do {                                                                 \
-      rc = set_smem(decode_umma_kernel<TYPE, DIM, OUT>, smem);           \
-      if (rc) return rc;                                                 \
-      launch_dependent(decode_umma_kernel<TYPE, DIM, OUT>, grid, kUmmaThreads, smem, stream, 1, tk, tv, p); \
+    const dim3 grid(p.inline_plan ? grid_items * a.kv_heads : std::min(static_cast<unsigned>(w.max_items) * a.kv_heads, wave), 1);
+#define B200ATTN_LAUNCH_UMMA(TYPE, DIM, OUT)                                  \
+    do {                                                                      \
+      auto* kernel = p.inline_plan ? decode_umma_kernel<TYPE, DIM, OUT, true> \
+                                   : decode_umma_kernel<TYPE, DIM, OUT, false>; \
+      if ((rc = set_smem(kernel, smem))) return rc;                           \
+      launch_dependent(kernel, grid, kUmmaThreads, smem, stream, 1, tk, tv, p); \
     } while (0)
     if (f32_out) {
       if (D == 128) B200ATTN_LAUNCH_UMMA(__half, 128, float); else B200ATTN_LAUNCH_UMMA(__half, 64, float);
