@@ -169,8 +169,7 @@ size_t b200attn_decode_workspace_bytes(const b200attn_decode_args_t* args);
 /*
  * Which way b200attn_decode (`is_static`: b200attn_decode_static) takes a call on a GPU of `sm_count` SMs: in clusters of 1, 2, 4
  * or 8 CTAs per (sequence, KV head) pair, in items that the CTAs plan for themselves (B200ATTN_ROUTE_INLINE) or behind the
- * planner's launch (B200ATTN_ROUTE_PLANNER; so are reported all calls of the tcgen05 kernel, more than 16 q rows per KV head
- * in 16 bits, although the CTAs of its short ones plan for themselves too).  Host arithmetic on the sizes; needs no GPU, reads no pointer.  No counterpart in
+ * planner's launch (B200ATTN_ROUTE_PLANNER).  Host arithmetic on the sizes; needs no GPU, reads no pointer.  No counterpart in
  * the reference.
  */
 int b200attn_decode_route(const b200attn_decode_args_t* args, int sm_count, int is_static);

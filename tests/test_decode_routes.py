@@ -88,7 +88,7 @@ def test_clusters_take_what_they_can_hold(sms):
                         c = route(layout, dtype, batch, qh, 1, 64, keys, m=m, sms=sms)
                         assert c in (PLANNER, INLINE, 1, 2, 4, 8)
                         if keys and qh * m > 16 and (dtype == "bf16" or m > 1):
-                            assert c == PLANNER
+                            assert c in (PLANNER, INLINE)
                         if batch > 96:
                             assert c != INLINE
                         if 1 < c <= 8:

@@ -2615,53 +2615,54 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows, bool a
   }
 }
 
-// Which way a pass of `rows` q rows per KV head goes: clusters (CTAs per pair), or items that the CTAs plan for themselves, or
-// (neither) items behind the planner.  More than sixteen rows of 16-bit elements always go to the tcgen05 kernel; those of fp32 are
-// planned (at six microseconds a tile and more a part is rarely short enough, and none was measured).
-//
-// Few (sequence, kv head) pairs: the CTAs plan for themselves (plan_inline, about a microsecond each) and the planner's
-// launch, 4 to 5 us in front of the kernel, goes.  The line is the number of merge tickets that fit into the header,
-// the only part of a workspace that may be relied on to be zero without a launch; beyond it a call streams for longer
-// and the planner is a smaller part of it.  fp32, which reads twice the bytes: twice as many pairs, with tickets of eight bits
-// where no pair can be cut into more items than those count, up to 300 MiB of keys and values (the most that there can be).  16
-// packed sequences of 100 to 4 096 keys, 8/8 heads, D 64 36.3 -> 32.4 us, 13 x 1 500 18.9 -> 15.5, 24 x 1 500 at D 128 in pages 43.8 ->
-// 38.7; 20 x 3 000 119 -> 113, but 20 x 10 000 281 -> 290 (64/8 heads, dense): the planner puts the last, shorter item of each
-// sequence behind all others, which is worth more than its launch there.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
-// keys of two heads 17.2 -> 13.0, four drafts for 16 short sequences 15.1 -> 12.9, 7 x 30 201 keys at 0.98 of the copy
-// bandwidth.  Not in the library's own array (`built_in`): nobody can zero that again after two calls have overlapped on it against
-// the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
-// in every call.
 // keys of all sequences, as many as there can be
 long long most_keys(const b200attn_decode_args_t& a) {
   if (a.layout == B200ATTN_RAGGED) return a.total_kv;
   return a.batch * (a.layout == B200ATTN_DENSE ? static_cast<long long>(a.max_kv) : a.table_stride * a.page_size);
 }
+
+// Bits of a merge ticket where the CTAs plan for themselves (plan_inline, about a microsecond each), 0 where the call needs the
+// planner's launch, 4 to 5 us in front of the kernel.
+//
+// Up to sixteen rows, and fp32: few (sequence, kv head) pairs.  The line is the number of merge tickets that fit into the header,
+// the only part of a workspace that may be relied on to be zero without a launch; beyond it a call streams for longer
+// and the planner is a smaller part of it.  Measured: one user 22.2 -> 17.7 us per (append, append, decode), 16 x 2 048
+// keys of two heads 17.2 -> 13.0, four drafts for 16 short sequences 15.1 -> 12.9, 7 x 30 201 keys at 0.98 of the copy
+// bandwidth.  fp32, which reads twice the bytes: twice as many pairs, with tickets of eight bits
+// where no pair can be cut into more items than those count, up to 300 MiB of keys and values (the most that there can be).  16
+// packed sequences of 100 to 4 096 keys, 8/8 heads, D 64 36.3 -> 32.4 us, 13 x 1 500 18.9 -> 15.5, 24 x 1 500 at D 128 in pages 43.8 ->
+// 38.7; 20 x 3 000 119 -> 113, but 20 x 10 000 281 -> 290 (64/8 heads, dense): the planner puts the last, shorter item of each
+// sequence behind all others, which is worth more than its launch there.
+//
+// More than sixteen rows (the tcgen05 kernel; two CTAs to an SM): the planner deals a batch out to the CTAs by keys, which no CTA can
+// see by itself (a batch cut into equal items leaves some CTAs without one), and a CTA's own plan takes longer the more sequences there
+// are.  So: up to 1 024 keys for each CTA, less 8 for every sequence.  40 rows, D 128, with the planner and without, in us: 12 x 300
+// keys of eight heads 15.7, 12.4; 1 x 2 000 22.9, 17.6; 10 x 2 590 39.0, 31.9; 38 x 1 557 of two heads 30.8, 25.7; 60 x 1 973 of one
+// 30.8, 26.8; 90 x 1 315 30.3, 30.0; and beyond the line 60 x 4 933 45.6, 47.9; 75 x 3 946 45.7, 49.8; 90 x 2 302 38.4, 44.3.
+//
+// Not in the library's own array: nobody can zero that again after two calls have overlapped on it against
+// the rules, and a ticket left over there would keep later calls from ever merging; the planner's tickets start at zero
+// in every call.
+int inline_plan_bits(const b200attn_decode_args_t& a, int sm_count, int rows) {
+  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads, keys = most_keys(a);
+  if (a.dtype != B200ATTN_F32 && rows > 16)
+    return pairs <= kInlinePairs && keys * a.kv_heads <= (1024 - 8ll * a.batch) * 2 * sm_count ? 16 : 0;
+  if (pairs <= kInlinePairs) return 16;
+  return a.dtype == B200ATTN_F32 && pairs <= kInlinePairs8 && a.batch <= kInlineBatch &&
+         decode_target_items(sm_count, a.kv_heads) + a.batch <= 255 &&
+         2 * keys * a.kv_heads * a.head_dim * 4 <= 300ll << 20 ? 8 : 0;
+}
+
+// Which way a pass of `rows` q rows per KV head goes: clusters (CTAs per pair), or items that the CTAs plan for themselves, or
+// (neither) items behind the planner.  More than sixteen rows of 16-bit elements always go to the tcgen05 kernel; those of fp32 are
+// planned (at six microseconds a tile and more a part is rarely short enough, and none was measured).
 struct Route { int cluster, inline_plan; };      // (inline_plan: the bits of a ticket)
 // `ask`: see clusters_held.
 Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in, bool ask) {
   Route r;
   r.cluster = rows <= 16 ? cluster_size(a, sm_count, rows, ask) : 0;
-  r.inline_plan = 0;
-  if (built_in || r.cluster || (a.dtype != B200ATTN_F32 && rows > 16)) return r;
-  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
-  if (pairs <= kInlinePairs) r.inline_plan = 16;
-  else if (a.dtype == B200ATTN_F32 && pairs <= kInlinePairs8 && a.batch <= kInlineBatch &&
-           decode_target_items(sm_count, a.kv_heads) + a.batch <= 255 &&
-           2 * most_keys(a) * a.kv_heads * a.head_dim * 4 <= 300ll << 20)
-    r.inline_plan = 8;
+  r.inline_plan = built_in || r.cluster ? 0 : inline_plan_bits(a, sm_count, rows);
   return r;
-}
-
-// Whether the CTAs of the tcgen05 kernel (16-bit elements, more than sixteen rows; two CTAs to an SM) plan for themselves too.
-//
-// The planner's launch was some 5 us of a call there.  But it deals a batch out to the CTAs by keys, which no CTA can see by itself (a
-// batch cut into equal items leaves some CTAs without one), and a CTA's own plan takes longer the more sequences there are.
-// So: up to 1 024 keys for each CTA, less 8 for every sequence.  40 rows, D 128, with the planner and without, in us: 12 x 300
-// keys of eight heads 15.7, 12.4; 1 x 2 000 22.9, 17.6; 10 x 2 590 39.0, 31.9; 38 x 1 557 of two heads 30.8, 25.7; 60 x 1 973 of one
-// 30.8, 26.8; 90 x 1 315 30.3, 30.0; and beyond the line 60 x 4 933 45.6, 47.9; 75 x 3 946 45.7, 49.8; 90 x 2 302 38.4, 44.3.
-bool wide_plans_itself(const b200attn_decode_args_t& a, int sm_count, int rows, bool built_in) {
-  return !built_in && a.dtype != B200ATTN_F32 && rows > 16 && static_cast<long long>(a.batch) * a.kv_heads <= kInlinePairs &&
-         most_keys(a) * a.kv_heads <= (1024 - 8ll * a.batch) * 2 * sm_count;
 }
 
 // `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
@@ -2701,9 +2702,8 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   const Route route = route_of(a, sm_count, p.rows, built_in, /*ask=*/true);
   p.cluster = route.cluster;
   p.inline_plan = route.inline_plan;
-  if (wide_plans_itself(a, sm_count, p.rows, built_in)) {
-    p.inline_plan = 16;
-    // Few sequences: items for one CTA an SM, not two, up to six of the shortest.  A second CTA on some of the SMs holds its neighbour up,
+  if (p.inline_plan && a.dtype != B200ATTN_F32 && p.rows > 16) {
+    // The tcgen05 kernel, few sequences: items for one CTA an SM, not two, up to six of the shortest.  A second CTA on some of the SMs holds its neighbour up,
     // and a merge, one CTA's work, is as long as a sequence has items: 1 x 8 000 keys of eight heads, 40 rows, D 128, 35.8 -> 25.7
     // us, 3 x 12 000 of two 45.6 -> 28.6, 1 x 30 000 of four, 64 rows, 71.2 -> 50.1.  (With any batch 12 x 1 400 in pages 21.0 ->
     // 23.6, 4 x 3 000 of eight, D 64, 16.0 -> 19.1.)
