@@ -811,9 +811,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           out_lb += ml.w * part_weight(ml.y, ref_b);
         }
       }
-      const float none = kMerge ? 0.f * (out_la + out_lb) : 0.f;      // (the NaN of a part that gave up shows)
-      const float inv_a = out_la > 0.f ? 1.f / out_la : none;
-      const float inv_b = out_lb > 0.f ? 1.f / out_lb : none;
+      // (a sum that is no number shows in its own row, also where no part has an accumulator)
+      const float inv_a = out_la > 0.f ? 1.f / out_la : kMerge ? 0.f * out_la : 0.f;
+      const float inv_b = out_lb > 0.f ? 1.f / out_lb : kMerge ? 0.f * out_lb : 0.f;
       // the 64 columns of block c: rows A and B as tmem_ld_16x256b_x8 gives them
       auto merge_parts = [&](uint32_t (&v)[32], int c) {
         if constexpr (kMerge) {
