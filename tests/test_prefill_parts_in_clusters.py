@@ -70,3 +70,24 @@ def test_rows_keep_to_themselves(d):
     assert not out[:, :, [3, 12]].any() and not want[:, :, [3, 12]].any()
     # (a warp with such a row takes its tiles in two passes: P and the output rounded to eight bits around another reference)
     torch.testing.assert_close(out[:, :, ~nan].float(), want[:, :, ~nan].float(), atol=2**-7, rtol=2**-7)
+
+
+@pytest.mark.parametrize("longest,d", [(760, 64), (1500, 64), (1500, 128)])
+@pytest.mark.parametrize("queries,causal", [(100, False), (700, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+def test_sequences_shorter_than_the_table(longest, d, queries, causal, dtype):
+    """An item of fewer tiles than the parts are worth is the first CTA's alone: every number of tiles up to the widest, also none."""
+    from kernels import flash_attention_v2
+
+    gen = torch.Generator().manual_seed(longest + d)
+    b, page = (13, 16) if queries == 100 else (2, 16)
+    lens = ([0, longest] + [n for t in range(1, 12) for n in (128 * t, 128 * t + 1) if n <= longest])[:b]
+    qs = [torch.randn((queries, 2, d), generator=gen).to(dtype).to(DEV) for _ in lens]
+    ks, vs = ([torch.randn((n, 1, d), generator=gen).to(dtype).to(DEV) for n in lens] for _ in range(2))
+    (kc, kt, n), (vc, vt, _) = (sdpa_ref.pack_paged(x, page, permute_seed=3, extra_pages=2, pad_value=-1, poison=float("nan")) for x in (ks, vs))
+    q = torch.stack([x.transpose(0, 1) for x in qs]).contiguous()
+    out = flash_attention_v2(q, kc, vc, is_causal=causal, kv_indptr=n, k_block_table=kt, v_block_table=vt, kv_page_size=page)
+    assert not out[0].any()
+    refs = sdpa_ref.prefill_reference(qs[1:], ks[1:], vs[1:], 2, 1, causal)
+    for i, ref in enumerate(refs, 1):
+        assert_close_both(out[i].transpose(0, 1), ref, dtype, max(1, lens[i]), f"{lens[i]} keys", strict=4e-3 if dtype == torch.float32 else None)

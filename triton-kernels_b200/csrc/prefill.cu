@@ -81,6 +81,7 @@ struct ItemWork {
   int m0[kSlots];      // first query row of each slot inside the sequence
   int nkv[kSlots];     // 128-key tiles each slot visits
   int nkv_max;
+  bool cut;            // (parts in clusters) the CTAs of the cluster share the item's keys; else the first of them does it alone
 };
 
 // shared-memory control block placed after the tiles
@@ -179,6 +180,7 @@ template <bool kParts> __device__ __forceinline__ ItemWork locate_item(const Pre
   w.kv_head_coord = 0;
   w.b = 0;
   w.nkv_max = 0;
+  w.cut = false;
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) {
     w.q_row0[s] = w.out_row0[s] = 0;
@@ -221,7 +223,7 @@ template <bool kParts> __device__ __forceinline__ ItemWork locate_item(const Pre
   return w;
 }
 
-__device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
+template <bool kParts> __device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
   if (p.layout == B200ATTN_RAGGED) {
     const int heads_per_item = p.head_pair ? 2 : 1;
     const int head_units = p.q_heads / heads_per_item;
@@ -255,7 +257,17 @@ __device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w,
       n = n < 0 ? 0 : (n > cap ? cap : n);
       w.len_k = static_cast<int>(n);
     }
-    if (p.kv_split_len > 0) {
+    // Parts in clusters: what the host cut is the longest that an item can be.  This one may be shorter, by its sequence's length or by
+    // its place under the diagonal, and not worth what the parts cost: every CTA of the cluster decides that by the same numbers,
+    // and the first takes the whole.  (64 queries over 100 keys in a table of 768, 8/2 heads, D 64: cut 11.1 us, not cut 7.4, a
+    // launch without clusters 7.3; over 700 in one of 1 536 13.0, 15.2 and, cut into parts in the workspace, 16.8.)
+    if constexpr (kParts) {
+      int tiles = (w.len_k + kBN - 1) / kBN;
+      if (p.is_causal) tiles = min(tiles, (min(w.m0[kSlots - 1] + kBM, w.len_q) + kBN - 1) / kBN);
+      w.cut = tiles >= p.cut_tiles;
+      if (!w.cut && w.kv_tok0 > 0) w.len_k = 0;
+    }
+    if (kParts ? w.cut : p.kv_split_len > 0) {
       // this item sees the keys [kv_tok0, kv_tok0 + kv_split_len) of the sequence only
       int local = w.len_k - w.kv_tok0;
       local = local < 0 ? 0 : (local > p.kv_split_len ? p.kv_split_len : local);
@@ -343,6 +355,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
   const uint32_t tmem = warp == kProducerWarp ? 0u : ctrl->tmem_base;   // (the producer never uses it)
   volatile int* abort_flag = &ctrl->abort_flag;
+  // Parts in clusters: every warp of the cluster takes part in two barriers (at the end of this kernel) whatever happens, so that none
+  // can wait for one that is not coming.  Where the item is not cut there is nothing to meet for: the warps arrive early and
+  // find the barriers completed later (both at the end cost that item 1.0 us, both at its start 1.3, as placed 0.1).
+  auto meet_arrive = [] { __syncwarp(); cluster_arrive_relaxed(); };
+  auto meet_again = [] { __syncwarp(); cluster_wait(); cluster_arrive_relaxed(); };
+  int met = 0;         // halves of the two barriers that this warp has been through
 
   if (warp == kProducerWarp) {
     // =========================== scheduler + TMA producer ===========================
@@ -391,7 +409,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           pg_k = first_pages(p.k_table, w);
           pg_v = first_pages(p.v_table, w);
         }
-        finish_item(p, w, item, lane);
+        finish_item<kParts>(p, w, item, lane);
       }
       if (lane == 0) {
         if (item >= 0) ctrl->sched_work[k & 1] = w;
@@ -399,6 +417,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         mbar_arrive(smem_u32(&ctrl->sched_full[k & 1]));
       }
       if (item < 0) break;
+      if (kParts && !w.cut) { meet_arrive(); met = 1; }
       const int* vtab = kPaged ? p.v_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
       const int* ktab = kPaged ? p.k_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
       auto read_page = [&](const int* tab, int first_box) -> int {
@@ -542,6 +561,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
         }
         if (pi == 0) ok = load_q(1);
+        if (kParts && pi == 1 && met == 1) { meet_again(); met = 3; }
       }
     }
     if (!ok) {
@@ -637,6 +657,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const int item = ctrl->sched_item[k & 1];
       if (item < 0) break;
       const ItemWork& wr = ctrl->sched_work[k & 1];
+      if (kParts && !wr.cut) { meet_arrive(); met = 1; }
       const int nkv0 = wr.nkv[0], nkv1 = wr.nkv[1], nkv_max = wr.nkv_max, len_k = wr.len_k;
       const int qbuf0 = (2 * k) % kQBufs, qbuf1 = (2 * k + 1) % kQBufs;
       const uint64_t qd0 = q_desc_of(qbuf0), qd1 = q_desc_of(qbuf1);
@@ -645,6 +666,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (ok && !pre_issued1) ok = start_slot(1, k, nkv1, pair_base);
       if (!ok) break;
       if (nkv_max > 0) mma_commit_lead(smem_u32(&ctrl->kv_empty[pair_base % kStages]), lead);
+      if (kParts && met == 1) { meet_again(); met = 3; }
       pre_issued0 = pre_issued1 = false;
       for (int j = 0; j < nkv_max && ok; ++j) {
         const int pr = pair_base + 1 + j;     // the pair {V_j, K_j+1}
@@ -751,6 +773,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     float out_ma = -INFINITY, out_mb = -INFINITY;   // ... and their references (kept for a merge)
     long long out_off = 0;   // element offset of row A's first output column
     long long out_stride = 0;   // elements between consecutive rows of the output
+    bool cut = true;         // (parts in clusters; a CTA that never saw its item sends its NaN)
     constexpr bool k16 = !std::is_same<OutT, float>::value;
     auto quad_max = [](float v) {
       v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
@@ -913,6 +936,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (!ok || *abort_flag) { ok = false; break; }
       const int item = ctrl->sched_item[k & 1];
       if (item < 0) break;
+      if (kParts && !ctrl->sched_work[0].cut) { meet_arrive(); meet_again(); }
       // (the few fields needed are read from shared memory where they are used, not held across the tile loop)
       const ItemWork& w = ctrl->sched_work[k & 1];
       const int n = w.nkv[s];
@@ -1097,6 +1121,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->p_ready[s]));
       }
+      if constexpr (kParts) cut = w.cut;
       if (!ok) break;
       // ---------------- the item's epilogue ----------------
       const int len_q = w.len_q;
@@ -1134,37 +1159,43 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // number there holds its own; one barrier of the cluster says that all tile buffers are done with, a second that the
       // parts have arrived.  (Every warp of the cluster meets at both; no wait before them is without a limit.)  A part that
       // gave up sends NaN.
-      if (ok && out_acc) ok = warp_wait(smem_u32(&ctrl->o_done[s]), out_phase);
-      if (!ok) out_la = out_lb = __int_as_float(0x7fc00000);
-      tc_fence_after();
-      __syncwarp();
-      cluster_arrive();
-      cluster_wait();
       const int rank = static_cast<int>(cluster_rank()), parts = p.cluster_parts;
-      const int owner = warp % parts;
-      if (owner != rank) {
-        const int from = rank < owner ? rank : rank - 1;
-        const uint4* const strip = peer_strip<D>(smem, warp / parts * (parts - 1) + from) + lane;
-        const uint32_t to = map_to_rank(smem_u32(strip), static_cast<uint32_t>(owner));
-        st_cluster_v4(to, __float_as_uint(out_ma), __float_as_uint(out_mb), __float_as_uint(out_la), __float_as_uint(out_lb));
+      if (!cut) {
+        __syncwarp();
+        cluster_wait();
+        if (ok && rank == 0) ok = write_out(std::false_type{});
+      } else {
+        if (ok && out_acc) ok = warp_wait(smem_u32(&ctrl->o_done[s]), out_phase);
+        if (!ok) out_la = out_lb = __int_as_float(0x7fc00000);
+        tc_fence_after();
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        const int owner = warp % parts;
+        if (owner != rank) {
+          const int from = rank < owner ? rank : rank - 1;
+          const uint4* const strip = peer_strip<D>(smem, warp / parts * (parts - 1) + from) + lane;
+          const uint32_t to = map_to_rank(smem_u32(strip), static_cast<uint32_t>(owner));
+          st_cluster_v4(to, __float_as_uint(out_ma), __float_as_uint(out_mb), __float_as_uint(out_la), __float_as_uint(out_lb));
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) {
-          uint32_t v[32];
-          if (out_acc) {
-            tmem_ld_16x256b_x8(tO + c * 64, v);
-            tmem_wait_ld();
-          } else {
+          for (int c = 0; c < D / 64; ++c) {
+            uint32_t v[32];
+            if (out_acc) {
+              tmem_ld_16x256b_x8(tO + c * 64, v);
+              tmem_wait_ld();
+            } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0u;
+              for (int i = 0; i < 32; ++i) v[i] = 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) st_cluster_v4(to + (1 + c * 8 + i) * 512, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
           }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) st_cluster_v4(to + (1 + c * 8 + i) * 512, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
         }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        if (owner == rank) write_out(std::true_type{});
       }
-      __syncwarp();
-      cluster_arrive();
-      cluster_wait();
-      if (owner == rank) write_out(std::true_type{});
     }
     if (!ok && lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
   }
@@ -1172,10 +1203,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   // ---------------- teardown ----------------
   if (kParts && warp >= kSoftmaxWarps) {
     __syncwarp();
-    cluster_arrive();
-    cluster_wait();
-    cluster_arrive();
-    cluster_wait();
+    if (met < 1) cluster_arrive();
+    if (met < 2) cluster_wait();
+    if (met < 3) cluster_arrive();
+    if (met < 4) cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
@@ -1301,8 +1332,9 @@ SplitPlan split_plan(const b200attn_prefill_args_t& a, int sm_count) {
 // long as some tiles, so the costs below, in 128-key steps of 1.6 us.  Queries of one block of rows over 4, 6 and 12 tiles, four items,
 // head_dim 64 12.2 -> 11.0, 15.4 -> 12.6, 17.4 -> 13.2 us; at head_dim 128 12 tiles 18.3 -> 16.7 (in eight parts), 16 tiles 15.6 -> 16.8, so
 // those keep their parts in the workspace.
-SplitPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const SplitPlan& other) {
-  SplitPlan sp{1, 0};
+struct ClusterPlan : SplitPlan { int cut_tiles; };     // (cut_tiles: see finish_item)
+ClusterPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const SplitPlan& other) {
+  ClusterPlan sp{{1, 0}, 0};
   if (a.layout == B200ATTN_RAGGED || a.batch <= 0 || a.max_q <= 0 || sm_count <= 0) return sp;
   const bool head_pair = (a.q_heads / a.kv_heads) % 2 == 0;
   const int item_rows = head_pair ? kBM : 2 * kBM;
@@ -1321,7 +1353,13 @@ SplitPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const Spl
     if (items > static_cast<long long>(held[i]) * sm_count / 148 || tiles < parts) break;
     const long long per = (tiles + parts - 1) / parts;
     const double cost = static_cast<double>(per) + cluster_cost[a.head_dim == 128][i];
-    if (cost < best) { best = cost; sp.parts = parts; sp.part_len = static_cast<int>(per * kBN); }
+    if (cost < best) {
+      best = cost;
+      sp.parts = parts;
+      sp.part_len = static_cast<int>(per * kBN);
+      // (beside one CTA alone, without a second launch, the parts at head_dim 128 cost a step less than the figures above)
+      sp.cut_tiles = static_cast<int>(std::min(tiles, static_cast<long long>(cost - (a.head_dim == 128 ? 1.0 : 0.0)) + 1));
+    }
   }
   return sp;
 }
@@ -1418,8 +1456,10 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
   p.kv_split_len = wsp.split.part_len;
   p.lse = nullptr;
   p.cluster_parts = 1;
-  if (const SplitPlan cp = cluster_plan(a, sm_count, wsp.split); cp.parts > 1) {
+  p.cut_tiles = 0;
+  if (const ClusterPlan cp = cluster_plan(a, sm_count, wsp.split); cp.parts > 1) {
     p.cluster_parts = cp.parts;
+    p.cut_tiles = cp.cut_tiles;
     p.kv_split = 1;
     p.kv_split_len = cp.part_len;
   }

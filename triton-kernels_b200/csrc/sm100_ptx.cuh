@@ -82,6 +82,8 @@ __device__ __forceinline__ void st_async_pair(uint32_t slot, uint32_t bar, uint3
 
 // Cluster-wide barrier in two halves; every thread of every CTA takes part.  (Only in grids launched with a cluster size.)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+// (where nothing was written that the others will read)
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
