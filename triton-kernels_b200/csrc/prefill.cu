@@ -773,7 +773,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     float out_ma = -INFINITY, out_mb = -INFINITY;   // ... and their references (kept for a merge)
     long long out_off = 0;   // element offset of row A's first output column
     long long out_stride = 0;   // elements between consecutive rows of the output
-    bool cut = true;         // (parts in clusters; a CTA that never saw its item sends its NaN)
+    bool seen = false, cut = true;      // (parts in clusters; a CTA that never saw its item sends NaN)
     constexpr bool k16 = !std::is_same<OutT, float>::value;
     auto quad_max = [](float v) {
       v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
@@ -1121,7 +1121,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->p_ready[s]));
       }
-      if constexpr (kParts) cut = w.cut;
+      if constexpr (kParts) { seen = true; cut = w.cut; }
       if (!ok) break;
       // ---------------- the item's epilogue ----------------
       const int len_q = w.len_q;
@@ -1158,7 +1158,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // their accumulator, row sums and references in fp32 into its tile buffers, register by register as the warp of the same
       // number there holds its own; one barrier of the cluster says that all tile buffers are done with, a second that the
       // parts have arrived.  (Every warp of the cluster meets at both; no wait before them is without a limit.)  A part that
-      // gave up sends NaN.
+      // gave up sends NaN, and fills the rows that are its own with it.
       const int rank = static_cast<int>(cluster_rank()), parts = p.cluster_parts;
       if (!cut) {
         __syncwarp();
@@ -1166,7 +1166,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (ok && rank == 0) ok = write_out(std::false_type{});
       } else {
         if (ok && out_acc) ok = warp_wait(smem_u32(&ctrl->o_done[s]), out_phase);
-        if (!ok) out_la = out_lb = __int_as_float(0x7fc00000);
+        if (!ok) {
+          out_la = out_lb = __int_as_float(0x7fc00000);
+          if (seen) {
+            const ItemWork& w = ctrl->sched_work[0];
+            out_rows = min(kBM, w.len_q - w.m0[s]);
+            out_stride = D;
+            out_off = (w.out_row0[s] + w.m0[s] + rowA) * D;
+          }
+        }
         tc_fence_after();
         __syncwarp();
         cluster_arrive();
