@@ -81,7 +81,6 @@ struct ItemWork {
   int m0[kSlots];      // first query row of each slot inside the sequence
   int nkv[kSlots];     // 128-key tiles each slot visits
   int nkv_max;
-  bool cut;            // (parts in clusters) the CTAs of the cluster share the item's keys; else the first of them does it alone
 };
 
 // shared-memory control block placed after the tiles
@@ -100,6 +99,7 @@ struct __align__(8) Control {
   ItemWork sched_work[2];   // decoded by the scheduler, read by every other warp
   uint32_t tmem_base;
   int abort_flag;
+  bool cut;                 // parts in clusters: see finish_item
 };
 
 template <int D>
@@ -180,7 +180,6 @@ template <bool kParts> __device__ __forceinline__ ItemWork locate_item(const Pre
   w.kv_head_coord = 0;
   w.b = 0;
   w.nkv_max = 0;
-  w.cut = false;
 #pragma unroll
   for (int s = 0; s < kSlots; ++s) {
     w.q_row0[s] = w.out_row0[s] = 0;
@@ -223,7 +222,9 @@ template <bool kParts> __device__ __forceinline__ ItemWork locate_item(const Pre
   return w;
 }
 
-template <bool kParts> __device__ __forceinline__ void finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
+// Whether the CTAs of a cluster share the item's keys; if not the first of them does it alone.  (false without parts in clusters)
+template <bool kParts> __device__ __forceinline__ bool finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
+  bool cut = false;
   if (p.layout == B200ATTN_RAGGED) {
     const int heads_per_item = p.head_pair ? 2 : 1;
     const int head_units = p.q_heads / heads_per_item;
@@ -264,10 +265,10 @@ template <bool kParts> __device__ __forceinline__ void finish_item(const Prefill
     if constexpr (kParts) {
       int tiles = (w.len_k + kBN - 1) / kBN;
       if (p.is_causal) tiles = min(tiles, (min(w.m0[kSlots - 1] + kBM, w.len_q) + kBN - 1) / kBN);
-      w.cut = tiles >= p.cut_tiles;
-      if (!w.cut && w.kv_tok0 > 0) w.len_k = 0;
+      cut = tiles >= p.cut_tiles;
+      if (!cut && w.kv_tok0 > 0) w.len_k = 0;
     }
-    if (kParts ? w.cut : p.kv_split_len > 0) {
+    if (kParts ? cut : p.kv_split_len > 0) {
       // this item sees the keys [kv_tok0, kv_tok0 + kv_split_len) of the sequence only
       int local = w.len_k - w.kv_tok0;
       local = local < 0 ? 0 : (local > p.kv_split_len ? p.kv_split_len : local);
@@ -286,6 +287,7 @@ template <bool kParts> __device__ __forceinline__ void finish_item(const Prefill
     w.nkv[s] = n;
     w.nkv_max = max(w.nkv_max, n);
   }
+  return cut;
 }
 
 // Parts in clusters: what a CTA sends of a strip of sixteen rows, a 16-byte piece per thread and register group: {references,
@@ -397,6 +399,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (!ok || *abort_flag) { ok = false; break; }
       }
       int item = -1;
+      bool cut = false;
       if (lane == 0) {
         item = k == 0 ? static_cast<int>(blockIdx.x) : static_cast<int>(gridDim.x) + atomicAdd(p.work_counter, 1);
         if (item >= p.total_items) item = -1;
@@ -409,15 +412,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           pg_k = first_pages(p.k_table, w);
           pg_v = first_pages(p.v_table, w);
         }
-        finish_item<kParts>(p, w, item, lane);
+        cut = finish_item<kParts>(p, w, item, lane);
       }
       if (lane == 0) {
         if (item >= 0) ctrl->sched_work[k & 1] = w;
+        if (kParts && item >= 0) ctrl->cut = cut;
         ctrl->sched_item[k & 1] = item;
         mbar_arrive(smem_u32(&ctrl->sched_full[k & 1]));
       }
       if (item < 0) break;
-      if (kParts && !w.cut) { meet_arrive(); met = 1; }
+      if (kParts && !cut) { meet_arrive(); met = 1; }
       const int* vtab = kPaged ? p.v_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
       const int* ktab = kPaged ? p.k_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
       auto read_page = [&](const int* tab, int first_box) -> int {
@@ -657,7 +661,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const int item = ctrl->sched_item[k & 1];
       if (item < 0) break;
       const ItemWork& wr = ctrl->sched_work[k & 1];
-      if (kParts && !wr.cut) { meet_arrive(); met = 1; }
+      if (kParts && !ctrl->cut) { meet_arrive(); met = 1; }
       const int nkv0 = wr.nkv[0], nkv1 = wr.nkv[1], nkv_max = wr.nkv_max, len_k = wr.len_k;
       const int qbuf0 = (2 * k) % kQBufs, qbuf1 = (2 * k + 1) % kQBufs;
       const uint64_t qd0 = q_desc_of(qbuf0), qd1 = q_desc_of(qbuf1);
@@ -936,7 +940,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (!ok || *abort_flag) { ok = false; break; }
       const int item = ctrl->sched_item[k & 1];
       if (item < 0) break;
-      if (kParts && !ctrl->sched_work[0].cut) { meet_arrive(); meet_again(); }
+      if (kParts && !ctrl->cut) { meet_arrive(); meet_again(); }
       // (the few fields needed are read from shared memory where they are used, not held across the tile loop)
       const ItemWork& w = ctrl->sched_work[k & 1];
       const int n = w.nkv[s];
@@ -1121,7 +1125,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->p_ready[s]));
       }
-      if constexpr (kParts) { seen = true; cut = w.cut; }
+      if constexpr (kParts) { seen = true; cut = ctrl->cut; }
       if (!ok) break;
       // ---------------- the item's epilogue ----------------
       const int len_q = w.len_q;
