@@ -1717,7 +1717,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         }
         const uint64_t vb = vdesc + static_cast<uint64_t>((stage * STAGE_BYTES + TILE_BYTES) >> 4);
         // A wait of a tile that ran out is noticed behind the MMAs, which then multiply whatever is there into this CTA's own
-        // tensor memory: votes between P and the next scores, and loops around waits that are nearly always over, are part of
+        // tensor memory (where the softmax warps take that for the unit's product, the teardown fills its rows with NaN): votes between P and the next scores, and loops around waits that are nearly always over, are part of
         // every tile's chain.  32 sequences of 1 to 33 thousand keys in pages, 40 rows per KV head, 310 -> 307 us, 32 x 8 192 keys
         // (dense) 206 -> 196, 8 of 1 to 4 thousand, 32/8 heads, 8 drafts, D 64 27.2 -> 25.9.
         bool good = mbar_wait_ready(smem_u32(&ctrl->p_ready), g & 1);
@@ -1739,7 +1739,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
       if (ok) unit_done(r);
     }
     if (!ok) {
-      if (lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; }
+      // (the softmax warps may have gone on since: no unit of the ring is known to be right)
+      if (lane == 0) { p.header[0] = DEV_ERR_WAIT_EXPIRED; *abort_flag = 1; ctrl->abort_round = 0; }
       // (what has been issued ends before tensor memory is given back)
       mma_commit_lead(smem_u32(&ctrl->drained), lead);
       warp_wait(smem_u32(&ctrl->drained), 0);
@@ -1784,7 +1785,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
     int owed_pair = -1, owed_round = 0;          // thread 0: pair whose ticket is still to be drawn, and its unit's round
     auto draw_owed_ticket = [&]() {
       if (tid != 0 || owed_pair < 0) return;
-      if (mbar_wait(smem_u32(&ctrl->rows_out), (merges - 1) & 1)) {
+      if (mbar_wait(smem_u32(&ctrl->rows_out), (merges - 1) & 1) && !*abort_flag) {
         __threadfence();                         // the rows the other softmax threads wrote before they arrived, too
         atomicAdd(p.counters + owed_pair, 1);
         atomicAdd(p.header + 3, 1);              // tickets drawn and not merged yet (a hint for the teardown)

@@ -338,6 +338,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         mbar_init(smem_u32(&ctrl->sched_empty[i]), kSoftmaxWarps + 1);
       }
       ctrl->abort_flag = 0;
+      ctrl->sched_item[0] = ctrl->sched_item[1] = -1;
       mbar_fence_init();
     }
     __syncwarp();
@@ -601,7 +602,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     bool pre_issued0 = false, pre_issued1 = false;   // first score tile of the coming item already issued
     // This warp's instructions between P and the commit of the next scores are part of every step's chain.  Inside the tile loop a
     // wait that ran out is noticed after the MMAs behind it have been issued (on whatever is there, into this CTA's own tensor
-    // memory), one vote for three waits: cycles per 128 x 128 tile and SM, 8 x 2 048 without a mask 1 840 -> 1 807, 2 x 2 048 causal
+    // memory; should that be read out for an item's product, the teardown takes it back), one vote for three waits: cycles per 128 x 128 tile and SM, 8 x 2 048 without a mask 1 840 -> 1 807, 2 x 2 048 causal
     // 2 144 -> 2 103 (all-zero inputs, so at full clock); at the power limit 74.7 -> 73.9 us.  Tried beside it: the code once per stage
     // of the ring, so that descriptors are constants in uniform registers (9 cycles, but 64 / 8 heads of 22 tokens took 2 % longer
     // with it), the commit of the P V behind that of the scores (nothing).
@@ -742,7 +743,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
       }
       if (nkv_max > 0) pair_base += nkv_max + 1;
-      if (lane == 0) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));
+      if (lane == 0 && ok) mbar_arrive(smem_u32(&ctrl->sched_empty[k & 1]));      // (else the teardown reads the slot)
       __syncwarp();
     }
     if (!ok) {
@@ -1169,7 +1170,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         cluster_wait();
         if (ok && rank == 0) ok = write_out(std::false_type{});
       } else {
-        if (ok && out_acc) ok = warp_wait(smem_u32(&ctrl->o_done[s]), out_phase);
+        if (ok && out_acc) ok = warp_wait(smem_u32(&ctrl->o_done[s]), out_phase) && !__any_sync(0xffffffffu, *abort_flag);
         if (!ok) {
           out_la = out_lb = __int_as_float(0x7fc00000);
           if (seen) {
@@ -1225,6 +1226,29 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
+  }
+  {
+    // A wait that ran out: the rows of the items in the scheduler's two slots, those that some warp has not done with among them, are
+    // unknown, and NaN says so.  (An item that its cluster shares is marked where its parts meet.  The thread and the control block
+    // are read anew: kept from above they cost every tile half a percent.)
+    unsigned t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    uintptr_t at = reinterpret_cast<uintptr_t>(smem_raw);
+    asm volatile("" : "+l"(at));
+    const Control* const c = reinterpret_cast<const Control*>(((at + 1023) & ~uintptr_t(1023)) + Plan::kCtrlOff);
+    if (c->abort_flag && !(kParts && (c->cut || c->sched_work[0].kv_tok0 > 0))) {
+      const OutT nan = ElemTraits<OutT>::from_float(__int_as_float(0x7fc00000));
+#pragma unroll 1
+      for (int k = 0; k < 2 * kSlots; ++k) {
+        if (c->sched_item[k & 1] < 0) continue;
+        const ItemWork& w = c->sched_work[k & 1];
+        const int s = k >> 1, rows = w.valid ? min(kBM, w.len_q - w.m0[s]) : 0;
+        const long long stride = p.layout == B200ATTN_RAGGED ? p.q_heads : 1;
+        OutT* const out = static_cast<OutT*>(p.out) + ((w.out_row0[s] + w.m0[s]) * stride + (stride > 1 ? w.q_head[s] : 0)) * D;
+#pragma unroll 1
+        for (int r = t / D; r < rows; r += kThreads / D) out[r * stride * D + t % D] = nan;
+      }
+    }
   }
 }
 
