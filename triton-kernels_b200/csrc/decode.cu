@@ -28,12 +28,12 @@
 //       CTAs of the warp-level or the fp32 kernel shares a (sequence, kv head) pair and merges through distributed shared
 //       memory; there, and only there, a CTA waits (with a limit) for the others of its cluster.
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 #include <type_traits>
 
 #include "cast.cuh"
 #include "common.cuh"
+#include "cluster_residency.h"
 #include "decode_launch.h"
 #include "launch.cuh"
 #include "sm100_ptx.cuh"
@@ -2512,39 +2512,6 @@ size_t simt_smem(int cluster, int rows, int D) {
 // fit three times up to ten rows, the fp32 kernel's up to seven).
 int ctas_per_sm(size_t smem) {
   return static_cast<int>(std::min<size_t>(3, 228 * 1024 / (smem + 1024 + 64)));
-}
-
-// Clusters of `c` CTAs, `per_sm` of them to an SM, that the GPU holds at once.  Those of four and eight leave SMs over in each of its
-// processing clusters: a call of 16 clusters of eight at one CTA per SM went in two waves and took 20.4 us instead of 15.4 planned
-// (two sequences of 4 096 keys, 32/8 heads, D 128).  The driver is asked once (`ask`; the answer depends on the device model
-// only); without a GPU the figures are those it gave for a B200.
-int clusters_held(int c, int per_sm, int sm_count, bool ask) {
-  if (c == 1) return per_sm * sm_count;
-  const int log_c = c == 2 ? 0 : c == 4 ? 1 : 2;
-  static std::atomic<int> known[3][3];
-  int n = ask ? known[log_c][per_sm - 1].load(std::memory_order_relaxed) : 0;
-  if (n > 0) return n;
-  static const int b200[3][3] = {{74, 148, 222}, {33, 71, 104}, {15, 33, 48}};
-  n = b200[log_c][per_sm - 1] * sm_count / 148;
-  if (!ask) return n;
-  auto kernel = decode_mma_kernel<__nv_bfloat16, 64, 2, 1, 160, 3, __nv_bfloat16, true>;
-  const size_t smem = (per_sm == 1 ? 120 : per_sm == 2 ? 80 : 60) * 1024;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(sm_count * 3 / c * c), 1, 1);
-  cfg.blockDim = dim3(32 * (kMmaSlices + 1), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = c;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int got = 0;
-  if (set_smem(kernel, smem) == 0 && cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) == cudaSuccess && got > 0) n = got;
-  else cudaGetLastError();                 // (no answer: the figures above stand)
-  known[log_c][per_sm - 1].store(n, std::memory_order_relaxed);
-  return n;
 }
 
 // What one CTA takes for a tile of 64 keys, alone on its SM, in ns.  (The fp32 kernel multiplies blocks of 1, 2 or 4 rows, each

@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "cast.cuh"
+#include "cluster_residency.h"
 #include "common.cuh"
 #include "launch.cuh"
 #include "prefill_launch.h"
@@ -1363,13 +1364,14 @@ SplitPlan split_plan(const b200attn_prefill_args_t& a, int sm_count) {
 }
 
 // The same with the parts of an item in a cluster, merged through distributed shared memory: for launches whose clusters are
-// all resident at once (one CTA to an SM: 74 of two, 33 of four, 15 of eight on a B200).  There is no second launch, and items
+// all resident at once (one CTA to an SM).  There is no second launch, and items
 // of four to seven tiles are worth cutting; but what a CTA sends, fp32 accumulators of 64 KB and more at head_dim 128, takes as
 // long as some tiles, so the costs below, in 128-key steps of 1.6 us.  Queries of one block of rows over 4, 6 and 12 tiles, four items,
 // head_dim 64 12.2 -> 11.0, 15.4 -> 12.6, 17.4 -> 13.2 us; at head_dim 128 12 tiles 18.3 -> 16.7 (in eight parts), 16 tiles 15.6 -> 16.8, so
 // those keep their parts in the workspace.
 struct ClusterPlan : SplitPlan { int cut_tiles; };     // (cut_tiles: see finish_item)
-ClusterPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const SplitPlan& other) {
+// `ask`: see clusters_held.
+ClusterPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const SplitPlan& other, bool ask) {
   ClusterPlan sp{{1, 0}, 0};
   if (a.layout == B200ATTN_RAGGED || a.batch <= 0 || a.max_q <= 0 || sm_count <= 0) return sp;
   const bool head_pair = (a.q_heads / a.kv_heads) % 2 == 0;
@@ -1383,10 +1385,9 @@ ClusterPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const S
   constexpr double kLaunchCost = 1.5, kGain = 0.4;
   const long long whole = (tiles + other.parts - 1) / other.parts;
   double best = static_cast<double>(whole) + (other.parts > 1 ? kLaunchCost : 0.0) - kGain;
-  static const int held[3] = {74, 33, 15};
   for (int i = 0; i < 3; ++i) {
     const int parts = 2 << i;
-    if (items > static_cast<long long>(held[i]) * sm_count / 148 || tiles < parts) break;
+    if (tiles < parts || items > clusters_held(parts, /*per_sm=*/1, sm_count, ask)) break;
     const long long per = (tiles + parts - 1) / parts;
     const double cost = static_cast<double>(per) + cluster_cost[a.head_dim == 128][i];
     if (cost < best) {
@@ -1493,7 +1494,7 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
   p.lse = nullptr;
   p.cluster_parts = 1;
   p.cut_tiles = 0;
-  if (const ClusterPlan cp = cluster_plan(a, sm_count, wsp.split); cp.parts > 1) {
+  if (const ClusterPlan cp = cluster_plan(a, sm_count, wsp.split, /*ask=*/true); cp.parts > 1) {
     p.cluster_parts = cp.parts;
     p.cut_tiles = cp.cut_tiles;
     p.kv_split = 1;
