@@ -43,6 +43,9 @@ enum { B200ATTN_DENSE = 0, B200ATTN_RAGGED = 1, B200ATTN_PAGED = 2 };
 
 /* b200attn_decode_route: 1 .. 8 are CTAs per (sequence, KV head) pair of a call in clusters */
 enum { B200ATTN_ROUTE_PLANNER = 0, B200ATTN_ROUTE_INLINE = 16 };
+/* b200attn_prefill_route: 1, or in how many parts (2, 4, 8) the CTAs of a cluster share an item; with this added, in how many (2 .. 8)
+   parts of the workspace every sequence's keys are cut */
+enum { B200ATTN_ROUTE_WORKSPACE = 32 };
 
 /* status codes */
 enum {
@@ -173,6 +176,13 @@ size_t b200attn_decode_workspace_bytes(const b200attn_decode_args_t* args);
  * the reference.
  */
 int b200attn_decode_route(const b200attn_decode_args_t* args, int sm_count, int is_static);
+
+/*
+ * Which way b200attn_prefill takes a call on a GPU of `sm_count` SMs: every item whole (1), the longest items shared by the CTAs of a
+ * cluster (2, 4 or 8; shorter ones stay whole), or in parts that a second launch merges (B200ATTN_ROUTE_WORKSPACE + their number).
+ * Host arithmetic on the sizes; needs no GPU, reads no pointer.  No counterpart in the reference.
+ */
+int b200attn_prefill_route(const b200attn_prefill_args_t* args, int sm_count);
 
 int b200attn_prefill(const b200attn_prefill_args_t* args, void* cuda_stream);
 int b200attn_decode(const b200attn_decode_args_t* args, void* cuda_stream);

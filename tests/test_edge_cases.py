@@ -213,7 +213,7 @@ def test_prefill_outlier_keys_move_the_exponent_reference(dtype, causal):
 @pytest.mark.gpu
 @pytest.mark.parametrize("layout", ["dense", "paged"])
 @pytest.mark.parametrize("shape", [(1, 8, 2, 128, 2048, False, 128), (1, 8, 8, 128, 4096, False, 64), (2, 4, 1, 200, 1000, False, 128),
-                                   (1, 2, 1, 2048, 2048, True, 128), (1, 4, 2, 1100, 1100, True, 64), (3, 2, 2, 128, 1280, False, 128)],
+                                   (1, 2, 1, 2048, 2048, True, 128), (1, 8, 2, 1100, 1100, True, 64), (3, 2, 2, 128, 1280, False, 128)],
                          ids=["b1-q128-kv2048", "b1-mha-kv4096-d64", "b2-q200-kv1000", "b1-causal-2048", "b1-causal-1100-d64", "b3-kv1280"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
 def test_prefill_few_work_items_split_kv(layout, shape, dtype):
@@ -225,8 +225,12 @@ def test_prefill_few_work_items_split_kv(layout, shape, dtype):
 
     from kernels import _native
     from test_attention import run_prefill
+    from test_prefill_routes import WORKSPACE, route
 
     b, qh, kvh, lq, lkv, causal, d = shape
+    # (in parts of the workspace, not shared by the CTAs of a cluster)
+    assert route(layout, {torch.bfloat16: "bf16", torch.float32: "fp32"}[dtype], *shape,
+                 sms=torch.cuda.get_device_properties(0).multi_processor_count) >= WORKSPACE + 2
     gen = torch.Generator().manual_seed(lq * 7 + lkv + qh)
     qs = [torch.randn((lq, qh, d), generator=gen).to(dtype).to(DEV) for _ in range(b)]
     if layout == "paged" and not causal:
@@ -239,7 +243,7 @@ def test_prefill_few_work_items_split_kv(layout, shape, dtype):
     outs = run_prefill(layout, qs, ks, vs, causal, permute=11, pad=-1, poison=float("nan"))
     for i in range(b):
         assert_close_both(outs[i], refs[i], dtype, kv_lens[i], f"seq {i}", strict=4e-3 if dtype == torch.float32 else None)
-    # the split really is in play for these shapes: the library asks for room for the parts
+    # the library asks for room for the parts
     a = _native.PrefillArgs()
     a.dtype, a.layout = _native.DTYPE_CODE[dtype], _native.DENSE
     a.batch, a.q_heads, a.kv_heads, a.max_q, a.max_kv, a.head_dim = b, qh, kvh, lq, lkv, d

@@ -6,6 +6,7 @@ import sys
 import pytest
 
 from test_decode_routes import route
+from test_prefill_routes import route as prefill_route
 
 CODE = """
 import sys
@@ -36,6 +37,7 @@ def test_first_call_is_recorded(shapes, mode):
     from kernels import _native
 
     assert route("dense", "bf16", 4, 32, 8, 128, 300) == 8
+    assert prefill_route("dense", "bf16", 1, 8, 2, 100, 600, False, 64) == 4
     done = subprocess.run([sys.executable, "-c", CODE.format(pkg=_native._PKG_ROOT, mode=mode, shapes=shapes)], capture_output=True,
                           text=True, timeout=300)
     assert done.returncode == 0 and "ok" in done.stdout, done.stderr[-2000:]

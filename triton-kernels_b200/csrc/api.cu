@@ -164,6 +164,11 @@ int b200attn_decode_route(const b200attn_decode_args_t* a, int sm_count, int is_
   return decode_route(*a, sm_count, is_static != 0);
 }
 
+int b200attn_prefill_route(const b200attn_prefill_args_t* a, int sm_count) {
+  if (!a || a->batch < 0 || a->q_heads <= 0 || a->kv_heads <= 0 || a->q_heads % a->kv_heads != 0 || sm_count <= 0) { set_error("prefill_route: bad arguments"); return B200ATTN_E_INVALID; }
+  return prefill_route(*a, sm_count);
+}
+
 int b200attn_prefill(const b200attn_prefill_args_t* a, void* cuda_stream) {
   if (!a) { set_error("args is null"); return B200ATTN_E_INVALID; }
   int rc = check_common(a->dtype, a->layout, a->batch, a->q_heads, a->kv_heads, a->head_dim);

@@ -1448,6 +1448,12 @@ WsPlan ws_plan(const b200attn_prefill_args_t& a, int sm_count) {
 
 size_t prefill_workspace_bytes(const b200attn_prefill_args_t& a, int sm_count) { return ws_plan(a, sm_count).total; }
 
+int prefill_route(const b200attn_prefill_args_t& a, int sm_count) {
+  const SplitPlan split = ws_plan(a, sm_count).split;
+  if (const int parts = cluster_plan(a, sm_count, split, /*ask=*/false).parts; parts > 1) return parts;
+  return split.parts > 1 ? B200ATTN_ROUTE_WORKSPACE + split.parts : 1;
+}
+
 int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream_t stream) {
   const WsPlan wsp = ws_plan(a_in, sm_count);
   const size_t need = wsp.total;

@@ -41,6 +41,8 @@ struct PrefillParams {
 };
 
 size_t prefill_workspace_bytes(const b200attn_prefill_args_t& a, int sm_count);
+// which way a call goes: see b200attn_prefill_route
+int prefill_route(const b200attn_prefill_args_t& a, int sm_count);
 int launch_prefill(const b200attn_prefill_args_t& a, int sm_count, cudaStream_t stream);
 
 }  // namespace b200attn
