@@ -1,9 +1,10 @@
 """fp32 decode calls of 97 to 192 (sequence, KV head) pairs plan inside the kernel too, with merge tickets of eight bits: either side of
-the line, pairs at every place of a header word, the most items that a pair can have, calls with tickets of either width in turn."""
+the line, pairs at every place of a header word, pairs of more than 128 items, calls with tickets of either width in turn."""
 import pytest
 import torch
 
 from helpers import assert_close_both
+from test_decode_planned import _route
 from test_decode_routes import INLINE, PLANNER, route
 from test_decode_without_planner import DEV, _call, _problem, _reference
 
@@ -28,11 +29,10 @@ def test_tickets_of_eight_bits(batch, qh, kvh, d, layout):
     gen = torch.Generator().manual_seed(batch * 7 + d)
     base = [1, 63, 64, 65, 129, 2500, 640, 1500]
     lens = [base[i % len(base)] for i in range(batch)]
-    lens[-1] = 9000                              # a pair of many items
+    lens[-1] = 9000 if layout == "ragged" else 2900          # a pair of many items (a table of 9 000 keys would be beyond 300 MiB)
     page = 16
     keys = -(-max(lens) // page) * page
-    if layout == "ragged":
-        assert route(layout, "fp32", batch, qh, kvh, d, 0, total=sum(lens)) in (INLINE, PLANNER)
+    assert _route(lens, layout, torch.float32, qh, kvh, d, page=page) == INLINE
     qs, ks, vs = _problem(gen, lens, qh, kvh, d, torch.float32)
     small = _problem(gen, [700, 90, 3000], 8, 2, d, torch.float32)     # sixteen bits
     ref, small_ref = _reference(qs, ks, vs, qh, kvh, 0), _reference(*small, 8, 2, 0)
@@ -41,3 +41,23 @@ def test_tickets_of_eight_bits(batch, qh, kvh, d, layout):
         other = _call(*small, layout, 0, page)
         assert_close_both(out, ref, torch.float32, keys, f"{layout} {batch}x{kvh}")
         assert_close_both(other, small_ref, torch.float32, 3000, layout)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("place", [0, 13, 27])
+def test_tickets_beyond_half_of_eight_bits(place):
+    """Pairs of more than 128 items, so that the highest bit of their tickets is drawn: the KV heads of one sequence, whose tickets are
+    neighbours in the header."""
+    from utils.launch_config import decode_items, decode_plan
+
+    gen = torch.Generator().manual_seed(place)
+    lens = [20] * 28
+    lens[place] = 67000
+    assert _route(lens, "ragged", torch.float32, 5, 5, 64) == INLINE
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    items = decode_items(decode_plan(sms, len(lens), 5, 5, 1, fp32=True), lens)
+    assert 128 < items[place] <= 255
+    qs, ks, vs = _problem(gen, lens, 5, 5, 64, torch.float32)
+    ref = _reference(qs, ks, vs, 5, 5, 0)
+    for _ in range(2):
+        assert_close_both(_call(qs, ks, vs, "ragged", 0), ref, torch.float32, max(lens))
