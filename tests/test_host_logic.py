@@ -183,18 +183,23 @@ def test_planning_mirror_agrees_with_the_library(qh, kvh, m, batch, d, fp32):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("qh,kvh,m,lens", [
-    (32, 8, 1, [8192]),                                   # one sequence: a single wave of short items
-    (32, 8, 1, [8192] * 16),                              # uniform batch that fits one wave of three-resident CTAs
-    (32, 8, 1, [4096] * 32),                              # ... and one that stays with two waves
-    (64, 8, 5, [8192] * 32),                              # speculative decode, uniform: one item per sequence
-    (64, 8, 5, [8192] * 4),
-    (8, 1, 5, [1500, 9000, 31000, 700, 16000, 12000]),    # one KV head (the eight-GPU shard)
-    (32, 8, 1, [600, 8000, 512, 4100, 7777, 2300, 900, 5000] * 8),   # uneven lengths, more sequences than one wave holds
+@pytest.mark.parametrize("qh,kvh,m,lens,planner", [
+    (32, 8, 1, [8192], False),                            # one sequence: a single wave of short items
+    (32, 8, 1, [8192] * 16, True),                        # uniform batch that fits one wave of three-resident CTAs
+    (32, 8, 1, [4096] * 32, True),                        # ... and one that stays with two waves
+    (64, 8, 5, [8192] * 32, True),                        # speculative decode, uniform: one item per sequence
+    (64, 8, 5, [8192] * 4, False),
+    (64, 8, 5, [9000], False),                            # few sequences: items for one CTA an SM
+    (64, 8, 5, [4000, 100, 3000], False),
+    (64, 8, 5, [35000], False),                           # ... of up to six of the shortest
+    (64, 8, 5, [36500], False),                           # ... and for two
+    (8, 1, 5, [1500, 9000, 31000, 700, 16000, 12000], False),        # one KV head (the eight-GPU shard)
+    (8, 1, 5, [1500, 9000, 131000, 700, 116000, 112000], True),
+    (32, 8, 1, [600, 8000, 512, 4100, 7777, 2300, 900, 5000] * 8, True),   # uneven lengths, more sequences than one wave holds
 ])
-def test_planner_chunk_matches_the_mirror(qh, kvh, m, lens):
-    """The chunk size and item count the device planner wrote into the workspace header are the ones
-    utils/launch_config.py derives from the same lengths (several waves or a single one)."""
+def test_plan_matches_the_mirror(qh, kvh, m, lens, planner):
+    """The chunk size and item count that the planner, or the first CTA of a call that plans for itself, wrote into the workspace
+    header are the ones utils/launch_config.py derives from the same lengths (several waves or a single one)."""
     from kernels import _native
     from kernels.decode import decode_attention
     from kernels.speculative_decode import speculative_decode_attention
@@ -216,7 +221,10 @@ def test_planner_chunk_matches_the_mirror(qh, kvh, m, lens):
     torch.cuda.synchronize()
     ws = _native._workspaces[(torch.cuda.current_device(), int(torch.cuda.current_stream().cuda_stream))]
     header = ws[:16].view(torch.int32).tolist()
-    plan = decode_plan(info.sm_count, len(lens), qh, kvh, m)
+    from test_decode_routes import INLINE, PLANNER, route
+
+    assert route("ragged", "bf16", len(lens), qh, kvh, 64, 0, m=m, total=total, sms=info.sm_count) == (PLANNER if planner else INLINE)
+    plan = decode_plan(info.sm_count, len(lens), qh, kvh, m, keys=total)
     assert header[0] == 0
     assert header[1] == decode_chunk_tokens(plan, lens)
     assert header[2] == sum(decode_items(plan, lens))

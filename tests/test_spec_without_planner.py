@@ -27,6 +27,9 @@ def test_route_on_either_side_of_the_lines(layout, dtype, sms):
         line = _line(batch, kvh, sms)
         assert way(batch, kvh, line) == INLINE
         assert way(batch, kvh, line + 1) == PLANNER
+        from utils.launch_config import tcgen05_plans_itself
+
+        assert tcgen05_plans_itself(sms, batch, kvh, batch * line) and not tcgen05_plans_itself(sms, batch, kvh, batch * (line + 1))
     # sixteen rows are another kernel's, without a line of keys
     assert way(1, 8, 100000, m=2) == INLINE
 

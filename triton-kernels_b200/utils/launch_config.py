@@ -61,7 +61,16 @@ def decode_workspace_bytes(plan: "DecodePlan", batch: int, kv_heads: int, head_d
     return off
 
 
-def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: int, fp32: bool = False) -> DecodePlan:
+def tcgen05_plans_itself(sm_count: int, batch: int, kv_heads: int, keys: int) -> bool:
+    """Whether a call of more than sixteen q rows per KV head in 16 bits goes without the planner's launch (csrc/decode.cu
+    inline_plan_bits); ``keys``: of all sequences, as many as there can be (a packed tensor's rows, a table's width for each)."""
+    return batch * kv_heads <= 96 and keys * kv_heads <= (1024 - 8 * batch) * 2 * sm_count
+
+
+def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: int, fp32: bool = False,
+                keys: Optional[int] = None) -> DecodePlan:
+    """``keys`` (see ``tcgen05_plans_itself``): with it, calls of the tcgen05 kernel that plan for themselves are planned as they do,
+    without dealing the batch out, and up to three short sequences in items for one CTA an SM; without it all are the planner's."""
     group = decode_pass_group(q_heads // kv_heads, q_len)
     rows = group * q_len
     # fp32 inputs of a speculative-decode call (several q rows per head) run the tensor-core kernels on fp16 copies
@@ -76,8 +85,12 @@ def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: i
     wide = rows > 16 and not fp32   # more than one 16-row tile: the tcgen05 kernel, two resident CTAs per SM (else three)
     wave = max(1, (sm_count * (2 if wide else 3)) // max(1, kv_heads))
     overhead = 448 if wide else 128
-    return DecodePlan(target, min_chunk, target + batch, tiles, slices, 32 * (tiles * slices + 1), wave, overhead,
-                      2 * sm_count // max(1, kv_heads) if wide else 0)
+    slots, max_items = 2 * sm_count // max(1, kv_heads) if wide else 0, target + batch
+    if wide and keys is not None and tcgen05_plans_itself(sm_count, batch, kv_heads, keys):
+        slots = 0
+        if batch <= 3 and keys * kv_heads <= 6 * min_chunk * sm_count:
+            target, wave = max(1, sm_count // kv_heads), 0
+    return DecodePlan(target, min_chunk, max_items, tiles, slices, 32 * (tiles * slices + 1), wave, overhead, slots)
 
 
 def _round_up(x: int, m: int) -> int:
