@@ -148,3 +148,27 @@ def test_calls_in_a_row_see_each_other(kvh, want):
 
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,qh,kvh,m,batch,width", [("fp32", 8, 8, 1, 24, 3200), ("fp32", 4, 4, 1, 26, 5888), ("bf16", 64, 8, 5, 12, 2848),
+                                                        ("fp16", 8, 1, 5, 90, 992), ("bf16", 8, 8, 1, 12, 8000)])
+def test_tables_wider_than_the_sequences(dtype, qh, kvh, m, batch, width):
+    """Grids are as large as the table's width asks for, and most CTAs of a call that plans for itself find that these lengths leave
+    nothing for them: no sequence at all, one key, items that end on and around the shortest (128 to 320 keys), one long sequence."""
+    kind = {v: k for k, v in NAMES.items()}[dtype]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert route("paged", dtype, batch, qh, kvh, 64, width, m=m, sms=sms) == INLINE
+    gen = torch.Generator().manual_seed(width)
+    for base in ([m], [128], [129, 127], [320, 321, 640, 639], [m + 1] * (batch - 1) + [width]):
+        lens = [base[i % len(base)] for i in range(batch)]
+        qs, ks, vs = _problem(gen, lens, qh, kvh, 64, kind, m if m > 1 else 0)
+        k, kt, n = sdpa_ref.pack_paged(ks, 16, permute_seed=1, extra_pages=2, pad_value=-1, poison=float("nan"))
+        v, vt, _ = sdpa_ref.pack_paged(vs, 16, permute_seed=2, extra_pages=2, pad_value=-1, poison=float("nan"))
+        kt, vt = (torch.nn.functional.pad(t, (0, width // 16 - t.shape[1]), value=-1).contiguous() for t in (kt, vt))
+        kw = dict(kv_indptr=n, k_block_table=kt, v_block_table=vt, kv_page_size=16)
+        from kernels import decode_attention, speculative_decode_attention
+
+        q = torch.stack(qs)
+        out = decode_attention(q, k, v, **kw) if m == 1 else speculative_decode_attention(q, k, v, causal=True, **kw)
+        ref = _reference(qs, ks, vs, qh, kvh, m if m > 1 else 0)
+        assert_close_both(out, ref, kind, max(lens), f"{base[:4]}")

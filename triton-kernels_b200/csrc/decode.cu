@@ -724,6 +724,10 @@ __device__ __forceinline__ bool plan_inline(const DecodeParams& p, int item, Inl
   long long t = 0;
 #pragma unroll
   for (int w = 0; w < kInlineBatch / 32; ++w) t += s.tot[w];
+  // The grid is as large as the longest sequences that there can be ask for, in pages by the table's width.  There are at most
+  // t / min_chunk + batch items: a CTA that these lengths leave nothing for goes without the plan.  (12 sequences of 142 keys in tables of
+  // 2 848, 64/8 heads, D 128, 5 drafts, 944 CTAs: 17.3 -> 12.1 us, behind the planner 15.0.)
+  if (static_cast<long long>(item - p.batch + 1) * p.min_chunk > t) return false;
   // candidate `lane` of either target; the warps share the sequences
   auto candidate = [&](int target) -> int {
     long long base = t <= 0x7fffffff ? (static_cast<unsigned>(t) + target - 1) / static_cast<unsigned>(target) : (t + target - 1) / target;
