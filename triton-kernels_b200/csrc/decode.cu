@@ -1721,9 +1721,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         }
         const uint64_t vb = vdesc + static_cast<uint64_t>((stage * STAGE_BYTES + TILE_BYTES) >> 4);
         // A wait of a tile that ran out is noticed behind the MMAs, which then multiply whatever is there into this CTA's own
-        // tensor memory (where the softmax warps take that for the unit's product, the teardown fills its rows with NaN): votes between P and the next scores, and loops around waits that are nearly always over, are part of
-        // every tile's chain.  32 sequences of 1 to 33 thousand keys in pages, 40 rows per KV head, 310 -> 307 us, 32 x 8 192 keys
-        // (dense) 206 -> 196, 8 of 1 to 4 thousand, 32/8 heads, 8 drafts, D 64 27.2 -> 25.9.
+        // tensor memory (where the softmax warps take that for the unit's product, the teardown fills its rows with NaN): votes between
+        // P and the next scores, and loops around waits that are nearly always over, are part of every tile's chain.  32 sequences of
+        // 1 to 33 thousand keys in pages, 40 rows per KV head, 335 -> 327 us, 32 x 8 192 keys (dense) 206 -> 196, 8 of 1 to 4 thousand,
+        // 32/8 heads, 8 drafts, D 64 27.2 -> 25.9.
         bool good = mbar_wait_ready(smem_u32(&ctrl->p_ready), g & 1);
         // (a PV that starts a new accumulator: the previous unit's O must have left tensor memory)
         if (tile == 0 && r > 0) good = mbar_wait(smem_u32(&ctrl->o_free), (r - 1) & 1) && good;
@@ -2527,7 +2528,7 @@ int tile_ns(const b200attn_decode_args_t& a, int rows) {
 
 // CTAs per (sequence, KV head) pair when the call runs without a plan, 0 when it is planned.  Up to eight CTAs share a pair,
 // as long as all of them are resident at once.  A planned call takes 9 to 12 us before its items' length counts, some 5 more when
-// the planner has a launch of its own (more pairs than kInlinePairs), and cuts the keys evenly over the GPU whatever the lengths are;
+// the planner has a launch of its own (`planner`: more than 96 pairs), and cuts the keys evenly over the GPU whatever the lengths are;
 // a call in clusters takes 3 us and its longest part.  So the line is drawn by the time of a part (tile_ns), of one as long as the
 // host can tell: dense, the length of all; paged, the table's width; ragged, the average, and the longest that there can be,
 // a sequence that holds all keys, has a line of its own.  The lines are where the sweep below found the last call that was not faster
@@ -2551,6 +2552,9 @@ int cluster_size(const b200attn_decode_args_t& a, int sm_count, int rows, bool a
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
   if (pairs <= 0) return 0;
   const bool ragged = a.layout == B200ATTN_RAGGED, dense = a.layout == B200ATTN_DENSE, fp32 = a.dtype == B200ATTN_F32;
+  // (fp32 calls of up to 192 pairs may have none either, but the lines are right for them as they are: with those for up to 96 pairs,
+  // 240 packed calls of 97 to 192 of 40 to 600 keys took 1.02 of their time, 13 x 200 of 8/8 heads, D 128, equal 9.9 -> 14.8 us, with one
+  // sequence of nearly all keys 24.4 -> 17.1)
   const bool planner = pairs > kInlinePairs;
   auto tiles_of = [](long long keys) { return (keys + kTileN - 1) / kTileN; };
   const long long tiles = tiles_of(ragged ? (a.total_kv + a.batch - 1) / a.batch
@@ -2603,8 +2607,10 @@ long long most_keys(const b200attn_decode_args_t& a) {
 // bandwidth.  fp32, which reads twice the bytes: twice as many pairs, with tickets of eight bits
 // where no pair can be cut into more items than those count, up to 300 MiB of keys and values (the most that there can be).  16
 // packed sequences of 100 to 4 096 keys, 8/8 heads, D 64 36.3 -> 32.4 us, 13 x 1 500 18.9 -> 15.5, 24 x 1 500 at D 128 in pages 43.8 ->
-// 38.7; 20 x 3 000 119 -> 113, but 20 x 10 000 281 -> 290 (64/8 heads, dense): the planner puts the last, shorter item of each
-// sequence behind all others, which is worth more than its launch there.
+// 38.7; 20 x 3 000 119 -> 113, but 20 x 10 000 (819 MB, 64/8 heads, dense) 281 -> 290: the planner puts the last, shorter item of each
+// sequence behind all others, which is worth more than its launch there.  (Between the two packed lengths from nothing to twice the
+// average still gained without it: 340 MB 0.93 to 1.01 of the time over twelve calls, 650 MB 0.95 to 1.00.  And in pages it is the
+// width of the table that counts: a server whose tables are as wide as its context limit keeps the planner.)
 //
 // More than sixteen rows (the tcgen05 kernel; two CTAs to an SM): the planner deals a batch out to the CTAs by keys, which no CTA can
 // see by itself (a batch cut into equal items leaves some CTAs without one), and a CTA's own plan takes longer the more sequences there

@@ -31,7 +31,7 @@
 // 1 077 -> 1 001; 8 x 2 048 without a mask 586 -> 546.
 //
 // Every mbarrier wait is bounded; on expiry the role records DEV_ERR_WAIT_EXPIRED
-// in the workspace header and falls through to the common teardown (TMEM is freed).
+// in the workspace header and falls through to the common teardown (TMEM is freed, rows that are not known become NaN).
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -308,7 +308,7 @@ __device__ __forceinline__ float part_weight(float m, float largest) { return m 
 // kPaged: the instantiation launched for paged K/V; only it carries the block-table read-ahead of the producer (in
 // the dense / ragged kernel that code, though never run, cost 1 % on the dense benchmark configuration).  The other
 // layout checks stay run-time checks.  kParts: the one launched in clusters that share an item (its epilogue costs the others
-// registers).
+// registers; of these only the form for pages at head_dim 128 spills, 16 bytes).
 template <typename T, int D, typename OutT, bool kPaged, bool kParts>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -1368,7 +1368,9 @@ SplitPlan split_plan(const b200attn_prefill_args_t& a, int sm_count) {
 // of four to seven tiles are worth cutting; but what a CTA sends, fp32 accumulators of 64 KB and more at head_dim 128, takes as
 // long as some tiles, so the costs below, in 128-key steps of 1.6 us.  Queries of one block of rows over 4, 6 and 12 tiles, four items,
 // head_dim 64 12.2 -> 11.0, 15.4 -> 12.6, 17.4 -> 13.2 us; at head_dim 128 12 tiles 18.3 -> 16.7 (in eight parts), 16 tiles 15.6 -> 16.8, so
-// those keep their parts in the workspace.
+// those keep their parts in the workspace.  (Two parts at head_dim 128 are never the cheapest: below eight tiles they do not pay, from
+// there on the workspace has them.  What a launch costs, and how short a part may be, is counted otherwise in split_plan: twelve tiles
+// could go in four workspace parts of three.)
 struct ClusterPlan : SplitPlan { int cut_tiles; };     // (cut_tiles: see finish_item)
 // `ask`: see clusters_held.
 ClusterPlan cluster_plan(const b200attn_prefill_args_t& a, int sm_count, const SplitPlan& other, bool ask) {
