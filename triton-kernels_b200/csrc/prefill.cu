@@ -223,9 +223,9 @@ template <bool kParts> __device__ __forceinline__ ItemWork locate_item(const Pre
   return w;
 }
 
-// Whether the CTAs of a cluster share the item's keys; if not the first of them does it alone.  (false without parts in clusters)
-template <bool kParts> __device__ __forceinline__ bool finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
-  bool cut = false;
+// Whether the CTAs of a cluster share the sequence's keys; if not the first of them does the item alone.
+template <bool kPaged, bool kParts> __device__ __forceinline__ bool finish_item(const PrefillParams& p, ItemWork& w, int item, int lane) {
+  bool cut = kParts;
   if (p.layout == B200ATTN_RAGGED) {
     const int heads_per_item = p.head_pair ? 2 : 1;
     const int head_units = p.q_heads / heads_per_item;
@@ -259,13 +259,14 @@ template <bool kParts> __device__ __forceinline__ bool finish_item(const Prefill
       n = n < 0 ? 0 : (n > cap ? cap : n);
       w.len_k = static_cast<int>(n);
     }
-    // Parts in clusters: what the host cut is the longest that an item can be.  This one may be shorter, by its sequence's length or by
-    // its place under the diagonal, and not worth what the parts cost: every CTA of the cluster decides that by the same numbers,
-    // and the first takes the whole.  (64 queries over 100 keys in a table of 768, 8/2 heads, D 64: cut 11.1 us, not cut 7.4, a
-    // launch without clusters 7.3; over 700 in one of 1 536 13.0, 15.2 and, cut into parts in the workspace, 16.8.)
-    if constexpr (kParts) {
+    // Parts in clusters: what the host cut is the longest that a sequence can be.  This one may be shorter, and its items not worth
+    // what the parts cost: every CTA of the cluster sees that by the same numbers, and the first takes the whole.  (64 queries over 100
+    // keys in a table of 768, 8/2 heads, D 64: cut 11.1 us, not cut 7.4, a launch without clusters 7.3; over 700 in one of 1 536 13.0, 15.2
+    // and, cut into parts in the workspace, 16.8.  Short items of a long sequence, under the diagonal, are cut with the others: their
+    // parts are through before those are.)
+    if constexpr (kParts && kPaged) {
       int tiles = (w.len_k + kBN - 1) / kBN;
-      if (p.is_causal) tiles = min(tiles, (min(w.m0[kSlots - 1] + kBM, w.len_q) + kBN - 1) / kBN);
+      if (p.is_causal) tiles = min(tiles, (w.len_q + kBN - 1) / kBN);
       cut = tiles >= p.cut_tiles;
       if (!cut && w.kv_tok0 > 0) w.len_k = 0;
     }
@@ -308,7 +309,8 @@ __device__ __forceinline__ float part_weight(float m, float largest) { return m 
 // kPaged: the instantiation launched for paged K/V; only it carries the block-table read-ahead of the producer (in
 // the dense / ragged kernel that code, though never run, cost 1 % on the dense benchmark configuration).  The other
 // layout checks stay run-time checks.  kParts: the one launched in clusters that share an item (its epilogue costs the others
-// registers; of these only the form for pages at head_dim 128 spills, 16 bytes).
+// registers; at the cap of 96 the forms for head_dim 128 spill, 52 bytes dense and 16 over pages.  That is not what they wait for: a
+// build whose form for 64 spilled 72 took 10.48 us for 512 causal tokens, the present one, which spills none, 10.46).
 template <typename T, int D, typename OutT, bool kPaged, bool kParts>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -359,6 +361,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   }
   const uint32_t tmem = warp == kProducerWarp ? 0u : ctrl->tmem_base;   // (the producer never uses it)
   volatile int* abort_flag = &ctrl->abort_flag;
+  // (the host knows the lengths of dense tensors: what it has cut is cut)
+  constexpr bool kMayBeWhole = kParts && kPaged;
   // Parts in clusters: every warp of the cluster takes part in two barriers (at the end of this kernel) whatever happens, so that none
   // can wait for one that is not coming.  Where the item is not cut there is nothing to meet for: the warps arrive early and
   // find the barriers completed later (both at the end cost that item 1.0 us, both at its start 1.3, as placed 0.1).
@@ -401,7 +405,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (!ok || *abort_flag) { ok = false; break; }
       }
       int item = -1;
-      bool cut = false;
+      bool cut = kParts;
       if (lane == 0) {
         item = k == 0 ? static_cast<int>(blockIdx.x) : static_cast<int>(gridDim.x) + atomicAdd(p.work_counter, 1);
         if (item >= p.total_items) item = -1;
@@ -414,16 +418,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           pg_k = first_pages(p.k_table, w);
           pg_v = first_pages(p.v_table, w);
         }
-        cut = finish_item<kParts>(p, w, item, lane);
+        cut = finish_item<kPaged, kParts>(p, w, item, lane);
       }
       if (lane == 0) {
         if (item >= 0) ctrl->sched_work[k & 1] = w;
-        if (kParts && item >= 0) ctrl->cut = cut;
+        if (kMayBeWhole && item >= 0) ctrl->cut = cut;
         ctrl->sched_item[k & 1] = item;
         mbar_arrive(smem_u32(&ctrl->sched_full[k & 1]));
       }
       if (item < 0) break;
-      if (kParts && !cut) { meet_arrive(); met = 1; }
+      if (kMayBeWhole && !cut) { meet_arrive(); met = 1; }
       const int* vtab = kPaged ? p.v_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
       const int* ktab = kPaged ? p.k_table + static_cast<long long>(w.b) * p.table_stride : nullptr;
       auto read_page = [&](const int* tab, int first_box) -> int {
@@ -567,7 +571,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
         }
         if (pi == 0) ok = load_q(1);
-        if (kParts && pi == 1 && met == 1) { meet_again(); met = 3; }
+        if (kMayBeWhole && pi == 1 && met == 1) { meet_again(); met = 3; }
       }
     }
     if (!ok) {
@@ -663,7 +667,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const int item = ctrl->sched_item[k & 1];
       if (item < 0) break;
       const ItemWork& wr = ctrl->sched_work[k & 1];
-      if (kParts && !ctrl->cut) { meet_arrive(); met = 1; }
+      if (kMayBeWhole && !ctrl->cut) { meet_arrive(); met = 1; }
       const int nkv0 = wr.nkv[0], nkv1 = wr.nkv[1], nkv_max = wr.nkv_max, len_k = wr.len_k;
       const int qbuf0 = (2 * k) % kQBufs, qbuf1 = (2 * k + 1) % kQBufs;
       const uint64_t qd0 = q_desc_of(qbuf0), qd1 = q_desc_of(qbuf1);
@@ -672,7 +676,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (ok && !pre_issued1) ok = start_slot(1, k, nkv1, pair_base);
       if (!ok) break;
       if (nkv_max > 0) mma_commit_lead(smem_u32(&ctrl->kv_empty[pair_base % kStages]), lead);
-      if (kParts && met == 1) { meet_again(); met = 3; }
+      if (kMayBeWhole && met == 1) { meet_again(); met = 3; }
       pre_issued0 = pre_issued1 = false;
       for (int j = 0; j < nkv_max && ok; ++j) {
         const int pr = pair_base + 1 + j;     // the pair {V_j, K_j+1}
@@ -942,7 +946,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (!ok || *abort_flag) { ok = false; break; }
       const int item = ctrl->sched_item[k & 1];
       if (item < 0) break;
-      if (kParts && !ctrl->cut) { meet_arrive(); meet_again(); }
+      if (kMayBeWhole && !ctrl->cut) { meet_arrive(); meet_again(); }
       // (the few fields needed are read from shared memory where they are used, not held across the tile loop)
       const ItemWork& w = ctrl->sched_work[k & 1];
       const int n = w.nkv[s];
@@ -1127,7 +1131,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->p_ready[s]));
       }
-      if constexpr (kParts) { seen = true; cut = ctrl->cut; }
+      if constexpr (kParts) { seen = true; cut = !kMayBeWhole || ctrl->cut; }
       if (!ok) break;
       // ---------------- the item's epilogue ----------------
       const int len_q = w.len_q;
@@ -1166,7 +1170,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // parts have arrived.  (Every warp of the cluster meets at both; no wait before them is without a limit.)  A part that
       // gave up sends NaN, and fills the rows that are its own with it.
       const int rank = static_cast<int>(cluster_rank()), parts = p.cluster_parts;
-      if (!cut) {
+      if (kMayBeWhole && !cut) {
         __syncwarp();
         cluster_wait();
         if (ok && rank == 0) ok = write_out(std::false_type{});
@@ -1237,7 +1241,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     uintptr_t at = reinterpret_cast<uintptr_t>(smem_raw);
     asm volatile("" : "+l"(at));
     const Control* const c = reinterpret_cast<const Control*>(((at + 1023) & ~uintptr_t(1023)) + Plan::kCtrlOff);
-    if (c->abort_flag && !(kParts && (c->cut || c->sched_work[0].kv_tok0 > 0))) {
+    if (c->abort_flag && !(kParts && (!kMayBeWhole || c->cut || c->sched_work[0].kv_tok0 > 0))) {
       const OutT nan = ElemTraits<OutT>::from_float(__int_as_float(0x7fc00000));
 #pragma unroll 1
       for (int k = 0; k < 2 * kSlots; ++k) {

@@ -34,7 +34,7 @@ struct PrefillParams {
   int head_pair;        // 1: the two slots of a work item are two q heads of one KV head over the same 128 rows
   int kv_split;         // parts every sequence's KV range is cut into that are merged by a second launch (1: not split so)
   int cluster_parts;    // parts that are the CTAs of a cluster (1: not split so)
-  int cut_tiles;        // items in clusters: the fewest KV tiles that the parts share
+  int cut_tiles;        // parts in clusters: the fewest KV tiles of a sequence that they share
   int kv_split_len;     // keys per part (a multiple of 128)
   float* lse;           // split only: log-sum-exp per (virtual sequence, q head, row), log2 domain
   float scale_log2;
