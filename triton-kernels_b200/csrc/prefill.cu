@@ -108,12 +108,22 @@ struct SmemPlan {
   static constexpr int kChunks = D / 64;                   // 128-byte column blocks per row
   static constexpr int kChunkBytes = kBN * 128;            // one column block of a 128-row tile
   static constexpr int kTileBytes = kChunks * kChunkBytes; // 128 x D 16-bit tile
+  // K and V of pages lie in groups of eight rows, [group][column block][row][128 B], so that one copy brings a page's rows whole (see
+  // make_kv_groups_map); all other tiles as [column block][row][128 B].
+  static constexpr int kGroupBytes = kChunks * 1024;
   static constexpr int kQOff = 0;
   static constexpr int kRingOff = kQBufs * kTileBytes;
   static constexpr int kCtrlOff = kRingOff + kRing * kTileBytes;
   static constexpr int kTotal = kCtrlOff + static_cast<int>(sizeof(Control));
   static_assert(kTotal + 1024 <= 227 * 1024, "shared memory of an SM (1 KiB for the alignment of the tiles)");
 };
+
+// K and V of pages: whether a box (a page's rows, up to a tile's) comes whole, by the 5-D map of make_kv_groups_map, instead of one
+// 64-column block at a time.  A box costs the producer a hundred cycles whatever it holds, and the sixteen copies of a tile of
+// 16-key pages at head_dim 128, twice a step, were as long as the step: causal, 4 x 2 048 tokens, 32/8 heads 166 -> 156 us, 2 x 4 096 289
+// -> 270, 4 x 252 11.8 -> 11.1; 128 queries over 2 048 keys 27.5 -> 26.4.  At head_dim 64 there is one block, and the 5-D copies
+// are slower than the 3-D ones (3 x 8 181 1 133 -> 1 160 us); so they are with boxes of less than a group (four keys 61 -> 66).
+__host__ __device__ constexpr bool group_boxes(int D, int box_rows) { return D > 64 && box_rows >= 8; }
 
 // The waits of a tile.  At head_dim 128 the first look is straight-line code (cycles per tile 1 807 -> 1 785); at 64 the softmax,
 // not the chain of waits, is what a step takes, and that costs (4 x 4 096 causal 362 -> 368 us).
@@ -394,6 +404,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     int pair_e = 0;       // K/V pairs issued so far, across items
     int q_uses = 0;       // Q tiles issued (or skipped) so far
     int pair_lo = 0;      // first pair of the current item
+    // where row r of a tile of pages lies, and whether a box comes in one copy
+    auto row_dst = [](int r) -> int { return Plan::kChunks == 1 ? r * 128 : (r >> 3) * Plan::kGroupBytes + (r & 7) * 128; };
+    const bool whole_boxes = group_boxes(D, p.box_rows);
     auto first_pages = [&](const int* table, const ItemWork& it) -> int {
       const long long tg = static_cast<long long>(lane << box_shift) + it.kv_tok0;
       const long long lp = page_pow2 ? tg >> page_shift : tg / p.page_size;
@@ -451,9 +464,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           const uint32_t bar = smem_u32(&ctrl->q_full[buf]);
           if (w.nkv[s] > 0) {
             mbar_arrive_expect_tx(bar, Plan::kTileBytes);
-            for (int c = 0; c < Plan::kChunks; ++c)
-              tma_load_3d(smem_base + Plan::kQOff + buf * Plan::kTileBytes + c * Plan::kChunkBytes, &tm_q, bar, c * 64,
-                          w.q_head_coord[s], static_cast<int>(w.q_row0[s] + w.m0[s]));
+            tma_load_4d(smem_base + Plan::kQOff + buf * Plan::kTileBytes, &tm_q, bar, 0, static_cast<int>(w.q_row0[s] + w.m0[s]), 0,
+                        w.q_head_coord[s]);
           } else {
             mbar_arrive(bar);   // keeps one q_full phase per use
           }
@@ -464,8 +476,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       };
       if (k >= 1 && lane == 0 && w.nkv[1] > 0) {
         // pull the second slot's Q into L2 now, so the copies issued once its buffer is free only pay an L2 round trip
-        for (int c = 0; c < Plan::kChunks; ++c)
-          tma_prefetch_3d(&tm_q, c * 64, w.q_head_coord[1], static_cast<int>(w.q_row0[1] + w.m0[1]));
+        tma_prefetch_4d(&tm_q, 0, static_cast<int>(w.q_row0[1] + w.m0[1]), 0, w.q_head_coord[1]);
       }
       ok = load_q(0);
       if (!ok) break;
@@ -492,14 +503,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (!kPaged) {
           if (lane == 0) {
             mbar_arrive_expect_tx(bar, (has_v ? Plan::kTileBytes : 0) + (has_k ? Plan::kTileBytes : 0));
-            for (int c = 0; c < Plan::kChunks; ++c) {
-              if (has_v)
-                tma_load_3d(vdst + c * Plan::kChunkBytes, &tm_v, bar, c * 64, w.kv_head_coord,
-                            static_cast<int>(w.kv_row0 + static_cast<long long>(jv) * kBN));
-              if (has_k)
-                tma_load_3d(kdst + c * Plan::kChunkBytes, &tm_k, bar, c * 64, w.kv_head_coord,
-                            static_cast<int>(w.kv_row0 + static_cast<long long>(jk) * kBN));
-            }
+            if (has_v) tma_load_4d(vdst, &tm_v, bar, 0, static_cast<int>(w.kv_row0 + static_cast<long long>(jv) * kBN), 0, w.kv_head_coord);
+            if (has_k) tma_load_4d(kdst, &tm_k, bar, 0, static_cast<int>(w.kv_row0 + static_cast<long long>(jk) * kBN), 0, w.kv_head_coord);
           }
         } else if (pf) {
           // one box per lane and operand from the entries read ahead
@@ -527,11 +532,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           const int rv = lane < nv ? row_of(ev, jv * kBN + (lane << box_shift)) : -1;
           if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(nk + nv) * p.box_rows * 128 * Plan::kChunks);
           __syncwarp();
-          for (int c = 0; c < Plan::kChunks; ++c) {
-            if (rv >= 0)
-              tma_load_3d(vdst + c * Plan::kChunkBytes + lane * p.box_rows * 128, &tm_v, bar, c * 64, w.kv_head_coord, rv);
-            if (rk >= 0)
-              tma_load_3d(kdst + c * Plan::kChunkBytes + lane * p.box_rows * 128, &tm_k, bar, c * 64, w.kv_head_coord, rk);
+          const int dst = row_dst(lane << box_shift);
+          if (whole_boxes) {
+            if (rv >= 0) tma_load_5d(vdst + dst, &tm_v, bar, 0, 0, 0, rv >> 3, w.kv_head_coord);
+            if (rk >= 0) tma_load_5d(kdst + dst, &tm_k, bar, 0, 0, 0, rk >> 3, w.kv_head_coord);
+          } else {
+            for (int c = 0; c < Plan::kChunks; ++c) {
+              if (rv >= 0) tma_load_3d(vdst + dst + c * 1024, &tm_v, bar, c * 64, w.kv_head_coord, rv);
+              if (rk >= 0) tma_load_3d(kdst + dst + c * 1024, &tm_k, bar, c * 64, w.kv_head_coord, rk);
+            }
           }
         } else {
           // one box of `box_rows` tokens per lane per round and operand; only pages that exist are fetched
@@ -562,11 +571,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           __syncwarp();
           int kk = 0;
           for (int i = lane; i < boxes; i += 32, ++kk) {
+            const int rv = rows_v[kk], rk = rows_k[kk], dst = row_dst(i * p.box_rows);    // (fewer than four rows)
             for (int c = 0; c < Plan::kChunks; ++c) {
-              if (rows_v[kk] >= 0)
-                tma_load_3d(vdst + c * Plan::kChunkBytes + i * p.box_rows * 128, &tm_v, bar, c * 64, w.kv_head_coord, rows_v[kk]);
-              if (rows_k[kk] >= 0)
-                tma_load_3d(kdst + c * Plan::kChunkBytes + i * p.box_rows * 128, &tm_k, bar, c * 64, w.kv_head_coord, rows_k[kk]);
+              if (rv >= 0) tma_load_3d(vdst + dst + c * 1024, &tm_v, bar, c * 64, w.kv_head_coord, rv);
+              if (rk >= 0) tma_load_3d(kdst + dst + c * 1024, &tm_k, bar, c * 64, w.kv_head_coord, rk);
             }
           }
         }
@@ -599,8 +607,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     bool ok = true;
     // Descriptor words are prepared once: the high words never change, the low words are a base
     // (start address >> 4) plus small constants, so issuing one MMA costs the single thread a few adds.
-    const uint64_t kdesc = make_smem_desc_sw128(smem_base, 16);                    // K-major operands (Q, K)
-    const uint64_t vdesc = make_smem_desc_sw128(smem_base, Plan::kChunkBytes);     // MN-major operand (V)
+    constexpr int kGroup = kPaged ? Plan::kGroupBytes : 1024;           // between groups of eight keys
+    constexpr int kBlock = kPaged ? 1024 : Plan::kChunkBytes;           // between column blocks
+    const uint64_t qdesc = make_smem_desc_sw128(smem_base, 16);                    // K-major operands (Q, K)
+    const uint64_t kdesc = make_smem_desc_sw128(smem_base, 16, kGroup);
+    const uint64_t vdesc = make_smem_desc_sw128(smem_base, kBlock, kGroup);        // MN-major operand (V)
     int pair_base = 0;            // pair that holds K_0 of the current item (pair j + 1 holds V_j and K_j+1)
     // per-slot state as scalars (an array indexed by the slot would live in local memory)
     int tiles_done0 = 0, tiles_done1 = 0;       // score tiles issued per slot so far (barrier phases run across items)
@@ -630,17 +641,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       return uniform(vdesc + static_cast<uint64_t>((Plan::kRingOff + (2 * (pr % kStages)) * Plan::kTileBytes) >> 4));
     };
     auto q_desc_of = [&](int buf) -> uint64_t {
-      return uniform(kdesc + static_cast<uint64_t>((Plan::kQOff + buf * Plan::kTileBytes) >> 4));
+      return uniform(qdesc + static_cast<uint64_t>((Plan::kQOff + buf * Plan::kTileBytes) >> 4));
     };
     auto issue_s = [&](int s, uint64_t qa, uint64_t kb) {
       // S_s = Q_s K^T : K-major A and B, D/16 k-steps
-      mma_ss_batch<D / 16>(tmem_S[s], qa, kb, idesc_s, 0u, lead);
+      mma_ss_batch<D / 16, kBlock / 16>(tmem_S[s], qa, kb, idesc_s, 0u, lead);
       mma_commit_lead(smem_u32(&ctrl->s_full[s]), lead);
     };
     auto issue_pv = [&](int s, uint64_t vb, bool first) {
       // O_s (+)= P_s V : A = packed 16-bit P, 32 TMEM columns at the start of each 64-column half of the S tile;
       // B = V, MN-major
-      mma_ts_batch8(tmem_O[s], tmem_S[s], vb, idesc_o, first ? 0u : 1u, lead);
+      mma_ts_batch8<2 * kGroup / 16>(tmem_O[s], tmem_S[s], vb, idesc_o, first ? 0u : 1u, lead);
       mma_commit_lead(smem_u32(&ctrl->o_done[s]), lead);
     };
 
@@ -694,8 +705,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             const int first = valid > 0 ? valid : 0;
             const int n16 = (kBN - first) * 8;  // 16-byte pieces per column block
             for (int c = 0; c < Plan::kChunks; ++c) {
-              uint4* dst = reinterpret_cast<uint4*>(vbuf + c * Plan::kChunkBytes + first * 128);
-              for (int i = lane; i < n16; i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+              if constexpr (kGroup == 1024) {
+                // (written out for this case: with the indices of the other one, never run in a whole tile, 3 x 8 192 causal tokens,
+                // 32/8 heads, head_dim 64, took 1 120 us instead of 1 064)
+                uint4* dst = reinterpret_cast<uint4*>(vbuf + c * kBlock + first * 128);
+                for (int i = lane; i < n16; i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+              } else {
+                for (int i = lane; i < n16; i += 32) {
+                  const int at = first * 8 + i;   // (eight pieces a row, 64 a group)
+                  *reinterpret_cast<uint4*>(vbuf + c * kBlock + (at >> 6) * kGroup + (at & 63) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                }
+              }
             }
             fence_proxy_async_smem();
             __syncwarp();
@@ -1523,28 +1543,34 @@ int launch_prefill(const b200attn_prefill_args_t& a_in, int sm_count, cudaStream
   CUtensorMap tq, tk, tv;
   int rc;
   dim3 grid;
+  const long long row_bytes = D * 2ll;
   long long total_items = 0;
   if (a.layout == B200ATTN_RAGGED) {
-    if ((rc = make_token_map(&tq, a.dtype, a.q, a.total_q, a.q_heads, D, kBM))) return rc;
-    if ((rc = make_token_map(&tk, a.dtype, a.k, a.total_kv, a.kv_heads, D, kBN))) return rc;
-    if ((rc = make_token_map(&tv, a.dtype, a.v, a.total_kv, a.kv_heads, D, kBN))) return rc;
+    if ((rc = make_kv_rows_map(&tq, a.dtype, a.q, a.total_q, a.q_heads, D, kBM, a.q_heads * row_bytes, row_bytes))) return rc;
+    if ((rc = make_kv_rows_map(&tk, a.dtype, a.k, a.total_kv, a.kv_heads, D, kBN, a.kv_heads * row_bytes, row_bytes))) return rc;
+    if ((rc = make_kv_rows_map(&tv, a.dtype, a.v, a.total_kv, a.kv_heads, D, kBN, a.kv_heads * row_bytes, row_bytes))) return rc;
     const long long pairs = a.total_q / item_rows + a.batch;
     total_items = pairs * head_units;
   } else {
     const long long q_rows = static_cast<long long>(a.batch) * a.q_heads * a.max_q;
-    if ((rc = make_token_map(&tq, a.dtype, a.q, q_rows, 1, D, kBM))) return rc;
+    if ((rc = make_kv_rows_map(&tq, a.dtype, a.q, q_rows, 1, D, kBM, row_bytes, row_bytes))) return rc;
     if (a.layout == B200ATTN_DENSE) {
       const long long kv_rows = static_cast<long long>(a.batch) * a.kv_heads * a.max_kv;
-      if ((rc = make_token_map(&tk, a.dtype, a.k, kv_rows, 1, D, kBN))) return rc;
-      if ((rc = make_token_map(&tv, a.dtype, a.v, kv_rows, 1, D, kBN))) return rc;
+      if ((rc = make_kv_rows_map(&tk, a.dtype, a.k, kv_rows, 1, D, kBN, row_bytes, row_bytes))) return rc;
+      if ((rc = make_kv_rows_map(&tv, a.dtype, a.v, kv_rows, 1, D, kBN, row_bytes, row_bytes))) return rc;
     } else {
       // largest power of two that divides the page size, capped at the tile: every box stays inside one page
       int box = 1;
       while (box < kBN && (a.page_size % (box * 2)) == 0) box *= 2;
       p.box_rows = box;
       p.num_pages = static_cast<int>(std::min<long long>(a.total_kv / a.page_size, 0x7fffffff));
-      if ((rc = make_token_map(&tk, a.dtype, a.k, a.total_kv, a.kv_heads, D, box))) return rc;
-      if ((rc = make_token_map(&tv, a.dtype, a.v, a.total_kv, a.kv_heads, D, box))) return rc;
+      if (group_boxes(D, box)) {
+        if ((rc = make_kv_groups_map(&tk, a.dtype, a.k, a.total_kv, a.kv_heads, D, box, a.kv_heads * row_bytes, row_bytes))) return rc;
+        if ((rc = make_kv_groups_map(&tv, a.dtype, a.v, a.total_kv, a.kv_heads, D, box, a.kv_heads * row_bytes, row_bytes))) return rc;
+      } else {
+        if ((rc = make_token_map(&tk, a.dtype, a.k, a.total_kv, a.kv_heads, D, box))) return rc;
+        if ((rc = make_token_map(&tv, a.dtype, a.v, a.total_kv, a.kv_heads, D, box))) return rc;
+      }
     }
     total_items = static_cast<long long>((a.max_q + item_rows - 1) / item_rows) * head_units * a.batch * p.kv_split * p.cluster_parts;
   }

@@ -140,9 +140,9 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, 
 }
 
 // brings the box into L2 only (no shared-memory destination, no completion to wait for)
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* m, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];\n"
-               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2)
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* m, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
 
@@ -150,6 +150,13 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* m, 
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
+
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2, int c3, int c4) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];\n"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
       : "memory");
 }
 
@@ -319,15 +326,15 @@ __device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
 }
 
 // ------------------------------ tcgen05.mma ----------------------------------
-// Shared-memory matrix descriptor, 128-byte swizzle, rows of 128 bytes packed
-// back to back (8-row groups every 1024 bytes).  `lbo_bytes` is the distance
+// Shared-memory matrix descriptor, 128-byte swizzle, groups of eight 128-byte rows
+// every `group_bytes`.  `lbo_bytes` is the distance
 // between 128-byte-wide column blocks of an MN-major operand (ignored for
 // K-major operands, where one MMA never leaves the 128-byte row).
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes) {
+__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t group_bytes = 1024) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);              // start address, bits [0,14)
   d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;          // leading byte offset, bits [16,30)
-  d |= static_cast<uint64_t>((1024u >> 4) & 0x3FFFu) << 32;              // stride byte offset, bits [32,46)
+  d |= static_cast<uint64_t>((group_bytes >> 4) & 0x3FFFu) << 32;        // stride byte offset, bits [32,46)
   d |= static_cast<uint64_t>(1) << 46;                                   // descriptor version (Blackwell)
   d |= static_cast<uint64_t>(2) << 61;                                   // layout: SWIZZLE_128B
   return d;
@@ -366,13 +373,13 @@ __device__ __forceinline__ uint32_t elect_one() {
   return r;
 }
 
-#define B200ATTN_SS_STEP(OFF)                                                                   \
-  "add.s64 a1, %1, " #OFF ";\n\tadd.s64 b1, %2, " #OFF ";\n\t"                                  \
+#define B200ATTN_SS_STEP(AOFF, BOFF)                                                            \
+  "add.s64 a1, %1, " #AOFF ";\n\tadd.s64 b1, %2, " BOFF ";\n\t"                                 \
   "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
 
-// D/16 k-steps of a K-major x K-major product whose operands are 128-row, 128-byte-swizzled tiles stored as
-// 64-element column blocks of 16 KiB: k-step kk starts (kk / 4) * 16 KiB + (kk % 4) * 32 bytes into both tiles.
-template <int KSTEPS>
+// D/16 k-steps of a K-major x K-major product of 128-row, 128-byte-swizzled tiles.  A is stored as 64-element column blocks
+// of 16 KiB: k-step kk starts (kk / 4) * 16 KiB + (kk % 4) * 32 bytes into the tile; B's column blocks are CHUNK16 * 16 bytes apart.
+template <int KSTEPS, int CHUNK16>
 __device__ __forceinline__ void mma_ss_batch(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                              uint32_t accumulate_first, uint32_t lead) {
   static_assert(KSTEPS == 4 || KSTEPS == 8, "head dimension 64 or 128");
@@ -381,37 +388,40 @@ __device__ __forceinline__ void mma_ss_batch(uint32_t d_tmem, uint64_t a_desc, u
         "{\n\t.reg .pred p, t, e;\n\t.reg .b64 a1, b1;\n\t"
         "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        B200ATTN_SS_STEP(2) B200ATTN_SS_STEP(4) B200ATTN_SS_STEP(6)
-        B200ATTN_SS_STEP(1024) B200ATTN_SS_STEP(1026) B200ATTN_SS_STEP(1028) B200ATTN_SS_STEP(1030)
-        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead) : "memory");
+        B200ATTN_SS_STEP(2, "2") B200ATTN_SS_STEP(4, "4") B200ATTN_SS_STEP(6, "6")
+        B200ATTN_SS_STEP(1024, "%6") B200ATTN_SS_STEP(1026, "%7") B200ATTN_SS_STEP(1028, "%8") B200ATTN_SS_STEP(1030, "%9")
+        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead),
+        "n"(CHUNK16), "n"(CHUNK16 + 2), "n"(CHUNK16 + 4), "n"(CHUNK16 + 6) : "memory");
   } else {
     asm volatile(
         "{\n\t.reg .pred p, t, e;\n\t.reg .b64 a1, b1;\n\t"
         "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-        B200ATTN_SS_STEP(2) B200ATTN_SS_STEP(4) B200ATTN_SS_STEP(6)
+        B200ATTN_SS_STEP(2, "2") B200ATTN_SS_STEP(4, "4") B200ATTN_SS_STEP(6, "6")
         "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead) : "memory");
   }
 }
 #undef B200ATTN_SS_STEP
 
-#define B200ATTN_TS_STEP(AOFF, BOFF)                                                            \
-  "add.u32 a1, %1, " #AOFF ";\n\tadd.s64 b1, %2, " #BOFF ";\n\t"                                \
+#define B200ATTN_TS_STEP(AOFF, BOPND)                                                           \
+  "add.u32 a1, %1, " #AOFF ";\n\tadd.s64 b1, %2, " BOPND ";\n\t"                                \
   "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
 
 // Eight k-steps (128 keys) of O += P V: A is packed 16-bit P, keys 0..63 in the 32 tensor-memory columns at `a_tmem`
-// and keys 64..127 in the 32 columns at `a_tmem + kPHalfStride`; B is an MN-major 128-row V tile, 16 rows (2 KiB)
+// and keys 64..127 in the 32 columns at `a_tmem + kPHalfStride`; B is an MN-major 128-row V tile, 16 rows (STEP16 * 16 bytes)
 // per k-step.
 constexpr uint32_t kPHalfStride = 64;
+template <int STEP16>
 __device__ __forceinline__ void mma_ts_batch8(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate_first, uint32_t lead) {
   asm volatile(
       "{\n\t.reg .pred p, t, e;\n\t.reg .b32 a1;\n\t.reg .b64 b1;\n\t"
       "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      B200ATTN_TS_STEP(8, 128) B200ATTN_TS_STEP(16, 256) B200ATTN_TS_STEP(24, 384)
-      B200ATTN_TS_STEP(64, 512) B200ATTN_TS_STEP(72, 640) B200ATTN_TS_STEP(80, 768) B200ATTN_TS_STEP(88, 896)
-      "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead) : "memory");
+      B200ATTN_TS_STEP(8, "%6") B200ATTN_TS_STEP(16, "%7") B200ATTN_TS_STEP(24, "%8")
+      B200ATTN_TS_STEP(64, "%9") B200ATTN_TS_STEP(72, "%10") B200ATTN_TS_STEP(80, "%11") B200ATTN_TS_STEP(88, "%12")
+      "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead), "n"(STEP16), "n"(2 * STEP16),
+      "n"(3 * STEP16), "n"(4 * STEP16), "n"(5 * STEP16), "n"(6 * STEP16), "n"(7 * STEP16) : "memory");
   static_assert(kPHalfStride == 64, "the offsets in the instruction list above");
 }
 #undef B200ATTN_TS_STEP

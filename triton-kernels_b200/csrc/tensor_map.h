@@ -16,4 +16,11 @@ int make_token_map(CUtensorMap* m, int dtype, const void* base, long long tokens
 int make_kv_rows_map(CUtensorMap* m, int dtype, const void* base, long long rows, int heads, int D, int box_rows,
                      long long row_stride_bytes, long long head_stride_bytes);
 
+// 5-D map over the same rows in groups of eight: dims (64 elements, 8 rows, D/64 column blocks, groups, heads); box = 64 x 8 x D/64 x
+// box_rows / 8 x 1, 128-byte swizzle, box_rows a multiple of eight.  One copy brings box_rows keys of one head as
+// [group][column block][row of the group][128 B], which, unlike the 4-D map's order, a tcgen05 descriptor can address across boxes of any
+// size: the groups of a column block lie at one distance in the whole tile.
+int make_kv_groups_map(CUtensorMap* m, int dtype, const void* base, long long rows, int heads, int D, int box_rows,
+                       long long row_stride_bytes, long long head_stride_bytes);
+
 }  // namespace b200attn
