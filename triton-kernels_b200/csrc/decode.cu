@@ -19,6 +19,8 @@
 //       written to tensor memory once per unit, P once per 64-key tile, so both MMAs take their A operand from TMEM
 //       and shared memory is read once per K/V byte.  Persistent: one wave of CTAs walks the unit list, the producer
 //       runs ahead across units.  Same planner and partial format; merges are claimed in the CTAs' teardown.
+//   decode_keyrows_kernel (decode_keyrows.cuh) : 17 to 64 q rows over long sequences.  The tensor-core tiles have keys as their rows
+//       and the q rows as their columns, so nothing is multiplied for rows that are not there.
 //   decode_simt_kernel : the fp32-input variant, fp32 FMA arithmetic like the reference's decode kernel.
 //   A unit whose sequence has a single chunk writes the output directly; otherwise it writes an (m, l, acc) partial
 //       and takes a ticket.  In the one-CTA-per-unit kernels (emit_and_merge) the CTA that draws the last ticket of
@@ -524,6 +526,13 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
       s_carry = 0;
       // (a cut moved to the end of a sequence makes a stretch up to min_chunk longer: without that in the estimate 47
       // sequences of 350 to 5 600 keys on one KV head were dealt out and took 48 us instead of 45)
+      // (One CTA to an SM: dealing out costs some 500 keys more, and the estimate has to favour it by a tenth.  Over 26 batches it gave 0.94 to
+      // 1.05 of the time without; by this rule 32 x 1 000 to 33 000 keys 292 -> 287 us, of 34 x 10 232 at D 64 166 instead of 171.
+      // Equal items end with the last round of CTAs, not half an item behind the average.)
+      if (p.one_cta) {
+        const float rounds = static_cast<float>((items0 + p.wave_items - 1) / p.wave_items) * (static_cast<float>(pick_chunk) + ovh);
+        best = 0.89f * fminf(best, rounds) - 500.f;
+      }
       const bool deal = p.slots > 1 && p.slots <= kPlanMaxSlots && cached && line < (1 << 30) && items0 > p.wave_items &&
                         static_cast<float>(line) / static_cast<float>(p.slots) + static_cast<float>(p.min_chunk) < best;
       s_slots = deal ? p.slots : 0;
@@ -1382,6 +1391,66 @@ __device__ __forceinline__ UmmaUnit umma_unit(const DecodeParams& p, int u) {
   return w;
 }
 
+// Merges.  A (sequence, kv head) pair whose chunks have all drawn their tickets is merged by whichever CTA claims
+// it while sweeping the ticket counters in its teardown, with all of its threads: CTAs that finish early take the pairs that
+// are complete, the CTA that draws a pair's last ticket sweeps after it did, so every pair is merged by the time
+// the last CTA leaves, and no CTA waits for another.  A CTA takes one pair per sweep and sweeps again as long as it
+// saw a complete pair; header[3] (tickets drawn and not merged) lets a CTA skip the sweep when there is nothing.
+template <typename OutT, int D, typename Ctrl>
+__device__ __forceinline__ void claim_merges(const DecodeParams& p, Ctrl* ctrl, int me) {
+  if (ctrl->abort_flag) return;
+  const int tid = threadIdx.x;
+  const int n_pairs = p.batch * p.kv_heads;
+  for (int sweep = 0; sweep < n_pairs + 64; ++sweep) {
+    if (tid == 0) {
+      ctrl->ready = *reinterpret_cast<volatile int*>(p.header + 3);
+      ctrl->n_reserved = 0;
+      ctrl->n_claimed = 0;
+    }
+    __syncthreads();
+    if (ctrl->ready <= 0) break;
+    for (int e = tid; e < n_pairs; e += static_cast<int>(blockDim.x)) {
+      const int pair = (e + me * 61) % n_pairs;            // CTAs start their sweeps at different pairs
+      const int b = pair / p.kv_heads;
+      const int n = p.item_start[b + 1] - p.item_start[b];
+      if (n > 1 && *reinterpret_cast<volatile int*>(p.counters + pair) == n &&
+          atomicAdd(&ctrl->n_reserved, 1) < kUmmaMaxClaims &&
+          atomicCAS(p.counters + pair, n, n + kMergeClaimed) == n) {
+        atomicSub(p.header + 3, n);
+        ctrl->claimed[atomicAdd(&ctrl->n_claimed, 1)] = pair;
+      }
+    }
+    __syncthreads();
+    if (ctrl->n_reserved == 0) break;                      // no complete pair in sight: whoever completes one sweeps
+    const int n_claimed = ctrl->n_claimed;
+    for (int i = 0; i < n_claimed; ++i) {
+      const int pair = ctrl->claimed[i];
+      const int b = pair / p.kv_heads, h = pair - b * p.kv_heads;
+      const int item0 = p.item_start[b];
+      OutT* out = static_cast<OutT*>(p.out) +
+                  ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
+      merge_chunks<OutT, D>(p, b, h, p.item_start[b + 1] - item0, item0, out, tid, static_cast<int>(blockDim.x));
+    }
+    __syncthreads();
+  }
+}
+
+// A bounded wait ran out: the rows of the unit whose rows were being written, and of the units this CTA had not
+// reached, are unknown.  They are filled with NaN (and their tickets are not drawn, so nobody merges over them):
+// the failure shows in the output as well as in the error word.  `unit_of(r)`: the CTA's r-th unit.
+template <typename OutT, int D, typename Ctrl, typename UnitOf>
+__device__ __forceinline__ void poison_units(const DecodeParams& p, Ctrl* ctrl, int n_units, UnitOf unit_of) {
+  const OutT nan_t = ElemTraits<OutT>::from_float(__int_as_float(0x7fc00000));
+  // (the slots of units that are not finished cannot have been reused by the producer)
+  for (int r = ctrl->abort_round; r < ctrl->published; ++r) {
+    if (ctrl->unit_ring[r % kUmmaUnitRing] >= n_units) break;
+    const UmmaUnit w = unit_of(r);
+    OutT* out = static_cast<OutT*>(p.out) +
+                ((static_cast<long long>(w.b) * p.q_heads + static_cast<long long>(w.h) * p.head_stride + p.head0) * p.q_len) * D;
+    for (int i = threadIdx.x; i < p.rows * D; i += static_cast<int>(blockDim.x)) out[i] = nan_t;
+  }
+}
+
 // T: element type of q, k, v as the kernel reads them; OutT: element type of the output rows (T, or float when the
 // inputs are fp16 copies of fp32 tensors).  kOwnPlan: no planner has run, and every CTA works out the one unit that is its own.
 template <typename T, int D, typename OutT, bool kOwnPlan>
@@ -2069,62 +2138,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
       return;
     }
   }
-  // Merges.  A (sequence, kv head) pair whose chunks have all drawn their tickets is merged by whichever CTA claims
-  // it while sweeping the ticket counters here, with all of its threads: CTAs that finish early take the pairs that
-  // are complete, the CTA that draws a pair's last ticket sweeps after it did, so every pair is merged by the time
-  // the last CTA leaves, and no CTA waits for another.  A CTA takes one pair per sweep and sweeps again as long as it
-  // saw a complete pair; header[3] (tickets drawn and not merged) lets a CTA skip the sweep when there is nothing.
-  if (!ctrl->abort_flag && !kOwnPlan) {
-    const int n_pairs = p.batch * p.kv_heads;
-    for (int sweep = 0; sweep < n_pairs + 64; ++sweep) {
-      if (tid == 0) {
-        ctrl->ready = *reinterpret_cast<volatile int*>(p.header + 3);
-        ctrl->n_reserved = 0;
-        ctrl->n_claimed = 0;
-      }
-      __syncthreads();
-      if (ctrl->ready <= 0) break;
-      for (int e = tid; e < n_pairs; e += static_cast<int>(blockDim.x)) {
-        const int pair = (e + me * 61) % n_pairs;            // CTAs start their sweeps at different pairs
-        const int b = pair / p.kv_heads;
-        const int n = p.item_start[b + 1] - p.item_start[b];
-        if (n > 1 && *reinterpret_cast<volatile int*>(p.counters + pair) == n &&
-            atomicAdd(&ctrl->n_reserved, 1) < kUmmaMaxClaims &&
-            atomicCAS(p.counters + pair, n, n + kMergeClaimed) == n) {
-          atomicSub(p.header + 3, n);
-          ctrl->claimed[atomicAdd(&ctrl->n_claimed, 1)] = pair;
-        }
-      }
-      __syncthreads();
-      if (ctrl->n_reserved == 0) break;                      // no complete pair in sight: whoever completes one sweeps
-      const int n_claimed = ctrl->n_claimed;
-      for (int i = 0; i < n_claimed; ++i) {
-        const int pair = ctrl->claimed[i];
-        const int b = pair / p.kv_heads, h = pair - b * p.kv_heads;
-        const int item0 = p.item_start[b];
-        OutT* out = static_cast<OutT*>(p.out) +
-                    ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
-        merge_chunks<OutT, D>(p, b, h, p.item_start[b + 1] - item0, item0, out, tid, static_cast<int>(blockDim.x));
-      }
-      __syncthreads();
-    }
-  }
-  if (ctrl->abort_flag) {
-    // A bounded wait ran out: the rows of the unit the softmax warps were in, and of the units this CTA had not
-    // reached, are unknown.  They are filled with NaN (and their tickets are not drawn, so nobody merges over them):
-    // the failure shows in the output as well as in the error word.
-    const OutT nan_t = ElemTraits<OutT>::from_float(__int_as_float(0x7fc00000));
-    // (the slots of units the softmax warps have not finished cannot have been reused by the producer)
-    for (int r = ctrl->abort_round; r < ctrl->published; ++r) {
-      const int u = ctrl->unit_ring[r % kUmmaUnitRing];
-      if (u >= n_units) break;
-      const UmmaUnit w = unit_of(u);
-      OutT* out = static_cast<OutT*>(p.out) +
-                  ((static_cast<long long>(w.b) * p.q_heads + static_cast<long long>(w.h) * p.head_stride + p.head0) * p.q_len) * D;
-      for (int i = tid; i < R * D; i += blockDim.x) out[i] = nan_t;
-    }
-  }
+  if (!kOwnPlan) claim_merges<OutT, D>(p, ctrl, me);
+  if (ctrl->abort_flag) poison_units<OutT, D>(p, ctrl, n_units, [&](int r) { return unit_of(ctrl->unit_ring[r % kUmmaUnitRing]); });
 }
+
+#include "decode_keyrows.cuh"
 
 // ---------------------------------------------------------------------------
 // fp32 kernel: fp32 FMA dot products.
@@ -2643,6 +2661,32 @@ Route route_of(const b200attn_decode_args_t& a, int sm_count, int rows, bool bui
   return r;
 }
 
+// largest power of two that divides the page size, at most a tile of 64: every box stays inside one page
+int page_box(const b200attn_decode_args_t& a) {
+  int box = kTileN;
+  if (a.layout == B200ATTN_PAGED) {
+    box = 1;
+    while (box < kTileN && (a.page_size % (box * 2)) == 0) box *= 2;
+  }
+  return box;
+}
+
+// Whether a planned pass of more than sixteen rows goes to decode_keyrows_kernel.  A unit there, a CTA's to itself, has some 2.5 us
+// beside its copies; decode_umma_kernel's take longer, but an SM has two CTAs.  So the line is the length of a sequence, 512 keys at
+// head_dim 128 and 1 024 at 64 (us, umma and keyrows, 40 rows of eight heads, D 128: 64 sequences of 250 keys 25.1, 28.4; of 400 33.5, 34.7;
+// of 600 41.9, 41.5; of 1 000 59.4, 57.6; 200 of 400 82.7, 78.9; D 64, 64 of 700 32.6, 39.7; of 1 000 41.3, 48.0; of 1 200 60.2, 51.8; of
+// 2 400 90.3, 86.4), and half of that where no SM has more than one unit (16 of 250 at D 128, 20 rows 22.7, 16.0; 40 rows 15.4, 15.8).
+// Pages say how long a sequence can be; twice the line is asked for, which sequences of any length up to that reach on average.
+// (Much shorter ones in such tables are slower for it: 64 of 20 keys in tables of 8 192 17.4, 23.0.  Both kernels launched, and the planner's
+// word for which of them stays, cost every call 4 to 6 us.)
+bool keyrows_suit(const b200attn_decode_args_t& a, int sm_count, int rows) {
+  if (a.dtype == B200ATTN_F32 || rows <= 16 || rows > kKrMaxRows || !keyrows_boxes(page_box(a))) return false;
+  if (inline_plan_bits(a, sm_count, rows)) return false;      // (also in the library's own array, where such a call is planned)
+  const bool one_each = static_cast<long long>(a.batch) * a.kv_heads <= sm_count;
+  const long long line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * (a.layout == B200ATTN_PAGED ? 2 : 1) / 2;
+  return most_keys(a) >= line * a.batch;
+}
+
 // `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
 int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, const DecodeWsLayout& w,
                        int pass_group, int head0, bool f32_out, bool built_in) {
@@ -2673,7 +2717,6 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   p.box_shift = 6;
   p.target_items = w.target_items; p.min_chunk = w.min_chunk; p.max_items = w.max_items;
   p.wave_items = w.wave_items; p.item_overhead = w.item_overhead;
-  p.slots = a.dtype != B200ATTN_F32 && p.rows > 16 ? 2 * sm_count / a.kv_heads : 0;
   p.scale_log2 = a.sm_scale * 1.4426950408889634f;
 
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
@@ -2690,6 +2733,18 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
       p.wave_items = 0;
     }
   }
+  // the kernels of many rows are persistent: two CTAs to an SM (planned for in decode_ws_layout), or one
+  const bool key_rows = keyrows_suit(a, sm_count, p.rows);
+  p.slots = a.dtype != B200ATTN_F32 && p.rows > 16 ? 2 * sm_count / a.kv_heads : 0;
+  if (key_rows) {
+    // Three units a CTA where there are enough to share, handed out longest first: us, against six and dealt out as for two CTAs, 128 x 1 500
+    // keys of two heads, 40 rows, D 128 51.7 -> 44.4, 34 x 10 232 of eight, 36 rows, D 64 171 -> 166, 200 x 300 to 4 000 in pages 91.8 -> 88.1.
+    // Very uneven batches are still dealt out (32 x 1 000 to 33 000 291 -> 286).
+    p.wave_items = std::max(1, sm_count / a.kv_heads);
+    p.target_items = std::max(1, 3 * sm_count / a.kv_heads);
+    p.slots = sm_count / a.kv_heads;
+  }
+  p.one_cta = key_rows;
   unsigned grid_items = static_cast<unsigned>(w.max_items);
   cudaError_t e = cudaSuccess;
   if (p.inline_plan) {
@@ -2723,11 +2778,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     // many q rows per KV head: one 128-row tcgen05 tile with Q and P in tensor memory
     CUtensorMap tk, tv;
     int rc = 0;
-    int box = kTileN;
-    if (a.layout == B200ATTN_PAGED) {
-      box = 1;
-      while (box < kTileN && (a.page_size % (box * 2)) == 0) box *= 2;
-    }
+    const int box = page_box(a);
     p.box_shift = 0;
     while ((1 << p.box_shift) < box) ++p.box_shift;
     long long tokens;
@@ -2738,11 +2789,26 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     if ((rc = make_token_map(&tv, a.dtype, a.v, tokens, heads, D, box))) return rc;
     const size_t stage_bytes = static_cast<size_t>(kUmmaStages) * 2 * kTileN * D * 2;
     const size_t smem = 1024 + stage_bytes + sizeof(UmmaCtrl);
-    // persistent: one wave of two CTAs per SM walks the unit list (fewer CTAs when the list cannot be longer)
-    const unsigned wave = 2u * static_cast<unsigned>(sm_count);
-    const dim3 grid(p.inline_plan ? grid_items * a.kv_heads : std::min(static_cast<unsigned>(w.max_items) * a.kv_heads, wave), 1);
+    // persistent: one wave walks the unit list (fewer CTAs when the list cannot be longer)
+    auto wave_of = [&](int ctas) { return dim3(std::min(static_cast<unsigned>(w.max_items) * a.kv_heads, static_cast<unsigned>(ctas))); };
+    const dim3 grid = p.inline_plan ? dim3(grid_items * a.kv_heads) : wave_of(2 * sm_count);
+    CUtensorMap tq, gk = tk, gv = tv;
+    if (key_rows) {
+      const long long q_rows = static_cast<long long>(a.batch) * a.q_heads * a.q_len;
+      if ((rc = make_token_map(&tq, a.dtype, a.q, q_rows, 1, D, (p.rows + 15) & ~15))) return rc;
+      if (D == 128 && a.layout == B200ATTN_PAGED) {
+        if ((rc = make_kv_groups_map(&gk, a.dtype, a.k, tokens, heads, D, box, heads * D * 2ll, D * 2ll))) return rc;
+        if ((rc = make_kv_groups_map(&gv, a.dtype, a.v, tokens, heads, D, box, heads * D * 2ll, D * 2ll))) return rc;
+      }
+    }
 #define B200ATTN_LAUNCH_UMMA(TYPE, DIM, OUT)                                  \
     do {                                                                      \
+      if (key_rows) {                                                         \
+        constexpr size_t bytes = KrPlan<DIM>::kTotal;                         \
+        if ((rc = set_smem(decode_keyrows_kernel<TYPE, DIM, OUT>, bytes))) return rc; \
+        launch_dependent(decode_keyrows_kernel<TYPE, DIM, OUT>, wave_of(sm_count), kKrThreads, bytes, stream, 1, tq, gk, gv, p); \
+        break;                                                                \
+      }                                                                       \
       auto* kernel = p.inline_plan ? decode_umma_kernel<TYPE, DIM, OUT, true> \
                                    : decode_umma_kernel<TYPE, DIM, OUT, false>; \
       if ((rc = set_smem(kernel, smem))) return rc;                           \
@@ -2786,11 +2852,7 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
     // tensor maps over K and V: (D, heads, tokens), one box = 64 elements x 1 head x box_rows keys
     CUtensorMap tk, tv;
     int rc = 0;
-    int box = kTileN;
-    if (a.layout == B200ATTN_PAGED) {
-      box = 1;
-      while (box < kTileN && (a.page_size % (box * 2)) == 0) box *= 2;
-    }
+    const int box = page_box(a);
     p.box_shift = 0;
     while ((1 << p.box_shift) < box) ++p.box_shift;
     if (a.layout == B200ATTN_DENSE) {

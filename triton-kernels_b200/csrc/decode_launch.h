@@ -55,6 +55,7 @@ struct DecodeParams {
   int item_overhead; // start-up and merge of a work item, in keys of streaming time (planner's cost estimate)
   int min_chunk;
   int max_items;
+  int one_cta;       // the persistent kernel has one CTA to an SM: see the planner's estimates
   int slots;         // persistent kernel: CTAs per KV head that the planner may deal the batch out to; 0: none
   int inline_plan;   // not 0: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs); the bits of a merge ticket
   int cluster;       // CTAs that share a (sequence, KV head) pair in the kernels without a plan; 0: items are planned

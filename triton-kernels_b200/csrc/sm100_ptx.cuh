@@ -35,6 +35,19 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
   return ok;
 }
 
+// whether the phase has completed, without waiting
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait: returns false when the phase has not completed after `limit` tries.  The loop lives in one asm
 // block - a completed phase costs the caller two instructions, which matters for a warp that has to share its issue
 // slots with busy neighbours - and every failed try suspends the thread in hardware for up to a microsecond or so,
@@ -120,6 +133,20 @@ __device__ __forceinline__ void grid_dep_launch_dependents() { asm volatile("gri
 __device__ __forceinline__ void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(ptr)); }
 __device__ __forceinline__ void named_bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void named_bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory"); }
+
+// meets the other threads of barrier `id` and tells whether any of them said yes
+__device__ __forceinline__ bool named_bar_any(int id, int count, bool mine) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.or.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(id), "r"(count), "r"(static_cast<uint32_t>(mine))
+      : "memory");
+  return r != 0;
+}
 
 // ------------------------------ proxies / fences ----------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -288,6 +315,13 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+// 8 columns, asynchronously (two of them may share a tmem_wait_ld_regs)
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -341,12 +375,12 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
 }
 
 // Instruction descriptor for kind::f16 (fp16/bf16 inputs, fp32 accumulate).
-//   ab_format: 0 = fp16, 1 = bf16;  b_mn_major: B operand is MN-major (N contiguous)
-__host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, int ab_format, int b_mn_major) {
+//   ab_format: 0 = fp16, 1 = bf16;  b_mn_major: B operand is MN-major (N contiguous); a_mn_major: A likewise
+__host__ __device__ constexpr uint32_t make_idesc_f16(int M, int N, int ab_format, int b_mn_major, int a_mn_major = 0) {
   return (1u << 4)                                     // accumulator format: fp32
          | (static_cast<uint32_t>(ab_format) << 7)     // A format
          | (static_cast<uint32_t>(ab_format) << 10)    // B format
-         | (0u << 15)                                  // A K-major (or TMEM)
+         | (static_cast<uint32_t>(a_mn_major) << 15)   // A major (K-major, or TMEM: 0)
          | (static_cast<uint32_t>(b_mn_major) << 16)   // B major
          | (static_cast<uint32_t>(N >> 3) << 17)
          | (static_cast<uint32_t>(M >> 4) << 24);
@@ -467,6 +501,54 @@ __device__ __forceinline__ void mma_ts_batch4(uint32_t d_tmem, uint32_t a_tmem, 
       "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead) : "memory");
 }
 #undef B200ATTN_TSK_STEP
+
+#define B200ATTN_KR_STEP(A, AOFF, B, BOFF)                                                      \
+  "add.s64 a1, " A ", " AOFF ";\n\tadd.s64 b1, " B ", " BOFF ";\n\t"                            \
+  "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
+
+// S^T = K Q^T, KSTEPS k-steps of 16 elements: A is a K-major tile of 128 keys, B the K-major q rows; the second 64 elements of a
+// row start at `a_block` and at 8 KiB (units of 16 bytes).
+template <int KSTEPS>
+__device__ __forceinline__ void mma_keys_by_rows(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint64_t a_block,
+                                                 uint32_t lead) {
+  static_assert(KSTEPS == 4 || KSTEPS == 8, "head dimension 64 or 128");
+  asm volatile(
+      "{\n\t.reg .pred p, t, e;\n\t.reg .b64 a1, b1;\n\t"
+      "setp.ne.b32 p, 0, 0;\n\tsetp.eq.b32 t, 0, 0;\n\tsetp.ne.b32 e, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      B200ATTN_KR_STEP("%1", "2", "%2", "2") B200ATTN_KR_STEP("%1", "4", "%2", "4") B200ATTN_KR_STEP("%1", "6", "%2", "6")
+      "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(lead) : "memory");
+  if constexpr (KSTEPS == 8) {
+    asm volatile(
+        "{\n\t.reg .pred t, e;\n\t.reg .b64 a1, b1;\n\t"
+        "setp.eq.b32 t, 0, 0;\n\tsetp.ne.b32 e, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, t;\n\t"
+        B200ATTN_KR_STEP("%1", "2", "%2", "2") B200ATTN_KR_STEP("%1", "4", "%2", "4") B200ATTN_KR_STEP("%1", "6", "%2", "6")
+        "}\n" ::"r"(d_tmem), "l"(a_desc + a_block), "l"(b_desc + 512), "r"(idesc), "r"(lead) : "memory");
+  }
+}
+// O^T += V^T P^T, `steps` k-steps of sixteen keys, at most eight: A is an MN-major V tile, `a_step` (units of 16 bytes) from 16 keys to the
+// next; B is P as MN-major rows of 128 bytes, a key each.
+__device__ __forceinline__ void mma_values_by_weights(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint64_t a_step,
+                                                      uint32_t accumulate_first, int steps, uint32_t lead) {
+  if (steps == 8) {
+    asm volatile(
+        "{\n\t.reg .pred p, t, e;\n\t.reg .b64 a1, b1;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        B200ATTN_KR_STEP("%1", "%6", "%2", "128") B200ATTN_KR_STEP("a1", "%6", "%2", "256") B200ATTN_KR_STEP("a1", "%6", "%2", "384")
+        B200ATTN_KR_STEP("a1", "%6", "%2", "512") B200ATTN_KR_STEP("a1", "%6", "%2", "640") B200ATTN_KR_STEP("a1", "%6", "%2", "768")
+        B200ATTN_KR_STEP("a1", "%6", "%2", "896")
+        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate_first), "r"(lead), "l"(a_step) : "memory");
+  } else {
+    for (int i = 0; i < steps; ++i)
+      asm volatile(
+          "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+          ::"r"(d_tmem), "l"(a_desc + i * a_step), "l"(b_desc + i * 128), "r"(idesc), "r"(i > 0 ? 1u : accumulate_first), "r"(lead) : "memory");
+  }
+}
+#undef B200ATTN_KR_STEP
 
 // tcgen05.commit issued by the lane whose `lead` is non-zero (warp converged)
 __device__ __forceinline__ void mma_commit_lead(uint32_t bar, uint32_t lead) {

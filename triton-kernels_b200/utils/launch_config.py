@@ -29,6 +29,7 @@ class DecodePlan:
     wave_items: int = 0      # items of one KV head resident at once (one wave); 0: a single wave is never planned
     item_overhead: int = 0   # start-up + merge of an item in keys of streaming time (the planner's cost estimate)
     slots: int = 0           # CTAs per KV head of the persistent kernel that a batch may be dealt out to
+    one_cta: bool = False    # that kernel has one CTA to an SM, not two
 
 
 def decode_pass_group(group: int, q_len: int) -> int:
@@ -67,10 +68,21 @@ def tcgen05_plans_itself(sm_count: int, batch: int, kv_heads: int, keys: int) ->
     return batch * kv_heads <= 96 and keys * kv_heads <= (1024 - 8 * batch) * 2 * sm_count
 
 
+def keyrows_suit(sm_count: int, batch: int, kv_heads: int, rows: int, keys: int, head_dim: int, page_size: Optional[int] = None) -> bool:
+    """Whether a call of 16-bit elements behind the planner goes to the kernel whose tiles have keys as their rows (csrc/decode.cu
+    keyrows_suit); ``keys`` as in ``tcgen05_plans_itself``, ``page_size`` for paged caches."""
+    if not 16 < rows <= 64 or (page_size is not None and page_size % 8):
+        return False
+    line = (512 << 7) // head_dim * (1 if batch * kv_heads <= sm_count else 2) * (2 if page_size is not None else 1) // 2
+    return keys >= line * batch
+
+
 def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: int, fp32: bool = False,
-                keys: Optional[int] = None) -> DecodePlan:
+                keys: Optional[int] = None, head_dim: int = 64, page_size: Optional[int] = None) -> DecodePlan:
     """``keys`` (see ``tcgen05_plans_itself``): with it, calls of the tcgen05 kernel that plan for themselves are planned as they do,
-    without dealing the batch out, and up to three short sequences in items for one CTA an SM; without it all are the planner's."""
+    without dealing the batch out, and up to three short sequences in items for one CTA an SM, and calls of the kernel with keys as rows
+    (``keyrows_suit``, which ``head_dim`` and ``page_size`` are for) as for that; without it all are the planner's, for the tcgen05 kernel
+    with two CTAs an SM."""
     group = decode_pass_group(q_heads // kv_heads, q_len)
     rows = group * q_len
     # fp32 inputs of a speculative-decode call (several q rows per head) run the tensor-core kernels on fp16 copies
@@ -90,6 +102,9 @@ def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: i
         slots = 0
         if batch <= 3 and keys * kv_heads <= 6 * min_chunk * sm_count:
             target, wave = max(1, sm_count // kv_heads), 0
+    elif wide and keys is not None and keyrows_suit(sm_count, batch, kv_heads, rows, keys, head_dim, page_size):
+        slots, target, wave = sm_count // kv_heads, max(1, 3 * sm_count // kv_heads), max(1, sm_count // kv_heads)
+        return DecodePlan(target, min_chunk, max_items, tiles, slices, 32 * (tiles * slices + 1), wave, overhead, slots, True)
     return DecodePlan(target, min_chunk, max_items, tiles, slices, 32 * (tiles * slices + 1), wave, overhead, slots)
 
 
@@ -129,6 +144,8 @@ def _plan_lengths(plan: DecodePlan, lens: Sequence[int]):
         w_chunk, _, w_biggest, found = _pick_chunk(plan, lens, plan.wave_items)
         if found and w_biggest + plan.item_overhead < best:
             best, chunk = w_biggest + plan.item_overhead, w_chunk
+    if plan.one_cta:
+        best = 0.89 * min(best, -(-items // plan.wave_items) * (chunk + plan.item_overhead)) - 500
     line = total + (len(lens) + plan.slots - 1) * plan.item_overhead
     dealt = (1 < plan.slots <= 512 and len(lens) <= 4096 and line < 1 << 30 and items > plan.wave_items
              and line / plan.slots + plan.min_chunk < best)
