@@ -385,6 +385,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (lane == 0) { prefetch_tensormap(&tm_q); prefetch_tensormap(&tm_k); prefetch_tensormap(&tm_v); }
     // the first item of a CTA is its own index (the grid never exceeds the item count); later ones are drawn
     ItemWork w = locate_item<kParts>(p, static_cast<int>(blockIdx.x));
+    // The first tiles of a dense item start for L2 here, while this CTA waits for the launches in front: where they lie follows from the
+    // arguments alone, and bringing lines into L2 reads nothing that a later write would not replace there.  (3 x 522 causal tokens, 32/8
+    // heads, 18.5 -> 18.3 us, 16 x 600 92.8 -> 92.0.)
+    if (!kPaged && p.layout == B200ATTN_DENSE && lane == 0) {
+      const int kv_row = static_cast<int>(w.kv_row0);
+      tma_prefetch_4d(&tm_q, 0, static_cast<int>(w.q_row0[0] + w.m0[0]), 0, w.q_head_coord[0]);
+      tma_prefetch_4d(&tm_k, 0, kv_row, 0, w.kv_head_coord);
+      tma_prefetch_4d(&tm_q, 0, static_cast<int>(w.q_row0[1] + w.m0[1]), 0, w.q_head_coord[1]);
+      tma_prefetch_4d(&tm_v, 0, kv_row, 0, w.kv_head_coord);
+    }
     // everything the other warps read or write outside this CTA follows an item published or a tile loaded below
     ptx::grid_dep_wait();
     bool ok = true;

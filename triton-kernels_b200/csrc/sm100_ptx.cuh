@@ -121,6 +121,11 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
+// brings `bytes` (a multiple of 16) at a 16-byte aligned address into L2
+__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(reinterpret_cast<uint64_t>(src)), "r"(bytes) : "memory");
+}
+
 // ------------------------------ programmatic dependent launch ----------------
 // A grid launched with programmatic stream serialisation may start while the grid before it in the stream is still
 // running; grid_dep_wait blocks until that grid has completed and its writes are visible (a no-op in a grid launched

@@ -479,6 +479,11 @@ softmax_pipe_kernel(const T* x, T* out, long long rows, long long cols, int stag
   if (tid == 0) {
     for (int i = 0; i < kPipeStages; ++i) ptx::mbar_init(smem_u32(&full[i]), 1);
     ptx::mbar_fence_init();
+    // The first row starts for L2 before the wait for the launches in front: where it lies is an argument, and bringing lines into L2 reads
+    // nothing that a later write would not replace there.  (Here and in the ring: 148 x 27 648 bf16 6.5 -> 4.5 us, 809 x 22 336 fp16 16.9
+    // -> 16.4, 8 000 x 20 000 fp32 227 -> 223, 2 450 x 81 603 285 -> 278.  In the kernels with a row in registers, whose later CTAs would do
+    // it too, 4 to 8 % slower.)
+    ptx::bulk_prefetch_l2(x + blockIdx.x * cols, static_cast<uint32_t>(n) * 16u);
   }
   __syncthreads();
   ptx::grid_dep_wait();
@@ -596,12 +601,17 @@ softmax_ring_kernel(const T* x, T* out, long long rows, long long cols, int slic
     }
     ptx::mbar_fence_init();
   }
-  if (csize > 1) cg::this_cluster().sync(); else __syncthreads();
-  ptx::grid_dep_wait();
-  ptx::grid_dep_launch_dependents();
   const long long row_step = gridDim.x / csize, r0 = blockIdx.x / csize;
   const int first = slice * rank;                          // this CTA's pieces of every row: first .. first + slice - 1
   auto my_pieces = [&](const RowSplit& sp) { return max(0, min(slice, sp.nv - first)); };
+  if (tid == 0) {
+    const RowSplit sp = split_row(x + r0 * cols, cols);
+    const int n = min(my_pieces(sp), kRingSlots * kRingChunk);
+    if (n > 0) ptx::bulk_prefetch_l2(reinterpret_cast<const uint4*>(x + r0 * cols + sp.head) + first, static_cast<uint32_t>(n) * 16u);
+  }
+  if (csize > 1) cg::this_cluster().sync(); else __syncthreads();
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch_dependents();
 
   if (warp == kRingWarps) {
     // ------------------------------ producer ------------------------------
