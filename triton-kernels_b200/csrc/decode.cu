@@ -50,6 +50,7 @@ constexpr int kMaxStages = 4;
 constexpr int kPlanThreads = 1024;
 constexpr int kPlanBuckets = 32;    // size classes of the execution order (longest items first)
 constexpr int kPlanLenCache = 4096; // sequences whose lengths the planner keeps in shared memory
+constexpr int kGroupedChunks = 20;  // chunks of a pair from which they are merged in two steps
 constexpr int kPlanMaxSlots = 512;  // slots of the persistent kernel that the planner deals out
 
 struct SeqInfo {
@@ -93,39 +94,50 @@ __device__ __forceinline__ void poison_rows(float* comb_o, float* comb_ml, int r
 }
 
 // ---------------------------------------------------------------------------
-// Merge of the n_chunks published partials of one (sequence, kv head) into its output rows, by the `nt` threads
+// Merge of published partials of one (sequence, kv head), into its output rows or into one partial, by the `nt` threads
 // t = 0 .. nt-1 of the CTA that drew the last ticket: g = max m; O = sum 2^(m-g) acc / sum 2^(m-g) l
-// (kernels/decode.py:186-197).  Leaves the ticket counter at zero for the next call.
+// (kernels/decode.py:186-197).
 // ---------------------------------------------------------------------------
-// Where the header holds a pair's ticket in a call without a planner launch.
-struct TicketPlace { unsigned* word; int shift; };
-__device__ __forceinline__ TicketPlace ticket_place(const DecodeParams& p, int pair) {
+// Where the header holds a pair's tickets in a call without a planner launch (`i`: 0, or 1 + the group of chunks).  (In the library's own
+// array the planner, which runs in every call there, puts them at zero.)
+struct TicketPlace { unsigned* word; int shift, bits; };
+__device__ __forceinline__ TicketPlace ticket_place(const DecodeParams& p, int pair, int i) {
+  unsigned* const words = reinterpret_cast<unsigned*>(p.header) + kTicketWord;
+  if (p.pair_tickets) {
+    const int at = pair * p.pair_tickets + i;
+    return {words + (at >> 2), (at & 3) * 8, 8};
+  }
   const int log_per_word = p.inline_plan == 8 ? 2 : 1;
-  return {reinterpret_cast<unsigned*>(p.header) + kTicketWord + (pair >> log_per_word), (pair & ((1 << log_per_word) - 1)) * p.inline_plan};
+  return {words + (pair >> log_per_word), (pair & ((1 << log_per_word) - 1)) * p.inline_plan, p.inline_plan};
 }
 // Draws the next merge ticket of a (sequence, kv head) pair.
-__device__ __forceinline__ int draw_ticket(const DecodeParams& p, int pair) {
-  if (!p.inline_plan) return atomicAdd(p.counters + pair, 1);
-  const TicketPlace t = ticket_place(p, pair);
-  return (atomicAdd(t.word, 1u << t.shift) >> t.shift) & ((1u << p.inline_plan) - 1);
+__device__ __forceinline__ int draw_ticket(const DecodeParams& p, int pair, int i = 0) {
+  if (!p.inline_plan && !p.pair_tickets) return atomicAdd(p.counters + pair, 1);
+  const TicketPlace t = ticket_place(p, pair, i);
+  return (atomicAdd(t.word, 1u << t.shift) >> t.shift) & ((1u << t.bits) - 1);
 }
 // Leaves the pair's ticket counter at zero for the next call; `n` tickets were drawn.
-__device__ __forceinline__ void reset_ticket(const DecodeParams& p, int pair, int n) {
-  if (!p.inline_plan) p.counters[pair] = 0;
-  else { const TicketPlace t = ticket_place(p, pair); atomicSub(t.word, static_cast<unsigned>(n) << t.shift); }
+__device__ __forceinline__ void reset_ticket(const DecodeParams& p, int pair, int n, int i = 0) {
+  if (!p.inline_plan && !p.pair_tickets) p.counters[pair] = 0;
+  else { const TicketPlace t = ticket_place(p, pair, i); atomicSub(t.word, static_cast<unsigned>(n) << t.shift); }
+}
+// Chunks of a group where a pair's chunks are merged in two steps, 0 where they are not (see publish_and_merge).
+__device__ __forceinline__ int merge_group(const DecodeParams& p, int n_chunks) {
+  if (!p.pair_tickets || n_chunks < kGroupedChunks) return 0;
+  const int groups = min(p.pair_tickets - 1, __float2int_rn(sqrtf(static_cast<float>(n_chunks))));
+  return (n_chunks + groups - 1) / groups;
 }
 
-template <typename T, int D>
-__device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h, int n_chunks, int item0, T* out,
-                                             int t, int nt) {
-  constexpr int D4 = D / 4;
+// The partials are in the slots slot0, slot0 + step, ...  `s_ml` not null: their merge goes to the first of them (shared memory for two
+// floats per row; every thread of the CTA takes part then), else to `out`.
+//
+// One pass with a running maximum, E output elements and 8 / E chunks per step: the loads of a step do not depend on each other or on
+// the running state, so they are in flight together (the merge is a chain of L2 round trips otherwise).  With eight chunks of one element
+// everywhere the kernels of many rows spill (40 rows, 8 x 2 500 keys 26.8 -> 29.4 us).
+template <typename T, int D, int E>
+__device__ __forceinline__ void merge_elements(const DecodeParams& p, long long slot0, int step, int n_chunks, T* out, int t, int nt, float* s_ml) {
+  constexpr int D4 = D / 4, CH = 8 / E;
   const int R = p.rows;
-  __threadfence();
-  // One pass with a running maximum, two output elements and four chunks per step: the 24 loads of a step do not
-  // depend on each other or on the running state, so they are in flight together (the merge is a chain of L2 round
-  // trips otherwise).
-  constexpr int E = 2;
-  const long long slot0 = static_cast<long long>(item0) * p.kv_heads + h;   // chunk k lives in slot0 + k * kv_heads
   const int total = R * D4;
   for (int idx0 = t; idx0 < total; idx0 += nt * E) {
     int r[E], d4[E];
@@ -143,15 +155,15 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h
       l[e] = 0.f;
       acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (int k0 = 0; k0 < n_chunks; k0 += 4) {
-      float mk[E][4], lk[E][4];
-      float4 o[E][4];
+    for (int k0 = 0; k0 < n_chunks; k0 += CH) {
+      float mk[E][CH], lk[E][CH];
+      float4 o[E][CH];
 #pragma unroll
       for (int e = 0; e < E; ++e) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < CH; ++j) {
           const bool on = k0 + j < n_chunks;
-          const long long s = slot0 + static_cast<long long>(on ? k0 + j : k0) * p.kv_heads;
+          const long long s = slot0 + static_cast<long long>(on ? k0 + j : k0) * step;
           const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (s * R + r[e]) * 2));
           o[e][j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + (s * R + r[e]) * D + d4[e] * 4));
           mk[e][j] = on ? ml.x : -INFINITY;
@@ -160,12 +172,14 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h
       }
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const float mn = fmaxf(fmaxf(mg[e], fmaxf(mk[e][0], mk[e][1])), fmaxf(mk[e][2], mk[e][3]));
+        float mn = mg[e];
+#pragma unroll
+        for (int j = 0; j < CH; ++j) mn = fmaxf(mn, mk[e][j]);
         const float keep = (mg[e] == -INFINITY) ? 0.f : fast_exp2(mg[e] - mn);
         acc[e].x *= keep; acc[e].y *= keep; acc[e].z *= keep; acc[e].w *= keep;
         l[e] *= keep;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < CH; ++j) {
           const float w = (mk[e][j] == -INFINITY) ? 0.f : fast_exp2(mk[e][j] - mn);
           acc[e].x += w * o[e][j].x; acc[e].y += w * o[e][j].y; acc[e].z += w * o[e][j].z; acc[e].w += w * o[e][j].w;
           l[e] += w * lk[e][j];
@@ -176,6 +190,12 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       if (!live[e]) continue;
+      if (s_ml) {
+        // (this thread alone has read and writes these four elements)
+        *reinterpret_cast<float4*>(p.part_o + (slot0 * R + r[e]) * D + d4[e] * 4) = acc[e];
+        if (d4[e] == 0) { s_ml[2 * r[e]] = mg[e]; s_ml[2 * r[e] + 1] = l[e]; }
+        continue;
+      }
       const float inv = l[e] > 0.f ? 1.f / l[e] : 0.f;
       T* dst = out + static_cast<long long>(r[e]) * D + d4[e] * 4;
       if constexpr (sizeof(T) == 2) {
@@ -188,7 +208,52 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h
       }
     }
   }
-  if (t == 0) reset_ticket(p, b * p.kv_heads + h, n_chunks);
+}
+// kFew: the kernel may have so few rows that a thread has one element; it then takes eight chunks at a time (55 chunks of one sequence
+// of 8 000 keys, 32/8 heads, 20.8 -> 19.7 us).
+template <typename T, int D, bool kFew>
+__device__ __forceinline__ void merge_chunks(const DecodeParams& p, long long slot0, int step, int n_chunks, T* out, int t, int nt, float* s_ml) {
+  __threadfence();
+  if (kFew && p.rows * (D / 4) <= nt) merge_elements<T, D, 1>(p, slot0, step, n_chunks, out, t, nt, s_ml);
+  else merge_elements<T, D, 2>(p, slot0, step, n_chunks, out, t, nt, s_ml);
+  if (s_ml) {
+    __syncthreads();                 // (every thread has read the references and sums that are written over)
+    for (int i = t; i < 2 * p.rows; i += nt) p.part_ml[slot0 * p.rows * 2 + i] = s_ml[i];
+  }
+}
+
+// Publishes chunk c of a pair, whose partial this CTA's threads have written, by a ticket; the last arrival merges (nobody waits).
+// A merge is one CTA's chain of L2 round trips, four chunks each, so that one long sequence alone was mostly that: its chunks are merged
+// in groups, about as many as a group has chunks, each by the last of its CTAs to arrive, and the groups by the last of those.
+// One sequence of 30 000 keys, us: 8/1 heads (235 chunks) 44.6 -> 19.9, 32/8 heads 37.1 -> 32.8; 6 of 30 271, 8/1 heads, 35.7 -> 30.9; 6 of
+// 6 607 to 26 430, 40 rows of one head 59.2 -> 33.6.  Below twenty chunks (kGroupedChunks) the second ticket costs what the shorter chains
+// save (18 chunks 38.1 us and 38.7; 11 27.4 and 28.2).  `s_word`, `s_ml` (two floats per row): shared memory.
+template <typename T, int D, bool kFew>
+__device__ __forceinline__ void publish_and_merge(const DecodeParams& p, int b, int h, int c, int n_chunks, int item0, T* out, int* s_word,
+                                                  float* s_ml) {
+  const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x), pair = b * p.kv_heads + h;
+  const long long slot0 = static_cast<long long>(item0) * p.kv_heads + h;   // chunk k lives in slot0 + k * kv_heads
+  __threadfence();
+  __syncthreads();
+  const int group = merge_group(p, n_chunks);
+  int n = n_chunks, step = p.kv_heads;
+  if (group > 0) {
+    const int g = c / group, size = min(group, n_chunks - g * group);
+    if (t == 0) *s_word = draw_ticket(p, pair, 1 + g);
+    __syncthreads();
+    if (*s_word != size - 1) return;
+    merge_chunks<T, D, kFew>(p, slot0 + static_cast<long long>(g * group) * step, step, size, out, t, nt, s_ml);
+    if (t == 0) reset_ticket(p, pair, size, 1 + g);
+    __threadfence();
+    __syncthreads();
+    n = (n_chunks + group - 1) / group;
+    step *= group;
+  }
+  if (t == 0) *s_word = draw_ticket(p, pair);
+  __syncthreads();
+  if (*s_word != n - 1) return;
+  merge_chunks<T, D, kFew>(p, slot0, step, n, out, t, nt, nullptr);
+  if (t == 0) reset_ticket(p, pair, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -198,7 +263,7 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, int b, int h
 // ---------------------------------------------------------------------------
 template <typename T, int D>
 __device__ __forceinline__ void emit_and_merge(const DecodeParams& p, int b, int h, int c, int n_chunks,
-                                               int item0, const float* comb_o, const float* comb_ml,
+                                               int item0, const float* comb_o, float* comb_ml,
                                                int KS, int rows_pad, int* s_ticket) {
   constexpr int D4 = D / 4;
   const int R = p.rows;
@@ -239,13 +304,7 @@ __device__ __forceinline__ void emit_and_merge(const DecodeParams& p, int b, int
   }
   if (n_chunks == 1) return;
 
-  // publish the partial, draw a ticket; the last arrival merges (nobody waits)
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) *s_ticket = draw_ticket(p, b * p.kv_heads + h);
-  __syncthreads();
-  if (*s_ticket != n_chunks - 1) return;
-  merge_chunks<T, D>(p, b, h, n_chunks, item0, out, threadIdx.x, blockDim.x);
+  publish_and_merge<T, D, true>(p, b, h, c, n_chunks, item0, out, s_ticket, comb_ml);
 }
 
 // ---------------------------------------------------------------------------
@@ -539,6 +598,7 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     }
   }
   for (int i = tid; i < p.batch * p.kv_heads; i += kPlanThreads) p.counters[i] = 0;
+  if (p.pair_tickets && tid < 64 - kTicketWord) p.header[kTicketWord + tid] = 0;      // (the library's own array)
   __syncthreads();
   const int chunk = s_chunk;
 
@@ -1429,7 +1489,9 @@ __device__ __forceinline__ void claim_merges(const DecodeParams& p, Ctrl* ctrl, 
       const int item0 = p.item_start[b];
       OutT* out = static_cast<OutT*>(p.out) +
                   ((static_cast<long long>(b) * p.q_heads + static_cast<long long>(h) * p.head_stride + p.head0) * p.q_len) * D;
-      merge_chunks<OutT, D>(p, b, h, p.item_start[b + 1] - item0, item0, out, tid, static_cast<int>(blockDim.x));
+      const int n = p.item_start[b + 1] - item0;
+      merge_chunks<OutT, D, false>(p, static_cast<long long>(item0) * p.kv_heads + h, p.kv_heads, n, out, tid, static_cast<int>(blockDim.x), nullptr);
+      if (tid == 0) reset_ticket(p, pair, n);
     }
     __syncthreads();
   }
@@ -2126,15 +2188,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 2) decode_umma_kernel(const __gr
         for (int i = tid; i < R * D; i += blockDim.x) p.part_o[slot * R * D + i] = __int_as_float(0x7fc00000);
         for (int i = tid; i < R * 2; i += blockDim.x) p.part_ml[slot * R * 2 + i] = __int_as_float(0x7fc00000);
       }
-      __threadfence();
-      __syncthreads();
-      if (tid == 0) ctrl->ready = draw_ticket(p, w.b * p.kv_heads + w.h);
-      __syncthreads();
-      if (ctrl->ready == w.n_chunks - 1) {
-        OutT* out = static_cast<OutT*>(p.out) +
-                    ((static_cast<long long>(w.b) * p.q_heads + static_cast<long long>(w.h) * p.head_stride + p.head0) * p.q_len) * D;
-        merge_chunks<OutT, D>(p, w.b, w.h, w.n_chunks, w.item0, out, tid, static_cast<int>(blockDim.x));
-      }
+      OutT* out = static_cast<OutT*>(p.out) +
+                  ((static_cast<long long>(w.b) * p.q_heads + static_cast<long long>(w.h) * p.head_stride + p.head0) * p.q_len) * D;
+      publish_and_merge<OutT, D, false>(p, w.b, w.h, w.c, w.n_chunks, w.item0, out, &ctrl->ready, reinterpret_cast<float*>(smem));
       return;
     }
   }
@@ -2723,6 +2779,12 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
   const Route route = route_of(a, sm_count, p.rows, built_in, /*ask=*/true);
   p.cluster = route.cluster;
   p.inline_plan = route.inline_plan;
+  // (a byte counts a group's chunks, and the chunks of a pair that is merged in one step)
+  constexpr int kTicketBytes = (64 - kTicketWord) * 4;
+  p.pair_tickets = 0;
+  // (in the library's own array such calls are planned, but merged alike)
+  if ((p.inline_plan || (built_in && (a.dtype == B200ATTN_F32 || p.rows <= 16))) && pairs > 0 && pairs <= kTicketBytes / 4 && w.max_items <= 255 * (kTicketBytes / pairs - 1))
+    p.pair_tickets = static_cast<int>(kTicketBytes / pairs);
   if (p.inline_plan && a.dtype != B200ATTN_F32 && p.rows > 16) {
     // The tcgen05 kernel, few sequences: items for one CTA an SM, not two, up to six of the shortest.  A second CTA on some of the SMs holds its neighbour up,
     // and a merge, one CTA's work, is as long as a sequence has items: 1 x 8 000 keys of eight heads, 40 rows, D 128, 35.8 -> 25.7

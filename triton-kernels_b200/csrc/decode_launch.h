@@ -58,6 +58,7 @@ struct DecodeParams {
   int one_cta;       // the persistent kernel has one CTA to an SM: see the planner's estimates
   int slots;         // persistent kernel: CTAs per KV head that the planner may deal the batch out to; 0: none
   int inline_plan;   // not 0: no planner launch, every CTA works out its own item (few (sequence, KV head) pairs); the bits of a merge ticket
+  int pair_tickets;  // such calls of few pairs, and those in the own array: header bytes of a pair, the first its merge ticket, the others those of groups of its chunks; else 0
   int cluster;       // CTAs that share a (sequence, KV head) pair in the kernels without a plan; 0: items are planned
   int stages;        // K/V stages of a CTA of the warp-level kernel in a cluster
   float scale_log2;  // sm_scale * log2(e)
