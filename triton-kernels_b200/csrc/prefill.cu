@@ -713,19 +713,23 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // shared memory, the next sequence, poisoned page tails): zero them so 0 * x stays 0
             unsigned char* vbuf = smem + Plan::kRingOff + (2 * (pr % kStages)) * Plan::kTileBytes;
             const int first = valid > 0 ? valid : 0;
-            const int n16 = (kBN - first) * 8;  // 16-byte pieces per column block
-            for (int c = 0; c < Plan::kChunks; ++c) {
-              if constexpr (kGroup == 1024) {
+            if constexpr (kGroup == 1024) {
+              const int n16 = (kBN - first) * 8;  // 16-byte pieces per column block
+              for (int c = 0; c < Plan::kChunks; ++c) {
                 // (written out for this case: with the indices of the other one, never run in a whole tile, 3 x 8 192 causal tokens,
                 // 32/8 heads, head_dim 64, took 1 120 us instead of 1 064)
                 uint4* dst = reinterpret_cast<uint4*>(vbuf + c * kBlock + first * 128);
                 for (int i = lane; i < n16; i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
-              } else {
-                for (int i = lane; i < n16; i += 32) {
-                  const int at = first * 8 + i;   // (eight pieces a row, 64 a group)
-                  *reinterpret_cast<uint4*>(vbuf + c * kBlock + (at >> 6) * kGroup + (at & 63) * 16) = make_uint4(0u, 0u, 0u, 0u);
-                }
               }
+            } else {
+              // the rest of a group, then whole groups, which lie one behind the other (piece by piece, with an index for each, 7 x 20 tokens
+              // took 8.8 us instead of 8.2)
+              for (int c = 0; c < Plan::kChunks; ++c) {
+                uint4* dst = reinterpret_cast<uint4*>(vbuf + c * kBlock + (first >> 3) * kGroup + (first & 7) * 128);
+                for (int i = lane; i < (-first & 7) * 8; i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
+              }
+              uint4* dst = reinterpret_cast<uint4*>(vbuf + ((first + 7) >> 3) * kGroup);
+              for (int i = lane; i < (kBN / 8 - ((first + 7) >> 3)) * (kGroup / 16); i += 32) dst[i] = make_uint4(0u, 0u, 0u, 0u);
             }
             fence_proxy_async_smem();
             __syncwarp();
