@@ -598,7 +598,6 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     }
   }
   for (int i = tid; i < p.batch * p.kv_heads; i += kPlanThreads) p.counters[i] = 0;
-  if (p.pair_tickets && tid < 64 - kTicketWord) p.header[kTicketWord + tid] = 0;      // (the library's own array)
   __syncthreads();
   const int chunk = s_chunk;
 
@@ -760,6 +759,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
     p.header[3] = 0;          // tickets drawn and not merged yet (tcgen05 kernel)
     p.header[4] = 0;          // units drawn beyond the CTAs' first ones (tcgen05 kernel)
     p.header[5] = 0;
+  } else if (p.pair_tickets && tid >= 64 && tid < 128 - kTicketWord) {
+    p.header[kTicketWord + tid - 64] = 0;      // (the library's own array)
   }
 }
 

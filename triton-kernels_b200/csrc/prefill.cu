@@ -121,8 +121,8 @@ struct SmemPlan {
 // K and V of pages: whether a box (a page's rows, up to a tile's) comes whole, by the 5-D map of make_kv_groups_map, instead of one
 // 64-column block at a time.  A box costs the producer a hundred cycles whatever it holds, and the sixteen copies of a tile of
 // 16-key pages at head_dim 128, twice a step, were as long as the step: causal, 4 x 2 048 tokens, 32/8 heads 166 -> 156 us, 2 x 4 096 289
-// -> 270, 4 x 252 11.8 -> 11.1; 128 queries over 2 048 keys 27.5 -> 26.4.  At head_dim 64 there is one block, and the 5-D copies
-// are slower than the 3-D ones (3 x 8 181 1 133 -> 1 160 us); so they are with boxes of less than a group (four keys 61 -> 66).
+// -> 270, 4 x 252 11.8 -> 11.1; 128 queries over 2 048 keys 27.5 -> 26.4.  At head_dim 64 there is one block, and nothing to
+// gain; boxes of less than a group would come in pieces (four keys 61 -> 66).
 __host__ __device__ constexpr bool group_boxes(int D, int box_rows) { return D > 64 && box_rows >= 8; }
 
 // The waits of a tile.  At head_dim 128 the first look is straight-line code (cycles per tile 1 807 -> 1 785); at 64 the softmax,
