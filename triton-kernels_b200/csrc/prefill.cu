@@ -388,7 +388,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // The first tiles of a dense item start for L2 here, while this CTA waits for the launches in front: where they lie follows from the
     // arguments alone, and bringing lines into L2 reads nothing that a later write would not replace there.  (3 x 522 causal tokens, 32/8
     // heads, 18.5 -> 18.3 us, 16 x 600 92.8 -> 92.0.)
-    if (!kPaged && p.layout == B200ATTN_DENSE && lane == 0) {
+    if (!kPaged && p.layout == B200ATTN_DENSE && p.max_kv > 0 && lane == 0) {
       const int kv_row = static_cast<int>(w.kv_row0);
       tma_prefetch_4d(&tm_q, 0, static_cast<int>(w.q_row0[0] + w.m0[0]), 0, w.q_head_coord[0]);
       tma_prefetch_4d(&tm_k, 0, kv_row, 0, w.kv_head_coord);
