@@ -77,7 +77,7 @@ LENS = [0, 1, 3, 15, 16, 17, 63, 64, 65, 111, 112, 113, 127, 128, 129, 143, 144,
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
 def test_lengths_and_pages(layout, page, d, causal):
-    lens = [n for n in LENS if n == 0 or n >= 3 or not causal] + [2600 + 7 * i for i in range(76)]
+    lens = [n for n in LENS if n == 0 or n >= 3 or not causal] + [(2600 if d == 128 else 5700) + 7 * i for i in range(78)]
     keys = sum(lens) if layout == "ragged" else len(lens) * -(-max(lens) // page) * page
     _takes_it(len(lens), 2, 24, keys, d, page)
     _run(layout, torch.bfloat16, 16, 2, 3, d, lens, causal, page=page or 16)

@@ -2734,14 +2734,17 @@ int page_box(const b200attn_decode_args_t& a) {
 // of 600 41.9, 41.5; of 1 000 59.4, 57.6; 200 of 400 82.7, 78.9; D 64, 64 of 700 32.6, 39.7; of 1 000 41.3, 48.0; of 1 200 60.2, 51.8; of
 // 2 400 90.3, 86.4), and half of that where no SM has more than one unit (16 of 250 at D 128, 20 rows 22.7, 16.0; 40 rows 15.4, 15.8).
 // Pages say how long a sequence can be; twice the line is asked for, which sequences of any length up to that reach on average.
+// And each SM needs 2 048 keys (D 64 4 096) where some have more than one unit: shorter calls end with a round that is mostly empty, or cut their
+// sequences for it (100 x 1 000 keys of two heads, 48 rows, 44.2 us, umma 30.5; 20 x 300 to 2 500 of eight 44.4, 41.5; 40 x 600 to 2 500 62.9, 68.8).
 // (Much shorter ones in such tables are slower for it: 64 of 20 keys in tables of 8 192 17.4, 23.0.  Both kernels launched, and the planner's
 // word for which of them stays, cost every call 4 to 6 us.)
 bool keyrows_suit(const b200attn_decode_args_t& a, int sm_count, int rows) {
   if (a.dtype == B200ATTN_F32 || rows <= 16 || rows > kKrMaxRows || !keyrows_boxes(page_box(a))) return false;
   if (inline_plan_bits(a, sm_count, rows)) return false;      // (also in the library's own array, where such a call is planned)
   const bool one_each = static_cast<long long>(a.batch) * a.kv_heads <= sm_count;
-  const long long line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * (a.layout == B200ATTN_PAGED ? 2 : 1) / 2;
-  return most_keys(a) >= line * a.batch;
+  const long long twice = a.layout == B200ATTN_PAGED ? 2 : 1, line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * twice / 2;
+  const long long keys = most_keys(a);
+  return keys >= line * a.batch && (one_each || keys * a.kv_heads * a.head_dim >= (2048ll << 7) * twice * sm_count);
 }
 
 // `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32

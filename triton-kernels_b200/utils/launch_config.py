@@ -73,8 +73,9 @@ def keyrows_suit(sm_count: int, batch: int, kv_heads: int, rows: int, keys: int,
     keyrows_suit); ``keys`` as in ``tcgen05_plans_itself``, ``page_size`` for paged caches."""
     if not 16 < rows <= 64 or (page_size is not None and page_size % 8):
         return False
-    line = (512 << 7) // head_dim * (1 if batch * kv_heads <= sm_count else 2) * (2 if page_size is not None else 1) // 2
-    return keys >= line * batch
+    one_each, twice = batch * kv_heads <= sm_count, 2 if page_size is not None else 1
+    line = (512 << 7) // head_dim * (1 if one_each else 2) * twice // 2
+    return keys >= line * batch and (one_each or keys * kv_heads * head_dim >= (2048 << 7) * twice * sm_count)
 
 
 def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: int, fp32: bool = False,
