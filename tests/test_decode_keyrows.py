@@ -36,24 +36,31 @@ def _reference(q, k, v, causal):
     return torch.softmax(s, -1).nan_to_num(0.0) @ vv
 
 
-def _run(layout, dtype, qh, kvh, m, d, lens, causal, page=16, seed=0):
+def _run(layout, dtype, qh, kvh, m, d, lens, causal, page=16, seed=0, width=0, again=0):
+    """`width`: keys that the tables have room for, where that is more than the longest sequence; `again`: further calls, of which the
+    same bits are expected."""
     g = torch.Generator(device="cuda").manual_seed(seed + qh + m)
     q = torch.randn((len(lens), qh, m, d), generator=g, device="cuda").to(dtype)
     ks, vs = ([torch.randn((n, kvh, d), generator=g, device="cuda").clamp(-5, 5).to(dtype) for n in lens] for _ in range(2))
     if layout == "dense":
         k, v = (torch.stack(x).transpose(1, 2).contiguous() for x in (ks, vs))
-        out = speculative_decode_attention(q, k, v, causal=causal)
+        call = lambda: speculative_decode_attention(q, k, v, causal=causal)
     elif layout == "ragged":
         # NaN behind the last sequence; a tile that ends in one sequence holds the next one's rows
         pad = torch.full((130, kvh, d), float("nan"), device="cuda", dtype=dtype)
         k, v = (torch.cat(x + [pad])[: sum(lens)] for x in (ks, vs))
-        out = speculative_decode_attention(q, k, v, causal=causal,
-                                           kv_indptr=torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda())
+        indptr = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
+        call = lambda: speculative_decode_attention(q, k, v, causal=causal, kv_indptr=indptr)
     else:
         kc, kt, ln = sdpa_ref.pack_paged(ks, page, permute_seed=1, extra_pages=2, pad_value=-1, poison=float("nan"))
         vc, vt, _ = sdpa_ref.pack_paged(vs, page, permute_seed=2, extra_pages=2, pad_value=-1, poison=float("nan"))
-        out = speculative_decode_attention(q, kc, vc, causal=causal, kv_indptr=ln.cuda(), k_block_table=kt.cuda(),
-                                           v_block_table=vt.cuda(), kv_page_size=page)
+        kt, vt = (torch.nn.functional.pad(t, (0, max(0, width // page - t.shape[1])), value=-1).cuda() for t in (kt, vt))
+        ln = ln.cuda()
+        call = lambda: speculative_decode_attention(q, kc, vc, causal=causal, kv_indptr=ln, k_block_table=kt, v_block_table=vt,
+                                                    kv_page_size=page)
+    out = call()
+    for _ in range(again):
+        assert torch.equal(call(), out)
     assert torch.isfinite(out).all()
     for i, n in enumerate(lens):
         ref = _reference(q[i], ks[i], vs[i], causal)
@@ -89,6 +96,52 @@ def test_long_sequences_are_cut_and_merged(dtype, layout):
     lens = [20000] * 13 if layout == "dense" else [3, 70000, 128, 9000, 33333, 20001, 64, 15000, 500, 40000, 7, 25000, 1]
     _takes_it(13, 8, 40, sum(lens), 128, 16 if layout == "paged" else None)
     _run(layout, dtype, 64, 8, 5, 128, lens, causal=False, seed=1)
+
+
+def _with_empty(batch, empty, order, length):
+    """Lengths of `batch` sequences, `empty` tenths of them zero, in runs or scattered; the others length(i)."""
+    blank = [i % 10 < empty for i in range(batch)]
+    if order == "scattered":
+        blank = [blank[p] for p in torch.randperm(batch, generator=torch.Generator().manual_seed(empty)).tolist()]
+    return [0 if b else length(i) for i, b in enumerate(blank)]
+
+
+def _run_with_empty(lens, kvh, d, dealt, page=None, width=0):
+    from kernels._native import check_device_errors
+    from utils.launch_config import decode_cuts, decode_plan
+
+    keys = sum(lens) if page is None else len(lens) * width
+    _takes_it(len(lens), kvh, 24, keys, d, page)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    plan = decode_plan(sms, len(lens), 8 * kvh, kvh, 3, keys=keys, head_dim=d, page_size=page)
+    assert (decode_cuts(plan, lens) is not None) == dealt
+    _run("ragged" if page is None else "paged", torch.bfloat16, 8 * kvh, kvh, 3, d, lens, causal=False, width=width, again=20)
+    check_device_errors()
+
+
+# what the sequences with keys are, in tables of 16 384: several tiles, one tile, mostly one tile and a few that are cut
+KEYS = {"long": [700, 1300, 640], "one tile": [20, 128, 100, 7], "cut": [30, 9000, 100, 64, 128]}
+
+
+@pytest.mark.parametrize("empty", [3, 6, 9])
+@pytest.mark.parametrize("order", ["runs", "scattered"])
+@pytest.mark.parametrize("kind", ["long", "one tile", "cut", "packed"])
+@pytest.mark.parametrize("kvh,d", [(1, 128), (2, 64), (8, 128)])
+def test_empty_sequences(empty, order, kind, kvh, d):
+    """Longest-first order hands the units of sequences without keys out behind all others, `kvh` for each."""
+    batch, lengths = 320 // kvh, KEYS["cut" if kind == "packed" else kind]
+    lens = _with_empty(batch, empty, order, lambda i: lengths[i // 3 % len(lengths)])
+    if kind == "packed":       # as many keys as the call needs to go there, most of them in the last sequence
+        lens[-1] += max(0, 1100 * 128 // d * batch - sum(lens))
+    _run_with_empty(lens, kvh, d, False, *(() if kind == "packed" else (16, 16384)))
+
+
+@pytest.mark.parametrize("order", ["runs", "scattered"])
+@pytest.mark.parametrize("kvh,d,empty", [(1, 128, 6), (2, 64, 3), (2, 64, 6), (8, 128, 3)])
+def test_empty_sequences_dealt_out(kvh, d, empty, order):
+    """A CTA's units are those of its stretch of the batch: a run of empty sequences comes one behind the other."""
+    lens = _with_empty(60 // kvh + 20, empty, order, lambda i: 1000 + i * 7919 % 33000)
+    _run_with_empty(lens, kvh, d, True)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])

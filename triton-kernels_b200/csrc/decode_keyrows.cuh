@@ -36,17 +36,24 @@ constexpr int kKrRingBytes = 160 * 1024;
 constexpr int kKrMaxSlots = 10;
 constexpr float kKrMaxWeight = 1024.0f;      // P fits 16 bits, and the reference lies at most ten powers of two below the maximum
 
+// A wait asks for a phase by its parity, so a barrier must not complete its next phase before all who wait for this one have seen
+// it.  Beside each: what keeps that (g: a tile of the CTA, r: a unit, those of an even and an odd number having barriers of their own).
 struct __align__(16) KrCtrl {
-  uint64_t full[kKrMaxSlots], empty[kKrMaxSlots];
-  uint64_t q_full[2], q_empty[2];
-  uint64_t s_full[2];     // MMA warp -> softmax warps (commit): scores of a tile
-  uint64_t p_ready;       // softmax warps -> MMA warp: P of a tile
-  uint64_t o_done[2];     // (commit): a unit's last
-  uint64_t o_free[2];     // output warps: the accumulator and the sums have been read
-  uint64_t l_ready[2];    // softmax warps -> output warps: a unit's sums and references
+  uint64_t full[kKrMaxSlots];    // copies -> MMA warp: a tile.  The next one's copies wait for `empty`
+  // MMA warp -> copies, softmax warps (commit): a tile is consumed.  The next one here comes by copies that waited for this.  The softmax warps
+  // wait for V of g - 1 before P of g; the next tile in its slot, K of g + 3 at the earliest, is asked for behind P of g + 1
+  uint64_t empty[kKrMaxSlots];
+  uint64_t q_full[2];     // copies -> MMA warp: a unit's Q.  r + 2 waits for q_empty of r
+  uint64_t q_empty[2];    // MMA warp -> copies (commit, every unit).  r + 2 needs q_full of r + 2
+  uint64_t s_full[2];     // MMA warp -> softmax warps (commit): scores of a tile.  g + 2 is asked for after P of g
+  uint64_t p_ready;       // softmax warps -> MMA warp: P of a tile.  P of g + 1 waits for the product of g
+  uint64_t o_done[2];     // MMA warp -> output warps (commit): a unit's last, with or without keys.  r + 2 waits for o_free of r
+  uint64_t o_free[2];     // output warps -> MMA, softmax warps: the accumulator and the sums have been read.  r + 2 needs o_done and l_ready of r + 2
+  uint64_t l_ready[2];    // softmax warps -> output warps: a unit's sums and references.  r + 2 waits for o_free of r
   uint64_t rows_out;      // output warps: partial rows are written and fenced
-  uint64_t drained;
-  uint64_t may_draw[2];   // copies of K -> scheduler: the end of a unit (of that parity) is near
+  uint64_t drained;       // once
+  uint64_t may_draw[2];   // copies of K -> scheduler: the end of a unit (of that parity) is near.  Units behind r are published after the wait in r
+  // scheduler -> all others, and back: a unit's record.  r + 4 waits for all of them to be done with r
   uint64_t unit_full[kUmmaUnitRing], unit_empty[kUmmaUnitRing];
   UmmaUnit unit[kUmmaUnitRing];
   int unit_ring[kUmmaUnitRing];
@@ -423,7 +430,12 @@ __global__ void __launch_bounds__(kKrThreads, 1) decode_keyrows_kernel(const __g
         if (!ok) break;
       }
       ahead = false;
-      if (n == 0) mma_commit_lead(smem_u32(&ctrl->o_done[r & 1]), lead);
+      if (n == 0) {
+        // (like a unit with keys, whose first product waits for this: else o_done completes twice before its waiters have looked)
+        if (r >= 2) ok = warp_wait(smem_u32(&ctrl->o_free[r & 1]), ((r >> 1) - 1) & 1) && !*abort_flag;
+        if (!ok) break;
+        mma_commit_lead(smem_u32(&ctrl->o_done[r & 1]), lead);
+      }
       for (int tile = 0; tile < n && ok; ++tile, ++g) {
         const bool last = tile + 1 == n;
         bool good = true;
