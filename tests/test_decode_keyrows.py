@@ -144,6 +144,25 @@ def test_empty_sequences_dealt_out(kvh, d, empty, order):
     _run_with_empty(lens, kvh, d, True)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("heads,m", [(8, 3), (8, 5), (8, 8)])
+@pytest.mark.parametrize("kvh", [1, 2, 8])
+def test_short_ends_of_cut_sequences(kvh, heads, m, d):
+    """Every sequence is a chunk of the shortest and twenty keys.  Those ends come last, and a CTA finishes one after the other: a pair's
+    ticket may be drawn when all four output warps have written the unit's rows (at head_dim 64 two of them have none to write)."""
+    from kernels._native import check_device_errors
+    from utils.launch_config import decode_chunk_tokens, decode_cuts, decode_plan
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    batch, width = 3 * sms // kvh // 2, 16384
+    plan = decode_plan(sms, batch, heads * kvh, kvh, m, keys=batch * width, head_dim=d, page_size=16)
+    lens = [plan.min_chunk + 20] * batch
+    assert decode_cuts(plan, lens) is None and decode_chunk_tokens(plan, lens) == plan.min_chunk
+    _takes_it(batch, kvh, heads * m, batch * width, d, 16)
+    _run("paged", torch.bfloat16, heads * kvh, kvh, m, d, lens, causal=False, width=width, again=40)
+    check_device_errors()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
 @pytest.mark.parametrize("qh,kvh,m", [(16, 2, 5), (6, 2, 7), (32, 4, 8)])
 @pytest.mark.parametrize("step", [0, 2.9, 3.1, 9.9, 10.1, 16.5, 40])

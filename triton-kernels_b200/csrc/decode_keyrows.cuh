@@ -50,7 +50,7 @@ struct __align__(16) KrCtrl {
   uint64_t o_done[2];     // MMA warp -> output warps (commit): a unit's last, with or without keys.  r + 2 waits for o_free of r
   uint64_t o_free[2];     // output warps -> MMA, softmax warps: the accumulator and the sums have been read.  r + 2 needs o_done and l_ready of r + 2
   uint64_t l_ready[2];    // softmax warps -> output warps: a unit's sums and references.  r + 2 waits for o_free of r
-  uint64_t rows_out;      // output warps: partial rows are written and fenced
+  uint64_t rows_out;      // output warps, all of them on both sides: a cut unit's partial rows are written and fenced
   uint64_t drained;       // once
   uint64_t may_draw[2];   // copies of K -> scheduler: the end of a unit (of that parity) is near.  Units behind r are published after the wait in r
   // scheduler -> all others, and back: a unit's record.  r + 4 waits for all of them to be done with r
@@ -723,14 +723,14 @@ __global__ void __launch_bounds__(kKrThreads, 1) decode_keyrows_kernel(const __g
         __threadfence();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->rows_out));
-        if (quad == 0) {
-          ok = warp_wait(smem_u32(&ctrl->rows_out), merges & 1) && !*abort_flag;
-          if (!ok) break;
-          if (lane == 0) {
-            __threadfence();
-            atomicAdd(p.counters + w.b * p.kv_heads + w.h, 1);
-            atomicAdd(p.header + 3, 1);              // tickets drawn and not merged yet (a hint for the teardown)
-          }
+        // (all four warps: one that went on could arrive for its next unit in the place of one that still writes this unit's rows.  The
+        // accumulator and the sums are given back already, so nothing but these warps waits)
+        ok = warp_wait(smem_u32(&ctrl->rows_out), merges & 1) && !*abort_flag;
+        if (!ok) break;
+        if (quad == 0 && lane == 0) {
+          __threadfence();
+          atomicAdd(p.counters + w.b * p.kv_heads + w.h, 1);
+          atomicAdd(p.header + 3, 1);              // tickets drawn and not merged yet (a hint for the teardown)
         }
         ++merges;
       }
