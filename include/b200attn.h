@@ -241,6 +241,13 @@ int b200attn_selftest_wait_expiry(int device, void* workspace, uint32_t tries, v
 int b200attn_selftest_cluster_expiry(int device, void* workspace, float* out, uint32_t tries, int late, void* cuda_stream);
 
 /*
+ * Self-test of what a CTA of the persistent decode kernels leaves when it gives up after `published` (1..64) entries of its unit list,
+ * the last of them the end mark if `ended`: out (64 rows of 64 floats, device; unit r is row r) becomes NaN in the rows of all units
+ * that may be unfinished, which are those of the last four entries from `abort_round` on.  No counterpart in the reference.
+ */
+int b200attn_selftest_abandoned_units(int device, float* out, int published, int ended, int abort_round, void* cuda_stream);
+
+/*
  * Paged KV-cache append: copies the new rows of every sequence into the pages its block table names.
  *   src        [total_rows, heads, head_dim]  new K (or V) rows of all sequences, packed
  *   src_indptr [B+1] prefix sums over src rows;  dst_pos [B] position in each sequence of its first new row

@@ -74,3 +74,20 @@ def test_cluster_selftest_rejects_what_it_cannot_bound():
     w, o = C.c_void_p(ws.data_ptr()), C.c_void_p(out.data_ptr())
     for args in ((w, o, 0), (w, o, (1 << 14) + 1), (None, o, 16), (w, None, 16)):
         assert lib.b200attn_selftest_cluster_expiry(dev, *args, 1, stream) == -1
+
+
+@pytest.mark.parametrize("ended", [0, 1])
+@pytest.mark.parametrize("published", [1, 2, 4, 5, 6, 7, 8, 9, 13])
+@pytest.mark.parametrize("abort_round", [0, 3, 6, 1 << 30])
+def test_every_unfinished_unit_of_a_cta_that_gave_up_is_nan(published, ended, abort_round):
+    """A persistent decode CTA holds the last four entries of its list, the end mark among them; which of those units are finished
+    is known from `abort_round` on (0: of none)."""
+    from kernels import _native
+
+    out = torch.zeros((64, 64), device="cuda")
+    _native.check(_native.lib().b200attn_selftest_abandoned_units(torch.cuda.current_device(), C.c_void_p(out.data_ptr()), published, ended,
+                                                                  abort_round, C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                  "b200attn_selftest_abandoned_units")
+    want = torch.zeros(64, dtype=torch.bool)
+    want[max(0, published - 4, abort_round): published - ended] = True
+    assert torch.equal(torch.isnan(out).all(1).cpu(), want) and (out[~want.cuda()] == 0).all()

@@ -259,6 +259,17 @@ int b200attn_selftest_cluster_expiry(int device, void* workspace, float* out, ui
   return launch_cluster_selftest(static_cast<int*>(workspace), out, tries, late != 0, static_cast<cudaStream_t>(cuda_stream));
 }
 
+int b200attn_selftest_abandoned_units(int device, float* out, int published, int ended, int abort_round, void* cuda_stream) {
+  if (!out) { set_error("selftest: null pointer"); return B200ATTN_E_INVALID; }
+  if (published < 1 || published > 64 || abort_round < 0) { set_error("selftest: %d entries, abort round %d", published, abort_round); return B200ATTN_E_INVALID; }
+  b200attn_device_info_t info = {};
+  int rc;
+  if ((rc = check_arch(device, &info))) return rc;
+  DeviceGuard guard;
+  if ((rc = guard.enter(device))) return rc;
+  return launch_abandoned_units_selftest(out, published, ended, abort_round, static_cast<cudaStream_t>(cuda_stream));
+}
+
 int b200attn_paged_append(const b200attn_paged_append_args_t* a, void* cuda_stream) {
   if (!a) { set_error("args is null"); return B200ATTN_E_INVALID; }
   if (a->batch < 0 || a->total_rows < 0 || a->cache_rows < 0 || a->table_stride < 0 || a->page_size <= 0) { set_error("paged_append: negative extent or bad page size"); return B200ATTN_E_INVALID; }

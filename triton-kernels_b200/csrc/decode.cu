@@ -1504,8 +1504,9 @@ __device__ __forceinline__ void claim_merges(const DecodeParams& p, Ctrl* ctrl, 
 template <typename OutT, int D, typename Ctrl, typename UnitOf>
 __device__ __forceinline__ void poison_units(const DecodeParams& p, Ctrl* ctrl, int n_units, UnitOf unit_of) {
   const OutT nan_t = ElemTraits<OutT>::from_float(__int_as_float(0x7fc00000));
-  // (the slots of units that are not finished cannot have been reused by the producer)
-  for (int r = ctrl->abort_round; r < ctrl->published; ++r) {
+  // The slots of units that are not finished cannot have been reused, so those units are among the ring's: from its oldest on, where
+  // abort_round lies further back (0: nobody knows), and in their order, in which the end mark is the last.
+  for (int r = max(ctrl->abort_round, ctrl->published - kUmmaUnitRing); r < ctrl->published; ++r) {
     if (ctrl->unit_ring[r % kUmmaUnitRing] >= n_units) break;
     const UmmaUnit w = unit_of(r);
     OutT* out = static_cast<OutT*>(p.out) +
@@ -3080,6 +3081,31 @@ __global__ void __launch_bounds__(64) cluster_expiry_selftest_kernel(const Decod
   if (part.rank == 0 && threadIdx.x == 0) static_cast<float*>(p.out)[D] = ptx::mbar_try_wait(smem_u32(&recv_bar), 0) ? 1.f : 0.f;
 }
 }  // namespace
+
+// Self-test of what a CTA of the persistent kernels does when it gives up: `published` entries, the last of them the end mark if `ended`,
+// unit r being sequence r with one row of 64; the rows that its poison_units fills become NaN.
+namespace {
+__global__ void __launch_bounds__(64) abandoned_units_selftest_kernel(const DecodeParams p, int published, int ended, int abort_round) {
+  __shared__ UmmaCtrl ctrl;
+  const int n_units = published - (ended ? 1 : 0);
+  if (threadIdx.x == 0) {
+    for (int r = max(0, published - kUmmaUnitRing); r < published; ++r) ctrl.unit_ring[r % kUmmaUnitRing] = r;
+    ctrl.published = published;
+    ctrl.abort_round = abort_round;
+  }
+  __syncthreads();
+  poison_units<float, 64>(p, &ctrl, n_units, [&](int r) { UmmaUnit w = {}; w.b = ctrl.unit_ring[r % kUmmaUnitRing]; return w; });
+}
+}  // namespace
+
+int launch_abandoned_units_selftest(float* out, int published, int ended, int abort_round, cudaStream_t stream) {
+  DecodeParams p = {};
+  p.out = out;
+  p.q_heads = p.kv_heads = p.head_stride = p.q_len = p.rows = 1;
+  abandoned_units_selftest_kernel<<<1, 64, 0, stream>>>(p, published, ended, abort_round);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? B200ATTN_OK : cuda_fail(e, "abandoned-units selftest kernel launch");
+}
 
 int launch_cluster_selftest(int* header, float* out, uint32_t tries, int late, cudaStream_t stream) {
   DecodeParams p = {};

@@ -92,5 +92,6 @@ int decode_route(const b200attn_decode_args_t& a, int sm_count, bool built_in);
 int launch_decode_static(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream);
 int check_decode_static(int device, cudaStream_t stream, int32_t* code);
 int launch_cluster_selftest(int* header, float* out, uint32_t tries, int late, cudaStream_t stream);
+int launch_abandoned_units_selftest(float* out, int published, int ended, int abort_round, cudaStream_t stream);
 
 }  // namespace b200attn

@@ -38,6 +38,7 @@ EXPORTS = (
     "b200attn_decode_static_check",
     "b200attn_selftest_wait_expiry",
     "b200attn_selftest_cluster_expiry",
+    "b200attn_selftest_abandoned_units",
     "b200attn_paged_append",
     "b200attn_softmax",
     "b200attn_check_workspace",
@@ -192,6 +193,8 @@ def lib() -> C.CDLL:
         handle.b200attn_selftest_wait_expiry.restype = C.c_int
         handle.b200attn_selftest_cluster_expiry.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_uint32, C.c_int, C.c_void_p]
         handle.b200attn_selftest_cluster_expiry.restype = C.c_int
+        handle.b200attn_selftest_abandoned_units.argtypes = [C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
+        handle.b200attn_selftest_abandoned_units.restype = C.c_int
         handle.b200attn_paged_append.argtypes = [C.POINTER(PagedAppendArgs), C.c_void_p]
         handle.b200attn_paged_append.restype = C.c_int
         handle.b200attn_softmax.argtypes = [C.POINTER(SoftmaxArgs), C.c_void_p]
