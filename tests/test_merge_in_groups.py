@@ -71,3 +71,21 @@ def test_groups_in_a_recorded_call():
         graph.replay()
         torch.cuda.synchronize()
         assert (out.double() - refs).abs().max().item() <= ATOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("qh,kvh,m,d", [(8, 1, 1, 128), (16, 1, 1, 64), (8, 1, 5, 128), (24, 1, 1, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("batch", [1, 5, 60])
+def test_an_infinite_value_stays_infinite(batch, dtype, qh, kvh, m, d):
+    """One key of each sequence has an infinite element of V: the weight of every key is positive, and so the output's element is that
+    infinity, whatever number of chunks the sequence is merged from."""
+    for n in (1500, 2500, 3000, 4000, 7000, 12000):
+        g = torch.Generator(device="cuda").manual_seed(n)
+        k, v = (torch.randn((batch, kvh, n, d), generator=g, device="cuda").to(dtype) for _ in range(2))
+        q = torch.randn((batch, qh, d) if m == 1 else (batch, qh, m, d), generator=g, device="cuda").to(dtype)
+        at = torch.arange(batch, device="cuda")
+        v[at, 0, at * 977 % n, 7] = float("inf")
+        v[at, 0, at * 977 % n, 9] = float("-inf")
+        out = decode_attention(q, k, v) if m == 1 else speculative_decode_attention(q, k, v, causal=False)
+        assert (out[..., 7] == float("inf")).all() and (out[..., 9] == float("-inf")).all(), n
+        assert torch.isfinite(out[..., [i for i in range(d) if i not in (7, 9)]]).all(), n

@@ -162,11 +162,15 @@ __device__ __forceinline__ void merge_elements(const DecodeParams& p, long long 
       for (int e = 0; e < E; ++e) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-          const bool on = k0 + j < n_chunks;
-          const long long s = slot0 + static_cast<long long>(on ? k0 + j : k0) * step;
-          const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (s * R + r[e]) * 2));
-          o[e][j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + (s * R + r[e]) * D + d4[e] * 4));
-          mk[e][j] = on ? ml.x : -INFINITY;
+          // (nothing where there is no chunk, not another chunk with a weight of 0: that may hold infinities)
+          const long long s = slot0 + static_cast<long long>(k0 + j) * step;
+          float2 ml = make_float2(-INFINITY, 0.f);
+          o[e][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (k0 + j < n_chunks) {
+            ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (s * R + r[e]) * 2));
+            o[e][j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + (s * R + r[e]) * D + d4[e] * 4));
+          }
+          mk[e][j] = ml.x;
           lk[e][j] = ml.y;
         }
       }
