@@ -178,6 +178,12 @@ size_t b200attn_decode_workspace_bytes(const b200attn_decode_args_t* args);
 int b200attn_decode_route(const b200attn_decode_args_t* args, int sm_count, int is_static);
 
 /*
+ * Of a call behind the planner's launch, which kernel it plans for: 1 where the tensor-core tiles have keys as their rows (17 to 64 q rows
+ * per KV head over long sequences), 0 for every other call.  Arguments and limits as of b200attn_decode_route.
+ */
+int b200attn_decode_keys_as_rows(const b200attn_decode_args_t* args, int sm_count, int is_static);
+
+/*
  * Which way b200attn_prefill takes a call on a GPU of `sm_count` SMs: every item whole (1), the longest items shared by the CTAs of a
  * cluster (2, 4 or 8; shorter ones stay whole), or in parts that a second launch merges (B200ATTN_ROUTE_WORKSPACE + their number).
  * Host arithmetic on the sizes; needs no GPU, reads no pointer.  No counterpart in the reference.

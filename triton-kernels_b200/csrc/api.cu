@@ -164,6 +164,13 @@ int b200attn_decode_route(const b200attn_decode_args_t* a, int sm_count, int is_
   return decode_route(*a, sm_count, is_static != 0);
 }
 
+int b200attn_decode_keys_as_rows(const b200attn_decode_args_t* a, int sm_count, int is_static) {
+  const int route = b200attn_decode_route(a, sm_count, is_static);
+  if (route < 0) return route;
+  if (a->head_dim != 64 && a->head_dim != 128) { set_error("decode_keys_as_rows: head_dim %d", a->head_dim); return B200ATTN_E_UNSUPPORTED; }
+  return route == B200ATTN_ROUTE_PLANNER && decode_keys_as_rows(*a, sm_count, is_static != 0);
+}
+
 int b200attn_prefill_route(const b200attn_prefill_args_t* a, int sm_count) {
   if (!a || a->batch < 0 || a->q_heads <= 0 || a->kv_heads <= 0 || a->q_heads % a->kv_heads != 0 || sm_count <= 0) { set_error("prefill_route: bad arguments"); return B200ATTN_E_INVALID; }
   return prefill_route(*a, sm_count);

@@ -2962,11 +2962,21 @@ int launch_decode_pass(const b200attn_decode_args_t& a, int sm_count, cudaStream
 }
 }  // namespace
 
-int decode_route(const b200attn_decode_args_t& a, int sm_count, bool built_in) {
+// the call as its passes see it: fp32 inputs that are copied are fp16
+static b200attn_decode_args_t as_launched(const b200attn_decode_args_t& a, int sm_count, bool built_in) {
   b200attn_decode_args_t b = a;
   if (decode_ws_layout(a, sm_count, /*allow_cast=*/!built_in).cast_kv_elems > 0) b.dtype = B200ATTN_F16;
-  const Route r = route_of(b, sm_count, decode_pass_group(a.q_heads / a.kv_heads, a.q_len) * a.q_len, built_in, /*ask=*/false);
+  return b;
+}
+
+int decode_route(const b200attn_decode_args_t& a, int sm_count, bool built_in) {
+  const Route r = route_of(as_launched(a, sm_count, built_in), sm_count, decode_pass_group(a.q_heads / a.kv_heads, a.q_len) * a.q_len, built_in,
+                           /*ask=*/false);
   return r.cluster ? r.cluster : r.inline_plan ? B200ATTN_ROUTE_INLINE : B200ATTN_ROUTE_PLANNER;
+}
+
+bool decode_keys_as_rows(const b200attn_decode_args_t& a, int sm_count, bool built_in) {
+  return keyrows_suit(as_launched(a, sm_count, built_in), sm_count, decode_pass_group(a.q_heads / a.kv_heads, a.q_len) * a.q_len);
 }
 
 // ---------------------------------------------------------------------------

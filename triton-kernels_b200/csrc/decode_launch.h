@@ -89,6 +89,8 @@ DecodeWsLayout decode_ws_layout(const b200attn_decode_args_t& a, int sm_count, b
 int launch_decode(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream, bool built_in = false);
 // which way a call goes: see b200attn_decode_route
 int decode_route(const b200attn_decode_args_t& a, int sm_count, bool built_in);
+// whether its passes behind the planner are decode_keyrows_kernel's: see b200attn_decode_keys_as_rows
+bool decode_keys_as_rows(const b200attn_decode_args_t& a, int sm_count, bool built_in);
 int launch_decode_static(const b200attn_decode_args_t& a, int sm_count, cudaStream_t stream);
 int check_decode_static(int device, cudaStream_t stream, int32_t* code);
 int launch_cluster_selftest(int* header, float* out, uint32_t tries, int late, cudaStream_t stream);

@@ -31,6 +31,7 @@ EXPORTS = (
     "b200attn_prefill_workspace_bytes",
     "b200attn_decode_workspace_bytes",
     "b200attn_decode_route",
+    "b200attn_decode_keys_as_rows",
     "b200attn_prefill_route",
     "b200attn_prefill",
     "b200attn_decode",
@@ -179,6 +180,8 @@ def lib() -> C.CDLL:
         handle.b200attn_decode_workspace_bytes.restype = C.c_size_t
         handle.b200attn_decode_route.argtypes = [C.POINTER(DecodeArgs), C.c_int, C.c_int]
         handle.b200attn_decode_route.restype = C.c_int
+        handle.b200attn_decode_keys_as_rows.argtypes = [C.POINTER(DecodeArgs), C.c_int, C.c_int]
+        handle.b200attn_decode_keys_as_rows.restype = C.c_int
         handle.b200attn_prefill_route.argtypes = [C.POINTER(PrefillArgs), C.c_int]
         handle.b200attn_prefill_route.restype = C.c_int
         handle.b200attn_prefill.argtypes = [C.POINTER(PrefillArgs), C.c_void_p]
