@@ -36,9 +36,9 @@ def _reference(q, k, v, causal):
     return torch.softmax(s, -1).nan_to_num(0.0) @ vv
 
 
-def _run(layout, dtype, qh, kvh, m, d, lens, causal, page=16, seed=0, width=0, again=0):
-    """`width`: keys that the tables have room for, where that is more than the longest sequence; `again`: further calls, of which the
-    same bits are expected."""
+def _run(layout, dtype, qh, kvh, m, d, lens, causal, page=16, seed=0, width=0, again=0, cache=0):
+    """`width`: keys that the tables have room for, where that is more than the longest sequence; `cache`: rows of the cache, where that
+    is more than the sequences'; `again`: further calls, of which the same bits are expected."""
     g = torch.Generator(device="cuda").manual_seed(seed + qh + m)
     q = torch.randn((len(lens), qh, m, d), generator=g, device="cuda").to(dtype)
     ks, vs = ([torch.randn((n, kvh, d), generator=g, device="cuda").clamp(-5, 5).to(dtype) for n in lens] for _ in range(2))
@@ -52,10 +52,15 @@ def _run(layout, dtype, qh, kvh, m, d, lens, causal, page=16, seed=0, width=0, a
         indptr = torch.tensor([0] + lens).cumsum(0).to(torch.int32).cuda()
         call = lambda: speculative_decode_attention(q, k, v, causal=causal, kv_indptr=indptr)
     else:
-        kc, kt, ln = sdpa_ref.pack_paged(ks, page, permute_seed=1, extra_pages=2, pad_value=-1, poison=float("nan"))
-        vc, vt, _ = sdpa_ref.pack_paged(vs, page, permute_seed=2, extra_pages=2, pad_value=-1, poison=float("nan"))
+        spare = max(2, cache // page - sum(-(-n // page) for n in lens))
+        kc, kt, ln = sdpa_ref.pack_paged(ks, page, permute_seed=1, extra_pages=spare, pad_value=-1, poison=float("nan"))
+        vc, vt, _ = sdpa_ref.pack_paged(vs, page, permute_seed=2, extra_pages=spare, pad_value=-1, poison=float("nan"))
         kt, vt = (torch.nn.functional.pad(t, (0, max(0, width // page - t.shape[1])), value=-1).cuda() for t in (kt, vt))
         ln = ln.cuda()
+        from test_decode_keyrows_rule import _args, _ask
+
+        asked = _args("paged", "bf16", len(lens), qh, kvh, d, kt.shape[1] * page, m, page, kc.shape[0])
+        assert _ask(asked, sms=torch.cuda.get_device_properties(0).multi_processor_count)[1] == 1
         call = lambda: speculative_decode_attention(q, kc, vc, causal=causal, kv_indptr=ln, k_block_table=kt, v_block_table=vt,
                                                     kv_page_size=page)
     out = call()
@@ -106,6 +111,17 @@ def _with_empty(batch, empty, order, length):
     return [0 if b else length(i) for i, b in enumerate(blank)]
 
 
+def _cache_for(batch, qh, kvh, m, d, width, page=16):
+    """Rows of the smallest cache, in units of 4 096, before which the library takes such a call to the kernel."""
+    from test_decode_keyrows_rule import _args, _ask
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for cache in range(4096, batch * width + 1, 4096):
+        if _ask(_args("paged", "bf16", batch, qh, kvh, d, width, m, page, cache), sms=sms)[1] == 1:
+            return cache
+    raise AssertionError("not that kernel's, whatever the cache")
+
+
 def _run_with_empty(lens, kvh, d, dealt, page=None, width=0):
     from kernels._native import check_device_errors
     from utils.launch_config import decode_cuts, decode_plan
@@ -115,7 +131,8 @@ def _run_with_empty(lens, kvh, d, dealt, page=None, width=0):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     plan = decode_plan(sms, len(lens), 8 * kvh, kvh, 3, keys=keys, head_dim=d, page_size=page)
     assert (decode_cuts(plan, lens) is not None) == dealt
-    _run("ragged" if page is None else "paged", torch.bfloat16, 8 * kvh, kvh, 3, d, lens, causal=False, width=width, again=20)
+    _run("ragged" if page is None else "paged", torch.bfloat16, 8 * kvh, kvh, 3, d, lens, causal=False, width=width, again=20,
+         cache=0 if page is None else _cache_for(len(lens), 8 * kvh, kvh, 3, d, width, page))
     check_device_errors()
 
 
@@ -159,7 +176,8 @@ def test_short_ends_of_cut_sequences(kvh, heads, m, d):
     lens = [plan.min_chunk + 20] * batch
     assert decode_cuts(plan, lens) is None and decode_chunk_tokens(plan, lens) == plan.min_chunk
     _takes_it(batch, kvh, heads * m, batch * width, d, 16)
-    _run("paged", torch.bfloat16, heads * kvh, kvh, m, d, lens, causal=False, width=width, again=40)
+    _run("paged", torch.bfloat16, heads * kvh, kvh, m, d, lens, causal=False, width=width, again=40,
+         cache=_cache_for(batch, heads * kvh, kvh, m, d, width))
     check_device_errors()
 
 

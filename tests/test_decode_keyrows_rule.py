@@ -8,7 +8,7 @@ import pytest
 from test_decode_routes import PLANNER, SMS
 
 
-def _args(layout, dtype, batch, qh, kvh, d, keys, m, page=16):
+def _args(layout, dtype, batch, qh, kvh, d, keys, m, page=16, cache=None):
     from kernels import _native
 
     a = _native.DecodeArgs()
@@ -17,7 +17,7 @@ def _args(layout, dtype, batch, qh, kvh, d, keys, m, page=16):
     a.batch, a.q_heads, a.kv_heads, a.head_dim, a.q_len = batch, qh, kvh, d, m
     a.max_kv = keys
     a.page_size, a.table_stride = page, -(-keys // page)
-    a.total_kv = batch * keys
+    a.total_kv = batch * keys if cache is None else cache
     return a
 
 
@@ -33,7 +33,7 @@ def _says(layout, a, sms=SMS):
 
     keys = a.total_kv if layout == "ragged" else a.batch * (a.max_kv if layout == "dense" else a.table_stride * a.page_size)
     rows = decode_pass_group(a.q_heads // a.kv_heads, a.q_len) * a.q_len
-    return keyrows_suit(sms, a.batch, a.kv_heads, rows, keys, a.head_dim, a.page_size if layout == "paged" else None)
+    return keyrows_suit(sms, a.batch, a.kv_heads, rows, keys, a.head_dim, *((a.page_size, a.total_kv) if layout == "paged" else ()))
 
 
 @pytest.mark.parametrize("layout", ["dense", "ragged", "paged"])
@@ -71,3 +71,18 @@ def test_calls_that_plan_for_themselves_or_mean_nothing():
         for name, value in bad.items():
             setattr(a, name, value)
         assert _ask(a)[1] < 0, bad
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("kvh,batch", [(8, 16), (8, 64), (8, 256), (2, 64), (2, 256), (1, 320)])
+def test_a_cache_holds_no_more_keys_than_it_has_rows(kvh, batch, d):
+    """Wide tables in front of a cache that only has room for short sequences: what counts is the cache, to a key."""
+    line = (192 if batch * kvh <= SMS else 384) * 128 // d * batch
+    if batch * kvh > SMS:
+        line = max(line, -(-1536 * 128 * SMS // (kvh * d)))
+    for cache in (0, batch * 20, line - 1, line, batch * 8192):
+        a = _args("paged", "bf16", batch, 8 * kvh, kvh, d, 8192, 5, cache=cache)
+        route, key_rows = _ask(a)
+        assert route == PLANNER and key_rows == _says("paged", a) == (cache >= line), cache
+    # a longer table does not make such sequences longer
+    assert _ask(_args("paged", "bf16", batch, 8 * kvh, kvh, d, 1 << 20, 5, cache=batch * 20)) == (PLANNER, 0)

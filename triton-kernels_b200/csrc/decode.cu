@@ -2738,18 +2738,26 @@ int page_box(const b200attn_decode_args_t& a) {
 // head_dim 128 and 1 024 at 64 (us, umma and keyrows, 40 rows of eight heads, D 128: 64 sequences of 250 keys 25.1, 28.4; of 400 33.5, 34.7;
 // of 600 41.9, 41.5; of 1 000 59.4, 57.6; 200 of 400 82.7, 78.9; D 64, 64 of 700 32.6, 39.7; of 1 000 41.3, 48.0; of 1 200 60.2, 51.8; of
 // 2 400 90.3, 86.4), and half of that where no SM has more than one unit (16 of 250 at D 128, 20 rows 22.7, 16.0; 40 rows 15.4, 15.8).
-// Pages say how long a sequence can be; twice the line is asked for, which sequences of any length up to that reach on average.
+// Tables of pages say how long a sequence can be; twice the line is asked of them, which sequences of any length up to that reach on average.
+// And the cache says how many keys there can be in all, where no sequences share pages.  Three quarters of the line are asked of that, so
+// that short sequences in wide tables stay with decode_umma_kernel where the cache is no larger than they need: us, keyrows and umma, tables of
+// 8 192 keys, eight heads, 40 rows, D 128, 64 x 20 keys 22.8, 17.2; 256 x 20 59.2, 39.0; 64 x 250 28.5, 23.9; 256 x 250 78.4, 71.2; 24 rows, D 64,
+// 256 x 20 58.1, 32.9; 128 x 500 53.6, 47.4; 19 x 250 (152 units for 148 SMs) 26.3, 15.5.  Of the whole line 64 x 1 000, D 64, would take 56.2 in
+// place of 48.4, 128 x 1 000 of two heads, 32 rows, D 128 37.0 in place of 34.6.
 // And each SM needs 2 048 keys (D 64 4 096) where some have more than one unit: shorter calls end with a round that is mostly empty, or cut their
 // sequences for it (100 x 1 000 keys of two heads, 48 rows, 44.2 us, umma 30.5; 20 x 300 to 2 500 of eight 44.4, 41.5; 40 x 600 to 2 500 62.9, 68.8).
-// (Much shorter ones in such tables are slower for it: 64 of 20 keys in tables of 8 192 17.4, 23.0.  Both kernels launched, and the planner's
-// word for which of them stays, cost every call 4 to 6 us.)
+// (Much shorter ones in wide tables of a large cache are slower for it: the same calls.  Both kernels launched, and the planner's word for
+// which of them stays, cost every call 4 to 6 us.)
 bool keyrows_suit(const b200attn_decode_args_t& a, int sm_count, int rows) {
   if (a.dtype == B200ATTN_F32 || rows <= 16 || rows > kKrMaxRows || !keyrows_boxes(page_box(a))) return false;
   if (inline_plan_bits(a, sm_count, rows)) return false;      // (also in the library's own array, where such a call is planned)
   const bool one_each = static_cast<long long>(a.batch) * a.kv_heads <= sm_count;
-  const long long twice = a.layout == B200ATTN_PAGED ? 2 : 1, line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * twice / 2;
-  const long long keys = most_keys(a);
-  return keys >= line * a.batch && (one_each || keys * a.kv_heads * a.head_dim >= (2048ll << 7) * twice * sm_count);
+  auto enough = [&](long long keys, int quarters) {        // ... of the line
+    const long long line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * quarters / 8;
+    return keys >= line * a.batch && (one_each || keys * a.kv_heads * a.head_dim >= (512ll << 7) * quarters * sm_count);
+  };
+  if (a.layout != B200ATTN_PAGED) return enough(most_keys(a), 4);
+  return enough(most_keys(a), 8) && enough(a.total_kv, 3);
 }
 
 // `f32_out`: the inputs are the fp16 copies of fp32 tensors and the output rows are fp32
