@@ -134,6 +134,9 @@ __device__ __forceinline__ int merge_group(const DecodeParams& p, int n_chunks) 
 // One pass with a running maximum, E output elements and 8 / E chunks per step: the loads of a step do not depend on each other or on
 // the running state, so they are in flight together (the merge is a chain of L2 round trips otherwise).  With eight chunks of one element
 // everywhere the kernels of many rows spill (40 rows, 8 x 2 500 keys 26.8 -> 29.4 us).
+// What a step reads in the place of a chunk that is not there.  (Zeros; a constant would let the compiler make branches of the loads:
+// 16 x 9 943 keys of two heads, twelve rows, 42.0 -> 43.4 us, 1 x 30 000 of one head 19.4 -> 20.1.)
+__device__ float4 g_no_chunk;
 template <typename T, int D, int E>
 __device__ __forceinline__ void merge_elements(const DecodeParams& p, long long slot0, int step, int n_chunks, T* out, int t, int nt, float* s_ml) {
   constexpr int D4 = D / 4, CH = 8 / E;
@@ -162,15 +165,13 @@ __device__ __forceinline__ void merge_elements(const DecodeParams& p, long long 
       for (int e = 0; e < E; ++e) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-          // (nothing where there is no chunk, not another chunk with a weight of 0: that may hold infinities)
-          const long long s = slot0 + static_cast<long long>(k0 + j) * step;
-          float2 ml = make_float2(-INFINITY, 0.f);
-          o[e][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (k0 + j < n_chunks) {
-            ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (s * R + r[e]) * 2));
-            o[e][j] = __ldcg(reinterpret_cast<const float4*>(p.part_o + (s * R + r[e]) * D + d4[e] * 4));
-          }
-          mk[e][j] = ml.x;
+          const bool on = k0 + j < n_chunks;
+          const long long s = slot0 + static_cast<long long>(on ? k0 + j : k0) * step;
+          const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (s * R + r[e]) * 2));
+          // (zeros where there is no chunk, not another chunk with a weight of 0: that may hold infinities)
+          const float4* const from = on ? reinterpret_cast<const float4*>(p.part_o + (s * R + r[e]) * D + d4[e] * 4) : &g_no_chunk;
+          o[e][j] = __ldcg(from);
+          mk[e][j] = on ? ml.x : -INFINITY;
           lk[e][j] = ml.y;
         }
       }
