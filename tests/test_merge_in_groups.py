@@ -89,3 +89,25 @@ def test_an_infinite_value_stays_infinite(batch, dtype, qh, kvh, m, d):
         out = decode_attention(q, k, v) if m == 1 else speculative_decode_attention(q, k, v, causal=False)
         assert (out[..., 7] == float("inf")).all() and (out[..., 9] == float("-inf")).all(), n
         assert torch.isfinite(out[..., [i for i in range(d) if i not in (7, 9)]]).all(), n
+
+
+@pytest.mark.parametrize("dtype,qh,kvh,m,d", [(torch.bfloat16, 8, 1, 1, 64), (torch.float32, 8, 2, 1, 128), (torch.float16, 32, 8, 1, 128),
+                                              (torch.bfloat16, 8, 1, 2, 128), (torch.bfloat16, 8, 1, 4, 128)])
+@pytest.mark.parametrize("chunks", [25, 26, 27, 39, 40, 41])
+def test_either_side_of_the_lines(chunks, dtype, qh, kvh, m, d):
+    """Pairs of as many chunks as are merged in one step and in groups: 26 are the first where a thread has more than one element of the
+    output, 40 where it has one."""
+    from utils.launch_config import decode_items, decode_plan
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for n in range(1500, 40000, 128):
+        lens = [n, 700]
+        plan = decode_plan(sms, 2, qh, kvh, m, fp32=dtype == torch.float32, keys=sum(lens), head_dim=d)
+        if decode_items(plan, lens)[0] == chunks:
+            break
+    else:
+        pytest.skip("no length of that many chunks")
+    run, refs = _call(dtype, qh, kvh, m, d, lens)
+    first = run()
+    assert (first.double() - refs).abs().max().item() <= ATOL[dtype]
+    assert torch.equal(run(), first)

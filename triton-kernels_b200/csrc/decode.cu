@@ -50,7 +50,8 @@ constexpr int kMaxStages = 4;
 constexpr int kPlanThreads = 1024;
 constexpr int kPlanBuckets = 32;    // size classes of the execution order (longest items first)
 constexpr int kPlanLenCache = 4096; // sequences whose lengths the planner keeps in shared memory
-constexpr int kGroupedChunks = 20;  // chunks of a pair from which they are merged in two steps
+constexpr int kGroupedChunks = 26;  // chunks of a pair from which they are merged in two steps
+constexpr int kGroupedChunksFew = 40; // ... where a thread has one element and takes eight chunks at a time
 constexpr int kPlanMaxSlots = 512;  // slots of the persistent kernel that the planner deals out
 
 struct SeqInfo {
@@ -122,8 +123,8 @@ __device__ __forceinline__ void reset_ticket(const DecodeParams& p, int pair, in
   else { const TicketPlace t = ticket_place(p, pair, i); atomicSub(t.word, static_cast<unsigned>(n) << t.shift); }
 }
 // Chunks of a group where a pair's chunks are merged in two steps, 0 where they are not (see publish_and_merge).
-__device__ __forceinline__ int merge_group(const DecodeParams& p, int n_chunks) {
-  if (!p.pair_tickets || n_chunks < kGroupedChunks) return 0;
+__device__ __forceinline__ int merge_group(const DecodeParams& p, int n_chunks, bool few) {
+  if (!p.pair_tickets || n_chunks < (few ? kGroupedChunksFew : kGroupedChunks)) return 0;
   const int groups = min(p.pair_tickets - 1, __float2int_rn(sqrtf(static_cast<float>(n_chunks))));
   return (n_chunks + groups - 1) / groups;
 }
@@ -231,8 +232,10 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, long long sl
 // A merge is one CTA's chain of L2 round trips, four chunks each, so that one long sequence alone was mostly that: its chunks are merged
 // in groups, about as many as a group has chunks, each by the last of its CTAs to arrive, and the groups by the last of those.
 // One sequence of 30 000 keys, us: 8/1 heads (235 chunks) 44.6 -> 19.9, 32/8 heads 37.1 -> 32.8; 6 of 30 271, 8/1 heads, 35.7 -> 30.9; 6 of
-// 6 607 to 26 430, 40 rows of one head 59.2 -> 33.6.  Below twenty chunks (kGroupedChunks) the second ticket costs what the shorter chains
-// save (18 chunks 38.1 us and 38.7; 11 27.4 and 28.2).  `s_word`, `s_ml` (two floats per row): shared memory.
+// 6 607 to 26 430, 40 rows of one head 59.2 -> 33.6.  With fewer chunks the second ticket costs more than the shorter chains save; in one step and
+// in groups, us: 22 chunks, 20 rows, D 128 18.0, 18.7; 23 25.9, 26.7; 24, 16 rows 24.7, 25.0; 27 24.2, 23.4; 30, 32 rows 22.9, 21.1; with eight
+// chunks a step, 4 rows, D 128, 27 15.5, 16.6; 30 17.0, 17.9; 36 17.9, 17.9; 55 18.0, 16.9; fp32 21 18.8, 20.5; 33 20.3, 20.9; 40 21.7, 21.7.
+// `s_word`, `s_ml` (two floats per row): shared memory.
 template <typename T, int D, bool kFew>
 __device__ __forceinline__ void publish_and_merge(const DecodeParams& p, int b, int h, int c, int n_chunks, int item0, T* out, int* s_word,
                                                   float* s_ml) {
@@ -240,7 +243,7 @@ __device__ __forceinline__ void publish_and_merge(const DecodeParams& p, int b, 
   const long long slot0 = static_cast<long long>(item0) * p.kv_heads + h;   // chunk k lives in slot0 + k * kv_heads
   __threadfence();
   __syncthreads();
-  const int group = merge_group(p, n_chunks);
+  const int group = merge_group(p, n_chunks, kFew && p.rows * (D / 4) <= nt);
   int n = n_chunks, step = p.kv_heads;
   if (group > 0) {
     const int g = c / group, size = min(group, n_chunks - g * group);
