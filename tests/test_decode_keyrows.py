@@ -126,10 +126,13 @@ def _run_with_empty(lens, kvh, d, dealt, page=None, width=0):
     from kernels._native import check_device_errors
     from utils.launch_config import decode_cuts, decode_plan
 
+    from test_decode_keyrows_rule import _args, _ask
+
     keys = sum(lens) if page is None else len(lens) * width
     _takes_it(len(lens), kvh, 24, keys, d, page)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    plan = decode_plan(sms, len(lens), 8 * kvh, kvh, 3, keys=keys, head_dim=d, page_size=page)
+    plan = decode_plan(sms, len(lens), 8 * kvh, kvh, 3, keys=keys, head_dim=d, page_size=page, equal=False)
+    assert page is not None or _ask(_args("ragged", "bf16", len(lens), 8 * kvh, kvh, d, 0, 3, cache=keys), sms=sms)[1] == 1
     assert (decode_cuts(plan, lens) is not None) == dealt
     _run("ragged" if page is None else "paged", torch.bfloat16, 8 * kvh, kvh, 3, d, lens, causal=False, width=width, again=20,
          cache=0 if page is None else _cache_for(len(lens), 8 * kvh, kvh, 3, d, width, page))
@@ -157,7 +160,7 @@ def test_empty_sequences(empty, order, kind, kvh, d):
 @pytest.mark.parametrize("kvh,d,empty", [(1, 128, 6), (2, 64, 3), (2, 64, 6), (8, 128, 3)])
 def test_empty_sequences_dealt_out(kvh, d, empty, order):
     """A CTA's units are those of its stretch of the batch: a run of empty sequences comes one behind the other."""
-    lens = _with_empty(60 // kvh + 20, empty, order, lambda i: 1000 + i * 7919 % 33000)
+    lens = _with_empty(60 // kvh + 20 if d == 128 else 80, empty, order, lambda i: 1000 + i * 7919 % 33000)
     _run_with_empty(lens, kvh, d, True)
 
 

@@ -33,7 +33,8 @@ def _says(layout, a, sms=SMS):
 
     keys = a.total_kv if layout == "ragged" else a.batch * (a.max_kv if layout == "dense" else a.table_stride * a.page_size)
     rows = decode_pass_group(a.q_heads // a.kv_heads, a.q_len) * a.q_len
-    return keyrows_suit(sms, a.batch, a.kv_heads, rows, keys, a.head_dim, *((a.page_size, a.total_kv) if layout == "paged" else ()))
+    return keyrows_suit(sms, a.batch, a.kv_heads, rows, keys, a.head_dim, *((a.page_size, a.total_kv) if layout == "paged" else ()),
+                        equal=layout == "dense")
 
 
 @pytest.mark.parametrize("layout", ["dense", "ragged", "paged"])
@@ -78,11 +79,22 @@ def test_calls_that_plan_for_themselves_or_mean_nothing():
 def test_a_cache_holds_no_more_keys_than_it_has_rows(kvh, batch, d):
     """Wide tables in front of a cache that only has room for short sequences: what counts is the cache, to a key."""
     line = (192 if batch * kvh <= SMS else 384) * 128 // d * batch
+    never = d == 64 and batch * kvh <= SMS
     if batch * kvh > SMS:
         line = max(line, -(-1536 * 128 * SMS // (kvh * d)))
     for cache in (0, batch * 20, line - 1, line, batch * 8192):
         a = _args("paged", "bf16", batch, 8 * kvh, kvh, d, 8192, 5, cache=cache)
         route, key_rows = _ask(a)
-        assert route == PLANNER and key_rows == _says("paged", a) == (cache >= line), cache
+        assert route == PLANNER and key_rows == _says("paged", a) == (cache >= line and not never), cache
     # a longer table does not make such sequences longer
     assert _ask(_args("paged", "bf16", batch, 8 * kvh, kvh, d, 1 << 20, 5, cache=batch * 20)) == (PLANNER, 0)
+
+
+@pytest.mark.parametrize("kvh", [1, 2])
+def test_short_heads_want_a_sequence_for_an_sm(kvh):
+    """At head_dim 64, up to one pair an SM: only sequences of one length that two thirds of the SMs have one of."""
+    for batch in (96 // kvh, 98 // kvh, 100 // kvh, 148 // kvh, 150 // kvh):
+        for layout in ("dense", "ragged", "paged"):
+            route, key_rows = _ask(_args(layout, "bf16", batch, 8 * kvh, kvh, 64, 9000, 5))
+            pairs = batch * kvh
+            assert route == PLANNER and key_rows == (pairs > SMS or (layout == "dense" and 3 * pairs >= 2 * SMS)), (batch, layout)

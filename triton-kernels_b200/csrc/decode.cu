@@ -2755,7 +2755,12 @@ int page_box(const b200attn_decode_args_t& a) {
 bool keyrows_suit(const b200attn_decode_args_t& a, int sm_count, int rows) {
   if (a.dtype == B200ATTN_F32 || rows <= 16 || rows > kKrMaxRows || !keyrows_boxes(page_box(a))) return false;
   if (inline_plan_bits(a, sm_count, rows)) return false;      // (also in the library's own array, where such a call is planned)
-  const bool one_each = static_cast<long long>(a.batch) * a.kv_heads <= sm_count;
+  const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
+  const bool one_each = pairs <= sm_count;
+  // At head_dim 64 sequences that have to be cut for the SMs are slower here whatever their lengths (packed, 12 x 6 000 keys of eight heads, 40
+  // rows 59.5 and 73.2, 35 x 6 000 of two 46.3, 51.8, 88 x 4 000 of one 37.0, 44.8; of uneven lengths 110 x 2 500 33.0, 40.3; two or more to an
+  // SM are 0.95 of the time): only equal ones, of which nearly every SM has one, stay whole (120 x 2 400 39.5, 32.0; 148 x 8 000 76.4, 69.5).
+  if (one_each && a.head_dim == 64 && (a.layout != B200ATTN_DENSE || pairs * 3 < sm_count * 2ll)) return false;
   auto enough = [&](long long keys, int quarters) {        // ... of the line
     const long long line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * quarters / 8;
     return keys >= line * a.batch && (one_each || keys * a.kv_heads * a.head_dim >= (512ll << 7) * quarters * sm_count);

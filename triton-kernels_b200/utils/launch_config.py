@@ -69,13 +69,15 @@ def tcgen05_plans_itself(sm_count: int, batch: int, kv_heads: int, keys: int) ->
 
 
 def keyrows_suit(sm_count: int, batch: int, kv_heads: int, rows: int, keys: int, head_dim: int, page_size: Optional[int] = None,
-                 cache_keys: Optional[int] = None) -> bool:
+                 cache_keys: Optional[int] = None, equal: bool = True) -> bool:
     """Whether a call of 16-bit elements behind the planner goes to the kernel whose tiles have keys as their rows (csrc/decode.cu
     keyrows_suit); ``keys`` as in ``tcgen05_plans_itself``; for paged caches ``page_size`` and the rows of the cache (None: as many as
-    it takes)."""
+    it takes); ``equal``: a dense batch, whose sequences have one length."""
     if not 16 < rows <= 64 or (page_size is not None and page_size % 8):
         return False
     one_each = batch * kv_heads <= sm_count
+    if one_each and head_dim == 64 and (not equal or page_size is not None or batch * kv_heads * 3 < sm_count * 2):
+        return False
 
     def enough(n: int, quarters: int) -> bool:
         line = (512 << 7) // head_dim * (1 if one_each else 2) * quarters // 8
@@ -87,10 +89,11 @@ def keyrows_suit(sm_count: int, batch: int, kv_heads: int, rows: int, keys: int,
 
 
 def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: int, fp32: bool = False,
-                keys: Optional[int] = None, head_dim: int = 64, page_size: Optional[int] = None, cache_keys: Optional[int] = None) -> DecodePlan:
+                keys: Optional[int] = None, head_dim: int = 64, page_size: Optional[int] = None, cache_keys: Optional[int] = None,
+                equal: bool = True) -> DecodePlan:
     """``keys`` (see ``tcgen05_plans_itself``): with it, calls of the tcgen05 kernel that plan for themselves are planned as they do,
     without dealing the batch out, and up to three short sequences in items for one CTA an SM, and calls of the kernel with keys as rows
-    (``keyrows_suit``, which ``head_dim``, ``page_size`` and ``cache_keys`` are for) as for that; without it all are the planner's, for the tcgen05 kernel
+    (``keyrows_suit``, which ``head_dim`` and what follows it are for) as for that; without it all are the planner's, for the tcgen05 kernel
     with two CTAs an SM."""
     group = decode_pass_group(q_heads // kv_heads, q_len)
     rows = group * q_len
@@ -111,7 +114,7 @@ def decode_plan(sm_count: int, batch: int, q_heads: int, kv_heads: int, q_len: i
         slots = 0
         if batch <= 3 and keys * kv_heads <= 6 * min_chunk * sm_count:
             target, wave = max(1, sm_count // kv_heads), 0
-    elif wide and keys is not None and keyrows_suit(sm_count, batch, kv_heads, rows, keys, head_dim, page_size, cache_keys):
+    elif wide and keys is not None and keyrows_suit(sm_count, batch, kv_heads, rows, keys, head_dim, page_size, cache_keys, equal):
         slots, target, wave = sm_count // kv_heads, max(1, 3 * sm_count // kv_heads), max(1, sm_count // kv_heads)
         return DecodePlan(target, min_chunk, max_items, tiles, slices, 32 * (tiles * slices + 1), wave, overhead, slots, True)
     return DecodePlan(target, min_chunk, max_items, tiles, slices, 32 * (tiles * slices + 1), wave, overhead, slots)
