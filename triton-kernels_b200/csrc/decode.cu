@@ -234,7 +234,7 @@ __device__ __forceinline__ void merge_chunks(const DecodeParams& p, long long sl
 // One sequence of 30 000 keys, us: 8/1 heads (235 chunks) 44.6 -> 19.9, 32/8 heads 37.1 -> 32.8; 6 of 30 271, 8/1 heads, 35.7 -> 30.9; 6 of
 // 6 607 to 26 430, 40 rows of one head 59.2 -> 33.6.  With fewer chunks the second ticket costs more than the shorter chains save; in one step and
 // in groups, us: 22 chunks, 20 rows, D 128 18.0, 18.7; 23 25.9, 26.7; 24, 16 rows 24.7, 25.0; 27 24.2, 23.4; 30, 32 rows 22.9, 21.1; with eight
-// chunks a step, 4 rows, D 128, 27 15.5, 16.6; 30 17.0, 17.9; 36 17.9, 17.9; 55 18.0, 16.9; fp32 21 18.8, 20.5; 33 20.3, 20.9; 40 21.7, 21.7.
+// chunks a step, 4 rows, D 128, 27 15.5, 16.6; 30 17.0, 17.9; 36 17.9, 17.9; 55 18.0, 16.9; fp32 21 18.8, 20.5; 33 20.3, 20.9.
 // `s_word`, `s_ml` (two floats per row): shared memory.
 template <typename T, int D, bool kFew>
 __device__ __forceinline__ void publish_and_merge(const DecodeParams& p, int b, int h, int c, int n_chunks, int item0, T* out, int* s_word,
@@ -2757,9 +2757,10 @@ bool keyrows_suit(const b200attn_decode_args_t& a, int sm_count, int rows) {
   if (inline_plan_bits(a, sm_count, rows)) return false;      // (also in the library's own array, where such a call is planned)
   const long long pairs = static_cast<long long>(a.batch) * a.kv_heads;
   const bool one_each = pairs <= sm_count;
-  // At head_dim 64 sequences that have to be cut for the SMs are slower here whatever their lengths (packed, 12 x 6 000 keys of eight heads, 40
-  // rows 59.5 and 73.2, 35 x 6 000 of two 46.3, 51.8, 88 x 4 000 of one 37.0, 44.8; of uneven lengths 110 x 2 500 33.0, 40.3; two or more to an
-  // SM are 0.95 of the time): only equal ones, of which nearly every SM has one, stay whole (120 x 2 400 39.5, 32.0; 148 x 8 000 76.4, 69.5).
+  // At head_dim 64 sequences that have to be cut for the SMs are slower here (us, umma and keyrows, packed, 40 rows, 12 x 6 000 keys of eight heads
+  // 47.3, 56.7; 35 x 6 000 of two 40.4, 42.8; 88 x 4 000 of one 37.6, 43.9; lengths of a sixteenth to twice 2 500, 110 of one head 34.2, 40.6; where
+  // SMs have more than one pair such lengths take 0.95 of umma's time).  Only equal ones, of which most SMs have one, stay whole, and only of a
+  // dense batch is that known (120 x 2 400 39.5, 32.0; 148 x 8 000 76.4, 69.5; packed, 110 x 2 500 would be 37.7, 33.3).
   if (one_each && a.head_dim == 64 && (a.layout != B200ATTN_DENSE || pairs * 3 < sm_count * 2ll)) return false;
   auto enough = [&](long long keys, int quarters) {        // ... of the line
     const long long line = (512 << 7) / a.head_dim * (one_each ? 1 : 2) * quarters / 8;
