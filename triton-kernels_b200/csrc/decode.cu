@@ -593,9 +593,10 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
       s_carry = 0;
       // (a cut moved to the end of a sequence makes a stretch up to min_chunk longer: without that in the estimate 47
       // sequences of 350 to 5 600 keys on one KV head were dealt out and took 48 us instead of 45)
-      // (One CTA to an SM: dealing out costs some 500 keys more, and the estimate has to favour it by a tenth.  Over 26 batches it gave 0.94 to
-      // 1.05 of the time without; by this rule 32 x 1 000 to 33 000 keys 292 -> 287 us, of 34 x 10 232 at D 64 166 instead of 171.
-      // Equal items end with the last round of CTAs, not half an item behind the average.)
+      // (One CTA to an SM: equal items end with the last round of CTAs, not half an item behind the average.  CTAs of a batch that is
+      // dealt out cannot take over from one another, as those that draw units longest first do: where the estimates alone favoured it, it took
+      // 0.90 to 1.17 of the time, 1.007 over 45 batches, and they did not tell which.  So it has to be ahead by about as much as they are
+      // wrong, a tenth and one item's overhead, some 500 keys.  What is left are long, very uneven batches: 2 of the 45, 0.99 of the time each.)
       if (p.one_cta) {
         const float rounds = static_cast<float>((items0 + p.wave_items - 1) / p.wave_items) * (static_cast<float>(pick_chunk) + ovh);
         best = 0.89f * fminf(best, rounds) - 500.f;

@@ -319,7 +319,7 @@ __device__ __forceinline__ float part_weight(float m, float largest) { return m 
 // kPaged: the instantiation launched for paged K/V; only it carries the block-table read-ahead of the producer (in
 // the dense / ragged kernel that code, though never run, cost 1 % on the dense benchmark configuration).  The other
 // layout checks stay run-time checks.  kParts: the one launched in clusters that share an item (its epilogue costs the others
-// registers; at the cap of 96 the forms for head_dim 128 spill, 52 bytes dense and 16 over pages.  That is not what they wait for: a
+// registers; at the cap of 96 the forms for head_dim 128 spill, 8 bytes dense and 16 over pages.  That is not what they wait for: a
 // build whose form for 64 spilled 72 took 10.48 us for 512 causal tokens, the present one, which spills none, 10.46).
 template <typename T, int D, typename OutT, bool kPaged, bool kParts>
 __global__ void __launch_bounds__(kThreads, 1)
